@@ -239,7 +239,7 @@ __device__ __forceinline__ void run_phase(const CUtensorMap* tmW, const CUtensor
     const float* ws = PH == 1 ? a.w1s : a.w2s;
     uint32_t kbc = 0;
     bool ok = true;
-    int ready_tile = -1, loaded_tile = -1;
+    int ready_tile = -1, loaded_tile = -1, ready_e = -1;
     float ws_next = 0.f;
     bool have_ws_next = false;
     for (int w = first; w < last && ok; w += step) {
@@ -253,6 +253,15 @@ __device__ __forceinline__ void run_phase(const CUtensorMap* tmW, const CUtensor
         bar_epi();
         if (!*sh.epi_flag) break;  // the producer records the timeout
         ready_tile = tile;
+      }
+      if (PH == 1 && a.exp_gate && e != ready_e) {
+        // the row scales are read with plain loads below: they have landed when the expert's arrival word is full (the
+        // producer's wait on the same word orders only the TMA loads)
+        const uint32_t need = (uint32_t)(sh.goff[e + 1] - sh.goff[e]) * (uint32_t)a.exp_parts;
+        if (tid == 0) *sh.epi_flag = wait_flag_ge_sys(a.exp_cnt + e, need) ? 1 : 0;
+        bar_epi();
+        if (!*sh.epi_flag) break;  // the producer records the timeout
+        ready_e = e;
       }
       if (PH == 1 || tile != loaded_tile) {
         // activation scales (and, in phase 2, the owner / slot of every row) depend on the token tile only; a CTA's

@@ -419,3 +419,28 @@ def test_timed_out_wait_poisons_the_object_until_reset():
     finally:
         for h in heaps:
             h.close()
+
+
+def test_one_launch_layer_on_new_inputs_matches_its_phases():
+    """The layer in one launch (dispatch inside, GEMM tiles starting as their expert's rows land) gives the bytes of its
+    four phases run one after the other, also when nothing in the slab is left over from an earlier call: a tile that
+    reads a row or its scales before they have landed shows."""
+    from umdk_b200.ops.ep_ll import EpLowLatency, ExpertWeights
+    from umdk_b200.parallel.symm import SymmetricHeap
+    T, H, F, E, K = 96, 2048, 256, 16, 8
+    w = ExpertWeights(*(t.cuda() for t in _weights(E, H, F, seed=3))).to_tiled()
+    for seed in range(4):
+        xs, idxs, ws = _inputs(1, T, H, E, K, seed=seed)
+        x, idx, tw = xs[0].cuda() * (seed + 1), idxs[0].cuda(), ws[0].cuda()
+        res = []
+        for masks in ((4, 8, 1, 2), (15,)):
+            heap = SymmetricHeap(EpLowLatency.heap_bytes(1, E, K, H, T))
+            st = EpLowLatency(heap, E, K, H, F, T)
+            out = torch.zeros(T, H, dtype=torch.bfloat16, device="cuda")
+            for pm in masks:
+                st._fused(w, idx, tw, out, phase_mask=pm, x=x)
+            torch.cuda.synchronize()
+            st.check()
+            heap.close()
+            res.append(out)
+        assert torch.equal(res[0], res[1])
