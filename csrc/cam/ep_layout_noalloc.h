@@ -27,7 +27,8 @@
 //   * All calls on one device share the array. Two calls whose kernels may overlap on the GPU (different streams
 //     without an ordering between them) race on it; keep calls on one stream or order them with events.
 //   * Nothing in the array has to survive between calls. The barrier words are reset on the caller's stream at the
-//     start of every call; the histogram part is fully rewritten by the kernel before it is read.
+//     start of every call that uses them (two CTAs and more); the histogram part is fully rewritten by the kernel
+//     before it is read.
 //   * The entry point itself calls no cudaMalloc, cudaFree or allocating library routine, on the first call or
 //     later; the only memory event is the driver's one-time module load described above.
 #pragma once

@@ -198,3 +198,10 @@ def test_notify_matches_dispatch_counts(R, T, E, K):
     finally:
         for h in heaps:
             h.close()
+
+
+@pytest.mark.parametrize("T,K,E,R", [(1024, 8, 256, 8), (1025, 16, 96, 32), (2049, 3, 64, 1), (70, 2, 6000, 4)])
+def test_layout_cta_and_warp_edges(T, K, E, R):
+    """One CTA exactly full, one token more (a second CTA behind the grid barrier), and so many experts that the
+    histograms of fewer warps fill the shared memory."""
+    test_layout_matches_reference(T, K, E, R)
