@@ -205,3 +205,39 @@ def test_layout_cta_and_warp_edges(T, K, E, R):
     """One CTA exactly full, one token more (a second CTA behind the grid barrier), and so many experts that the
     histograms of fewer warps fill the shared memory."""
     test_layout_matches_reference(T, K, E, R)
+
+
+@pytest.mark.parametrize("T,H,E,K,quant", [
+    (1, 128, 8, 1, True), (33, 2176, 16, 4, True), (300, 7168, 64, 8, True), (33, 2176, 16, 4, False),
+    (129, 128, 5, 3, False),
+])
+def test_single_rank_short_path_matches_exchange(T, H, E, K, quant):
+    """A group of one rank takes kernels without an exchange; the two halves of a call take the exchanging ones. Same
+    bytes from both, with dropped slots, tokens routed nowhere and alternating use of the two on one state."""
+    xs, idxs, ws = _make_inputs(1, T, H, E, K, seed=T, drop=True)
+    idxs[0][T // 2] = -1
+    heaps, (st,) = _virtual_states(1, E, K, H, cap=T + 3)
+    try:
+        for rnd in range(2):
+            x, idx, w = xs[0].cuda() + rnd, idxs[0].cuda(), ws[0].cuda()
+            want = st.dispatch(x, idx, w, quant=quant, phase_mask=1, row_info=True)
+            want = st.dispatch(x, idx, w, quant=quant, phase_mask=2, out=want)
+            got = st.dispatch(x, idx, w, quant=quant, sync_counts=True, row_info=True)
+            n, a = int(want.counts[0]), int(want.counts[1])
+            assert got.num_recv == n and got.per_expert == want.recv_tokens_per_expert.tolist()
+            assert torch.equal(got.counts[:5], want.counts[:5])
+            for f in ("recv_x", "recv_scales", "expand_idx"):
+                u, v = getattr(got, f), getattr(want, f)
+                assert u is None and v is None or torch.equal(u[:n].view(torch.uint8), v[:n].view(torch.uint8)), f
+            for f in ("recv_count", "recv_tokens_per_expert", "row_expert", "row_weight"):
+                assert torch.equal(getattr(got, f), getattr(want, f)), f
+            assert torch.equal(got.recv_meta[:a], want.recv_meta[:a])
+            y = torch.randn(got.recv_x.shape[0], H, device="cuda").to(torch.bfloat16)
+            for weights in (True, False):
+                o = torch.full((T, H), float("nan"), dtype=torch.bfloat16, device="cuda")
+                st.combine(y, want, apply_weights=weights, phase_mask=1, out=o)
+                st.combine(y, want, apply_weights=weights, phase_mask=2, out=o)
+                assert torch.equal(st.combine(y, got, apply_weights=weights), o)
+        st.check()
+    finally:
+        heaps[0].close()

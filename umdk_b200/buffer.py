@@ -165,19 +165,9 @@ class Buffer:
                 return self._dispatch_static(st, x, topk_idx, topk_weights, use_fp8, el, async_finish)
             out = st.dispatch(x.contiguous(), topk_idx.contiguous(),
                               topk_weights.contiguous() if topk_weights is not None else None, quant=use_fp8,
-                              sync_counts=True)
-            n = out.num_recv
-            per_expert = out.recv_tokens_per_expert.tolist()
-            rows_le = torch.repeat_interleave(torch.arange(el, device=x.device),
-                                              out.recv_tokens_per_expert.to(x.device))
-            # per-row weights travel in the arrival metadata; rebuild them in row order
-            recv_w = torch.zeros(n, dtype=torch.float32, device=x.device)
-            a = int(out.counts[1].item())
-            meta = out.recv_meta[:a]
-            rows = meta[:, 2:2 + K].reshape(-1).long()
-            wbits = meta[:, 2 + K:2 + 2 * K].reshape(-1).contiguous().view(torch.float32)
-            sel = rows >= 0
-            recv_w[rows[sel]] = wbits[sel]
+                              sync_counts=True, row_info=True)
+            n, per_expert = out.num_recv, out.per_expert
+            rows_le, recv_w = out.row_expert[:n], out.row_weight[:n]
             recv_x = (out.recv_x[:n], out.recv_scales[:n]) if use_fp8 else out.recv_x[:n]
             h = DispatchHandle("gpu", topk_idx, topk_weights, T, gpu=out)
             ev = EventOverlap(torch.cuda.current_stream().record_event()) if async_finish else EventOverlap()
@@ -190,26 +180,13 @@ class Buffer:
 
     def _dispatch_static(self, st, x, topk_idx, topk_weights, use_fp8, el, async_finish):
         """Dispatch whose results keep their worst-case sizes; every count stays on the device."""
-        T, K = topk_idx.shape
+        T = topk_idx.shape[0]
         out = st.dispatch(x.contiguous(), topk_idx.contiguous(),
-                          topk_weights.contiguous() if topk_weights is not None else None, quant=use_fp8)
-        dev = x.device
-        n_cap, a_cap = out.recv_x.shape[0], out.recv_meta.shape[0]
-        ends = out.recv_tokens_per_expert.cumsum(0)                       # [E_local] row where each expert ends
-        rows_le = torch.searchsorted(ends, torch.arange(n_cap, device=dev), right=True)
-        rows_le = torch.where(rows_le < el, rows_le, torch.full_like(rows_le, -1))
-        # weights ride in the arrival metadata; rows of arrivals that did not happen are sent to a spare slot
-        arrived = (torch.arange(a_cap, device=dev) < out.counts[1]).unsqueeze(1)
-        rows = out.recv_meta[:, 2:2 + K].long()
-        wbits = out.recv_meta[:, 2 + K:2 + 2 * K].contiguous().view(torch.float32)
-        ok = arrived & (rows >= 0) & (rows < n_cap)
-        recv_w = torch.zeros(n_cap + 1, dtype=torch.float32, device=dev)
-        recv_w.scatter_(0, torch.where(ok, rows, torch.full_like(rows, n_cap)).reshape(-1),
-                        torch.where(ok, wbits, torch.zeros_like(wbits)).reshape(-1))
+                          topk_weights.contiguous() if topk_weights is not None else None, quant=use_fp8, row_info=True)
         recv_x = (out.recv_x, out.recv_scales) if use_fp8 else out.recv_x
         h = DispatchHandle("gpu", topk_idx, topk_weights, T, gpu=out)
         ev = EventOverlap(torch.cuda.current_stream().record_event()) if async_finish else EventOverlap()
-        return recv_x, rows_le, recv_w[:n_cap], out.recv_tokens_per_expert, h, ev
+        return recv_x, out.row_expert, out.row_weight, out.recv_tokens_per_expert, h, ev
 
     @_trace.traced("umdk.buffer.combine")
     def combine(self, x: torch.Tensor, handle: DispatchHandle, topk_weights: Optional[torch.Tensor] = None,

@@ -33,6 +33,7 @@ class _DispatchParams(ctypes.Structure):
         ("recv_count", ctypes.c_void_p), ("recv_per_expert", ctypes.c_void_p), ("recv_meta", ctypes.c_void_p),
         ("counts_dev", ctypes.c_void_p), ("counts_host", ctypes.c_void_p),
         ("ctrl", ctypes.c_void_p), ("status", ctypes.c_void_p), ("diag", ctypes.c_void_p),
+        ("row_expert", ctypes.c_void_p), ("row_weight", ctypes.c_void_p), ("per_expert_host", ctypes.c_void_p),
     ]
 
 
@@ -74,7 +75,11 @@ def check_status(status: torch.Tensor, what: str = "kernel", owner=None):
     """Reads the 4-int status record (synchronises) and raises if a kernel reported an error. ``owner`` (an object
     with the ``Recoverable`` mix-in) is marked poisoned: a kernel that gave up on a wait may have left its shared
     counters and epoch words half-updated, so further launches are refused until ``owner.reset()``."""
-    s = status.tolist()
+    _raise_status(status.tolist(), status, what, owner)
+
+
+def _raise_status(s, status: torch.Tensor, what: str, owner=None):
+    """Raises for the record ``s`` (host values of the device record ``status``) if it holds an error."""
     if s[0] != 0:
         status.zero_()
         msg = (f"{what}: {_CODES.get(s[0], s[0])} in phase {_PHASES.get(s[1], s[1])} "
@@ -174,6 +179,9 @@ class DispatchResult:
     num_tokens: int
     quant: bool
     num_recv: Optional[int] = None       # host value of N when the caller asked for it
+    row_expert: Optional[torch.Tensor] = None   # [n_cap] int64 local expert of every row (-1 behind the received ones)
+    row_weight: Optional[torch.Tensor] = None   # [n_cap] fp32 routing weight of every row (0 behind them)
+    per_expert: Optional[List[int]] = None      # host values of recv_tokens_per_expert, with num_recv
 
 
 def layout(topk_idx: torch.Tensor, num_experts: int, num_ranks: int, scratch=None, bar=None, status=None,
@@ -232,7 +240,9 @@ class EpNormal(Recoverable):
         self.status = torch.zeros(4, dtype=torch.int32, device=dev)
         self.layout_bar = torch.zeros(2, dtype=torch.int32, device=dev)
         self.layout_scratch = torch.empty(((cap + 31) // 32) * (num_experts + self.R), dtype=torch.int32, device=dev)
-        self.mirror = HostMirror(8)
+        # counts of the last call in mapped host memory: 8 ints, then the rows per local expert (int64)
+        self.mirror = HostMirror(8 + 2 * (num_experts // self.R))
+        self.status_host = torch.zeros(4, dtype=torch.int32, pin_memory=True)
         # diagnose mode: the kernels record how long (ns) this rank waited for each source rank's data; gather the
         # rows of all ranks into a matrix and pass it to examples/utils.py:diagnose_matrix to find a slow rank or link
         # (the reference's in-kernel wait statistics: moe_dispatch_normal.h:489-529, moe_combine_normal.h:259-280)
@@ -287,9 +297,10 @@ class EpNormal(Recoverable):
     def dispatch(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_weights: Optional[torch.Tensor],
                  lay: Optional[LayoutResult] = None, quant: bool = True, n_cap: Optional[int] = None,
                  a_cap: Optional[int] = None, phase_mask: int = 3, out: Optional[DispatchResult] = None,
-                 sync_counts: bool = False) -> DispatchResult:
+                 sync_counts: bool = False, row_info: bool = False) -> DispatchResult:
         """Runs notify + quantise + push + expand. ``phase_mask`` 1 / 2 run only the send / receive half (used to
-        drive several virtual ranks from one process on one GPU)."""
+        drive several virtual ranks from one process on one GPU). ``row_info``: the kernel also writes the local expert
+        and the routing weight of every row (``row_expert``, ``row_weight`` of a new result)."""
         self._guard()
         assert x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous()
         T, H = x.shape
@@ -312,7 +323,10 @@ class EpNormal(Recoverable):
                 torch.empty(self.E, dtype=torch.int32, device=dev),
                 torch.empty(self.E // self.R, dtype=torch.int64, device=dev),
                 torch.empty(a_cap, 2 * K + 2, dtype=torch.int32, device=dev),
-                torch.zeros(4 + MAX_RANKS, dtype=torch.int32, device=dev), lay, topk_idx, topk_weights, T, quant)
+                torch.empty(4 + MAX_RANKS, dtype=torch.int32, device=dev), lay, topk_idx, topk_weights, T, quant)
+            if row_info:
+                out.row_expert = torch.empty(n_cap, dtype=torch.int64, device=dev)
+                out.row_weight = torch.empty(n_cap, dtype=torch.float32, device=dev)
         p = _DispatchParams()
         p.R, p.rank, p.E, p.K, p.H, p.cap, p.quant, p.T = self.R, self.rank, self.E, K, H, self.cap, int(quant), T
         p.n_cap, p.a_cap = out.recv_x.shape[0], out.recv_meta.shape[0]
@@ -330,13 +344,20 @@ class EpNormal(Recoverable):
         p.counts_dev, p.counts_host = out.counts.data_ptr(), self.mirror.dev_ptr
         p.ctrl, p.status = self.ctrl.data_ptr(), self.status.data_ptr()
         p.diag = self.diag_dispatch.data_ptr() if self.diagnose else None
+        if out.row_expert is not None:
+            p.row_expert, p.row_weight = out.row_expert.data_ptr(), out.row_weight.data_ptr()
+        p.per_expert_host = self.mirror.dev_ptr + 32
         rc = self.lib.umdk_ep_dispatch(ctypes.byref(p), _native.stream_ptr())
         if rc != 0:
             raise RuntimeError(f"umdk_ep_dispatch failed: {rc}")
         if sync_counts and (phase_mask & 2):
+            # one wait for everything the host reads: the counts lie in mapped memory, the status record comes along
+            self.status_host.copy_(self.status, non_blocking=True)
             torch.cuda.current_stream().synchronize()
-            check_status(self.status, "ep_dispatch", owner=self)
-            out.num_recv = int(self.mirror.host[0])
+            _raise_status(self.status_host.tolist(), self.status, "ep_dispatch", owner=self)
+            host = self.mirror.host
+            out.num_recv = int(host[0])
+            out.per_expert = host[8:8 + 2 * (self.E // self.R):2]   # low words: counts are far below 2^31
         return out
 
     @_trace.traced("umdk.ep.combine")
