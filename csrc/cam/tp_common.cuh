@@ -175,7 +175,9 @@ __device__ __forceinline__ void tp_copy_role_bulk(const TpArgs& a, int n_copy, i
       st_release_sys(reinterpret_cast<uint64_t*>(a.peers.base[threadIdx.x] + a.ready_off[slot]) + a.rank, tag);
     }
   }
-  for (int i = 0; i < a.R; ++i) {
+  // The GEMM reads the own shard where the caller has it: its counter only keeps step (the single-CTA kernel waits on it).
+  if (threadIdx.x == 0 && *s_ok) red_add_release_gpu(&a.chunk_done[a.rank], 1u);
+  for (int i = 1; i < a.R; ++i) {
     const int src = (a.rank + i) % a.R;
     if (threadIdx.x == 0) {
       const uint64_t* f = reinterpret_cast<const uint64_t*>(a.peers.base[a.rank] + a.ready_off[slot]) + src;

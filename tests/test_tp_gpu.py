@@ -150,3 +150,26 @@ def test_two_shot_allreduce_single_rank():
         assert torch.equal(out, x)
     finally:
         heap.close()
+
+
+def test_single_rank_pairs_and_single_ctas_alternate():
+    """One rank on CTA pairs reads its own tensor and stores the product itself; the single-CTA kernel goes through the heap.
+    Both keep the shared counters in step, so they can follow each other on one state."""
+    from umdk_b200.ops.tp import TpComm
+    from umdk_b200.parallel.symm import SymmetricHeap
+    g = torch.Generator().manual_seed(0)
+    Ts, K, N = 512, 320, 768
+    heap = SymmetricHeap(TpComm.heap_bytes(1, Ts, K, N))
+    try:
+        comm = TpComm(heap, Ts, K, N)
+        w = (torch.randn(N, K, generator=g) * 0.05).to(torch.bfloat16).cuda()
+        for single in (False, True, False, False, True):
+            comm.single_cta = single
+            x = torch.randn(Ts, K, generator=g).to(torch.bfloat16).cuda()
+            want = x.float() @ w.float().t()
+            ag, rs = comm.ag_gemm(x, w), comm.gemm_rs(x, w)
+            torch.cuda.synchronize()
+            comm.check()
+            assert _rel(ag, want) < 5e-3 and _rel(rs, want) < 5e-3
+    finally:
+        heap.close()
