@@ -444,3 +444,34 @@ def test_one_launch_layer_on_new_inputs_matches_its_phases():
             heap.close()
             res.append(out)
         assert torch.equal(res[0], res[1])
+
+
+@pytest.mark.parametrize("T,H,E,K", [(1, 128, 4, 1), (37, 2176, 40, 5), (128, 7168, 256, 8), (256, 1024, 33, 16)])
+def test_single_rank_short_path_matches_exchange(T, H, E, K):
+    """Low-latency dispatch and combine of one rank (no count exchange, rows summed where they lie) against the two
+    halves of the exchanging kernels: the same bytes, alternating on one state."""
+    from umdk_b200.ops.ep_ll import EpLowLatency
+    from umdk_b200.parallel.symm import SymmetricHeap
+    xs, idxs, ws = _inputs(1, T, H, E, K, seed=T)
+    heap = SymmetricHeap(EpLowLatency.heap_bytes(1, E, K, H, T + 2))
+    try:
+        st = EpLowLatency(heap, E, K, H, 256, T + 2)
+        n = int((idxs[0] >= 0).sum())
+        y = torch.randn(st.n_cap, H, device="cuda").to(torch.bfloat16)
+        for rnd in range(2):
+            x, idx, w = xs[0].cuda() + rnd, idxs[0].cuda(), ws[0].cuda()
+            outs = []
+            for masks in ((1, 2), (3,)):
+                for pm in masks:
+                    st.dispatch(x, idx, phase_mask=pm)
+                rows = [v[:n].clone() for v in st.slab_views()] + [st.group_off.clone(), st.recv_per_expert.clone()]
+                out = torch.full((T, H), float("nan"), dtype=torch.bfloat16, device="cuda")
+                for pm in masks:
+                    st.combine(y, idx, w, out=out, phase_mask=pm)
+                assert int(st.exp_cnt.abs().sum()) == 0
+                outs.append(rows + [out])
+            for u, v in zip(*outs):
+                assert torch.equal(u.view(torch.uint8), v.view(torch.uint8))
+        st.check()
+    finally:
+        heap.close()
