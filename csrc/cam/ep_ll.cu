@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kLLThreads, 1) ep_ll_combine_kernel(const LLCo
 // The same for a group of ONE rank: every row already lies in this GPU's memory, so the weighted sum reads it where it is.
 // Each CTA inverts the row metadata (row -> slot) into a slot -> row table in shared memory (a few KB), which replaces
 // the pass through the combine buffer, the completion flags and the grid-wide wait on them. Bound by latency: one table,
-// one round of row loads. Measured: 1024 rows of 7168 to 128 tokens 34.8 -> 15.0 us.
+// one round of row loads. Measured: 1024 rows of 7168 to 128 tokens 34.8 -> 12.9 us.
 constexpr int kLLLocalSlots = 11264;   // [T * K] ints in 44 KB of shared memory
 __global__ void __launch_bounds__(kLLThreads, 1) ep_ll_combine_local_kernel(const LLCombineArgs a) {
   extern __shared__ int s_rowof[];
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kLLThreads, 1) ep_ll_combine_local_kernel(cons
     for (int i = 0; i < 4; ++i) po[i] = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
     reinterpret_cast<int4*>(a.out + (size_t)t * g.H)[v] = o;
   }
-  if (cta_done_is_last(&a.ctrl[2], gridDim.x)) {   // the call ends: arrival words back to zero, next epoch
+  if (cta_done_is_last(&a.ctrl[2], gridDim.x, false)) {   // the call ends: arrival words back to zero, next epoch
     uint32_t* exp_cnt = reinterpret_cast<uint32_t*>(self + a.off.exp_cnt[0]);
     for (int i = threadIdx.x; i < g.E_local; i += blockDim.x) exp_cnt[i] = 0;
     if (threadIdx.x == 0) a.ctrl[0] += 1;

@@ -676,13 +676,6 @@ __global__ void __launch_bounds__(kEpThreads, 1) ep_dispatch_local_kernel(const 
       a.counts_dev[2] = arrivals;
       a.counts_dev[3] = 0;
       a.counts_dev[4] = 0;
-      if (a.counts_host) {
-        a.counts_host[0] = run;
-        a.counts_host[1] = arrivals;
-        a.counts_host[2] = arrivals;
-        __threadfence_system();
-        a.counts_host[4] = (int)(a.ctrl[0] + 1);
-      }
       if (a.diag) a.diag[0] = 0;
       if (run > a.n_cap || arrivals > a.a_cap)
         umdk_set_status(a.status, UMDK_ERR_OVERFLOW, UMDK_PH_DISPATCH_COUNT, run, arrivals);
@@ -802,8 +795,16 @@ __global__ void __launch_bounds__(kEpThreads, 1) ep_dispatch_local_kernel(const 
       }
     }
   }
+  if (a.counts_host && blockIdx.x == 0 && threadIdx.x == 0) {   // last: nothing here has to wait for the host's memory
+    const int arrivals = a.num_per_rank[0];
+    a.counts_host[0] = s_total;
+    a.counts_host[1] = arrivals;
+    a.counts_host[2] = arrivals;
+    __threadfence_system();
+    a.counts_host[4] = (int)(a.ctrl[0] + 1);
+  }
   // the epoch advances as in the exchanging kernel, so that the two can follow each other
-  if (cta_done_is_last(&a.ctrl[2], gridDim.x) && threadIdx.x == 0) a.ctrl[0] += 1;
+  if (cta_done_is_last(&a.ctrl[2], gridDim.x, false) && threadIdx.x == 0) a.ctrl[0] += 1;
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -1125,7 +1126,7 @@ __global__ void __launch_bounds__(kEpThreads, 1) ep_combine_local_kernel(const C
     if (a.in_rank[t]) continue;
     for (int v = lane; v < nvec; v += 32) reinterpret_cast<int4*>(a.out + (size_t)t * g.H)[v] = make_int4(0, 0, 0, 0);
   }
-  if (cta_done_is_last(&a.ctrl[5], gridDim.x) && threadIdx.x == 0) a.ctrl[3] += 1;
+  if (cta_done_is_last(&a.ctrl[5], gridDim.x, false) && threadIdx.x == 0) a.ctrl[3] += 1;
 }
 
 }  // namespace

@@ -566,16 +566,18 @@ moe_fused_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constant
 
   // ---- combine tail ----
   if (a.phase_mask & 1) {
-    if (cta_done_is_last(&a.ctrl[1], gridDim.x)) {
+    if (cta_done_is_last(&a.ctrl[1], gridDim.x, a.R > 1)) {
       // Every CTA is through with the slab: the arrival words go back to zero BEFORE the combine flags go out - a
       // peer starts its next call (and adds to these words again) only after it has seen this rank's flag.
       if (a.exp_cnt != nullptr)
         for (int i = threadIdx.x; i < a.G; i += blockDim.x) a.exp_cnt[i] = 0;
       for (int i = threadIdx.x; i < tiles; i += blockDim.x) a.tile_done[i] = 0;  // counters start from zero next call
-      __threadfence_system();
+      fence_for(a.R > 1);
       __syncthreads();
       if (threadIdx.x < a.R) {
-        st_release_sys(reinterpret_cast<uint64_t*>(a.peers.base[threadIdx.x] + a.comb_flag_off) + a.rank, tag);
+        uint64_t* flag = reinterpret_cast<uint64_t*>(a.peers.base[threadIdx.x] + a.comb_flag_off) + a.rank;
+        if (a.R > 1) st_release_sys(flag, tag);
+        else st_release_gpu(flag, tag);
       }
     }
   }
@@ -594,7 +596,7 @@ moe_fused_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constant
     ll_weighted_reduce<kThreads>(self + a.comb_buf_off, a.topk_idx, a.topk_w, a.out, a.share_out, a.T, a.Kt, a.H);
   }
   stamp(5);
-  if (cta_done_is_last(&a.ctrl[2], gridDim.x)) {
+  if (cta_done_is_last(&a.ctrl[2], gridDim.x, a.R > 1)) {
     if (threadIdx.x == 0) a.ctrl[0] = epoch + 1;
   }
 }

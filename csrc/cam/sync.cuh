@@ -76,20 +76,28 @@ __device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t num_ctas) {
   return s_ok != 0;
 }
 
+// Fence for stores that other GPUs read (`peers`) or only this one. A call that stays on this GPU passes false: at system
+// scope the fence waits for every store in flight beyond the GPU's own memory system.
+__device__ __forceinline__ void fence_for(bool peers) {
+  if (peers) __threadfence_system();
+  else __threadfence();
+}
+
 // "Last CTA" detector: every CTA calls it once when its part of a phase is complete (all threads, after their
 // stores). Returns true in exactly one CTA - the last to arrive - and resets the counter for the next launch.
-__device__ __forceinline__ bool cta_done_is_last(uint32_t* counter, uint32_t num_ctas) {
+// `peers`: other GPUs read what this phase stored (see fence_for).
+__device__ __forceinline__ bool cta_done_is_last(uint32_t* counter, uint32_t num_ctas, bool peers = true) {
   __shared__ int s_last;
-  // All threads' stores are ordered before the barrier; one system-scope fence by the thread that signals then
-  // orders them (cumulatively) before the counter update, the same shape as a cooperative grid barrier.
+  // All threads' stores are ordered before the barrier; one fence by the thread that signals then orders them
+  // (cumulatively) before the counter update, the same shape as a cooperative grid barrier.
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence_system();
+    fence_for(peers);
     const uint32_t old = atomicAdd(counter, 1u);
     s_last = (old == num_ctas - 1) ? 1 : 0;
     if (s_last) {
       *counter = 0;
-      __threadfence_system();
+      fence_for(peers);
     }
   }
   __syncthreads();
