@@ -54,22 +54,20 @@ class _CountingLib:
     """Proxy over the ctypes library that counts calls of kernel-launching entry points."""
 
     def __init__(self, lib: ctypes.CDLL):
-        object.__setattr__(self, "_lib", lib)
-        object.__setattr__(self, "_wrapped", {})
+        self._lib = lib
 
     def __getattr__(self, name):
+        # first use of an entry point only: what is found becomes an attribute of the proxy
         fn = getattr(self._lib, name)
         n = _KERNEL_ENTRY_POINTS.get(name)
-        if n is None:
-            return fn
-        w = self._wrapped.get(name)
-        if w is None:
-            def w(*args, _fn=fn, _n=n):
+        if n is not None:
+            def counted(*args, _fn=fn, _n=n):
                 global LAUNCH_COUNT
                 LAUNCH_COUNT += _n
                 return _fn(*args)
-            self._wrapped[name] = w
-        return w
+            fn = counted
+        setattr(self, name, fn)
+        return fn
 
 
 _cam_proxy = None
@@ -118,5 +116,15 @@ def ptr(t) -> ctypes.c_void_p:
 
 
 def stream_ptr() -> ctypes.c_void_p:
-    import torch
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream of the current device, without building a torch stream object for it (that costs a launch's worth
+    of host time per call)."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        torch.cuda.init()
+        dev, raw = torch.cuda.current_device, torch._C._cuda_getCurrentRawStream
+        _raw_stream = lambda: raw(dev())
+    return ctypes.c_void_p(_raw_stream())
+
+
+_raw_stream = None

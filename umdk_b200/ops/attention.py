@@ -2,6 +2,8 @@
 CTAs per (sequence, key-list split), the feature dimensions divided between them."""
 from __future__ import annotations
 
+import ctypes
+import functools
 from typing import Optional, Tuple
 
 import torch
@@ -12,6 +14,11 @@ HEADS = 128
 DIM = 576
 DIM_V = 512
 PAGE = 64
+
+
+@functools.lru_cache(maxsize=None)
+def _sm_count(device: int) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
 
 
 def sparse_mla_decode(q: torch.Tensor, kv_pages: torch.Tensor, block_table: torch.Tensor, indices: torch.Tensor,
@@ -40,7 +47,7 @@ def sparse_mla_decode(q: torch.Tensor, kv_pages: torch.Tensor, block_table: torc
         status = torch.zeros(4, dtype=torch.int32, device=dev)
     # one CTA pair resolves at most 2064 selected rows up front: longer key lists need more splits
     if num_splits <= 0:
-        sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        sms = _sm_count(dev.index)
         num_splits = max(1, min(sms // (2 * B), topk // (4 * 48), 16))
     num_splits = max(num_splits, int(lib.umdk_sparse_mla_min_splits(topk)))
     if workspace is not None and workspace[0].shape[1] != num_splits:
@@ -51,7 +58,6 @@ def sparse_mla_decode(q: torch.Tensor, kv_pages: torch.Tensor, block_table: torc
             workspace = (torch.empty(B, num_splits, HEADS, DIM_V, dtype=torch.float32, device=dev),
                          torch.empty(B, num_splits, HEADS, dtype=torch.float32, device=dev))
         po, pl = workspace
-    import ctypes
     rc = lib.umdk_sparse_mla_decode(
         _native.ptr(q), _native.ptr(kv_pages), _native.ptr(block_table), _native.ptr(indices),
         _native.ptr(seq_lens), _native.ptr(out), _native.ptr(lse), _native.ptr(po), _native.ptr(pl),

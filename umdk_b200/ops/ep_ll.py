@@ -199,6 +199,18 @@ class EpLowLatency(Recoverable):
         # the call here); part of what reset() clears
         from ..utils.rawtensor import from_ptr
         self.exp_cnt = from_ptr(self._local(self.lay.exp_cnt), (self.E_local,), torch.int32, dev)
+        self._slab = None
+        # the fields of the argument blocks that no call changes; every call works on a copy
+        self._dispatch_base = self._base(_LLDispatchParams(), recv_per_expert=self.recv_per_expert)
+        self._combine_base = self._base(_LLCombineParams())
+
+    def _base(self, p, **tensors):
+        p.R, p.rank, p.E, p.K, p.H, p.T_cap = self.R, self.rank, self.E, self.K, self.H, self.T_cap
+        for i, pp in enumerate(self.heap.peer_ptrs):
+            p.peers[i] = pp
+        for name, t in dict(tensors, group_off=self.group_off, ctrl=self.ctrl, status=self.status).items():
+            setattr(p, name, t.data_ptr())
+        return p
 
     @staticmethod
     def heap_bytes(R: int, E: int, K: int, H: int, T_cap: int, fold_shared: bool = False) -> int:
@@ -225,13 +237,17 @@ class EpLowLatency(Recoverable):
         return self.heap.local_ptr + off
 
     def slab_views(self):
-        """(slab_x fp8 [n_cap, H], slab_s fp32 [n_cap, H/128], slab_meta int32 [n_cap, 2]) as torch tensors."""
+        """(slab_x fp8 [n_cap, H], slab_s fp32 [n_cap, H/128], slab_meta int32 [n_cap, 2]) as torch tensors (made once:
+        adopting three raw pointers costs the host as much as launching the dispatch)."""
+        if self._slab is not None:
+            return self._slab
         from ..utils.rawtensor import from_ptr
         x = from_ptr(self._local(self.lay.slab_x), (self.n_cap, self.H), torch.uint8, self.device).view(
             torch.float8_e4m3fn)
         s = from_ptr(self._local(self.lay.slab_s), (self.n_cap, self.H // 128), torch.float32, self.device)
         m = from_ptr(self._local(self.lay.slab_meta), (self.n_cap, 2), torch.int32, self.device)
-        return x, s, m
+        self._slab = (x, s, m)
+        return self._slab
 
     # -- kernels -------------------------------------------------------------------------------------------------
     @_trace.traced("umdk.ep_ll.dispatch")
@@ -245,18 +261,13 @@ class EpLowLatency(Recoverable):
             2 * (((T + 31) // 32) * self.E + 2 * T * self.K) <= 160 * 1024
         if lay is None and not inline:
             lay = ep_layout(topk_idx, self.E, self.R, self.layout_scratch, self.layout_bar, self.status)
-        p = _LLDispatchParams()
-        p.R, p.rank, p.E, p.K, p.H, p.T_cap, p.T = self.R, self.rank, self.E, self.K, self.H, self.T_cap, T
-        p.num_ctas, p.phase_mask = self.dispatch_ctas, phase_mask
-        for i, pp in enumerate(self.heap.peer_ptrs):
-            p.peers[i] = pp
+        p = _LLDispatchParams.from_buffer_copy(self._dispatch_base)
+        p.T, p.num_ctas, p.phase_mask = T, self.dispatch_ctas, phase_mask
         p.x, p.topk_idx = x.data_ptr(), topk_idx.data_ptr()
         if lay is not None:
             p.send_idx, p.num_per_expert = lay.send_token_idx.data_ptr(), lay.num_tokens_per_expert.data_ptr()
         else:
             p.send_idx = p.num_per_expert = None
-        p.group_off, p.recv_per_expert = self.group_off.data_ptr(), self.recv_per_expert.data_ptr()
-        p.ctrl, p.status = self.ctrl.data_ptr(), self.status.data_ptr()
         rc = self.lib.umdk_ep_ll_dispatch(ctypes.byref(p), _native.stream_ptr())
         if rc != 0:
             raise RuntimeError(f"umdk_ep_ll_dispatch failed: {rc}")
@@ -274,14 +285,9 @@ class EpLowLatency(Recoverable):
         T = topk_idx.shape[0]
         if out is None:
             out = torch.empty(T, self.H, dtype=torch.bfloat16, device=y.device)
-        p = _LLCombineParams()
-        p.R, p.rank, p.E, p.K, p.H, p.T_cap, p.T = self.R, self.rank, self.E, self.K, self.H, self.T_cap, T
-        p.num_ctas, p.phase_mask = num_ctas, phase_mask
-        for i, pp in enumerate(self.heap.peer_ptrs):
-            p.peers[i] = pp
-        p.y, p.group_off = y.data_ptr(), self.group_off.data_ptr()
-        p.topk_idx, p.topk_w, p.out = topk_idx.data_ptr(), topk_w.data_ptr(), out.data_ptr()
-        p.ctrl, p.status = self.ctrl.data_ptr(), self.status.data_ptr()
+        p = _LLCombineParams.from_buffer_copy(self._combine_base)
+        p.T, p.num_ctas, p.phase_mask = T, num_ctas, phase_mask
+        p.y, p.topk_idx, p.topk_w, p.out = y.data_ptr(), topk_idx.data_ptr(), topk_w.data_ptr(), out.data_ptr()
         rc = self.lib.umdk_ep_ll_combine(ctypes.byref(p), _native.stream_ptr())
         if rc != 0:
             raise RuntimeError(f"umdk_ep_ll_combine failed: {rc}")
