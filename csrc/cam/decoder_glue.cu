@@ -50,21 +50,35 @@ add_rmsnorm_kernel(const __nv_bfloat16* __restrict__ x_in, const __nv_bfloat16* 
   __shared__ float red[kNormThreads / 32];
   const int t = blockIdx.x;
   const int nvec = H >> 3;
+  // Every load of the row is issued before the first is used (x_out may be x_in, so the compiler cannot move a later
+  // load above the store of an earlier vector): one round trip to memory instead of one per vector of a thread. 64 rows of
+  // 7168 with two addends: 5.4 -> 2.8 us.
+  uint4 xu[kMaxVecPerThread], au[kMaxVecPerThread], bu[kMaxVecPerThread], wu[kMaxVecPerThread];
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+#pragma unroll
+  for (int i = 0; i < kMaxVecPerThread; ++i) {
+    const int j = threadIdx.x + i * kNormThreads;
+    const bool in = j < nvec;
+    xu[i] = in ? reinterpret_cast<const uint4*>(x_in + (size_t)t * ld_in)[j] : zero;
+    au[i] = in && a != nullptr ? reinterpret_cast<const uint4*>(a + (size_t)t * H)[j] : zero;
+    bu[i] = in && b != nullptr ? reinterpret_cast<const uint4*>(b + (size_t)t * H)[j] : zero;
+    wu[i] = in ? reinterpret_cast<const uint4*>(w)[j] : zero;
+  }
   float v[kMaxVecPerThread][8];
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < kMaxVecPerThread; ++i) {
     const int j = threadIdx.x + i * kNormThreads;
     if (j < nvec) {
-      unpack8(reinterpret_cast<const uint4*>(x_in + (size_t)t * ld_in)[j], v[i]);
+      unpack8(xu[i], v[i]);
       float e[8];
       if (a != nullptr) {
-        unpack8(reinterpret_cast<const uint4*>(a + (size_t)t * H)[j], e);
+        unpack8(au[i], e);
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[i][q] += e[q];
       }
       if (b != nullptr) {
-        unpack8(reinterpret_cast<const uint4*>(b + (size_t)t * H)[j], e);
+        unpack8(bu[i], e);
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[i][q] += e[q];
       }
@@ -83,7 +97,7 @@ add_rmsnorm_kernel(const __nv_bfloat16* __restrict__ x_in, const __nv_bfloat16* 
     const int j = threadIdx.x + i * kNormThreads;
     if (j < nvec) {
       float g[8];
-      unpack8(reinterpret_cast<const uint4*>(w)[j], g);
+      unpack8(wu[i], g);
 #pragma unroll
       for (int q = 0; q < 8; ++q) v[i][q] = v[i][q] * inv * g[q];
       reinterpret_cast<uint4*>(h + (size_t)t * H)[j] = pack8(v[i]);
