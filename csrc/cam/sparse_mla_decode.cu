@@ -16,16 +16,23 @@
 //   and accumulates its own 256 output columns O[128 x 256] += P[128 x 48] * V[48 x own latent dims]  (3 MMAs),
 //   reading V from the SAME gathered tile through an MN-major descriptor.
 // Splitting by dimension halves the resident Q (80 KB instead of 144 KB), which makes room for a three-stage ring
-// of key tiles, and halves the Q*K^T work of each SM. Roles inside a CTA (13 warps):
-//   warps 0-3  softmax: tcgen05.ld of S, add the partner's partial, exp2, P to shared memory, lazy rescale of O
-//   warps 9-12 exchange: tcgen05.ld of the same S and asynchronous stores of it into the partner's shared memory,
+// of key tiles, and halves the Q*K^T work of each SM. Q moves to TMEM before the first chunk and P never leaves it: both
+// are A operands read out of TMEM, so that shared memory (128 bytes a clock) only feeds the key tiles to the MMAs.
+// TMEM columns: two S buffers of 48 (P takes the first 24 of its S), Q 160, O 256. Roles inside a CTA (20 warps):
+//   warps 0-7  softmax in two sets of four (half of a chunk's keys each): tcgen05.ld of S, add the partner's partial,
+//              common maximum of the sets, exp2, P to TMEM, lazy rescale of O
+//   warps 8-11 exchange: tcgen05.ld of the same S and asynchronous stores of it into the partner's shared memory,
 //              so that the round trip between the two CTAs is off the softmax warps' critical path
-//   warp  4    one thread issues every MMA: Q*K^T of chunk c+1 is issued BEFORE P*V of chunk c, so the tensor
-//              pipe works on the next scores while the softmax of the current chunk runs (S is double-buffered)
-//   warp  5    gather producer: TMA tile::gather4 copies (four selected rows x 128 bytes per instruction, written
+//   warp  12   MMA issuer (one elected thread)
+//   warps 13-19 gather producers: TMA tile::gather4 copies (four selected rows x 128 bytes per instruction, written
 //              in the 128-byte-swizzled layout the MMA descriptors expect), completion counted in bytes on the
-//              stage's barrier. Gathering with 16-byte cp.async was measured first: an SM sustains only about
-//              10 bytes per clock of such loads (2800 cycles for a 30 KB tile), whatever the access pattern
+//              stage's barrier. A warp issues its lanes' copies some 80 cycles apart and different warps side by side:
+//              48-key tiles of 640-byte pieces from 128 CTAs take 96 us for 2048 keys out of one warp, 57 us out of two,
+//              45 us out of four or more (3.7 TB/s of random 640-byte reads; 22 bytes per SM and clock when they hit
+//              L2). Gathering with 16-byte cp.async reaches the same 15 - 19 bytes with 16 warps, plain loads half of it.
+// What bounds it now: the softmax chain of a chunk (about 2600 cycles with its waits, the exp2 part 1240 of them), next
+// to 1600 cycles of DRAM time for the rows and some 1200 of MMAs. Batch 64, 2048 of 32768 keys: 94 -> 79 us; Q as an A
+// operand in shared memory alone kept one thread issuing MMAs for 2240 cycles a chunk.
 // All row addresses of the split are resolved once, up front, into shared memory (index -> page -> row).
 // The running maximum is only raised when it grows by more than 8 (in log2 units); P then stays below 2^8 and the
 // accumulated O needs rescaling only a few times per row instead of in most chunks.
@@ -48,21 +55,29 @@ constexpr int kQSlabBytes = kHeads * 128;        // 16 KB
 constexpr int kKSlabBytes = kChunk * 128;        // 6 KB
 constexpr int kQBytes = kMaxSlabs * kQSlabBytes; // 81920
 constexpr int kStageBytes = kMaxSlabs * kKSlabBytes;  // 30720
-constexpr int kPBytes = kHeads * 128;            // 16 KB (96 of every 128 bytes used)
 constexpr int kXBytes = kChunk * kHeads * 4;     // 24 KB, [key / 4][head][4] fp32
 constexpr int kMaxChunks = 43;                   // 2064 keys per split at most
 constexpr int kMaxKeys = kMaxChunks * kChunk;
-constexpr int kThreads = 416;
-constexpr int kProducerWarps = 4;   // warps 5..8 issue the gather copies: the TMA unit takes them faster from several warps
+constexpr int kSets = 2;            // softmax warp sets: set s (warps 4s .. 4s + 3) takes keys [24 s, 24 s + 24) of a chunk
+constexpr int kSetKeys = kChunk / kSets;
+constexpr int kSoftWarps = 4 * kSets;
+constexpr int kExchangeWarp = kSoftWarps;        // warps 8..11
+constexpr int kMmaWarp = kExchangeWarp + 4;      // warp 12
+constexpr int kProducerWarp = kMmaWarp + 1;      // warps 13..19
+constexpr int kProducerWarps = 7;
+constexpr int kThreads = 32 * (kProducerWarp + kProducerWarps);
+constexpr int kRowsPerThread = (kMaxKeys + kThreads - 1) / kThreads;
 constexpr int kTmemCols = 512;
-constexpr int kColS = 0;                         // two S buffers of 64 columns (48 used)
-constexpr int kColO = 128;
+constexpr int kColS = 0;                         // two S buffers of kChunk columns
+constexpr int kColQ = 2 * kChunk;                // Q as bf16 pairs, 32 columns per 64-dim slab
+constexpr int kColO = 256;
+static_assert(kColQ + kMaxSlabs * 32 <= kColO, "TMEM budget");
 constexpr int kOffK = kQBytes;
-constexpr int kOffP = kOffK + kStages * kStageBytes;
-constexpr int kOffX = kOffP + kPBytes;
+constexpr int kOffX = kOffK + kStages * kStageBytes;
 constexpr int kOffRows = kOffX + kXBytes;
 constexpr int kOffMask = kOffRows + kMaxKeys * 4;   // one 64-bit validity mask per chunk
-constexpr int kOffTail = kOffMask + ((kMaxChunks * 8 + 63) / 64) * 64;
+constexpr int kOffMax = kOffMask + ((kMaxChunks * 8 + 63) / 64) * 64;   // [2][kSets][128] chunk maxima of the sets
+constexpr int kOffTail = kOffMax + 2 * kSets * kHeads * 4;
 constexpr int kSmemBytes = 1024 + kOffTail + 256;
 static_assert(kSmemBytes <= 232448, "shared memory budget");
 static_assert(kStageBytes % 1024 == 0 && kKSlabBytes % 1024 == 0, "swizzle atoms must stay 1024-byte aligned");
@@ -86,19 +101,6 @@ struct MlaArgs {
   long long* diag;
 };
 
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
 // Bounded waits that also leave when either CTA of the pair has raised the abort flag.
 template <bool kCluster>
 __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
@@ -131,12 +133,27 @@ __device__ __forceinline__ void tma_gather4(void* smem_dst, const CUtensorMap* m
       "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(col), "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w)
       : "memory");
 }
-// Arrival on the partner's barrier WITHOUT release semantics. A release at cluster scope waits until every store this
-// thread has in flight (the asynchronous remote stores above all) is acknowledged, which was measured at about 3000
-// cycles per chunk. The barrier it is used for (`partner may overwrite my exchange buffer`) only has to follow this
-// warp's LOADS of that buffer, and those have completed once their values were used: instructions issue in order.
-__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+// D[tmem] (+)= A[tmem] * B[smem]; issued by ONE thread. A: lane = row, each 32-bit column two consecutive K elements.
+__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_x8(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st_x4(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3])
+               : "memory");
 }
 // 2^x with the special-function unit's native approximation (2 ulp; -inf gives 0): P is rounded to bf16 anyway.
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -148,6 +165,22 @@ __device__ __forceinline__ void st_cluster_u32(uint32_t cluster_addr, uint32_t v
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
 
+// Barrier of the softmax warps that also joins a decision: true on all of them or on none.
+__device__ __forceinline__ bool bar_softmax_and(bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.u32 q, %1, 0;\n"
+      "barrier.cta.red.and.pred p, 1, %2, q;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(r)
+      : "r"(ok ? 1u : 0u), "n"(32 * kSoftWarps)
+      : "memory");
+  return r != 0;
+}
+
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV,
                          const MlaArgs a) {
@@ -155,10 +188,10 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* q_sm = smem;
   uint8_t* k_sm = smem + kOffK;
-  uint8_t* p_sm = smem + kOffP;
   float* x_sm = reinterpret_cast<float*>(smem + kOffX);
   int* rows_sm = reinterpret_cast<int*>(smem + kOffRows);
   unsigned long long* mask_sm = reinterpret_cast<unsigned long long*>(smem + kOffMask);
+  float* max_sm = reinterpret_cast<float*>(smem + kOffMax);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kOffTail);
   uint64_t* bar_q = bars;            // 1
   // Arrivals are one per WARP: the lanes order their own accesses before a __syncwarp() and lane 0 arrives, so a
@@ -167,16 +200,17 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   uint64_t* bar_full = bars + 1;     // kStages, one arrival that expects the tile's bytes from the TMA gathers
   uint64_t* bar_empty = bars + 4;    // kStages, one commit
   uint64_t* bar_s = bars + 7;        // 2, one commit
-  uint64_t* bar_sfree = bars + 9;    // 2, arrivals of the 4 softmax warps and the 4 exchange warps
-  uint64_t* bar_p = bars + 11;       // 4 softmax-warp arrivals
+  uint64_t* bar_xld = bars + 9;      // 2, 4 exchange-warp arrivals: they have read this S buffer, P may take its place
+  uint64_t* bar_p = bars + 11;       // 8 softmax-warp arrivals
   uint64_t* bar_o = bars + 12;       // one commit
   uint64_t* bar_xfull = bars + 13;   // one local arrival that expects the 24 KB the partner's st.async stores deliver
-  uint64_t* bar_xfree = bars + 14;   // 4 arrivals from the partner's softmax warps: its X may be overwritten
+  uint64_t* bar_xfree = bars + 14;   // 8 arrivals from the partner's softmax warps: its X may be overwritten
   uint64_t* bar_fin = bars + 15;     // one commit (drain on the abort path)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* bar_qt = bars + 16;      // 8 softmax-warp arrivals: Q is in TMEM
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int b = blockIdx.y;
   const int half = static_cast<int>(cluster_ctarank());   // == blockIdx.x & 1
   const int split = blockIdx.x >> 1;
@@ -195,45 +229,61 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bar_s[i], 1);
-      mbar_init(&bar_sfree[i], 8);
+      mbar_init(&bar_xld[i], 4);
     }
-    mbar_init(bar_p, 4);
+    mbar_init(bar_p, kSoftWarps);
     mbar_init(bar_o, 1);
     mbar_init(bar_xfull, 1);
-    mbar_init(bar_xfree, 4);
+    mbar_init(bar_xfree, kSoftWarps);
     mbar_init(bar_fin, 1);
+    mbar_init(bar_qt, kSoftWarps);
     mbar_fence_init();
-    tma_prefetch_desc(&tmQ);
-    tma_prefetch_desc(&tmKV);
     *s_abort = 0;
+    fence_proxy_async_smem();   // the barrier's initial state, before the copy engine counts on it
+    // Q is on its way while the rows are resolved
+    mbar_expect_tx(bar_q, static_cast<uint32_t>(n_slabs) * kQSlabBytes);
+    for (int j = 0; j < n_slabs; ++j) {
+      const int dim0 = j < 4 ? half * 256 + j * 64 : 512;
+      tma_load_2d(q_sm + j * kQSlabBytes, &tmQ, bar_q, dim0, b * kHeads);
+    }
+    tma_prefetch_desc(&tmKV);
   }
-  if (warp == 4) {
+  if (warp == kMmaWarp) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
-  // resolve every selected row of this split once: index -> page -> row number in the pool (-1 = masked)
-  for (int k = tid; k < num_chunks * kChunk; k += kThreads) {
-    const int kpos = k_begin + k;
-    int idx = kpos < k_end ? a.indices[(size_t)b * a.topk + kpos] : -1;
-    if (idx < 0 || idx >= seq_len) idx = -1;
-    int row = -1;
-    if (idx >= 0) {
-      const int pg = idx / kPage;
-      const int page = pg < a.max_pages ? a.block_table[(size_t)b * a.max_pages + pg] : -1;
-      if (page < 0 || page >= a.num_pages) {
-        umdk_set_status(a.status, UMDK_ERR_OVERFLOW, UMDK_PH_NONE, b, idx);
-      } else {
-        row = page * kPage + (idx % kPage);
-      }
+  // Resolve every selected row of this split once: index -> page -> row number in the pool (-1 = masked). All indices of a
+  // thread are loaded before the first page lookup, so that the split pays two round trips to memory and not two per step.
+  {
+    int idx[kRowsPerThread], page[kRowsPerThread];
+#pragma unroll
+    for (int i = 0; i < kRowsPerThread; ++i) {
+      const int kpos = k_begin + tid + i * kThreads;
+      idx[i] = kpos < k_end ? a.indices[(size_t)b * a.topk + kpos] : -1;
     }
-    rows_sm[k] = row;
+#pragma unroll
+    for (int i = 0; i < kRowsPerThread; ++i) {
+      if (idx[i] >= seq_len) idx[i] = -1;
+      const int pg = idx[i] / kPage;
+      page[i] = idx[i] >= 0 && pg < a.max_pages ? a.block_table[(size_t)b * a.max_pages + pg] : -1;
+    }
+#pragma unroll
+    for (int i = 0; i < kRowsPerThread; ++i) {
+      const int k = tid + i * kThreads;
+      if (k >= num_chunks * kChunk) break;
+      int row = -1;
+      if (idx[i] >= 0) {
+        if (page[i] < 0 || page[i] >= a.num_pages) umdk_set_status(a.status, UMDK_ERR_OVERFLOW, UMDK_PH_NONE, b, idx[i]);
+        else row = page[i] * kPage + (idx[i] % kPage);
+      }
+      rows_sm[k] = row;
+    }
   }
   __syncthreads();
-  for (int c = tid; c < num_chunks; c += kThreads) {   // bit j of mask c: key j of chunk c takes part
-    unsigned long long m = 0;
-    for (int j = 0; j < kChunk; ++j)
-      if (rows_sm[c * kChunk + j] >= 0) m |= 1ull << j;
-    mask_sm[c] = m;
+  for (int c = warp; c < num_chunks; c += kThreads / 32) {   // bit j of mask c: key j of chunk c takes part
+    const uint32_t lo = __ballot_sync(0xffffffffu, rows_sm[c * kChunk + lane] >= 0);
+    const uint32_t hi = __ballot_sync(0xffffffffu, lane < kChunk - 32 && rows_sm[c * kChunk + 32 + (lane & 15)] >= 0);
+    if (lane == 0) mask_sm[c] = static_cast<unsigned long long>(hi) << 32 | lo;
   }
   tc_fence_before();
   __syncthreads();
@@ -250,14 +300,39 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   };
 
   if (num_chunks > 0) {
-    if (warp < 4) {
+    if (warp < kSoftWarps) {
       // ===================================== softmax ======================================================
-      const int head = tid;   // == TMEM lane
-      const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+      // Two sets of four warps share the heads (a thread per head and set) and split the keys of a chunk: one thread
+      // walking 48 keys alone is a chain of some 1100 cycles a chunk, longer than everything it waits for.
+      const int set = warp >> 2;
+      const int head = (warp & 3) * 32 + lane;   // == TMEM lane
+      const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+      const int key0 = set * kSetKeys;
       if (tid == 0) mbar_expect_tx(bar_xfull, kXBytes);   // arms the first phase; re-armed after every chunk
       const uint32_t peer_xfree = map_to_cta(bar_xfree, peer);
       float m_run = -INFINITY, l_run = 0.f;
-      bool ok = true;
+      // Q moves from shared memory into TMEM once: as the A operand of every Q * K^T step it would otherwise be read out
+      // of shared memory again for each chunk (80 KB for 48 keys, more than everything else together), and the shared
+      // memory's 128 bytes a clock are what this kernel runs out of first.
+      bool ok = __all_sync(0xffffffffu, wait_bar<false>(bar_q, 0, s_abort));
+      if (!ok) give_up(UMDK_PH_TMA_FULL, 0);
+      for (int j = set; j < n_slabs; j += kSets) {
+        const uint8_t* qrow = q_sm + j * kQSlabBytes + head * 128;
+        uint32_t w[32];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const uint4 v = *reinterpret_cast<const uint4*>(qrow + ((u ^ (head & 7)) << 4));
+          w[4 * u] = v.x;
+          w[4 * u + 1] = v.y;
+          w[4 * u + 2] = v.z;
+          w[4 * u + 3] = v.w;
+        }
+        tmem_st_x32(lane_addr + kColQ + j * 32, w);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_qt);
       const bool dg = a.diag != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0;
       long long dt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       long long t_prev = dg ? clock64() : 0;
@@ -268,52 +343,57 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           t_prev = t;
         }
       };
-      for (int c = 0; c < num_chunks && ok; ++c) {
+      // A wait that runs out in one warp must not leave the others at their next barrier: every warp walks on to the
+      // barrier of the chunk (or of the epilogue), which makes the decision common, before it leaves.
+      for (int c = 0; c < num_chunks; ++c) {
         const int sb = c & 1;
-        if (!__all_sync(0xffffffffu, wait_bar<false>(&bar_s[sb], (c >> 1) & 1, s_abort))) {
-          give_up(UMDK_PH_TMEM_FULL, c);
-          ok = false;
-          break;
+        if (ok) {
+          ok = __all_sync(0xffffffffu, wait_bar<false>(&bar_s[sb], (c >> 1) & 1, s_abort));
+          if (!ok) give_up(UMDK_PH_TMEM_FULL, c);
         }
         lap(0);
         tc_fence_after();
-        uint32_t sr[kChunk];
-        tmem_ld_x16(lane_addr + kColS + sb * 64, sr);
-        tmem_ld_x16(lane_addr + kColS + sb * 64 + 16, sr + 16);
-        tmem_ld_x16(lane_addr + kColS + sb * 64 + 32, sr + 32);
+        uint32_t sr[kSetKeys];
+        tmem_ld_x16(lane_addr + kColS + sb * kChunk + key0, sr);
+        tmem_ld_x8(lane_addr + kColS + sb * kChunk + key0 + 16, sr + 16);
         tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bar_sfree[sb]);
         lap(1);
         // the partner's partial comes in through the exchange warps of the other CTA
-        if (!__all_sync(0xffffffffu, wait_bar<true>(bar_xfull, c & 1, s_abort))) {
-          give_up(UMDK_PH_GROUP_READY, 1000 + c);
-          ok = false;
-          break;
+        if (ok) {
+          ok = __all_sync(0xffffffffu, wait_bar<true>(bar_xfull, c & 1, s_abort));
+          if (!ok) give_up(UMDK_PH_GROUP_READY, 1000 + c);
         }
         lap(4);
         // S = own partial + partner's partial (raw dot products; the scale is folded into the exponent below)
-        const unsigned long long valid = mask_sm[c];
-        float mx = -INFINITY;
+        float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        const float4* xp = reinterpret_cast<const float4*>(x_sm) + (key0 / 4) * kHeads + head;
 #pragma unroll
-        for (int j4 = 0; j4 < kChunk / 4; ++j4) {
-          const float4 xv = reinterpret_cast<const float4*>(x_sm)[j4 * kHeads + head];
-          const float xs4[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int j = 4 * j4 + u;
-            float t = __uint_as_float(sr[j]) + xs4[u];
-            if (!((valid >> j) & 1ull)) t = -INFINITY;
-            sr[j] = __float_as_uint(t);
-            mx = fmaxf(mx, t);
-          }
+        for (int j4 = 0; j4 < kSetKeys / 4; ++j4) {
+          const float4 xv = xp[j4 * kHeads];
+          sr[4 * j4] = __float_as_uint(__uint_as_float(sr[4 * j4]) + xv.x);
+          sr[4 * j4 + 1] = __float_as_uint(__uint_as_float(sr[4 * j4 + 1]) + xv.y);
+          sr[4 * j4 + 2] = __float_as_uint(__uint_as_float(sr[4 * j4 + 2]) + xv.z);
+          sr[4 * j4 + 3] = __float_as_uint(__uint_as_float(sr[4 * j4 + 3]) + xv.w);
         }
+        const uint32_t valid = static_cast<uint32_t>(mask_sm[c] >> key0) & ((1u << kSetKeys) - 1u);
+        if (valid != (1u << kSetKeys) - 1u) {   // the same for every thread of the set
+#pragma unroll
+          for (int j = 0; j < kSetKeys; ++j)
+            if (!((valid >> j) & 1u)) sr[j] = __float_as_uint(-INFINITY);
+        }
+#pragma unroll
+        for (int j = 0; j < kSetKeys; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], __uint_as_float(sr[j]));
+        float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
         // every lane's loads of x_sm have returned (mx depends on them); keep the arrival behind that dependence
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 0));
-        if (tid == 0 && c + 1 < num_chunks) mbar_expect_tx(bar_xfull, kXBytes);   // next phase, before the partner may send
+        max_sm[(sb * kSets + set) * kHeads + head] = mx;
+        ok = bar_softmax_and(ok);   // both sets' maxima are in place
+        if (!ok) break;
+        // re-armed before the partner may send again (its permission needs this warp's arrival below)
+        if (tid == 0 && c + 1 < num_chunks) mbar_expect_tx(bar_xfull, kXBytes);
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster_relaxed(peer_xfree);
+        mx = fmaxf(mx, max_sm[(sb * kSets + (set ^ 1)) * kHeads + head]);
         mx *= a.scale_log2;   // scale_log2 > 0: the maximum of the scaled scores
         // lazy maximum: raise it only when it grows by more than 8 (P stays below 2^8)
         float alpha = 1.f;
@@ -324,29 +404,37 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           m_run = m_new;
         }
         const float neg_m = m_run == -INFINITY ? 0.f : -m_run;
-        float sum = 0.f;
-        uint32_t pk[kChunk / 2];
+        float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+        uint32_t pk[kSetKeys / 2];
 #pragma unroll
-        for (int j = 0; j < kChunk / 2; ++j) {
+        for (int j = 0; j < kSetKeys / 2; ++j) {
           const float p0 = ex2_approx(fmaf(__uint_as_float(sr[2 * j]), a.scale_log2, neg_m));
           const float p1 = ex2_approx(fmaf(__uint_as_float(sr[2 * j + 1]), a.scale_log2, neg_m));
-          sum += p0 + p1;
+          sum4[j & 3] += p0 + p1;
           const __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);
           pk[j] = *reinterpret_cast<const uint32_t*>(&hh);
         }
-        l_run = l_run * alpha + sum;
+        l_run = l_run * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));   // of this set's keys
         lap(5);
         // P(c) overwrites P(c-1) and O may be rescaled: P(c-1) * V must have finished
-        if (c >= 1 && !__all_sync(0xffffffffu, wait_bar<false>(bar_o, (c - 1) & 1, s_abort))) {
-          give_up(UMDK_PH_TMEM_EMPTY, c);
-          ok = false;
-          break;
+        if (c >= 1) {
+          ok = __all_sync(0xffffffffu, wait_bar<false>(bar_o, (c - 1) & 1, s_abort));
+          if (!ok) {
+            give_up(UMDK_PH_TMEM_EMPTY, c);
+            continue;
+          }
+        }
+        // S(c) has been read by both sets (the barrier above) and by the exchange warps
+        ok = __all_sync(0xffffffffu, wait_bar<false>(&bar_xld[sb], (c >> 1) & 1, s_abort));
+        if (!ok) {
+          give_up(UMDK_PH_TMEM_EMPTY, 500 + c);
+          continue;
         }
         lap(6);
         tc_fence_after();
         if (c >= 1 && __any_sync(0xffffffffu, alpha != 1.f)) {
 #pragma unroll 1
-          for (int c0 = 0; c0 < 256; c0 += 32) {
+          for (int c0 = set * 128; c0 < set * 128 + 128; c0 += 32) {   // each set scales its half of the columns
             uint32_t o[32];
             tmem_ld_x32(lane_addr + kColO + c0, o);
             tmem_ld_wait();
@@ -356,12 +444,11 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           }
           tmem_st_wait();
         }
-        uint8_t* prow = p_sm + head * 128;
-#pragma unroll
-        for (int j8 = 0; j8 < kChunk / 8; ++j8)
-          *reinterpret_cast<uint4*>(prow + ((j8 ^ (head & 7)) << 4)) =
-              make_uint4(pk[4 * j8], pk[4 * j8 + 1], pk[4 * j8 + 2], pk[4 * j8 + 3]);
-        fence_proxy_async_smem();
+        // P takes the place of S as the A operand of P * V (key pairs in 24 of S's 48 columns): through shared memory the
+        // store and its proxy fence alone took some 800 cycles a chunk next to the MMAs' operand reads
+        tmem_st_x8(lane_addr + kColS + sb * kChunk + set * (kSetKeys / 2), pk);
+        tmem_st_x4(lane_addr + kColS + sb * kChunk + set * (kSetKeys / 2) + 8, pk + 8);
+        tmem_st_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_p);
@@ -371,20 +458,25 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         for (int i = 0; i < 8; ++i)
           if (i != 2 && i != 3) a.diag[i] = dt[i];
       }
-      // ---- epilogue: this CTA's 256 output columns ----
-      // (every decision below is warp-uniform: the TMEM loads are warp-collective)
-      if (ok && !__all_sync(0xffffffffu, wait_bar<false>(bar_o, (num_chunks - 1) & 1, s_abort))) {
-        give_up(UMDK_PH_TMEM_EMPTY, 2000);
-        ok = false;
+      // ---- epilogue: this CTA's 256 output columns, half of them per set ----
+      // (every decision below is the same for all eight warps: the TMEM loads are warp-collective)
+      if (ok) {
+        ok = __all_sync(0xffffffffu, wait_bar<false>(bar_o, (num_chunks - 1) & 1, s_abort));
+        if (!ok) give_up(UMDK_PH_TMEM_EMPTY, 2000);
       }
+      // both sets' sums; the last chunk used the other half of max_sm
+      max_sm[((num_chunks & 1) * kSets + set) * kHeads + head] = l_run;
+      ok = bar_softmax_and(ok);
+      l_run += max_sm[((num_chunks & 1) * kSets + (set ^ 1)) * kHeads + head];
       tc_fence_after();
       if (ok) {
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
         const float lse2 = l_run > 0.f ? m_run + log2f(l_run) : -INFINITY;
+        const int col0 = set * 128;
         if (a.num_splits == 1) {
           __nv_bfloat16* dst = a.out + ((size_t)b * kHeads + head) * kDimV + half * 256;
 #pragma unroll 1
-          for (int c0 = 0; c0 < 256; c0 += 32) {
+          for (int c0 = col0; c0 < col0 + 128; c0 += 32) {
             uint32_t o[32];
             tmem_ld_x32(lane_addr + kColO + c0, o);
             tmem_ld_wait();
@@ -400,11 +492,11 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
               *reinterpret_cast<uint4*>(dst + c0 + q * 8) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
             }
           }
-          if (half == 0 && a.lse) a.lse[(size_t)b * kHeads + head] = lse2 * 0.6931471805599453f;
+          if (half == 0 && set == 0 && a.lse) a.lse[(size_t)b * kHeads + head] = lse2 * 0.6931471805599453f;
         } else {
           float* dst = a.part_o + (((size_t)b * a.num_splits + split) * kHeads + head) * kDimV + half * 256;
 #pragma unroll 1
-          for (int c0 = 0; c0 < 256; c0 += 32) {
+          for (int c0 = col0; c0 < col0 + 128; c0 += 32) {
             uint32_t o[32];
             tmem_ld_x32(lane_addr + kColO + c0, o);
             tmem_ld_wait();
@@ -415,21 +507,19 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
                               __uint_as_float(o[q * 4 + 2]) * inv, __uint_as_float(o[q * 4 + 3]) * inv);
             }
           }
-          if (half == 0) a.part_lse[((size_t)b * a.num_splits + split) * kHeads + head] = lse2;
+          if (half == 0 && set == 0) a.part_lse[((size_t)b * a.num_splits + split) * kHeads + head] = lse2;
         }
       }
-    } else if (warp == 4) {
+    } else if (warp == kMmaWarp) {
       // ===================================== MMA issuer ===================================================
-      if (lane == 0) {
-        mbar_expect_tx(bar_q, static_cast<uint32_t>(n_slabs) * kQSlabBytes);
-        for (int j = 0; j < n_slabs; ++j) {
-          const int dim0 = j < 4 ? half * 256 + j * 64 : 512;
-          tma_load_2d(q_sm + j * kQSlabBytes, &tmQ, bar_q, dim0, b * kHeads);
-        }
+      if (elect_one()) {
         constexpr uint32_t idesc_qk = umma_idesc(kFmtBF16, kFmtBF16, kHeads, kChunk);
         constexpr uint32_t idesc_pv = umma_idesc(kFmtBF16, kFmtBF16, kHeads, 256, 0, 1);
-        bool ok = wait_bar<false>(bar_q, 0, s_abort);
+        bool ok = wait_bar<false>(bar_qt, 0, s_abort);
         if (!ok) give_up(UMDK_PH_TMA_FULL, 0);
+        const uint64_t k_desc = umma_desc_k_sw128(smem_u32(k_sm));
+        const uint64_t v_desc = umma_desc_mn_sw128(smem_u32(k_sm), kKSlabBytes, 1024);
+
         const bool dg = a.diag != nullptr && blockIdx.x == 0 && blockIdx.y == 0;
         long long dt[4] = {0, 0, 0, 0};
         const long long t_begin = dg ? clock64() : 0;
@@ -448,18 +538,23 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
             return false;
           }
           lap(0);
-          if (c >= 2 && !wait_bar<false>(&bar_sfree[c & 1], ((c >> 1) - 1) & 1, s_abort)) {
+          // S(c) overwrites S(c-2) and the P(c-2) in its place: P(c-2) * V has finished, and with it every reader of both
+          if (c >= 2 && !wait_bar<false>(bar_o, c & 1, s_abort)) {
             give_up(UMDK_PH_TMEM_EMPTY, 100 + c);
             return false;
           }
           lap(1);
           tc_fence_after();
-          const uint32_t d = tmem_base + kColS + (c & 1) * 64;
-          for (int j = 0; j < n_slabs; ++j) {
-            const uint64_t ad = umma_desc_k_sw128(smem_u32(q_sm + j * kQSlabBytes));
-            const uint64_t bd = umma_desc_k_sw128(smem_u32(k_sm + st * kStageBytes + j * kKSlabBytes));
+          const uint32_t d = tmem_base + kColS + (c & 1) * kChunk;
+          // one add per step: everything else about the operands is constant
+          const uint64_t bd = k_desc + st * (kStageBytes >> 4);
+          const uint32_t q = tmem_base + kColQ;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) umma_f16(d, ad + 2 * k, bd + 2 * k, idesc_qk, (j | k) ? 1u : 0u);
+          for (int j = 0; j < kMaxSlabs; ++j) {
+            if (j >= n_slabs) break;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              umma_f16_ta(d, q + j * 32 + k * 8, bd + j * (kKSlabBytes >> 4) + 2 * k, idesc_qk, (j | k) ? 1u : 0u);
           }
           umma_commit(&bar_s[c & 1]);
           lap(3);
@@ -477,13 +572,11 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           lap(2);
           tc_fence_after();
           const int st = c % kStages;
-          const uint32_t v_base = smem_u32(k_sm + st * kStageBytes);
+          const uint64_t vd = v_desc + st * (kStageBytes >> 4);
 #pragma unroll
-          for (int k = 0; k < kChunk / 16; ++k) {   // 16 keys per step: A advances 32 bytes, B two 8-key groups
-            const uint64_t ad = umma_desc_k_sw128(smem_u32(p_sm)) + 2 * k;
-            const uint64_t bd = umma_desc_mn_sw128(v_base + k * 2048, kKSlabBytes, 1024);
-            umma_f16(tmem_base + kColO, ad, bd, idesc_pv, (c | k) ? 1u : 0u);
-          }
+          for (int k = 0; k < kChunk / 16; ++k)   // 16 keys per step: A advances 8 columns, B two 8-key groups
+            umma_f16_ta(tmem_base + kColO, tmem_base + kColS + (c & 1) * kChunk + k * 8, vd + k * (2048 >> 4), idesc_pv,
+                        (c | k) ? 1u : 0u);
           umma_commit(&bar_empty[st]);
           umma_commit(bar_o);
           lap(3);
@@ -497,8 +590,8 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           mbar_wait(bar_fin, 0);
         }
       }
-    } else if (warp >= 9) {
-      // ===================================== exchange (warps 9..12) =======================================
+    } else if (warp >= kExchangeWarp && warp < kMmaWarp) {
+      // ===================================== exchange (warps 8..11) =======================================
       const int head = (warp & 3) * 32 + lane;   // == TMEM lane
       const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
       const uint32_t peer_x = map_to_cta(x_sm, peer) + static_cast<uint32_t>(head) * 16u;
@@ -514,13 +607,13 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         }
         tc_fence_after();
         uint32_t sr[kChunk];
-        tmem_ld_x16(lane_addr + kColS + sb * 64, sr);
-        tmem_ld_x16(lane_addr + kColS + sb * 64 + 16, sr + 16);
-        tmem_ld_x16(lane_addr + kColS + sb * 64 + 32, sr + 32);
+        tmem_ld_x16(lane_addr + kColS + sb * kChunk, sr);
+        tmem_ld_x16(lane_addr + kColS + sb * kChunk + 16, sr + 16);
+        tmem_ld_x16(lane_addr + kColS + sb * kChunk + 32, sr + 32);
         tmem_ld_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bar_sfree[sb]);
+        if (lane == 0) mbar_arrive(&bar_xld[sb]);
         if (dg) t_prev = clock64();
         // the partner's softmax warps must have read the previous partial out of their exchange buffer
         if (c >= 1 && !__all_sync(0xffffffffu, wait_bar<false>(bar_xfree, (c - 1) & 1, s_abort))) {
@@ -542,10 +635,10 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         a.diag[2] = dt[0];
         a.diag[3] = dt[1];
       }
-    } else if (warp >= 5 && warp < 5 + kProducerWarps) {
-      // ===================================== gather producers (warps 5..) =====================================
+    } else {
+      // ===================================== gather producers (warps 13..19) ==================================
       bool ok = true;
-      const bool dg = a.diag != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && lane == 0 && warp == 5;
+      const bool dg = a.diag != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && lane == 0 && warp == kProducerWarp;
       long long dt[3] = {0, 0, 0};
       long long t_prev = dg ? clock64() : 0;
       auto lap = [&](int i) {
@@ -566,11 +659,13 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           }
         }
         lap(1);
-        if (warp == 5 && lane == 0) mbar_expect_tx(&bar_full[st], static_cast<uint32_t>(n_slabs) * kKSlabBytes);
+        if (warp == kProducerWarp && lane == 0) mbar_expect_tx(&bar_full[st], static_cast<uint32_t>(n_slabs) * kKSlabBytes);
         __syncwarp();
         uint8_t* stage = k_sm + st * kStageBytes;
         const int4* rows4 = reinterpret_cast<const int4*>(rows_sm + c * kChunk);
-        for (int u = (warp - 5) * 32 + lane; u < n_inst; u += 32 * kProducerWarps) {
+        // A warp issues its lanes' copies one after the other, about 80 cycles apart, and different warps issue side by
+        // side: the copies of a tile are dealt over all producer warps (nine each) instead of filling two of them.
+        for (int u = lane * kProducerWarps + warp - kProducerWarp; u < n_inst; u += 32 * kProducerWarps) {
           const int grp = u / n_slabs, slab = u - grp * n_slabs;
           int4 r = rows4[grp];
           r.x = max(r.x, 0);   // masked keys read row 0: their scores are set to -inf before the softmax
@@ -601,37 +696,68 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 4) {
+  if (warp == kMmaWarp) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
   }
   cluster_sync_all();   // neither CTA leaves while the other may still write into its shared memory
 }
 
-// Joins the key-list splits: out = sum_i exp2(lse_i - lse) * o_i.
+// Joins the key-list splits: out = sum_i exp2(lse_i - lse) * o_i. One CTA per (sequence, head), four columns per thread; the
+// weights are made once per CTA and eight splits' partials are in flight at a time (bound by the latency of reading
+// num_splits x 2 KB per head out of L2).
 __global__ void __launch_bounds__(128) mla_merge_kernel(const float* __restrict__ part_o,
                                                         const float* __restrict__ part_lse,
                                                         __nv_bfloat16* __restrict__ out, float* __restrict__ lse,
                                                         int num_splits) {
-  const int bh = blockIdx.x;  // b * 128 + head
+  extern __shared__ float w_sm[];   // [num_splits]
+  const int bh = blockIdx.x;        // b * 128 + head
   const int b = bh / kHeads, head = bh % kHeads;
-  float mx = -INFINITY;
-  for (int s = 0; s < num_splits; ++s) mx = fmaxf(mx, part_lse[((size_t)b * num_splits + s) * kHeads + head]);
-  float den = 0.f;
-  for (int s = 0; s < num_splits; ++s) {
-    const float v = part_lse[((size_t)b * num_splits + s) * kHeads + head];
-    den += v == -INFINITY ? 0.f : exp2f(v - mx);
-  }
-  for (int d = threadIdx.x; d < kDimV; d += blockDim.x) {
-    float acc = 0.f;
-    for (int s = 0; s < num_splits; ++s) {
-      const float v = part_lse[((size_t)b * num_splits + s) * kHeads + head];
-      const float w = (v == -INFINITY || den == 0.f) ? 0.f : exp2f(v - mx) / den;
-      acc += w * part_o[(((size_t)b * num_splits + s) * kHeads + head) * kDimV + d];
+  const float4* po = reinterpret_cast<const float4*>(part_o + ((size_t)b * num_splits * kHeads + head) * kDimV) + threadIdx.x;
+  const size_t step = (size_t)kHeads * kDimV / 4;
+  float4 v[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+    if (u < num_splits) v[u] = __ldg(po + u * step);
+  if (threadIdx.x < 32) {
+    const float* pl = part_lse + (size_t)b * num_splits * kHeads + head;
+    float mx = -INFINITY;
+    for (int s = threadIdx.x; s < num_splits; s += 32) {
+      w_sm[s] = pl[(size_t)s * kHeads];
+      mx = fmaxf(mx, w_sm[s]);
     }
-    out[(size_t)bh * kDimV + d] = __float2bfloat16(acc);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    float den = 0.f;
+    for (int s = threadIdx.x; s < num_splits; s += 32) {
+      w_sm[s] = w_sm[s] == -INFINITY ? 0.f : exp2f(w_sm[s] - mx);
+      den += w_sm[s];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+    for (int s = threadIdx.x; s < num_splits; s += 32) w_sm[s] = den > 0.f ? w_sm[s] / den : 0.f;
+    if (threadIdx.x == 0 && lse) lse[bh] = den > 0.f ? (mx + log2f(den)) * 0.6931471805599453f : -INFINITY;
   }
-  if (threadIdx.x == 0 && lse) lse[bh] = den > 0.f ? (mx + log2f(den)) * 0.6931471805599453f : -INFINITY;
+  __syncthreads();
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s0 = 0; s0 < num_splits; s0 += 8) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (s0 + u >= num_splits) break;
+      if (s0 > 0) v[u] = __ldg(po + (s0 + u) * step);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (s0 + u >= num_splits) break;
+      const float w = w_sm[s0 + u];
+      acc.x = fmaf(w, v[u].x, acc.x);
+      acc.y = fmaf(w, v[u].y, acc.y);
+      acc.z = fmaf(w, v[u].z, acc.z);
+      acc.w = fmaf(w, v[u].w, acc.w);
+    }
+  }
+  __nv_bfloat162 o2[2] = {__floats2bfloat162_rn(acc.x, acc.y), __floats2bfloat162_rn(acc.z, acc.w)};
+  *reinterpret_cast<uint2*>(out + (size_t)bh * kDimV + threadIdx.x * 4) = *reinterpret_cast<const uint2*>(o2);
 }
 
 }  // namespace
@@ -688,7 +814,7 @@ UMDK_API int umdk_sparse_mla_decode(const void* q, const void* kv, const int* bl
   sparse_mla_decode_kernel<<<grid, kThreads, kSmemBytes, s>>>(tmQ, tmKV, a);
   UMDK_CUDA_CHECK(cudaGetLastError());
   if (num_splits > 1) {
-    mla_merge_kernel<<<B * kHeads, 128, 0, s>>>(part_o, part_lse, static_cast<__nv_bfloat16*>(out), lse, num_splits);
+    mla_merge_kernel<<<B * kHeads, 128, sizeof(float) * num_splits, s>>>(part_o, part_lse, static_cast<__nv_bfloat16*>(out), lse, num_splits);
     UMDK_CUDA_CHECK(cudaGetLastError());
   }
   return 0;

@@ -45,3 +45,38 @@ def test_sparse_mla_decode(B, ctx, topk, splits, inv):
     rel = ((out.float().cpu() - want).norm() / want.norm()).item()
     assert rel < 2e-2, (err, rel)
     assert torch.allclose(lse.cpu(), want_lse, atol=2e-2, rtol=1e-3)
+
+
+@pytest.mark.parametrize("B,topk,splits", [
+    (1, 1, 1), (2, 23, 1), (2, 25, 1), (1, 47, 1), (1, 49, 1), (2, 97, 2),   # around a set's 24 and a chunk's 48 keys
+    (1, 2064, 1),                                                            # all the rows one CTA pair resolves
+    (1, 480, 8), (1, 480, 9), (2, 1152, 24),                                 # the merge takes eight splits at a time
+])
+@pytest.mark.parametrize("kind", ["plain", "half_chunks", "growing"])
+def test_sparse_mla_decode_chunk_edges(B, topk, splits, kind):
+    """Chunk and set remainders; chunks in which one set's keys, or all keys, are masked; scores that grow along the key
+    list, so that the running maximum is raised and O rescaled in the middle of it."""
+    from umdk_b200.ops.attention import ref_sparse_mla_decode, sparse_mla_decode
+    q, kv, bt, idx = _case(B, 4096, topk, seed=topk + splits)
+    if kind == "half_chunks":
+        pos = torch.arange(topk)
+        idx[:, (pos // 24) % 4 == 0] = -1
+        idx[:, (pos // 48) % 4 == 1] = -1
+    if kind == "growing":   # every key is a multiple of the mean query: scores rise by some 30 (in log2 units) over the list
+        flat = kv.view(-1, 576)
+        mean = q.float().mean(1)
+        for b in range(B):
+            rows = bt[b].long()[idx[b].long() // 64] * 64 + idx[b].long() % 64
+            ramp = torch.linspace(0.0, 1.0, topk)[:, None] * 20.0 / mean[b].norm() ** 2 * 24
+            flat[rows] = (flat[rows].float() * 0.1 + ramp * mean[b]).to(torch.bfloat16)
+    scale = 576 ** -0.5
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    out, lse = sparse_mla_decode(q.cuda(), kv.cuda(), bt.cuda(), idx.cuda(), scale, num_splits=splits, status=status)
+    torch.cuda.synchronize()
+    assert status.tolist()[0] == 0, status.tolist()
+    want, want_lse = ref_sparse_mla_decode(q, kv, bt, idx, scale)
+    # P and the result are rounded to bf16 once each (2^-9 relative); the scores are exact fp32 sums of bf16 products
+    assert ((out.float().cpu() - want).norm() / want.norm().clamp_min(1e-9)).item() < 2e-2
+    assert torch.equal(torch.isinf(lse.cpu()), torch.isinf(want_lse))
+    ok = ~torch.isinf(want_lse)
+    assert torch.allclose(lse.cpu()[ok], want_lse[ok], atol=2e-2, rtol=1e-3)

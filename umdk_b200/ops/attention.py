@@ -29,7 +29,7 @@ def sparse_mla_decode(q: torch.Tensor, kv_pages: torch.Tensor, block_table: torc
     """q [B,128,576] bf16, kv_pages [P,64,576] bf16, block_table [B,max_pages] int32, indices [B,topk] int32
     (token positions; -1 = unused) -> (out [B,128,512] bf16, lse [B,128] fp32).
     ``num_splits`` 0 = as many splits of the key list as it takes to put a CTA pair on every SM (a batch of 64
-    already does with one split), each split keeping at least four 48-key chunks.
+    already does with one split), each split keeping at least two 48-key chunks, 24 splits at most.
     ``diag`` (int64 [16], device): the first CTA records how many cycles its roles spent in each of their waits and
     work sections (see MlaArgs::diag in the kernel source); for finding what bounds the pipeline."""
     lib = _native.cam()
@@ -48,7 +48,9 @@ def sparse_mla_decode(q: torch.Tensor, kv_pages: torch.Tensor, block_table: torc
     # one CTA pair resolves at most 2064 selected rows up front: longer key lists need more splits
     if num_splits <= 0:
         sms = _sm_count(dev.index)
-        num_splits = max(1, min(sms // (2 * B), topk // (4 * 48), 16))
+        # One sequence of 2048 keys: 10 splits 22.8 us, 16 splits 20.3, 22 splits 19.1, 43 splits 20.0 (a chunk each, twice
+        # the partials to join); 23 sequences of 1000 keys: 2 splits 35.7 us, 3 splits 30.7, 4 splits (a second wave) 46.3
+        num_splits = max(1, min(sms // (2 * B), topk // (2 * 48), 24))
     num_splits = max(num_splits, int(lib.umdk_sparse_mla_min_splits(topk)))
     if workspace is not None and workspace[0].shape[1] != num_splits:
         workspace = None
