@@ -12,12 +12,16 @@
 // product in TMEM (128 weight rows x 64 tokens); epilogue warps read it back with tcgen05.ld and accumulate
 // partial * w_scale * x_scale in fp32 registers while the next block's MMAs run into the other TMEM stage.
 //
+// Modes 0 and 1 normally run on CTA pairs (moe_gemm_pair.cu); this file keeps mode 2, mode 0 behind a start gate, and the
+// cases the pair kernel refuses.
+//
 // Role split per CTA (persistent, one CTA per SM): warp 0 TMA producer, warp 1 MMA issuer, warp 2 TMEM allocator,
 // warps 4-7 promotion + epilogue. The reference fuses the same chain on Ascend cube/vector cores with int8
 // operands and per-token scales (src/cam/comm_operator/ascend_kernels/fused_deep_moe/op_kernel/fused_deep_moe.h:354-448,
 // epilogue/block/block_epilogue_per_token_dequant_swiglu.h:255-283, gemm/kernel/post_swiglu_dynamic_quant.h:30-60,
 // epilogue/block/block_epilogue_per_token_dequant.hpp:199-250 for the combine-send epilogue).
 #include "ep_common.cuh"
+#include "moe_gemm_pair.cuh"
 #include "ptx.cuh"
 #include "sync.cuh"
 
@@ -545,6 +549,32 @@ UMDK_API int umdk_moe_gemm(const UmdkMoeGemmParams* p, void* stream) {
   a.status = p->status;
   a.phase_mask = p->phase_mask ? p->phase_mask : 3;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // Modes 0 and 1 run on CTA pairs, except behind a start gate (the low-latency layer's first GEMM), with one CTA, or with
+  // more experts than the pair kernel's tables hold. Tiles of 256 tokens where an expert has that many rows to fill them
+  // (average over the slab): 32 experts, hidden 7168, width 2048, narrow / wide in us, mode 0: 128 rows per expert 426 / 496,
+  // 256: 730 / 750, 512: 1311 / 1227; mode 1: 128: 206 / 209, 256: 358 / 323, 512: 664 / 574.
+  if (p->mode <= 1 && p->mode >= 0 && p->wait_n == 0) {
+    int grid = sm_count();
+    if (p->max_ctas > 0 && p->max_ctas < grid) grid = p->max_ctas;
+    grid &= ~1;
+    if (moe_gemm_pair_fits(p->G, grid)) {
+      MoePairArgs b;
+      b.G = a.G;
+      b.Nout = a.Nout;
+      b.K = a.K;
+      b.w_rows = a.w_rows;
+      b.n_rows_cap = a.n_rows_cap;
+      b.group_off = a.group_off;
+      b.xs = a.xs;
+      b.ws = a.ws;
+      b.hq = a.hq;
+      b.hs = a.hs;
+      b.y = a.y;
+      b.status = a.status;
+      const bool wide = p->n_rows_cap / p->G > (p->mode == 0 ? 384 : 160);
+      return moe_gemm_pair_launch(p->mode, wide, p->w, p->x, b, grid, s);
+    }
+  }
   switch (p->mode) {
     case 0: return launch<0>(p->w, p->x, a, s, p->max_ctas);
     case 1: return launch<1>(p->w, p->x, a, s, p->max_ctas);

@@ -1,0 +1,509 @@
+// Grouped (per-expert) fp8 GEMMs of the MoE FFN on CTA PAIRS (tcgen05.mma.cta_group::2): gate/up projection with SwiGLU
+// and fp8 re-quantisation (MODE 0) and down projection to bf16 rows (MODE 1), operand formats as in moe_gemm.cu.
+//
+// One item = 256 weight rows x up to NMAX tokens of one expert; each CTA of the pair stages 128 of the weight rows and
+// half of the tokens, and owns 128 rows x all tokens of the product. In MODE 0 the 128 rows of a CTA are 64 gate rows and
+// the 64 up rows of the same features, so that a pair finishes one 1x128 scale block: the per-token maxima of the two
+// halves cross once per item through distributed shared memory.
+//
+// What bounds it: every 128-wide K block must leave TMEM and be promoted in fp32 (partial * w_scale * x_scale), so MMA and
+// promotion pass the accumulators back and forth, and that round trip between the two SMs of a pair (about 4000 cycles)
+// times the 512 TMEM columns is the limit. Accumulators in flight hide it: eight of 64 tokens or two of 256. Eight warps
+// promote; the scale PRODUCTS are made once per (K block, token) by two further warps, which leaves one FMA per element
+// (skipping the FMAs altogether gains 7 % in MODE 0 and 30 % in MODE 1 at prefill sizes; the tensor cores' share is 30 %).
+// At decode sizes (tens of rows per expert) the weights bound it: the ring keeps 9 x 16 KB of them in flight per SM, and
+// items of half an SM pair's size fill the last wave (512 items on 148 CTAs left 14 % idle).
+// Measured against one CTA per tile (32 experts, hidden 7168, width 2048): 1024 rows 208 -> 187 us (MODE 0, 5.0 TB/s) and
+// 119 -> 91 us (MODE 1, 5.2 TB/s), 16384 rows 1237 -> 1227 us and 968 -> 574 us (840 TFLOP/s).
+#include "ep_common.cuh"
+#include "moe_gemm_pair.cuh"
+#include "ptx.cuh"
+
+namespace umdk {
+namespace {
+
+constexpr int kThreads = 384;
+constexpr int kEpiWarps = 8;
+constexpr int kBKB = 128;   // K bytes per block = one scale block = one swizzle atom
+
+template <int MODE, int NMAX>   // NMAX: 64 or 256 tokens
+struct Cfg {
+  static constexpr int kABytes = 128 * kBKB;
+  static constexpr int kBBytes = NMAX / 2 * kBKB;
+  static constexpr int kStageBytes = kABytes + kBBytes;
+  static constexpr int kStages = NMAX == 64 ? 9 : 5;
+  static constexpr int kBoxRows = NMAX == 64 ? 32 : 64;         // token rows per TMA box
+  static constexpr int kW = MODE == 0 ? 2 : 1;                  // scale rows per CTA (gate, up)
+  static constexpr int kScaleKb = NMAX == 64 ? 8 : 4;           // K blocks per scale stage
+  static constexpr int kScaleStages = NMAX == 64 ? 3 : 2;
+  static constexpr int kScaleFloats = kScaleKb * kW * NMAX;
+  static constexpr int kTmemStages = 512 / NMAX;                // accumulators in flight hide the hand-over between CTAs
+  static constexpr int kTmemCols = 512;
+  static constexpr int kTransBytes = 32 * 272;                  // per half: [32][136] bf16 or [32][65] fp32
+  static constexpr int kOffScale = kStages * kStageBytes;
+  static constexpr int kOffTrans = kOffScale + kScaleStages * kScaleFloats * 4;
+  static constexpr int kOffAmax = kOffTrans + 2 * kTransBytes;  // [2][NMAX] maxima of the partner's half
+  static constexpr int kOffBars = kOffAmax + 2 * NMAX * 4;
+  static constexpr int kNumBars = 2 * kStages + 2 * kTmemStages + 2 * kScaleStages + 2;
+  static constexpr int kOffTables = kOffBars + kNumBars * 8 + 16;
+};
+
+__device__ __forceinline__ uint32_t pack_fp8x4(float a, float b, float c, float d) {
+  const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
+  const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E4M3);
+  return (uint32_t)lo | ((uint32_t)hi << 16);
+}
+template <int R>
+__device__ __forceinline__ void regs_dec() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R));
+}
+template <int R>
+__device__ __forceinline__ void regs_inc() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R));
+}
+__device__ __forceinline__ void bar_half(int half) {
+  asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+}
+
+// The same barrier, joining a decision: true on all 128 threads or on none (a wait that ran out in one warp must not
+// leave the others at the next barrier).
+__device__ __forceinline__ bool bar_half_and(int half, bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.u32 q, %2, 0;\n"
+      "barrier.cta.red.and.pred p, %1, 128, q;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(r)
+      : "r"(1 + half), "r"(ok ? 1u : 0u)
+      : "memory");
+  return r != 0;
+}
+
+struct Item {
+  int e, j, row0, m, n;   // expert, feature tile, first row, valid rows, rows the MMA covers (multiple of 32)
+};
+
+template <int NMAX>
+__device__ __forceinline__ Item locate(const int* tile_pref, const int* goff, int G, int NT, int w) {
+  int lo = 0, hi = G;   // largest lo with tile_pref[lo] * NT <= w
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (tile_pref[mid] * NT <= w) lo = mid;
+    else hi = mid;
+  }
+  // the rows of an expert are cut into equal tiles (a multiple of 32 rows each), token tiles fastest: neighbouring
+  // pairs then read the same weight rows at the same time
+  const int ntt = tile_pref[lo + 1] - tile_pref[lo];
+  const int local = w - tile_pref[lo] * NT;
+  const int rows = goff[lo + 1] - goff[lo];
+  const int width = ((rows + ntt - 1) / ntt + 31) & ~31;
+  Item it;
+  it.e = lo;
+  it.j = local / ntt;
+  const int first = (local - it.j * ntt) * width;
+  it.row0 = goff[lo] + first;
+  it.m = min(width, rows - first);
+  it.n = (it.m + 31) & ~31;
+  return it;
+}
+
+template <int MODE, int NMAX>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
+                     const MoePairArgs a) {
+  using C = Cfg<MODE, NMAX>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  float* scale_sm = reinterpret_cast<float*>(smem + C::kOffScale);   // [stage][kb][gate/up][token]
+  float* amax_in = reinterpret_cast<float*>(smem + C::kOffAmax);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::kOffBars);
+  uint64_t* empty = full + C::kStages;
+  uint64_t* tfull = empty + C::kStages;
+  uint64_t* tempty = tfull + C::kTmemStages;
+  uint64_t* sfull = tempty + C::kTmemStages;
+  uint64_t* sempty = sfull + C::kScaleStages;
+  uint64_t* abar = sempty + C::kScaleStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(abar + 2);
+  int* tile_pref = reinterpret_cast<int*>(smem + C::kOffTables);   // [G + 1] token tiles before each expert
+  int* goff = tile_pref + a.G + 1;                                 // [G + 1]
+  __shared__ int s_ok;
+
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const uint32_t cta = cluster_ctarank();   // 0 = leader
+  const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  const int NT = MODE == 0 ? a.Nout / 128 : (a.Nout + 255) / 256;
+  const int kb_total = a.K / kBKB;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::kStages; ++s) {
+      mbar_init(&full[s], 1);    // leader's copy: one arrive (expect_tx) + the bytes of both CTAs
+      mbar_init(&empty[s], 1);   // one commit per CTA copy
+    }
+    for (int i = 0; i < C::kTmemStages; ++i) {
+      mbar_init(&tfull[i], 1);
+      mbar_init(&tempty[i], 2 * kEpiWarps);   // leader's copy: the promoting warps of both CTAs
+    }
+    for (int i = 0; i < 2; ++i) mbar_init(&abar[i], 1);   // one local arrive that expects the partner's maxima
+    for (int i = 0; i < C::kScaleStages; ++i) {
+      mbar_init(&sfull[i], 2);
+      mbar_init(&sempty[i], kEpiWarps);
+    }
+    mbar_fence_init();
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+    s_ok = 1;
+  }
+  if (warp == 2) {
+    tmem_alloc_pair(tmem_slot, C::kTmemCols);
+    tmem_relinquish_pair();
+  }
+  for (int i = threadIdx.x; i <= a.G; i += kThreads) goff[i] = a.group_off[i];
+  __syncthreads();
+  if (warp == 0) {   // exclusive scan of the token tiles per expert
+    int run = 0;
+    for (int e0 = 0; e0 < a.G; e0 += 32) {
+      const int e = e0 + lane;
+      int n = 0;
+      if (e < a.G) {
+        const int m = goff[e + 1] - goff[e];
+        if (m < 0 || goff[e] < 0 || goff[e + 1] > a.n_rows_cap) {
+          umdk_set_status(a.status, UMDK_ERR_OVERFLOW, UMDK_PH_GROUP_READY, e, goff[e + 1]);
+          s_ok = 0;
+        } else {
+          n = (m + NMAX - 1) / NMAX;
+        }
+      }
+      int x = n;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= d) x += y;
+      }
+      if (e < a.G) tile_pref[e] = run + x - n;
+      run += __shfl_sync(0xffffffffu, x, 31);
+    }
+    if (lane == 0) tile_pref[a.G] = run;
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();   // the peer's barriers exist before anything is signalled on them
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const int num_items = s_ok ? tile_pref[a.G] * NT : 0;
+
+  if (warp < 4) {
+    regs_dec<56>();
+    if (warp == 0) {
+      if (elect_one()) {
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int w = pair; w < num_items && ok; w += num_pairs) {
+          const Item it = locate<NMAX>(tile_pref, goff, a.G, NT, w);
+          const int nh = it.n / 2;
+          const int boxes = (nh + C::kBoxRows - 1) / C::kBoxRows;
+          const int xrow = it.row0 + (int)cta * nh;
+          const int wrow = it.e * a.w_rows + (MODE == 0 ? it.j * 128 + (int)cta * 64 : it.j * 256 + (int)cta * 128);
+          const uint32_t bytes = 2 * (C::kABytes + boxes * C::kBoxRows * kBKB);
+          for (int kb = 0; kb < kb_total; ++kb) {
+            if (!mbar_wait(&empty[s], ph ^ 1)) {
+              umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_EMPTY, w, kb);
+              ok = false;
+              break;
+            }
+            if (cta == 0) mbar_expect_tx(&full[s], bytes);
+            const uint32_t leader_full = map_to_cta(&full[s], 0);
+            uint8_t* st = smem + s * C::kStageBytes;
+            if (MODE == 0) {
+              tma_load_2d_pair(st, &tmW, leader_full, kb * kBKB, wrow);
+              tma_load_2d_pair(st + 64 * kBKB, &tmW, leader_full, kb * kBKB, wrow + a.Nout);
+            } else {
+              tma_load_2d_pair(st, &tmW, leader_full, kb * kBKB, wrow);
+            }
+            for (int b = 0; b < boxes; ++b)
+              tma_load_2d_pair(st + C::kABytes + b * C::kBoxRows * kBKB, &tmX, leader_full, kb * kBKB,
+                               xrow + b * C::kBoxRows);
+            if (++s == C::kStages) {
+              s = 0;
+              ph ^= 1;
+            }
+          }
+        }
+      }
+    } else if (warp == 1) {
+      if (cta == 0 && elect_one()) {
+        int s = 0;
+        uint32_t ph = 0, kbc = 0;
+        bool ok = true;
+        const uint64_t a_desc = umma_desc_k_sw128(smem_u32(smem));
+        for (int w = pair; w < num_items && ok; w += num_pairs) {
+          const Item it = locate<NMAX>(tile_pref, goff, a.G, NT, w);
+          const uint32_t idesc = umma_idesc(kFmtE4M3, kFmtE4M3, 256, it.n);
+          for (int kb = 0; kb < kb_total; ++kb, ++kbc) {
+            const int ts = kbc % C::kTmemStages;
+            if (!mbar_wait(&tempty[ts], ((kbc / C::kTmemStages) & 1) ^ 1)) {
+              umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_EMPTY, w, kb);
+              ok = false;
+              break;
+            }
+            if (!mbar_wait(&full[s], ph)) {
+              umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, kb);
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint64_t adesc = a_desc + s * (C::kStageBytes >> 4);
+            const uint64_t bdesc = adesc + (C::kABytes >> 4);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)   // 32 fp8 elements per MMA K step
+              umma_f8_pair(tmem_base + ts * NMAX, adesc + 2 * k, bdesc + 2 * k, idesc, k > 0 ? 1u : 0u);
+            umma_commit_both(smem_u32(&empty[s]));
+            umma_commit_both(smem_u32(&tfull[ts]));
+            if (++s == C::kStages) {
+              s = 0;
+              ph ^= 1;
+            }
+          }
+        }
+      }
+    } else {
+      // ---- scale products of the coming K blocks: x_scale[token] * w_scale[row block] ----
+      const int t64 = threadIdx.x - 64;
+      const int nsb = a.K / 128;
+      int ss = 0;
+      uint32_t sph = 0;
+      bool ok = true;
+      for (int w = pair; w < num_items && ok; w += num_pairs) {
+        const Item it = locate<NMAX>(tile_pref, goff, a.G, NT, w);
+        const int wsb = a.w_rows / 128;
+        const int blk = MODE == 0 ? it.j : min(2 * it.j + (int)cta, wsb - 1);
+        const float* ws0 = a.ws + ((size_t)it.e * wsb + blk) * nsb;
+        const float* ws1 = MODE == 0 ? ws0 + (size_t)(a.Nout / 128) * nsb : ws0;
+        for (int kb0 = 0; kb0 < kb_total; kb0 += C::kScaleKb) {
+          float xv[NMAX / 64][C::kScaleKb], w0[C::kScaleKb], w1[C::kScaleKb];
+#pragma unroll
+          for (int i = 0; i < C::kScaleKb; ++i) {
+            const bool in = kb0 + i < kb_total;
+            w0[i] = in ? __ldg(ws0 + kb0 + i) : 0.f;
+            w1[i] = MODE == 0 && in ? __ldg(ws1 + kb0 + i) : 0.f;
+          }
+#pragma unroll
+          for (int u = 0; u < NMAX / 64; ++u) {
+            const int t = t64 + 64 * u;
+#pragma unroll
+            for (int i = 0; i < C::kScaleKb; ++i)
+              xv[u][i] = t < it.m && kb0 + i < kb_total ? a.xs[(size_t)(it.row0 + t) * nsb + kb0 + i] : 0.f;
+          }
+          if (!__all_sync(0xffffffffu, mbar_wait(&sempty[ss], sph ^ 1))) {
+            umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_EMPTY, w, 10000 + kb0);
+            ok = false;
+            break;
+          }
+          float* dst = scale_sm + ss * C::kScaleFloats;
+#pragma unroll
+          for (int u = 0; u < NMAX / 64; ++u) {
+#pragma unroll
+            for (int i = 0; i < C::kScaleKb; ++i) {
+              dst[(i * C::kW) * NMAX + t64 + 64 * u] = xv[u][i] * w0[i];
+              if (MODE == 0) dst[(i * C::kW + C::kW - 1) * NMAX + t64 + 64 * u] = xv[u][i] * w1[i];
+            }
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sfull[ss]);
+          if (++ss == C::kScaleStages) {
+            ss = 0;
+            sph ^= 1;
+          }
+        }
+      }
+    }
+  } else {
+    regs_inc<224>();
+    // ---- promotion + epilogue: warp quarter q owns weight rows [32 q, 32 q + 32), `half` the lower / upper tokens ----
+    const int q = warp & 3, half = (warp - 4) >> 2;
+    const int tid = q * 32 + lane;   // == TMEM lane
+    constexpr int kBlocks = NMAX / 64;   // 32-token blocks per half
+    const int which = MODE == 0 ? q >> 1 : 0;   // 0: gate rows, 1: up rows
+    uint8_t* trans = smem + C::kOffTrans + half * C::kTransBytes;
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+    const uint32_t peer = cta ^ 1u;
+    int ss = 0, n_it = 0;
+    uint32_t sph = 0, kbc = 0;
+    bool ok = true;
+    for (int w = pair; w < num_items && ok; w += num_pairs, ++n_it) {
+      const Item it = locate<NMAX>(tile_pref, goff, a.G, NT, w);
+      const int nh = it.n / 2, col0 = half * nh;
+      const int par = n_it & 1;
+      if (MODE == 0 && warp == 4 && lane == 0) mbar_expect_tx(&abar[par], it.n * 4);
+      float acc[kBlocks * 32];
+#pragma unroll
+      for (int c = 0; c < kBlocks * 32; ++c) acc[c] = 0.f;
+      for (int kb0 = 0; kb0 < kb_total && ok; kb0 += C::kScaleKb) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&sfull[ss], sph))) {
+          umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, 10000 + kb0);
+          ok = false;
+          break;
+        }
+        const float* sc = scale_sm + ss * C::kScaleFloats + which * NMAX + col0;
+        const int kb1 = min(kb_total, kb0 + C::kScaleKb);
+        for (int kb = kb0; kb < kb1; ++kb, ++kbc, sc += C::kW * NMAX) {
+          const int ts = kbc % C::kTmemStages;
+          if (!__all_sync(0xffffffffu, mbar_wait(&tfull[ts], (kbc / C::kTmemStages) & 1))) {
+            umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, w, kb);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t taddr = lane_addr + ts * NMAX + col0;
+          uint32_t r[2][32];
+          tmem_ld_x32(taddr, r[0]);
+#pragma unroll
+          for (int b = 0; b < kBlocks; ++b) {
+            if (b * 32 >= nh) break;
+            tmem_ld_wait();
+            if ((b + 1) * 32 < nh) {
+              if (b + 1 < kBlocks) tmem_ld_x32(taddr + (b + 1) * 32, r[(b + 1) & 1]);
+            } else {   // everything of this stage is in registers: the next K block may overwrite it
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_cluster_relaxed(map_to_cta(&tempty[ts], 0));
+            }
+#pragma unroll
+            for (int c4 = 0; c4 < 8; ++c4) {
+              const float4 s4 = reinterpret_cast<const float4*>(sc + b * 32)[c4];
+              const int c = b * 32 + c4 * 4;
+              const uint32_t* rr = r[b & 1] + c4 * 4;
+              acc[c] = fmaf(__uint_as_float(rr[0]), s4.x, acc[c]);
+              acc[c + 1] = fmaf(__uint_as_float(rr[1]), s4.y, acc[c + 1]);
+              acc[c + 2] = fmaf(__uint_as_float(rr[2]), s4.z, acc[c + 2]);
+              acc[c + 3] = fmaf(__uint_as_float(rr[3]), s4.w, acc[c + 3]);
+            }
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sempty[ss]);
+        if (++ss == C::kScaleStages) {
+          ss = 0;
+          sph ^= 1;
+        }
+      }
+      ok = bar_half_and(half, ok);
+      if (!ok) break;
+      if (MODE == 1) {
+        const int feat0 = it.j * 256 + (int)cta * 128;
+        __nv_bfloat16* tb = reinterpret_cast<__nv_bfloat16*>(trans);
+#pragma unroll
+        for (int b = 0; b < kBlocks; ++b) {
+          if (b * 32 >= nh) break;
+#pragma unroll
+          for (int t = 0; t < 32; ++t) tb[t * 136 + tid] = __float2bfloat16(acc[b * 32 + t]);
+          bar_half(half);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int v = u * 128 + tid, t = v >> 4, tok = col0 + b * 32 + t;
+            if (b * 32 + t < nh && tok < it.m && feat0 < a.Nout) {
+              const int4 o = *reinterpret_cast<const int4*>(trans + t * 272 + (v & 15) * 16);
+              *reinterpret_cast<int4*>(a.y + (size_t)(it.row0 + tok) * a.Nout + feat0 + (v & 15) * 8) = o;
+            }
+          }
+          bar_half(half);
+        }
+      } else {
+        float* tf = reinterpret_cast<float*>(trans);   // [32 tokens][65]: up values, then h
+        const int f = (q & 1) * 32 + lane;             // feature inside this CTA's 64
+        const int t4 = tid >> 2, qq = tid & 3;         // afterwards: token and 16-feature quarter of a thread
+        float h[kBlocks][16], pm[kBlocks];
+        const uint32_t peer_amax = map_to_cta(amax_in + par * NMAX, peer);
+        const uint32_t peer_bar = map_to_cta(&abar[par], peer);
+#pragma unroll
+        for (int b = 0; b < kBlocks; ++b) {
+          if (b * 32 >= nh) break;
+          if (which == 1) {
+#pragma unroll
+            for (int t = 0; t < 32; ++t) tf[t * 65 + f] = acc[b * 32 + t];
+          }
+          bar_half(half);
+          if (which == 0) {
+#pragma unroll
+            for (int t = 0; t < 32; ++t) {
+              const float v = acc[b * 32 + t];
+              tf[t * 65 + f] = (v / (1.f + __expf(-v))) * tf[t * 65 + f];
+            }
+          }
+          bar_half(half);
+          float mx = 0.f;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            h[b][i] = tf[t4 * 65 + qq * 16 + i];
+            mx = fmaxf(mx, fabsf(h[b][i]));
+          }
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+          pm[b] = mx;
+          if (qq == 0 && b * 32 + t4 < nh) st_async_b32(peer_amax + (col0 + b * 32 + t4) * 4, __float_as_uint(mx), peer_bar);
+          if ((b + 1) * 32 < nh) bar_half(half);
+        }
+        ok = mbar_wait_cluster(&abar[par], (n_it >> 1) & 1);
+        if (!ok) umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_GROUP_READY, w, 20000);
+        ok = bar_half_and(half, ok);   // also: every read of the transposition buffer is done
+        if (!ok) break;
+#pragma unroll
+        for (int b = 0; b < kBlocks; ++b) {
+          const int tok = col0 + b * 32 + t4;
+          if (b * 32 + t4 < nh && tok < it.m) {
+            const float amax = fmaxf(fmaxf(pm[b], amax_in[par * NMAX + tok]), 1e-4f);
+            const float inv = 448.f / amax;
+            int4 o;
+            o.x = pack_fp8x4(h[b][0] * inv, h[b][1] * inv, h[b][2] * inv, h[b][3] * inv);
+            o.y = pack_fp8x4(h[b][4] * inv, h[b][5] * inv, h[b][6] * inv, h[b][7] * inv);
+            o.z = pack_fp8x4(h[b][8] * inv, h[b][9] * inv, h[b][10] * inv, h[b][11] * inv);
+            o.w = pack_fp8x4(h[b][12] * inv, h[b][13] * inv, h[b][14] * inv, h[b][15] * inv);
+            const size_t row = it.row0 + tok;
+            *reinterpret_cast<int4*>(a.hq + row * a.Nout + it.j * 128 + cta * 64 + qq * 16) = o;
+            if (cta == 0 && qq == 0) a.hs[row * (a.Nout / 128) + it.j] = amax * (1.f / 448.f);
+          }
+        }
+      }
+    }
+  }
+
+  // nobody leaves (or frees TMEM) while the peer may still signal this CTA's barriers or read its operands
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();
+  if (warp == 2) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, C::kTmemCols);
+  }
+}
+
+template <int MODE, int NMAX>
+int launch(const void* W, const void* X, const MoePairArgs& a, int grid, cudaStream_t stream) {
+  using C = Cfg<MODE, NMAX>;
+  CUtensorMap tmW, tmX;
+  if (make_tmap_2d(&tmW, TMAP_U8, W, a.K, (uint64_t)a.G * a.w_rows, a.K, kBKB, MODE == 0 ? 64 : 128, TMAP_SW_128B))
+    return -UMDK_ERR_BAD_ARG;
+  if (make_tmap_2d(&tmX, TMAP_U8, X, a.K, a.n_rows_cap, a.K, kBKB, C::kBoxRows, TMAP_SW_128B))
+    return -UMDK_ERR_BAD_ARG;
+  const size_t smem = 1024 + C::kOffTables + 2 * (size_t)(a.G + 1) * 4;
+  UMDK_CUDA_CHECK(cudaFuncSetAttribute(moe_gemm_pair_kernel<MODE, NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)smem));
+  moe_gemm_pair_kernel<MODE, NMAX><<<grid, kThreads, smem, stream>>>(tmW, tmX, a);
+  UMDK_CUDA_CHECK(cudaGetLastError());
+  return 0;
+}
+
+}  // namespace
+
+bool moe_gemm_pair_fits(int G, int grid) { return grid >= 2 && G <= 1024; }
+
+int moe_gemm_pair_launch(int mode, bool wide, const void* W, const void* X, const MoePairArgs& a, int grid,
+                         cudaStream_t stream) {
+  if (mode == 0) return wide ? launch<0, 256>(W, X, a, grid, stream) : launch<0, 64>(W, X, a, grid, stream);
+  return wide ? launch<1, 256>(W, X, a, grid, stream) : launch<1, 64>(W, X, a, grid, stream);
+}
+
+}  // namespace umdk

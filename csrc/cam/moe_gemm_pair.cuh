@@ -1,0 +1,26 @@
+// Entry of the CTA-pair grouped GEMM (moe_gemm_pair.cu) for the launcher in moe_gemm.cu.
+#pragma once
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace umdk {
+
+struct MoePairArgs {
+  int G, Nout, K, w_rows, n_rows_cap;
+  const int* group_off;    // [G + 1]
+  const float* xs;         // [n_rows_cap, K/128]
+  const float* ws;         // [G, w_rows/128, K/128]
+  uint8_t* hq;             // mode 0 out: [n_rows_cap, Nout] fp8
+  float* hs;               // mode 0 out: [n_rows_cap, Nout/128]
+  __nv_bfloat16* y;        // mode 1 out: [n_rows_cap, Nout]
+  int* status;
+};
+
+// Whether the pair kernel takes this call (a grid of at least one pair, tables of the experts fit in shared memory).
+bool moe_gemm_pair_fits(int G, int grid);
+// mode 0 or 1; `wide`: tiles of up to 256 tokens (else 64). `grid`: number of CTAs, even.
+int moe_gemm_pair_launch(int mode, bool wide, const void* W, const void* X, const MoePairArgs& a, int grid,
+                         cudaStream_t stream);
+
+}  // namespace umdk

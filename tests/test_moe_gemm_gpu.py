@@ -52,3 +52,18 @@ def test_grouped_ffn_matches_reference(G, counts, K, F, H):
     r_y = ref.ref_gemm2(hq.cpu(), hs.cpu(), c["off"], c["w2q"], c["w2s"])
     err = ref.mean_rel_err(y[:N].float().cpu(), r_y[:N])
     assert err < 5e-3, err
+
+
+# What the CTA-pair kernel can get wrong: one and several 64- / 256-token tiles and the remainders around 32 tokens (narrow
+# and wide tiles: the average of rows per expert picks them), K blocks that do not fill a scale stage, an odd number of
+# 128-row blocks in the down projection (the last pair has half a tile), empty experts.
+@pytest.mark.parametrize("G,counts,K,F,H", [
+    (3, [1, 31, 33], 128, 128, 128),
+    (4, [65, 64, 0, 32], 1152, 256, 384),
+    (1, [96], 640, 128, 384),
+    (2, [255, 257], 640, 128, 256),
+    (3, [300, 0, 513], 1152, 256, 384),
+    (2, [410, 385], 640, 256, 128),
+])
+def test_grouped_ffn_tile_edges(G, counts, K, F, H):
+    test_grouped_ffn_matches_reference(G, counts, K, F, H)
