@@ -240,11 +240,12 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     mbar_fence_init();
     *s_abort = 0;
     fence_proxy_async_smem();   // the barrier's initial state, before the copy engine counts on it
-    // Q is on its way while the rows are resolved
-    mbar_expect_tx(bar_q, static_cast<uint32_t>(n_slabs) * kQSlabBytes);
-    for (int j = 0; j < n_slabs; ++j) {
-      const int dim0 = j < 4 ? half * 256 + j * 64 : 512;
-      tma_load_2d(q_sm + j * kQSlabBytes, &tmQ, bar_q, dim0, b * kHeads);
+    if (num_chunks > 0) {   // Q is on its way while the rows are resolved; without keys nobody would wait for it
+      mbar_expect_tx(bar_q, static_cast<uint32_t>(n_slabs) * kQSlabBytes);
+      for (int j = 0; j < n_slabs; ++j) {
+        const int dim0 = j < 4 ? half * 256 + j * 64 : 512;
+        tma_load_2d(q_sm + j * kQSlabBytes, &tmQ, bar_q, dim0, b * kHeads);
+      }
     }
     tma_prefetch_desc(&tmKV);
   }
