@@ -506,13 +506,14 @@ struct UmdkMoeGemmParams {
 // long on a pair, which has half as many workers: with few items the pairs need a second wave where single CTAs have one,
 // and an odd number of 128-feature blocks leaves a mode-1 pair half idle. The rows of each expert are not known here:
 // single CTAs are taken where they win both for rows that share the buffer evenly and for random shares (half a tile more
-// per expert), and never with room for more than 128 per expert, where the buffer's size says little. Measured (us, single
+// per expert), and never with room for more than 128 per expert, where the buffer's size says little, or in mode 0 for more
+// than 64, which pairs take in one 256-token item (8 experts of 72 rows, 1024 of 2048: 28 / 21 us). Measured (us, single
 // / pairs): mode 0, 8 experts of 64 rows, 1280 features of 1152: 15.4 / 19.2, of 13 rows (a single CTA's masked rows cost
 // it more): 20.3 / 18.9; 32 experts of 64 rows, 2048 of 7168: 191 / 157; mode 1, 16 experts of 13 rows, 1152 of 2048: 14.3
 // / 19.5; 32 experts of 2 rows, 1152 of 2048: 22.4 / 25.3, of 256: 10.8 / 10.3; 7168 of 2048: 101 / 83.
 UMDK_API int umdk_moe_gemm_uses_pairs(int mode, int G, int Nout, int K, int rows, int ctas) {
   if (mode < 0 || mode > 1 || G < 1 || !moe_gemm_pair_fits(G, ctas & ~1)) return 0;
-  if (rows / G > 128) return 1;
+  if (rows / G > 128 || (mode == 0 && rows > 64 * (long)G)) return 1;
   const long even = rows > 64 * (long)G ? 2L * G : G;
   const long spread = rows > 32 * (long)G ? rows / 64 + G / 2 : G;
   for (const long tiles : {even, spread}) {

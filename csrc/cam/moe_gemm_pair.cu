@@ -1,21 +1,21 @@
 // Grouped (per-expert) fp8 GEMMs of the MoE FFN on CTA PAIRS (tcgen05.mma.cta_group::2): gate/up projection with SwiGLU
 // and fp8 re-quantisation (MODE 0) and down projection to bf16 rows (MODE 1), operand formats as in moe_gemm.cu.
 //
-// One item = 256 weight rows x up to NMAX tokens of one expert; each CTA of the pair stages 128 of the weight rows and
-// half of the tokens, and owns 128 rows x all tokens of the product. In MODE 0 the 128 rows of a CTA are 64 gate rows and
-// the 64 up rows of the same features, so that a pair finishes one 1x128 scale block: the per-token maxima of the two
-// halves cross once per item through distributed shared memory.
+// Every 128-wide K block must leave TMEM and be promoted in fp32 (partial * w_scale * x_scale): eight warps promote, the scale
+// PRODUCTS are made once per (K block, token) by two further warps. Two kinds of tile, picked from the rows that are there:
 //
-// What bounds it: every 128-wide K block must leave TMEM and be promoted in fp32 (partial * w_scale * x_scale), so MMA and
-// promotion pass the accumulators back and forth, and that round trip between the two SMs of a pair (about 4000 cycles)
-// times the 512 TMEM columns is the limit. Accumulators in flight hide it: eight of 64 tokens or two of 256. Eight warps
-// promote; the scale PRODUCTS are made once per (K block, token) by two further warps, which leaves one FMA per element
-// (skipping the FMAs altogether gains 7 % in MODE 0 and 30 % in MODE 1 at prefill sizes; the tensor cores' share is 30 %).
-// At decode sizes (tens of rows per expert) the weights bound it: the ring keeps 9 x 16 KB of them in flight per SM, and
-// items of half an SM pair's size fill the last wave (512 items on 148 CTAs left 14 % idle).
-// Measured against one CTA per tile (32 experts, hidden 7168, width 2048, rows spread unevenly, cold L2): 1024 rows 219 ->
-// 171 us (MODE 0, 5.5 TB/s) and 125 -> 99 us (MODE 1, 4.7 TB/s); 16384 rows 1231 -> 1188 us and 953 -> 513 us (940 TFLOP/s),
-// repeated under the power limit 1408 -> 1203 and 969 -> 521 us.
+// 64 tokens, the 256 weight rows of a pair on the MMA's M side (each CTA owns 128 of them x all tokens). For decode sizes (tens
+// of rows per expert), where the weights bound it: the ring keeps 9 x 16 KB of them in flight per SM. In MODE 0 the 128 rows of
+// a CTA are 64 gate rows and the 64 up rows of the same features, so that a pair finishes one 1x128 scale block: the
+// per-token maxima of the two halves cross once per item through distributed shared memory.
+//
+// 256 tokens on the M side (each CTA owns 128 of them x all 256 weight rows). With the weights there, a promoting thread needs
+// the scale of every COLUMN: a 16-byte broadcast load brings 512 bytes into a warp's registers, four cycles of the
+// shared-memory port, 1024 cycles a K block of 256 tokens for an MMA of 512. With the tokens there it needs one scale a K
+// block. Measured against 256-token tiles of the other kind (32 experts, hidden 7168, width 2048, 16384 rows spread unevenly):
+// 1188 -> 573 us (MODE 0) and 513 -> 328 us (MODE 1), 1.6 PFLOP/s; two promotions in one instruction (fma.rn.f32x2) are part
+// of it. A K block takes 900 cycles at 1.45 GHz under the power limit: the tensor cores 512, the rest is the promotion's chain
+// (wait, four to eight TMEM loads, 64 packed FMAs, release) of two warps a scheduler, which all but fills it.
 #include "ep_common.cuh"
 #include "fp8_block.cuh"
 #include "moe_gemm_pair.cuh"
@@ -28,62 +28,73 @@ constexpr int kThreads = 384;
 constexpr int kEpiWarps = 8;
 constexpr int kBKB = 128;   // K bytes per block = one scale block = one swizzle atom
 
-template <int MODE, int NMAX>   // NMAX: 64 or 256 tokens
+// Tiles with the WEIGHT ROWS on the MMA's M side and up to 64 tokens.
+constexpr int kTok = 64;
+template <int MODE>
 struct Cfg {
   static constexpr int kABytes = 128 * kBKB;
-  static constexpr int kBBytes = NMAX / 2 * kBKB;
+  static constexpr int kBBytes = kTok / 2 * kBKB;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = NMAX == 64 ? 9 : 5;
-  static constexpr int kBoxRows = NMAX == 64 ? 32 : 64;         // token rows per TMA box
+  static constexpr int kStages = 9;
+  static constexpr int kBoxRows = kTok / 2;                     // token rows per TMA box
   static constexpr int kW = MODE == 0 ? 2 : 1;                  // scale rows per CTA (gate, up)
-  static constexpr int kScaleKb = NMAX == 64 ? 8 : 4;           // K blocks per scale stage
-  static constexpr int kScaleStages = NMAX == 64 ? 3 : 2;
-  static constexpr int kScaleFloats = kScaleKb * kW * NMAX;
-  static constexpr int kTmemStages = 512 / NMAX;                // accumulators in flight hide the hand-over between CTAs
+  static constexpr int kScaleKb = 8;                            // K blocks per scale stage
+  static constexpr int kScaleStages = 3;
+  static constexpr int kScaleFloats = kScaleKb * kW * kTok;
+  static constexpr int kTmemStages = 512 / kTok;                // accumulators in flight hide the hand-over between CTAs
   static constexpr int kTransBytes = 32 * 272;                  // per half: [32][136] bf16 or [32][65] fp32
   static constexpr int kOffScale = kStages * kStageBytes;
   static constexpr int kOffTrans = kOffScale + kScaleStages * kScaleFloats * 4;
-  static constexpr int kOffAmax = kOffTrans + 2 * kTransBytes;  // [2][NMAX] maxima of the partner's half
-  static constexpr int kEnd = kOffAmax + 2 * NMAX * 4;
+  static constexpr int kOffAmax = kOffTrans + 2 * kTransBytes;  // [2][kTok] maxima of the partner's half
+  static constexpr int kEnd = kOffAmax + 2 * kTok * 4;
 };
 
-// Behind the buffers: barriers for either width (the counts are the same) and the tables.
+// Tiles with the TOKENS on the MMA's M side: one item = 256 tokens x 256 weight rows of one expert, each CTA of the pair owns 128
+// of the tokens (its TMEM lanes) x all 256 rows, as two accumulators of 128 columns per K block, one for each four of the
+// promoting warps - in MODE 0 64 gate rows and the up rows of the same features, so a thread has both factors of SwiGLU.
+template <int MODE>
+struct TokCfg {
+  static constexpr int kABytes = 128 * kBKB;
+  static constexpr int kBBytes = 64 * kBKB;   // per accumulator: half of its 128 weight rows
+  static constexpr int kStageBytes = kABytes + 2 * kBBytes;
+  static constexpr int kStages = 5;
+  static constexpr int kTmemStages = 4;       // 128 columns each: the MMAs are two accumulators ahead of the promotion
+  static constexpr int kScaleKb = 8;
+  static constexpr int kScaleStages = 2;
+  static constexpr int kScaleFloats = kScaleKb * 2 * 128;   // [kb][accumulator][token]
+  static constexpr int kTransBytes = 32 * 128;              // per warp
+  static constexpr int kOffScale = kStages * kStageBytes;
+  static constexpr int kOffTrans = kOffScale + kScaleStages * kScaleFloats * 4;
+  static constexpr int kOffAmax = kOffTrans + kEpiWarps * kTransBytes;   // [2][half][128]
+  static constexpr int kEnd = kOffAmax + 2 * 2 * 128 * 4;
+};
+
+// Behind the buffers: barriers for either kind of tile and the tables.
 struct Bars {
   uint64_t full[9], empty[9], tfull[8], tempty[8], sfull[3], sempty[3], abar[2], fin;
   uint32_t tmem_slot;
-  int wide, ok;
+  int tokens, ok;
 };
 template <int MODE>
 __host__ __device__ constexpr int off_bars() {
-  static_assert(Cfg<MODE, 64>::kEnd >= Cfg<MODE, 256>::kEnd, "either width's buffers fit in front of the barriers");
-  return Cfg<MODE, 64>::kEnd;
+  return Cfg<MODE>::kEnd > TokCfg<MODE>::kEnd ? Cfg<MODE>::kEnd : TokCfg<MODE>::kEnd;
 }
 template <int MODE>
 __host__ __device__ constexpr int off_tables() {
   return off_bars<MODE>() + (int)sizeof(Bars);
 }
 
-// Width of the tiles that the rows of one expert are cut into, at most nmax tokens each (a multiple of 32).
-__host__ __device__ __forceinline__ int tile_width(int rows, int nmax) {
-  const int tiles = (rows + nmax - 1) / nmax;
-  return tiles > 0 ? ((rows + tiles - 1) / tiles + 31) & ~31 : 0;
-}
-// Whether tiles of up to 256 tokens beat tiles of 64. A pair's time is its number of items times what one takes: in units of
-// a 64-token item, 1.3 + 0.0105 n for one of n tokens in MODE 0 and 1 + 0.0085 n in MODE 1, where n lies between the
-// average and the widest tile (the pairs that get the wide ones finish last). Narrow / wide in us (32 experts, 7168, 2048),
-// MODE 0: 256 rows for every expert 570 / 524, 512: 1130 / 1026, uneven 160: 426 / 514, uneven 512: 1174 / 1249; MODE 1:
-// 128 rows for every expert 158 / 178, uneven 160: 219 / 206, uneven 512: 603 / 525. Over 972 loads of nine shapes the
-// choice is 0.1 % off the faster width on average, 8 % at most. From the rows that are there, not from the buffer's size:
-// 30 rows per expert in room for 600 took 260 + 131 us in wide tiles, 184 + 100 in narrow ones. Without a division: it
+// Whether 256-token tiles (tokens on the M side) beat 64-token tiles (weight rows there). A pair's time is its number of items
+// times what one takes: 1.45 times as long in MODE 0 and 1.75 times in MODE 1 for a 256-token tile, however many tokens are in
+// either. 64 / 256 tokens in us (32 experts, 7168, 2048), MODE 0: 64 rows for every expert 168 / 251, uneven 72: 269 / 252,
+// 128: 315 / 256, uneven 512: 1284 / 584; MODE 1: 64 rows 90 / 143, uneven 72: 127 / 149, uneven 100: 157 / 146, uneven 512:
+// 619 / 328; 4 experts of 200 rows, 2048 of 1152: 34.5 / 16.9, 1152 of 2048: 19.9 / 18.0. Over 71 loads of six shapes the
+// choice is 6 % off the faster kind at most. From the rows that are there, not from the buffer's size. Without a division: it
 // stands between a CTA's start and its first load (inv_pairs = 1 / pairs; counts below 2^20).
-__host__ __device__ __forceinline__ bool wide_pays(int mode, int nt, int rows, int narrow_tiles, int wide_tiles, int widest,
-                                                   int pairs, float inv_pairs) {
-  const int narrow_waves = (int)((narrow_tiles * nt + pairs - 0.5f) * inv_pairs);
-  const int wide_waves = (int)((wide_tiles * nt + pairs - 0.5f) * inv_pairs);
-  // both sides times wide_tiles: n * wide_tiles is a mix of all rows and widest * wide_tiles
-  const float n = mode == 0 ? 0.25f * rows + 0.75f * widest * wide_tiles : 0.75f * rows + 0.25f * widest * wide_tiles;
-  const float item = mode == 0 ? 1.3f * wide_tiles + 0.0105f * n : 1.f * wide_tiles + 0.0085f * n;
-  return wide_waves * item < (float)narrow_waves * wide_tiles;
+__host__ __device__ __forceinline__ bool tokens_pay(int mode, int nt, int tiles64, int tiles256, int pairs, float inv_pairs) {
+  const int waves64 = (int)((tiles64 * nt + pairs - 0.5f) * inv_pairs);
+  const int waves256 = (int)((tiles256 * nt + pairs - 0.5f) * inv_pairs);
+  return waves256 * (mode == 0 ? 1.45f : 1.75f) < (float)waves64;
 }
 __host__ __device__ __forceinline__ int feature_tiles(int mode, int nout) {
   return mode == 0 ? nout / 128 : (nout + 255) / 256;
@@ -122,7 +133,6 @@ struct Item {
   int e, j, row0, m, n;   // expert, feature tile, first row, valid rows, rows the MMA covers (multiple of 32)
 };
 
-template <int NMAX>
 __device__ __forceinline__ Item locate(const int* tile_pref, const int* goff, int G, int NT, int w) {
   int lo = 0, hi = G;   // largest lo with tile_pref[lo] * NT <= w
   while (hi - lo > 1) {
@@ -146,15 +156,24 @@ __device__ __forceinline__ Item locate(const int* tile_pref, const int* goff, in
   return it;
 }
 
-// Everything behind the set-up, for one tile width.
-template <int MODE, int NMAX>
-__device__ __forceinline__ void pair_body(uint8_t* smem, const CUtensorMap& tmW, const CUtensorMap& tmX, const MoePairArgs& a,
+// v / (1 + exp(-v)) with the quotient rounded once more through its remainder (Markstein), which gives the rounded division
+// without its branches: 64 divisions a thread took 8 % of MODE 0 of the 256-token
+// tiles. A remainder that is not a number (v or the
+// divisor infinite) leaves the first quotient as it is.
+__device__ __forceinline__ float silu(float v) {
+  const float d = 1.f + __expf(-v);
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float q = v * r, e = fmaf(-q, d, v);
+  return fmaf(e == e ? e : -0.f, r, q);
+}
+
+// Everything behind the set-up, for 64-token tiles.
+template <int MODE>
+__device__ __forceinline__ void weight_body(uint8_t* smem, const CUtensorMap& tmW, const CUtensorMap& tmX, const MoePairArgs& a,
                                           Bars* bars, const int* tile_pref, const int* goff, int warp, int lane,
                                           uint32_t cta, uint32_t tmem_base) {
-  using C = Cfg<MODE, NMAX>;
-  // Both widths are in one kernel. What the compiler shares between them it keeps in registers all the way through the
-  // promotion; hiding that the addresses are the same took this form from 497 to 457 us (512 rows per expert, 7168 x 2048).
-  if constexpr (MODE == 1 && NMAX == 256) asm volatile("" : "+l"(smem), "+l"(bars));
+  using C = Cfg<MODE>;
   float* scale_sm = reinterpret_cast<float*>(smem + C::kOffScale);   // [stage][kb][gate/up][token]
   float* amax_in = reinterpret_cast<float*>(smem + C::kOffAmax);
   uint64_t* full = bars->full;
@@ -179,19 +198,17 @@ __device__ __forceinline__ void pair_body(uint8_t* smem, const CUtensorMap& tmW,
         uint32_t ph = 0;
         bool ok = true;
         for (int w = pair; w < num_items && ok; w += num_pairs) {
-          const Item it = locate<NMAX>(tile_pref, goff, a.G, NT, w);
+          const Item it = locate(tile_pref, goff, a.G, NT, w);
           const int nh = it.n / 2;
-          const int boxes = (nh + C::kBoxRows - 1) / C::kBoxRows;
           const int xrow = it.row0 + (int)cta * nh;
           const int wrow = it.e * a.w_rows + (MODE == 0 ? it.j * 128 + (int)cta * 64 : it.j * 256 + (int)cta * 128);
-          const uint32_t bytes = 2 * (C::kABytes + boxes * C::kBoxRows * kBKB);
           for (int kb = 0; kb < kb_total; ++kb) {
             if (!mbar_wait(&empty[s], ph ^ 1)) {
               umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_EMPTY, w, kb);
               ok = false;
               break;
             }
-            if (cta == 0) mbar_expect_tx(&full[s], bytes);
+            if (cta == 0) mbar_expect_tx(&full[s], 2 * C::kStageBytes);
             const uint32_t leader_full = map_to_cta(&full[s], 0);
             uint8_t* st = smem + s * C::kStageBytes;
             if (MODE == 0) {
@@ -200,9 +217,7 @@ __device__ __forceinline__ void pair_body(uint8_t* smem, const CUtensorMap& tmW,
             } else {
               tma_load_2d_pair(st, &tmW, leader_full, kb * kBKB, wrow);
             }
-            for (int b = 0; b < boxes; ++b)
-              tma_load_2d_pair(st + C::kABytes + b * C::kBoxRows * kBKB, &tmX, leader_full, kb * kBKB,
-                               xrow + b * C::kBoxRows);
+            tma_load_2d_pair(st + C::kABytes, &tmX, leader_full, kb * kBKB, xrow);
             if (++s == C::kStages) {
               s = 0;
               ph ^= 1;
@@ -217,7 +232,7 @@ __device__ __forceinline__ void pair_body(uint8_t* smem, const CUtensorMap& tmW,
         bool ok = true;
         const uint64_t a_desc = umma_desc_k_sw128(smem_u32(smem));
         for (int w = pair; w < num_items && ok; w += num_pairs) {
-          const Item it = locate<NMAX>(tile_pref, goff, a.G, NT, w);
+          const Item it = locate(tile_pref, goff, a.G, NT, w);
           const uint32_t idesc = umma_idesc(kFmtE4M3, kFmtE4M3, 256, it.n);
           for (int kb = 0; kb < kb_total; ++kb, ++kbc) {
             const int ts = kbc % C::kTmemStages;
@@ -236,7 +251,7 @@ __device__ __forceinline__ void pair_body(uint8_t* smem, const CUtensorMap& tmW,
             const uint64_t bdesc = adesc + (C::kABytes >> 4);
 #pragma unroll
             for (int k = 0; k < 4; ++k)   // 32 fp8 elements per MMA K step
-              umma_f8_pair(tmem_base + ts * NMAX, adesc + 2 * k, bdesc + 2 * k, idesc, k > 0 ? 1u : 0u);
+              umma_f8_pair(tmem_base + ts * kTok, adesc + 2 * k, bdesc + 2 * k, idesc, k > 0 ? 1u : 0u);
             umma_commit_both(smem_u32(&empty[s]));
             umma_commit_both(smem_u32(&tfull[ts]));
             if (++s == C::kStages) {
@@ -258,13 +273,13 @@ __device__ __forceinline__ void pair_body(uint8_t* smem, const CUtensorMap& tmW,
       uint32_t sph = 0;
       bool ok = true;
       for (int w = pair; w < num_items && ok; w += num_pairs) {
-        const Item it = locate<NMAX>(tile_pref, goff, a.G, NT, w);
+        const Item it = locate(tile_pref, goff, a.G, NT, w);
         const int wsb = a.w_rows / 128;
         const int blk = MODE == 0 ? it.j : min(2 * it.j + (int)cta, wsb - 1);
         const float* ws0 = a.ws + ((size_t)it.e * wsb + blk) * nsb;
         const float* ws1 = MODE == 0 ? ws0 + (size_t)(a.Nout / 128) * nsb : ws0;
         for (int kb0 = 0; kb0 < kb_total; kb0 += C::kScaleKb) {
-          float xv[NMAX / 64][C::kScaleKb], w0[C::kScaleKb], w1[C::kScaleKb];
+          float xv[C::kScaleKb], w0[C::kScaleKb], w1[C::kScaleKb];
 #pragma unroll
           for (int i = 0; i < C::kScaleKb; ++i) {
             const bool in = kb0 + i < kb_total;
@@ -272,12 +287,8 @@ __device__ __forceinline__ void pair_body(uint8_t* smem, const CUtensorMap& tmW,
             w1[i] = MODE == 0 && in ? __ldg(ws1 + kb0 + i) : 0.f;
           }
 #pragma unroll
-          for (int u = 0; u < NMAX / 64; ++u) {
-            const int t = t64 + 64 * u;
-#pragma unroll
-            for (int i = 0; i < C::kScaleKb; ++i)
-              xv[u][i] = t < it.m && kb0 + i < kb_total ? a.xs[(size_t)(it.row0 + t) * nsb + kb0 + i] : 0.f;
-          }
+          for (int i = 0; i < C::kScaleKb; ++i)
+            xv[i] = t64 < it.m && kb0 + i < kb_total ? a.xs[(size_t)(it.row0 + t64) * nsb + kb0 + i] : 0.f;
           if (!__all_sync(0xffffffffu, mbar_wait(&sempty[ss], sph ^ 1))) {
             umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_EMPTY, w, 10000 + kb0);
             ok = false;
@@ -285,12 +296,9 @@ __device__ __forceinline__ void pair_body(uint8_t* smem, const CUtensorMap& tmW,
           }
           float* dst = scale_sm + ss * C::kScaleFloats;
 #pragma unroll
-          for (int u = 0; u < NMAX / 64; ++u) {
-#pragma unroll
-            for (int i = 0; i < C::kScaleKb; ++i) {
-              dst[(i * C::kW) * NMAX + t64 + 64 * u] = xv[u][i] * w0[i];
-              if (MODE == 0) dst[(i * C::kW + C::kW - 1) * NMAX + t64 + 64 * u] = xv[u][i] * w1[i];
-            }
+          for (int i = 0; i < C::kScaleKb; ++i) {
+            dst[(i * C::kW) * kTok + t64] = xv[i] * w0[i];
+            if (MODE == 0) dst[(i * C::kW + C::kW - 1) * kTok + t64] = xv[i] * w1[i];
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(&sfull[ss]);
@@ -306,7 +314,6 @@ __device__ __forceinline__ void pair_body(uint8_t* smem, const CUtensorMap& tmW,
     // ---- promotion + epilogue: warp quarter q owns weight rows [32 q, 32 q + 32), `half` the lower / upper tokens ----
     const int q = warp & 3, half = (warp - 4) >> 2;
     const int tid = q * 32 + lane;   // == TMEM lane
-    constexpr int kBlocks = NMAX / 64;   // 32-token blocks per half
     const int which = MODE == 0 ? q >> 1 : 0;   // 0: gate rows, 1: up rows
     uint8_t* trans = smem + C::kOffTrans + half * C::kTransBytes;
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
@@ -315,22 +322,22 @@ __device__ __forceinline__ void pair_body(uint8_t* smem, const CUtensorMap& tmW,
     uint32_t sph = 0, kbc = 0;
     bool ok = true;
     for (int w = pair; w < num_items && ok; w += num_pairs, ++n_it) {
-      const Item it = locate<NMAX>(tile_pref, goff, a.G, NT, w);
+      const Item it = locate(tile_pref, goff, a.G, NT, w);
       const int nh = it.n / 2, col0 = half * nh;
       const int par = n_it & 1;
       if (MODE == 0 && warp == 4 && lane == 0) mbar_expect_tx(&abar[par], it.n * 4);
-      float acc[kBlocks * 32];
+      uint64_t acc[16];   // pairs of tokens
 #pragma unroll
-      for (int c = 0; c < kBlocks * 32; ++c) acc[c] = 0.f;
+      for (int c = 0; c < 16; ++c) acc[c] = 0;
       for (int kb0 = 0; kb0 < kb_total && ok; kb0 += C::kScaleKb) {
         if (!__all_sync(0xffffffffu, mbar_wait(&sfull[ss], sph))) {
           umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, 10000 + kb0);
           ok = false;
           break;
         }
-        const float* sc = scale_sm + ss * C::kScaleFloats + which * NMAX + col0;
+        const float* sc = scale_sm + ss * C::kScaleFloats + which * kTok + col0;
         const int kb1 = min(kb_total, kb0 + C::kScaleKb);
-        for (int kb = kb0; kb < kb1; ++kb, ++kbc, sc += C::kW * NMAX) {
+        for (int kb = kb0; kb < kb1; ++kb, ++kbc, sc += C::kW * kTok) {
           const int ts = kbc % C::kTmemStages;
           if (!__all_sync(0xffffffffu, mbar_wait(&tfull[ts], (kbc / C::kTmemStages) & 1))) {
             umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, w, kb);
@@ -338,30 +345,18 @@ __device__ __forceinline__ void pair_body(uint8_t* smem, const CUtensorMap& tmW,
             break;
           }
           tc_fence_after();
-          const uint32_t taddr = lane_addr + ts * NMAX + col0;
-          uint32_t r[2][32];
-          tmem_ld_x32(taddr, r[0]);
+          uint32_t r[32];
+          tmem_ld_x32(lane_addr + ts * kTok + col0, r);
+          tmem_ld_wait();
+          // everything of this stage is in registers: the next K block may overwrite it
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster_relaxed(map_to_cta(&tempty[ts], 0));
 #pragma unroll
-          for (int b = 0; b < kBlocks; ++b) {
-            if (b * 32 >= nh) break;
-            tmem_ld_wait();
-            if ((b + 1) * 32 < nh) {
-              if (b + 1 < kBlocks) tmem_ld_x32(taddr + (b + 1) * 32, r[(b + 1) & 1]);
-            } else {   // everything of this stage is in registers: the next K block may overwrite it
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive_cluster_relaxed(map_to_cta(&tempty[ts], 0));
-            }
-#pragma unroll
-            for (int c4 = 0; c4 < 8; ++c4) {
-              const float4 s4 = reinterpret_cast<const float4*>(sc + b * 32)[c4];
-              const int c = b * 32 + c4 * 4;
-              const uint32_t* rr = r[b & 1] + c4 * 4;
-              acc[c] = fmaf(__uint_as_float(rr[0]), s4.x, acc[c]);
-              acc[c + 1] = fmaf(__uint_as_float(rr[1]), s4.y, acc[c + 1]);
-              acc[c + 2] = fmaf(__uint_as_float(rr[2]), s4.z, acc[c + 2]);
-              acc[c + 3] = fmaf(__uint_as_float(rr[3]), s4.w, acc[c + 3]);
-            }
+          for (int c4 = 0; c4 < 8; ++c4) {
+            const ulonglong2 s4 = reinterpret_cast<const ulonglong2*>(sc)[c4];
+            acc[2 * c4] = fma_f32x2(pack_f32x2(r[4 * c4], r[4 * c4 + 1]), s4.x, acc[2 * c4]);
+            acc[2 * c4 + 1] = fma_f32x2(pack_f32x2(r[4 * c4 + 2], r[4 * c4 + 3]), s4.y, acc[2 * c4 + 1]);
           }
         }
         __syncwarp();
@@ -373,99 +368,404 @@ __device__ __forceinline__ void pair_body(uint8_t* smem, const CUtensorMap& tmW,
       }
       ok = bar_half_and(half, ok);
       if (!ok) break;
+      float v[32];
+#pragma unroll
+      for (int c = 0; c < 16; ++c) unpack_f32x2(acc[c], &v[2 * c], &v[2 * c + 1]);
       if (MODE == 1) {
         const int feat0 = it.j * 256 + (int)cta * 128;
         __nv_bfloat16* tb = reinterpret_cast<__nv_bfloat16*>(trans);
 #pragma unroll
-        for (int b = 0; b < kBlocks; ++b) {
-          if (b * 32 >= nh) break;
+        for (int t = 0; t < 32; ++t) tb[t * 136 + tid] = __float2bfloat16(v[t]);
+        bar_half(half);
 #pragma unroll
-          for (int t = 0; t < 32; ++t) tb[t * 136 + tid] = __float2bfloat16(acc[b * 32 + t]);
-          bar_half(half);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int v = u * 128 + tid, t = v >> 4, tok = col0 + b * 32 + t;
-            if (b * 32 + t < nh && tok < it.m && feat0 < a.Nout) {
-              const int4 o = *reinterpret_cast<const int4*>(trans + t * 272 + (v & 15) * 16);
-              *reinterpret_cast<int4*>(a.y + (size_t)(it.row0 + tok) * a.Nout + feat0 + (v & 15) * 8) = o;
-            }
+        for (int u = 0; u < 4; ++u) {
+          const int i = u * 128 + tid, t = i >> 4, tok = col0 + t;
+          if (t < nh && tok < it.m && feat0 < a.Nout) {
+            const int4 o = *reinterpret_cast<const int4*>(trans + t * 272 + (i & 15) * 16);
+            *reinterpret_cast<int4*>(a.y + (size_t)(it.row0 + tok) * a.Nout + feat0 + (i & 15) * 8) = o;
           }
-          bar_half(half);
         }
+        bar_half(half);
       } else {
         float* tf = reinterpret_cast<float*>(trans);   // [32 tokens][65]: up values, then h
         const int f = (q & 1) * 32 + lane;             // feature inside this CTA's 64
         const int t4 = tid >> 2, qq = tid & 3;         // afterwards: token and 16-feature quarter of a thread
-        float h[kBlocks][16], pm[kBlocks];
-        const uint32_t peer_amax = map_to_cta(amax_in + par * NMAX, peer);
+        const int tok = col0 + t4;
+        const uint32_t peer_amax = map_to_cta(amax_in + par * kTok, peer);
         const uint32_t peer_bar = map_to_cta(&abar[par], peer);
+        if (which == 1) {
 #pragma unroll
-        for (int b = 0; b < kBlocks; ++b) {
-          if (b * 32 >= nh) break;
-          if (which == 1) {
-#pragma unroll
-            for (int t = 0; t < 32; ++t) tf[t * 65 + f] = acc[b * 32 + t];
-          }
-          bar_half(half);
-          if (which == 0) {
-            // Rows behind the tile's own are zeros, which take the slow path of the division (an item of 13 rows lasted 3
-            // us longer than one of 64): any other number does for them.
-            const int own = it.m - col0 - b * 32;
-#pragma unroll
-            for (int t = 0; t < 32; ++t) {
-              const float v = t < own ? acc[b * 32 + t] : 1.f;
-              tf[t * 65 + f] = (v / (1.f + __expf(-v))) * tf[t * 65 + f];
-            }
-          }
-          bar_half(half);
-          float mx = 0.f;
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            h[b][i] = tf[t4 * 65 + qq * 16 + i];
-            mx = fmaxf(mx, fabsf(h[b][i]));
-          }
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-          pm[b] = mx;
-          if (qq == 0 && b * 32 + t4 < nh) st_async_b32(peer_amax + (col0 + b * 32 + t4) * 4, __float_as_uint(mx), peer_bar);
-          if ((b + 1) * 32 < nh) bar_half(half);
+          for (int t = 0; t < 32; ++t) tf[t * 65 + f] = v[t];
         }
+        bar_half(half);
+        if (which == 0) {
+#pragma unroll
+          for (int t = 0; t < 32; ++t) tf[t * 65 + f] = silu(v[t]) * tf[t * 65 + f];
+        }
+        bar_half(half);
+        float h[16], mx = 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          h[i] = tf[t4 * 65 + qq * 16 + i];
+          mx = fmaxf(mx, fabsf(h[i]));
+        }
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        if (qq == 0 && t4 < nh) st_async_b32(peer_amax + tok * 4, __float_as_uint(mx), peer_bar);
         ok = mbar_wait_cluster(&abar[par], (n_it >> 1) & 1);
         if (!ok) umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_GROUP_READY, w, 20000);
         ok = bar_half_and(half, ok);   // also: every read of the transposition buffer is done
         if (!ok) break;
-#pragma unroll
-        for (int b = 0; b < kBlocks; ++b) {
-          const int tok = col0 + b * 32 + t4;
-          if (b * 32 + t4 < nh && tok < it.m) {
-            const float amax = fmaxf(fmaxf(pm[b], amax_in[par * NMAX + tok]), 1e-4f);
-            const float inv = 448.f / amax;
-            int4 o;
-            o.x = pack_fp8x4(h[b][0] * inv, h[b][1] * inv, h[b][2] * inv, h[b][3] * inv);
-            o.y = pack_fp8x4(h[b][4] * inv, h[b][5] * inv, h[b][6] * inv, h[b][7] * inv);
-            o.z = pack_fp8x4(h[b][8] * inv, h[b][9] * inv, h[b][10] * inv, h[b][11] * inv);
-            o.w = pack_fp8x4(h[b][12] * inv, h[b][13] * inv, h[b][14] * inv, h[b][15] * inv);
-            const size_t row = it.row0 + tok;
-            *reinterpret_cast<int4*>(a.hq + row * a.Nout + it.j * 128 + cta * 64 + qq * 16) = o;
-            if (cta == 0 && qq == 0) a.hs[row * (a.Nout / 128) + it.j] = amax * (1.f / 448.f);
-          }
+        if (t4 < nh && tok < it.m) {
+          const float amax = fmaxf(fmaxf(mx, amax_in[par * kTok + tok]), 1e-4f);
+          const float inv = 448.f / amax;
+          int4 o;
+          o.x = pack_fp8x4(h[0] * inv, h[1] * inv, h[2] * inv, h[3] * inv);
+          o.y = pack_fp8x4(h[4] * inv, h[5] * inv, h[6] * inv, h[7] * inv);
+          o.z = pack_fp8x4(h[8] * inv, h[9] * inv, h[10] * inv, h[11] * inv);
+          o.w = pack_fp8x4(h[12] * inv, h[13] * inv, h[14] * inv, h[15] * inv);
+          const size_t row = it.row0 + tok;
+          *reinterpret_cast<int4*>(a.hq + row * a.Nout + it.j * 128 + cta * 64 + qq * 16) = o;
+          if (cta == 0 && qq == 0) a.hs[row * (a.Nout / 128) + it.j] = amax * (1.f / 448.f);
         }
       }
     }
   }
 }
 
-// kBoth: both tile widths, picked by wide_pays; else tiles of 64 tokens.
+__device__ __forceinline__ Item locate_tokens(const int* tile_pref, const int* goff, int G, int NT, int w) {
+  int lo = 0, hi = G;   // largest lo with tile_pref[lo] * NT <= w
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (tile_pref[mid] * NT <= w) lo = mid;
+    else hi = mid;
+  }
+  const int ntt = tile_pref[lo + 1] - tile_pref[lo];
+  const int local = w - tile_pref[lo] * NT;
+  Item it;
+  it.e = lo;
+  it.j = local / ntt;   // token tiles fastest
+  const int first = (local - it.j * ntt) * 256;
+  it.row0 = goff[lo] + first;
+  it.m = min(256, goff[lo + 1] - it.row0);
+  it.n = 256;
+  return it;
+}
+
+// Barrier of the two warps that share a quarter's tokens, joining a decision.
+__device__ __forceinline__ bool bar_quarter_and(int q, bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.u32 q, %2, 0;\n"
+      "barrier.cta.red.and.pred p, %1, 64, q;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(r)
+      : "r"(1 + q), "r"(ok ? 1u : 0u)
+      : "memory");
+  return r != 0;
+}
+
+template <int MODE>
+__device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW, const CUtensorMap& tmX, const MoePairArgs& a,
+                                           Bars* bars, const int* tile_pref, const int* goff, int warp, int lane,
+                                           uint32_t cta, uint32_t tmem_base) {
+  using C = TokCfg<MODE>;
+  // Both kinds of tile are in one kernel. What the compiler shares between them it keeps in registers all the way through the
+  // promotion: hide that the addresses are the same.
+  asm volatile("" : "+l"(smem), "+l"(bars));
+  static_assert(C::kStages <= 9 && C::kTmemStages <= 8 && C::kScaleStages <= 3, "barriers");
+  const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  const int NT = feature_tiles(MODE, a.Nout);
+  const int kb_total = a.K / kBKB;
+  const int num_items = bars->ok ? tile_pref[a.G] * NT : 0;
+
+  if (warp < 4) {
+    regs_dec<MODE == 0 ? 56 : 80>();
+    if (warp == 0) {
+      if (elect_one()) {
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int w = pair; w < num_items && ok; w += num_pairs) {
+          const Item it = locate_tokens(tile_pref, goff, a.G, NT, w);
+          const int xrow = it.row0 + (int)cta * 128;
+          // columns of an accumulator: 64 weight rows of the leader, 64 of its partner
+          const int wrow = it.e * a.w_rows + (MODE == 0 ? it.j * 128 + (int)cta * a.Nout : it.j * 256 + (int)cta * 64);
+          const int wstep = MODE == 0 ? 64 : 128;
+          for (int kb = 0; kb < kb_total; ++kb) {
+            if (!mbar_wait(&bars->empty[s], ph ^ 1)) {
+              umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_EMPTY, w, kb);
+              ok = false;
+              break;
+            }
+            if (cta == 0) mbar_expect_tx(&bars->full[s], 2 * C::kStageBytes);
+            const uint32_t leader_full = map_to_cta(&bars->full[s], 0);
+            uint8_t* st = smem + s * C::kStageBytes;
+            tma_load_2d_pair(st, &tmX, leader_full, kb * kBKB, xrow);
+            tma_load_2d_pair(st + C::kABytes, &tmW, leader_full, kb * kBKB, wrow);
+            tma_load_2d_pair(st + C::kABytes + C::kBBytes, &tmW, leader_full, kb * kBKB, wrow + wstep);
+            if (++s == C::kStages) {
+              s = 0;
+              ph ^= 1;
+            }
+          }
+        }
+      }
+    } else if (warp == 1) {
+      if (cta == 0 && elect_one()) {
+        constexpr uint32_t idesc = umma_idesc(kFmtE4M3, kFmtE4M3, 256, 128);
+        int s = 0;
+        uint32_t ph = 0, n = 0;   // n: accumulators so far
+        bool ok = true;
+        const uint64_t a_desc = umma_desc_k_sw128(smem_u32(smem));
+        for (int w = pair; w < num_items && ok; w += num_pairs) {
+          for (int kb = 0; kb < kb_total && ok; ++kb) {
+            if (!mbar_wait(&bars->full[s], ph)) {
+              umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, kb);
+              ok = false;
+              break;
+            }
+            const uint64_t adesc = a_desc + s * (C::kStageBytes >> 4);
+#pragma unroll
+            for (int u = 0; u < 2; ++u, ++n) {
+              const int ts = n % C::kTmemStages;
+              if (!mbar_wait(&bars->tempty[ts], ((n / C::kTmemStages) & 1) ^ 1)) {
+                umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_EMPTY, w, kb);
+                ok = false;
+                break;
+              }
+              tc_fence_after();
+              const uint64_t bdesc = adesc + ((C::kABytes + u * C::kBBytes) >> 4);
+#pragma unroll
+              for (int k = 0; k < 4; ++k)   // 32 fp8 elements per MMA K step
+                umma_f8_pair(tmem_base + ts * 128, adesc + 2 * k, bdesc + 2 * k, idesc, k > 0 ? 1u : 0u);
+              if (u == 1) umma_commit_both(smem_u32(&bars->empty[s]));
+              umma_commit_both(smem_u32(&bars->tfull[ts]));
+            }
+            if (++s == C::kStages) {
+              s = 0;
+              ph ^= 1;
+            }
+          }
+        }
+        umma_commit_pair(map_to_cta(&bars->fin, 0));   // as in weight_body
+        if (!mbar_wait(&bars->fin, 0)) umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, -1, 0);
+      }
+    } else {
+      // ---- scale products of the coming K blocks for this CTA's 128 tokens ----
+      float* scale_sm = reinterpret_cast<float*>(smem + C::kOffScale);
+      const int t64 = threadIdx.x - 64;
+      const int nsb = a.K / 128, wsb = a.w_rows / 128;
+      int ss = 0;
+      uint32_t sph = 0;
+      bool ok = true;
+      for (int w = pair; w < num_items && ok; w += num_pairs) {
+        const Item it = locate_tokens(tile_pref, goff, a.G, NT, w);
+        const float* ws0 = a.ws + ((size_t)it.e * wsb + (MODE == 0 ? it.j : 2 * it.j)) * nsb;
+        const float* ws1 = MODE == 0 ? ws0 + (size_t)(a.Nout / 128) * nsb : 2 * it.j + 1 < wsb ? ws0 + nsb : ws0;
+        for (int kb0 = 0; kb0 < kb_total; kb0 += C::kScaleKb) {
+          float w0[C::kScaleKb], w1[C::kScaleKb], xv[C::kScaleKb];
+          const float* xs = a.xs + (size_t)(it.row0 + (int)cta * 128 + t64) * nsb + kb0;
+          const int rows = it.m - (int)cta * 128 - t64;   // token t64 + 64 u is this expert's where 64 u < rows
+#pragma unroll
+          for (int i = 0; i < C::kScaleKb; ++i) {
+            const bool in = kb0 + i < kb_total;
+            w0[i] = in ? __ldg(ws0 + kb0 + i) : 0.f;
+            w1[i] = in ? __ldg(ws1 + kb0 + i) : 0.f;
+            xv[i] = in && rows > 0 ? xs[i] : 0.f;
+          }
+          if (!__all_sync(0xffffffffu, mbar_wait(&bars->sempty[ss], sph ^ 1))) {
+            umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_EMPTY, w, 10000 + kb0);
+            ok = false;
+            break;
+          }
+          float* dst = scale_sm + ss * C::kScaleFloats + t64;
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+#pragma unroll
+            for (int i = 0; i < C::kScaleKb; ++i) {
+              dst[(i * 2) * 128 + 64 * u] = xv[i] * w0[i];
+              dst[(i * 2 + 1) * 128 + 64 * u] = xv[i] * w1[i];
+              if (u == 0) xv[i] = kb0 + i < kb_total && rows > 64 ? xs[(size_t)64 * nsb + i] : 0.f;
+            }
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->sfull[ss]);
+          if (++ss == C::kScaleStages) {
+            ss = 0;
+            sph ^= 1;
+          }
+        }
+      }
+    }
+  } else {
+    regs_inc<MODE == 0 ? 224 : 208>();
+    // ---- promotion + epilogue: warp quarter q owns tokens [32 q, 32 q + 32), `u` the accumulator of every K block ----
+    const int q = warp & 3, u = (warp - 4) >> 2;
+    const int tid = q * 32 + lane;   // == TMEM lane == token of this CTA
+    float* amax_sm = reinterpret_cast<float*>(smem + C::kOffAmax);
+    uint8_t* trans = smem + C::kOffTrans + (warp - 4) * C::kTransBytes;
+    // 32-bit addresses only: the accumulators and the loads in flight take 160 to 192 registers, and one value kept in local memory
+    // costs a cache access in every K block
+    const uint32_t bars_sm = smem_u32(bars);
+    const uint32_t tfull = bars_sm + offsetof(Bars, tfull) + u * 8;
+    const uint32_t tempty = map_to_cta(&bars->tempty[u], 0);
+    const uint32_t cols = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + u * 128;
+    const uint32_t scales = smem_u32(smem + C::kOffScale) + tid * 4;
+    int ss = 0, n_it = 0;
+    uint32_t sph = 0, n = 0;   // n: K blocks so far; block n is in accumulator u + 2 (n & 1)
+    bool ok = true;
+    // Columns per load. Measured in us, 16384 rows (7168 x 2048, 32 experts), 32 / 16 columns: MODE 0 573 / 594, MODE 1 414 / 334
+    // (its longer epilogue and 64 columns in flight do not fit into the registers together).
+    constexpr int kCols = MODE == 0 ? 32 : 16, kLoads = 128 / kCols;
+    uint32_t r[2][kCols];
+    auto load = [&](uint32_t addr, uint32_t* dst) {
+      if constexpr (kCols == 32) tmem_ld_x32(addr, dst);
+      else tmem_ld_x16(addr, dst);
+    };
+    // waits for the accumulator of K block i and starts the load of its first columns
+    auto take = [&](uint32_t i, int w) {
+      ok = mbar_wait(tfull + (i & 1) * 16, (i >> 1) & 1);
+      if (!ok) umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, w, (int)i);
+      tc_fence_after();
+      load(cols + (i & 1) * 256, r[0]);
+    };
+    for (int w = pair; w < num_items && ok; w += num_pairs, ++n_it) {
+      uint64_t acc[64];   // pairs of columns; MODE 0: 64 gate features, then the same 64 up
+#pragma unroll
+      for (int c = 0; c < 64; ++c) acc[c] = 0;
+      take(n, w);
+      for (int left = kb_total; left > 0 && ok;) {
+        if (!__all_sync(0xffffffffu, mbar_wait(bars_sm + (uint32_t)offsetof(Bars, sfull) + ss * 8, sph))) {
+          umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, 10000 + left);
+          ok = false;
+          break;
+        }
+        uint32_t sc = scales + ss * C::kScaleFloats * 4;
+        const uint32_t end = sc + min(left, C::kScaleKb) * 1024;
+        left -= C::kScaleKb;
+#pragma unroll 1
+        for (; sc < end && ok; ++n, sc += 1024) {
+          const uint32_t f0 = ld_shared_u32(sc + (MODE == 0 ? 0 : u * 512));
+          const uint32_t f1 = MODE == 0 ? ld_shared_u32(sc + 512) : f0;
+#pragma unroll
+          for (int b = 0; b < kLoads; ++b) {   // the load of the next columns runs behind the FMAs of these
+            tmem_ld_wait();
+            if (b + 1 < kLoads) {
+              load(cols + (n & 1) * 256 + (b + 1) * kCols, r[(b + 1) & 1]);
+            } else {   // all of it is in registers: the MMAs may overwrite it
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_cluster_relaxed<2>(tempty + (n & 1) * 16);
+              if (left > 0 || sc + 1024 < end) take(n + 1, w);
+            }
+            const uint64_t f = b < kLoads / 2 ? pack_f32x2(f0, f0) : pack_f32x2(f1, f1);
+#pragma unroll
+            for (int c = 0; c < kCols / 2; ++c) {
+              uint64_t& d = acc[b * (kCols / 2) + c];
+              d = fma_f32x2(pack_f32x2(r[b & 1][2 * c], r[b & 1][2 * c + 1]), f, d);
+            }
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->sempty[ss]);
+        if (++ss == C::kScaleStages) {
+          ss = 0;
+          sph ^= 1;
+        }
+      }
+      const Item it = locate_tokens(tile_pref, goff, a.G, NT, w);
+      const int rows = min(32, it.m - ((int)cta * 128 + q * 32));   // valid tokens of this warp (may be negative)
+      const size_t row0 = (size_t)it.row0 + (int)cta * 128 + q * 32;
+      if (MODE == 1) {
+        if (!ok) break;
+        const int feat0 = it.j * 256 + u * 128;
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {   // 64 features at a time
+          __syncwarp();
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            int4 o;
+            __nv_bfloat162* po = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              float x, y;
+              unpack_f32x2(acc[p * 32 + c * 4 + i], &x, &y);
+              po[i] = __floats2bfloat162_rn(x, y);
+            }
+            *reinterpret_cast<int4*>(trans + lane * 128 + ((c ^ (lane & 7)) << 4)) = o;
+          }
+          __syncwarp();
+          if (feat0 < a.Nout) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int t = i * 4 + (lane >> 3), seg = lane & 7;
+              const int4 o = *reinterpret_cast<const int4*>(trans + t * 128 + ((seg ^ (t & 7)) << 4));
+              if (t < rows) *reinterpret_cast<int4*>(a.y + (row0 + t) * a.Nout + feat0 + p * 64 + seg * 8) = o;
+            }
+          }
+        }
+      } else {
+        float mx = 0.f;
+        const bool own = lane < rows;
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+          float g[2], up[2];
+          unpack_f32x2(acc[c], &g[0], &g[1]);
+          unpack_f32x2(acc[32 + c], &up[0], &up[1]);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            g[i] = silu(g[i]) * up[i];
+            mx = fmaxf(mx, fabsf(g[i]));
+          }
+          acc[c] = pack_f32x2(__float_as_uint(g[0]), __float_as_uint(g[1]));
+        }
+        float* am = amax_sm + (n_it & 1) * 256;
+        am[u * 128 + tid] = mx;
+        ok = bar_quarter_and(q, ok);
+        if (!ok) break;
+        const float amax = fmaxf(fmaxf(mx, am[(u ^ 1) * 128 + tid]), 1e-4f);
+        const float inv = 448.f / amax;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t o[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            float x[4];
+            unpack_f32x2(acc[c * 8 + i * 2], &x[0], &x[1]);
+            unpack_f32x2(acc[c * 8 + i * 2 + 1], &x[2], &x[3]);
+            o[i] = pack_fp8x4(x[0] * inv, x[1] * inv, x[2] * inv, x[3] * inv);
+          }
+          *reinterpret_cast<int4*>(trans + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) = make_int4(o[0], o[1], o[2], o[3]);
+        }
+        if (u == 0 && own) a.hs[(row0 + lane) * (a.Nout / 128) + it.j] = amax * (1.f / 448.f);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int t = i * 8 + (lane >> 2), seg = lane & 3;
+          const int4 o = *reinterpret_cast<const int4*>(trans + t * 64 + ((seg ^ ((t >> 1) & 3)) << 4));
+          if (t < rows) *reinterpret_cast<int4*>(a.hq + (row0 + t) * a.Nout + it.j * 128 + u * 64 + seg * 16) = o;
+        }
+        __syncwarp();
+      }
+    }
+  }
+}
+
+// kBoth: both kinds of tile, picked by tokens_pay; else tiles of 64 tokens.
 template <int MODE, bool kBoth>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX32,
-                     const __grid_constant__ CUtensorMap tmX64, const MoePairArgs a) {
+                     const __grid_constant__ CUtensorMap tmW64, const __grid_constant__ CUtensorMap tmX128, const MoePairArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   Bars* bars = reinterpret_cast<Bars*>(smem + off_bars<MODE>());
   int* goff = reinterpret_cast<int*>(smem + off_tables<MODE>());   // [G + 1]
-  int* pref_narrow = goff + a.G + 1;                               // [G + 1] token tiles of 64 before each expert
-  int* pref_wide = pref_narrow + a.G + 1;                          // the same of 256
+  int* pref64 = goff + a.G + 1;                                    // [G + 1] tiles of 64 tokens before each expert
+  int* pref256 = pref64 + a.G + 1;                                 // the same of 256
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();   // 0 = leader
@@ -488,7 +788,10 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
     mbar_fence_init();
     tma_prefetch_desc(&tmW);
     tma_prefetch_desc(&tmX32);
-    if (kBoth) tma_prefetch_desc(&tmX64);
+    if (kBoth) {
+      tma_prefetch_desc(&tmW64);
+      tma_prefetch_desc(&tmX128);
+    }
   }
   if (warp == 2) {
     tmem_alloc_pair(&bars->tmem_slot, 512);
@@ -497,7 +800,7 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
   for (int i = threadIdx.x; i <= a.G; i += kThreads) goff[i] = a.group_off[i];
   __syncthreads();
   if (warp == 0) {
-    int narrow = 0, wide = 0, widest = 0, bad = 0;   // exclusive scans of the token tiles per expert, for either width
+    int sum64 = 0, sum256 = 0, bad = 0;   // exclusive scans of the token tiles per expert, for either kind
     for (int e0 = 0; e0 < a.G; e0 += 32) {
       const int e = e0 + lane;
       int m = e < a.G ? goff[e + 1] - goff[e] : 0;
@@ -507,7 +810,6 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         m = 0;
       }
       const int n = (m + 63) / 64, w = (m + 255) / 256;
-      if (kBoth) widest = max(widest, tile_width(m, 256));
       int x = n, y = w;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
@@ -518,21 +820,19 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         }
       }
       if (e < a.G) {
-        pref_narrow[e] = narrow + x - n;
-        if (kBoth) pref_wide[e] = wide + y - w;
+        pref64[e] = sum64 + x - n;
+        if (kBoth) pref256[e] = sum256 + y - w;
       }
-      narrow += __shfl_sync(0xffffffffu, x, 31);
-      if (kBoth) wide += __shfl_sync(0xffffffffu, y, 31);
+      sum64 += __shfl_sync(0xffffffffu, x, 31);
+      if (kBoth) sum256 += __shfl_sync(0xffffffffu, y, 31);
     }
     bad = __any_sync(0xffffffffu, bad);
-    if (kBoth) widest = __reduce_max_sync(0xffffffffu, widest);
     if (lane == 0) {
-      pref_narrow[a.G] = narrow;
+      pref64[a.G] = sum64;
       bars->ok = !bad;
       if (kBoth) {
-        pref_wide[a.G] = wide;
-        bars->wide = wide_pays(MODE, feature_tiles(MODE, a.Nout), goff[a.G] - goff[0], narrow, wide, widest, gridDim.x >> 1,
-                               a.inv_pairs);
+        pref256[a.G] = sum256;
+        bars->tokens = tokens_pay(MODE, feature_tiles(MODE, a.Nout), sum64, sum256, gridDim.x >> 1, a.inv_pairs);
       }
     }
   }
@@ -541,12 +841,12 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
   cluster_sync_all();   // the peer's barriers exist before anything is signalled on them
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_slot;
-  bool wide = false;
+  bool tokens = false;
   if constexpr (kBoth) {
-    wide = bars->wide;
-    if (wide) pair_body<MODE, 256>(smem, tmW, tmX64, a, bars, pref_wide, goff, warp, lane, cta, tmem_base);
+    tokens = bars->tokens;
+    if (tokens) token_body<MODE>(smem, tmW64, tmX128, a, bars, pref256, goff, warp, lane, cta, tmem_base);
   }
-  if (!wide) pair_body<MODE, 64>(smem, tmW, tmX32, a, bars, pref_narrow, goff, warp, lane, cta, tmem_base);
+  if (!tokens) weight_body<MODE>(smem, tmW, tmX32, a, bars, pref64, goff, warp, lane, cta, tmem_base);
 
   // nobody leaves (or frees TMEM) while the peer may still signal this CTA's barriers or read its operands
   tc_fence_before();
@@ -560,16 +860,19 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
 
 template <int MODE, bool kBoth>
 int launch(const void* W, const void* X, const MoePairArgs& a, int grid, cudaStream_t stream) {
-  CUtensorMap tmW, tmX32, tmX64;
-  if (make_tmap_2d(&tmW, TMAP_U8, W, a.K, (uint64_t)a.G * a.w_rows, a.K, kBKB, MODE == 0 ? 64 : 128, TMAP_SW_128B))
+  CUtensorMap tmW, tmX32, tmW64, tmX128;
+  if (make_tmap_2d(&tmW, TMAP_U8, W, a.K, (uint64_t)a.G * a.w_rows, a.K, kBKB, MODE == 0 ? 64 : 128, TMAP_SW_128B) ||
+      make_tmap_2d(&tmX32, TMAP_U8, X, a.K, a.n_rows_cap, a.K, kBKB, Cfg<MODE>::kBoxRows, TMAP_SW_128B))
     return -UMDK_ERR_BAD_ARG;
-  if (make_tmap_2d(&tmX32, TMAP_U8, X, a.K, a.n_rows_cap, a.K, kBKB, Cfg<MODE, 64>::kBoxRows, TMAP_SW_128B) ||
-      make_tmap_2d(&tmX64, TMAP_U8, X, a.K, a.n_rows_cap, a.K, kBKB, Cfg<MODE, 256>::kBoxRows, TMAP_SW_128B))
+  tmW64 = tmW;
+  tmX128 = tmX32;
+  if (kBoth && (make_tmap_2d(&tmW64, TMAP_U8, W, a.K, (uint64_t)a.G * a.w_rows, a.K, kBKB, 64, TMAP_SW_128B) ||
+                make_tmap_2d(&tmX128, TMAP_U8, X, a.K, a.n_rows_cap, a.K, kBKB, 128, TMAP_SW_128B)))
     return -UMDK_ERR_BAD_ARG;
   const size_t smem = 1024 + off_tables<MODE>() + (kBoth ? 3 : 2) * (size_t)(a.G + 1) * 4;
   UMDK_CUDA_CHECK(cudaFuncSetAttribute(moe_gemm_pair_kernel<MODE, kBoth>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem));
-  moe_gemm_pair_kernel<MODE, kBoth><<<grid, kThreads, smem, stream>>>(tmW, tmX32, tmX64, a);
+  moe_gemm_pair_kernel<MODE, kBoth><<<grid, kThreads, smem, stream>>>(tmW, tmX32, tmW64, tmX128, a);
   UMDK_CUDA_CHECK(cudaGetLastError());
   return 0;
 }
@@ -581,29 +884,46 @@ bool moe_gemm_pair_fits(int G, int grid) { return grid >= 2 && G <= 1024; }
 int moe_gemm_pair_launch(int mode, const void* W, const void* X, const MoePairArgs& args, int grid, cudaStream_t stream) {
   MoePairArgs a = args;
   a.inv_pairs = 1.f / (grid / 2);
-  // Choosing takes 0.3 - 0.5 us: left out where wide tiles pay for no number of rows that the buffer holds for every expert (up
-  // to 128 of them they never do; few items fill one wave of narrow tiles).
-  const int nt = feature_tiles(mode, a.Nout), most = a.n_rows_cap / a.G;
-  bool both = most > 1024;
-  for (int m = 129; m <= most && !both; m += 32)
-    both = wide_pays(mode, nt, m * a.G, (m + 63) / 64 * a.G, (m + 255) / 256 * a.G, tile_width(m, 256), grid / 2, a.inv_pairs);
+  // Choosing takes 0.3 - 0.5 us: left out where hardly an expert has more than one tile of 64 tokens.
+  const bool both = a.n_rows_cap > 32 * a.G;
   if (both) return mode == 0 ? launch<0, true>(W, X, a, grid, stream) : launch<1, true>(W, X, a, grid, stream);
   return mode == 0 ? launch<0, false>(W, X, a, grid, stream) : launch<1, false>(W, X, a, grid, stream);
 }
 
 }  // namespace umdk
 
-// Token width of the tiles that the kernel takes for these rows per expert (host memory, [G + 1]) where it has the choice:
-// 64 or 256.
+// Whether a launch that has the choice takes 256-token tiles with the tokens on the MMA's M side (1) for these rows per expert
+// (host memory, [G + 1]), or 64-token tiles (0).
+UMDK_API int umdk_moe_gemm_tokens_on_m(int mode, int G, int Nout, const int* group_off, int num_ctas) {
+  if (mode < 0 || mode > 1 || G < 1 || Nout < 128 || num_ctas < 2) return -UMDK_ERR_BAD_ARG;
+  int tiles64 = 0, tiles256 = 0;
+  for (int e = 0; e < G; ++e) {
+    const int m = group_off[e + 1] - group_off[e];
+    tiles64 += (m + 63) / 64;
+    tiles256 += (m + 255) / 256;
+  }
+  const int pairs = num_ctas / 2;
+  return umdk::tokens_pay(mode, umdk::feature_tiles(mode, Nout), tiles64, tiles256, pairs, 1.f / pairs) ? 1 : 0;
+}
+
+// The better width, 64 or 256 tokens, of tiles with the weight rows on the M side for these rows per expert (host memory,
+// [G + 1]): a pair's time is its number of items times what one takes, in units of a 64-token item 1.3 + 0.0105 n for one of n
+// tokens in MODE 0 and 1 + 0.0085 n in MODE 1, where n lies between the average and the widest tile. Only the 64 are launched:
+// where 256 win, and in many places where they don't, tiles with the tokens on the M side are faster still.
 UMDK_API int umdk_moe_gemm_tile_tokens(int mode, int G, int Nout, const int* group_off, int num_ctas) {
   if (mode < 0 || mode > 1 || G < 1 || Nout < 128 || num_ctas < 2) return -UMDK_ERR_BAD_ARG;
-  int narrow = 0, wide = 0, widest = 0;
+  int tiles64 = 0, tiles256 = 0, widest = 0;
   for (int e = 0; e < G; ++e) {
-    const int m = group_off[e + 1] - group_off[e], w = umdk::tile_width(m, 256);
-    narrow += (m + 63) / 64;
-    wide += (m + 255) / 256;
+    const int m = group_off[e + 1] - group_off[e], tiles = (m + 255) / 256;
+    tiles64 += (m + 63) / 64;
+    tiles256 += tiles;
+    const int w = tiles > 0 ? ((m + tiles - 1) / tiles + 31) & ~31 : 0;
     widest = w > widest ? w : widest;
   }
   const int pairs = num_ctas / 2, nt = umdk::feature_tiles(mode, Nout);
-  return umdk::wide_pays(mode, nt, group_off[G] - group_off[0], narrow, wide, widest, pairs, 1.f / pairs) ? 256 : 64;
+  const int waves64 = (tiles64 * nt + pairs - 1) / pairs, waves256 = (tiles256 * nt + pairs - 1) / pairs;
+  const float rows = (float)(group_off[G] - group_off[0]), most = (float)widest * tiles256;
+  const float n = mode == 0 ? 0.25f * rows + 0.75f * most : 0.75f * rows + 0.25f * most;   // times the number of tiles
+  const float item = mode == 0 ? 1.3f * tiles256 + 0.0105f * n : 1.f * tiles256 + 0.0085f * n;
+  return waves256 * item < (float)waves64 * tiles256 ? 256 : 64;
 }

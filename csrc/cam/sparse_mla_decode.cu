@@ -105,10 +105,10 @@ struct MlaArgs {
 // Bounded waits that also leave when either CTA of the pair has raised the abort flag.
 template <bool kCluster>
 __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  if (kCluster ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
+  if (kCluster ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(smem_u32(bar), parity)) return true;
   const long long t0 = clock64();
   uint32_t spins = 0;
-  while (!(kCluster ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity))) {
+  while (!(kCluster ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(smem_u32(bar), parity))) {
     if ((++spins & 31u) == 0) {
       if (*abort_flag) return false;
       if (clock64() - t0 > kSpinLimitCycles) return false;

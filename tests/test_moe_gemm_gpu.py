@@ -122,6 +122,47 @@ def test_single_ctas_match_the_pairs(G, counts, K, F, H):
     assert all(torch.equal(u, v) for u, v in zip(*res))
 
 
+# 256-token tiles: rows around one and two CTAs' 128 and around a tile, a partner without rows, empty experts, K blocks that do
+# not fill a scale stage or fill several, fewer K blocks than accumulators, an odd number of 128-row blocks (half a last tile)
+@pytest.mark.parametrize("G,counts,K,F,H", [
+    (3, [256, 129, 255], 128, 128, 128),
+    (4, [257, 0, 128, 300], 1152, 256, 384),
+    (2, [512, 127], 1024, 128, 640),
+    (5, [1, 640, 31, 256, 33], 384, 384, 256),
+])
+def test_token_major_tiles_match_single_ctas(G, counts, K, F, H):
+    """One CTA pair takes the 256-token tiles here; ``max_ctas=1`` is the single-CTA kernel, which promotes the K blocks in the
+    same order: the same bytes. The oracle as in the tests above."""
+    import ctypes
+    from umdk_b200 import _native
+    from umdk_b200.ops import moe_gemm
+    c = _case(G, counts, K, F, H, seed=G + 2)
+    dev, N = "cuda", c["N"]
+    offs = (ctypes.c_int * (G + 1))(*c["off"].tolist())
+    for mode, nout in ((0, F), (1, H)):
+        assert _native.cam().umdk_moe_gemm_tokens_on_m(mode, G, nout, offs, 2) == 1
+        assert _native.cam().umdk_moe_gemm_uses_pairs(mode, G, nout, K if mode == 0 else F, N + 7, 2) == 1
+    status = torch.zeros(4, dtype=torch.int32, device=dev)
+    off, xq, xs, w1q, w1s, w2q, w2s = (c[k].to(dev) for k in ("off", "xq", "xs", "w1q", "w1s", "w2q", "w2s"))
+    xq.view(torch.uint8)[N:] = 0x7f   # NaN behind the last expert
+    res = []
+    for max_ctas in (1, 2):
+        hq = torch.full((N + 7, F), 0x55, dtype=torch.uint8, device=dev).view(torch.float8_e4m3fn)
+        hs = torch.full((N + 7, F // 128), 7.0, device=dev)
+        y = torch.full((N + 7, H), 7.0, dtype=torch.bfloat16, device=dev)
+        moe_gemm.gemm1_swiglu_quant(xq, xs, off, w1q, w1s, status, hq, hs, max_ctas=max_ctas)
+        moe_gemm.gemm2(hq, hs, off, w2q, w2s, status, y, max_ctas=max_ctas)
+        res.append((hq.view(torch.uint8), hs, y))   # the rows behind the experts' own among them: nobody writes those
+    torch.cuda.synchronize()
+    assert status.tolist()[0] == 0, status.tolist()
+    assert all(torch.equal(u, v) for u, v in zip(*res))
+    r_h = ref.ref_gemm1_swiglu_quant(c["xq"], c["xs"], c["off"], c["w1q"], c["w1s"])[2]
+    got_h = ref.dequant_fp8_1x128(res[1][0][:N].view(torch.float8_e4m3fn).cpu(), res[1][1][:N].cpu())
+    assert ref.mean_rel_err(got_h, r_h[:N]) < 0.04
+    r_y = ref.ref_gemm2(res[1][0].view(torch.float8_e4m3fn).cpu(), res[1][1].cpu(), c["off"], c["w2q"], c["w2s"])
+    assert ref.mean_rel_err(res[1][2][:N].float().cpu(), r_y[:N]) < 5e-3
+
+
 def test_more_experts_than_the_pairs_take():
     """1100 experts, a few of them with rows: the single-CTA kernel against the oracle of the hit experts."""
     from umdk_b200.ops import moe_gemm
