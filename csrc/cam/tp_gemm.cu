@@ -304,7 +304,7 @@ struct UmdkTpGemmParams {
   uint32_t* ctrl;        // [0] epoch, [1] done counter
   int* status;
   int phase_mask;        // 0 = 3 (everything); see TpArgs
-  int impl;              // 0 = CTA pairs where the shape allows (Ts and N multiples of 256), 1 = one CTA per tile
+  int impl;              // 0 = CTA pairs, 1 = one CTA per tile
 };
 
 // Symmetric-heap bytes a rank needs: MODE 0 regions (two shards + flags) followed by MODE 1 regions.
@@ -347,14 +347,18 @@ UMDK_API int umdk_tp_gemm(const UmdkTpGemmParams* p, void* stream) {
   a.phase_mask = p->phase_mask ? p->phase_mask : 3;
   const int M = p->R * p->Ts;
   const void* A = p->mode == 0 ? p->xg : p->a_local;
-  if (p->impl == 0 && a.phase_mask != 4 && (p->Ts % 256) == 0 && (p->N % 256) == 0) {
+  if (p->impl == 0 && a.phase_mask != 4) {
     int grid = sm_count();
     if (p->max_ctas > 0 && p->max_ctas < grid) grid = p->max_ctas;
     grid &= ~1;
     // whole pairs take the copy role; the bulk-copy engine needs few of them (default 4 pairs)
-    a.n_copy = p->n_copy > 0 ? ((p->n_copy + 1) & ~1) : 8;
-    if (grid <= a.n_copy + 1) return -UMDK_ERR_BAD_ARG;
-    return tp_gemm_2sm_launch(a, A, p->w, p->out, grid, static_cast<cudaStream_t>(stream));
+    const int n_copy = p->n_copy > 0 ? ((p->n_copy + 1) & ~1) : 8;
+    if (grid > n_copy + 1) {
+      a.n_copy = n_copy;
+      return tp_gemm_2sm_launch(a, A, p->w, p->out, grid, static_cast<cudaStream_t>(stream));
+    }
+    if (p->Ts % 256 == 0) return -UMDK_ERR_BAD_ARG;
+    // few CTAs (max_ctas) and an odd number of 128-row blocks: one CTA per tile
   }
   CUtensorMap tmA, tmB, tmC;
   if (make_tmap_2d(&tmA, TMAP_BF16, A, p->K, M, (uint64_t)p->K * 2, BK, BM, TMAP_SW_128B)) return -UMDK_ERR_BAD_ARG;

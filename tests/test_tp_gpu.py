@@ -64,6 +64,49 @@ def test_gemm_reduce_scatter(R, Ts, Kr, N, single_cta):
             h.close()
 
 
+# tiles of 64, 128 and 256 columns; an even and an odd number of 128-row blocks, one block only, fewer K steps than the ring
+# holds and more
+@pytest.mark.parametrize("R,Ts,K,N,columns", [(1, 128, 64, 256, 64), (1, 384, 704, 512, 64), (1, 640, 192, 2560, 128),
+                                              (1, 1536, 576, 4096, 128), (1, 1408, 2048, 2816, 256), (2, 384, 320, 512, 64),
+                                              (3, 640, 192, 768, 128), (2, 1152, 1024, 1536, 256)])
+def test_tile_columns_and_odd_row_blocks(R, Ts, K, N, columns):
+    from umdk_b200 import _native
+    from umdk_b200.ops.tp import TpComm
+    from umdk_b200.parallel.symm import SymmetricHeap
+    pairs = (torch.cuda.get_device_properties(0).multi_processor_count & ~1) // 2 - (4 if R > 1 else 0)
+    assert _native.cam().umdk_tp_tile_columns(0, R, Ts, N, K, 3, pairs) == columns
+    g = torch.Generator().manual_seed(Ts)
+    xs = [torch.randn(Ts, K, generator=g).to(torch.bfloat16).cuda() for _ in range(R)]
+    ws = [(torch.randn(N, K, generator=g) * 0.05).to(torch.bfloat16).cuda() for _ in range(R)]
+    ys = [torch.randn(R * Ts, K, generator=g).to(torch.bfloat16).cuda() for _ in range(R)]
+    heaps = SymmetricHeap.virtual(TpComm.heap_bytes(R, Ts, K, N), R)
+    try:
+        comms = [TpComm(h, Ts, K, N) for h in heaps]
+        for rnd in range(2):
+            for r in range(R):
+                comms[r].ag_gemm(xs[r], ws[r], phase_mask=4)
+            outs = [comms[r].ag_gemm(xs[r], ws[r]) for r in range(R)]
+            if R == 1:
+                sums = [comms[0].gemm_rs(ys[0], ws[0])]
+            else:
+                sums = [comms[r].gemm_rs(ys[r], ws[r], phase_mask=1) for r in range(R)]
+                for r in range(R):
+                    comms[r].gemm_rs(ys[r], ws[r], out=sums[r], phase_mask=2)
+            torch.cuda.synchronize()
+            xall = torch.cat(xs).float()
+            full = sum(ys[s].float() @ ws[s].float().t() for s in range(R))
+            for r in range(R):
+                comms[r].check()
+                # results are rounded to bf16 once (2^-9 relative at most); R > 1 rounds every partial sum too
+                assert _rel(outs[r], xall @ ws[r].float().t()) < 5e-3
+                assert _rel(sums[r], full[r * Ts:(r + 1) * Ts]) < 1e-2
+            xs = [x + 1 for x in xs]
+            ys = [y * 0.5 + 0.25 for y in ys]
+    finally:
+        for h in heaps:
+            h.close()
+
+
 @pytest.mark.parametrize("R,n", [(1, 4096), (2, 1 << 16), (4, 1 << 18), (8, 64 * 1024)])
 def test_one_shot_allreduce_virtual_ranks(R, n):
     from umdk_b200.ops.tp import AllReduce

@@ -84,7 +84,7 @@ class TpComm(Recoverable):
         if n_copy <= 0:
             n_copy = 16
         self.n_copy, self.max_ctas = n_copy, max_ctas
-        # False: CTA pairs (256 x 256 tiles) where Ts and N are multiples of 256; True: always one CTA per tile
+        # False: CTA pairs; True: one CTA per tile
         self.single_cta = single_cta
 
     @staticmethod
