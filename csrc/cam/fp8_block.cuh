@@ -42,4 +42,15 @@ __device__ __forceinline__ int4 quant16(const float* f, float* scale) {
   return q;
 }
 
+// v / (1 + exp(-v)) with the quotient rounded once more through its remainder (Markstein), which gives the rounded division
+// without its branches (a zero, as rows behind a tile's own hold, takes the slowest of them: 14000 cycles for 32 tokens a
+// thread). A remainder that is not a number (v or the divisor infinite) leaves the first quotient as it is.
+__device__ __forceinline__ float silu(float v) {
+  const float d = 1.f + __expf(-v);
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float q = v * r, e = fmaf(-q, d, v);
+  return fmaf(e == e ? e : -0.f, r, q);
+}
+
 }  // namespace umdk

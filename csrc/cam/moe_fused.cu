@@ -14,7 +14,8 @@
 // Work split: phase-1 items are dealt round-robin; phase-2 items (about 1/7 of the cost each) are dealt in
 // contiguous ranges sized so that every CTA ends at the same time, the CTAs with fewer phase-1 items taking the
 // earliest (first ready) phase-2 items. Roles per CTA as in moe_gemm.cu: TMA producer warp, single-thread MMA issuer,
-// TMEM allocator warp, eight promotion/epilogue warps (two per scheduler, so one hides the other's TMEM-load latency).
+// two warps that fetch scales ahead, eight promotion/epilogue warps (two per scheduler, so one hides the other's TMEM-load
+// latency). MMAs and promotion cover 16, 32 or 64 token columns, whatever the tile has.
 // Same math and operand formats as moe_gemm.cu modes 0 and 2.
 // Reference counterpart: the fused_deep_moe operator (src/cam/comm_operator/ascend_kernels/fused_deep_moe/op_kernel/
 // fused_deep_moe.h:354-448), whose cube cores likewise wait per expert group for arrived tokens
@@ -22,17 +23,24 @@
 // unbounded spin, here with a cycle budget and a status record.
 #include "ep_ll_dispatch.cuh"
 
+#include <type_traits>
+
 namespace umdk {
 namespace {
 
 constexpr int TT = 64;
 constexpr int BMW = 128;
 constexpr int BKB = 128;
-constexpr int kThreads = 384;      // TMA, MMA, TMEM-allocator and one spare warp + 8 promotion / epilogue warps
+constexpr int kThreads = 384;      // TMA, MMA and two scale warps (one of them allocates TMEM) + 8 promotion / epilogue warps
 constexpr int kEpiThreads = 256;
-constexpr int kTransStride = 129;
+constexpr int kTransStride = 132;   // conflict-free for the promotion's stores and for 16-byte loads of a token
 constexpr int kRingBytes = 4 * (2 * BMW * BKB + TT * BKB);  // 160 KB: 4 x 40 KB (phase 1) or 6 x 24 KB (phase 2)
-constexpr int kTmemCols = 256;
+constexpr int kTmemCols = 512;
+constexpr int kScaleKb = 8;        // K blocks per scale stage: [kb][token] activation scales, then [kb][gate / up] weight scales
+constexpr int kScaleStages = 4;
+constexpr int kScaleFloats = kScaleKb * TT + 2 * kScaleKb;
+constexpr int kTmemStages = 4;
+constexpr int kPhaseBars = 2 * 6 + 2 * kTmemStages + 2 * kScaleStages;
 
 struct FusedArgs {
   int G, F, H;             // local experts, FFN width, hidden size
@@ -83,18 +91,44 @@ struct P {
 
 struct Shared {
   float* trans;
-  float* xs_sm;
-  float* ws_sm;
+  float* scales;   // [kScaleStages][kScaleFloats]
   float* amax_sm;
   int* tile_pref;
   int* goff;
-  int* epi_flag;
-  int* meta_sm;    // [TT][2] owner rank and slot of the rows of the current token tile (phase 2)
-  uint64_t* bars;  // per phase: full[6], empty[6], tfull[2], tempty[2] = 16 barriers
+  uint64_t* bars;  // per phase: full[6], empty[6], tfull[4], tempty[4], sfull[4], sempty[4]
   uint8_t* ring;
 };
 
 __device__ __forceinline__ void bar_epi() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// The same barrier, joining a decision: true on all 256 threads or on none (a wait that ran out in one warp must not leave the
+// others at the next barrier).
+__device__ __forceinline__ bool bar_epi_and(bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.u32 q, %1, 0;\n"
+      "barrier.cta.red.and.pred p, 1, 256, q;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(r)
+      : "r"(ok ? 1u : 0u)
+      : "memory");
+  return r != 0;
+}
+// Token columns that the MMAs of a tile of m rows cover; the halves of the promoting warps take 8, 16 or 32 of them.
+__device__ __forceinline__ int tile_columns(int m) { return m <= 16 ? 16 : m <= 32 ? 32 : TT; }
+
+// 32 lanes x N columns: lanes 0..15 of the warp's in r[0], 16..31 in r[1] (see tmem_ld_16x256b_x1 for the order).
+template <int N>
+__device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t (*r)[N / 2]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if constexpr (N == 8) tmem_ld_16x256b_x1(addr + (h << 20), r[h]);
+    else if constexpr (N == 16) tmem_ld_16x256b_x2(addr + (h << 20), r[h]);
+    else tmem_ld_16x256b_x4(addr + (h << 20), r[h]);
+  }
+}
 __device__ __forceinline__ void locate_tile(const int* tile_pref, const int* goff, int G, int tile, int* e, int* row0,
                                             int* m) {
   int lo = 0, hi = G;
@@ -119,11 +153,14 @@ __device__ __forceinline__ void run_phase(const CUtensorMap* tmW, const CUtensor
   const int w_rows = PH == 1 ? 2 * a.F : a.H;
   const int NT = Nout / BMW;
   const int kb_total = K / BKB;
-  uint64_t* full = sh.bars + (PH - 1) * 16;
+  uint64_t* full = sh.bars + (PH - 1) * kPhaseBars;
   uint64_t* empty = full + 6;
   uint64_t* tfull = full + 12;
-  uint64_t* tempty = full + 14;
+  uint64_t* tempty = tfull + kTmemStages;
+  uint64_t* sfull = tempty + kTmemStages;
+  uint64_t* sempty = sfull + kScaleStages;
   const int NT1 = a.F / BMW;
+  const int nsb = K / 128, wsb = w_rows / 128;
 
   if (warp == 0) {
     if (elect_one()) {
@@ -183,15 +220,17 @@ __device__ __forceinline__ void run_phase(const CUtensorMap* tmW, const CUtensor
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc(kFmtE4M3, kFmtE4M3, BMW, TT);
       int s = 0;
       uint32_t ph = 0, kbc = 0;
       bool ok = true;
+      const uint64_t desc0 = umma_desc_k_sw128(smem_u32(sh.ring));
       for (int w = first; w < last && ok; w += step) {
+        int e, row0, m;
+        locate_tile(sh.tile_pref, sh.goff, a.G, w / NT, &e, &row0, &m);
+        const uint32_t idesc = umma_idesc(kFmtE4M3, kFmtE4M3, BMW, tile_columns(m));
         for (int kb = 0; kb < kb_total; ++kb, ++kbc) {
-          const int ts = kbc & 1;
-          const uint32_t tph = (kbc >> 1) & 1;
-          if (!mbar_wait(&tempty[ts], tph ^ 1)) {
+          const int ts = kbc % kTmemStages;
+          if (!mbar_wait(&tempty[ts], ((kbc / kTmemStages) & 1) ^ 1)) {
             umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_EMPTY, w, kb);
             ok = false;
             break;
@@ -202,10 +241,9 @@ __device__ __forceinline__ void run_phase(const CUtensorMap* tmW, const CUtensor
             break;
           }
           tc_fence_after();
-          const uint32_t sa = smem_u32(sh.ring + s * C::kStageBytes);
-          const uint64_t adesc = umma_desc_k_sw128(sa);
-          const uint64_t adesc_u = umma_desc_k_sw128(sa + BMW * BKB);
-          const uint64_t bdesc = umma_desc_k_sw128(sa + C::kABytes);
+          const uint64_t adesc = desc0 + s * (C::kStageBytes >> 4);
+          const uint64_t adesc_u = adesc + (BMW * BKB >> 4);
+          const uint64_t bdesc = adesc + (C::kABytes >> 4);
           const uint32_t d = tmem_base + ts * C::kTmemStageCols;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
@@ -221,165 +259,199 @@ __device__ __forceinline__ void run_phase(const CUtensorMap* tmW, const CUtensor
         }
       }
     }
-  } else if (warp >= 4) {
-    // Eight promotion / epilogue warps. TMEM lane = weight row of the tile; a warp may only touch the 32 lanes
-    // selected by (warp index mod 4), so warps 4..7 and 8..11 cover the same rows and split the 64 token columns.
-    const int ew = warp - 4;
-    const int q = warp & 3, hh = ew >> 2;
-    const int tid = ew * 32 + lane;         // 0..255 inside the epilogue group
-    const int wrow = q * 32 + lane;         // weight row of this thread inside the 128-row tile
-    constexpr int HC = TT / 2;              // token columns per thread
-    const int nsb = K / 128;
-    const int wsb = w_rows / 128;
+  } else if (warp < 4) {
+    // ---- scales of the coming K blocks: thread t fetches those of token t, eight blocks at a time, stages ahead of the
+    // promotion (fetched by the promoting warps at the start of every item they took 2300 - 9500 cycles of it) ----
+    const int t = threadIdx.x - 64;
     const float* xs = PH == 1 ? a.xs : a.hs;
     const float* ws = PH == 1 ? a.w1s : a.w2s;
-    uint32_t kbc = 0;
+    int ss = 0, ready = -1;
+    uint32_t sph = 0;
     bool ok = true;
-    int ready_tile = -1, loaded_tile = -1, ready_e = -1;
-    float ws_next = 0.f;
-    bool have_ws_next = false;
     for (int w = first; w < last && ok; w += step) {
       int e, row0, m;
-      const int tile = w / NT;
+      const int tile = w / NT, j = w - tile * NT;
       locate_tile(sh.tile_pref, sh.goff, a.G, tile, &e, &row0, &m);
-      const int j = w % NT;
-      if (PH == 2 && tile != ready_tile) {
-        // the scales of the intermediate rows are read with plain loads below: order them after the phase-1 writers
-        if (tid == 0) *sh.epi_flag = wait_flag_ge_gpu(&a.tile_done[tile], (uint32_t)NT1) ? 1 : 0;
-        bar_epi();
-        if (!*sh.epi_flag) break;  // the producer records the timeout
-        ready_tile = tile;
-      }
-      if (PH == 1 && a.exp_gate && e != ready_e) {
-        // the row scales are read with plain loads below: they have landed when the expert's arrival word is full (the
-        // producer's wait on the same word orders only the TMA loads)
+      // The same waits as the producer's (which records a timeout): they order the loads below, and through the barriers
+      // whatever the promoting warps read, behind the rows' arrival or the phase-1 writers.
+      if (PH == 1 && a.exp_gate && e != ready) {
         const uint32_t need = (uint32_t)(sh.goff[e + 1] - sh.goff[e]) * (uint32_t)a.exp_parts;
-        if (tid == 0) *sh.epi_flag = wait_flag_ge_sys(a.exp_cnt + e, need) ? 1 : 0;
-        bar_epi();
-        if (!*sh.epi_flag) break;  // the producer records the timeout
-        ready_e = e;
+        if (!__all_sync(0xffffffffu, wait_flag_ge_sys(a.exp_cnt + e, need))) break;
+        ready = e;
       }
-      if (PH == 1 || tile != loaded_tile) {
-        // activation scales (and, in phase 2, the owner / slot of every row) depend on the token tile only; a CTA's
-        // phase-2 items walk the weight tiles of one token tile back to back, so they are fetched once per tile
-        for (int i = tid; i < TT * kb_total; i += kEpiThreads) {
-          const int t = i / kb_total, kb = i - t * kb_total;
-          // phase 2 reads scales written by other SMs during this launch: bypass L1
-          sh.xs_sm[kb * TT + t] = t < m ? __ldcg(xs + (size_t)(row0 + t) * nsb + kb) : 0.f;
-        }
-        if (PH == 2 && tid < 2 * TT) sh.meta_sm[tid] = (tid >> 1) < m ? a.row_meta[2 * row0 + tid] : -1;
-        loaded_tile = tile;
+      if (PH == 2 && tile != ready) {
+        if (!__all_sync(0xffffffffu, wait_flag_ge_gpu(&a.tile_done[tile], (uint32_t)NT1))) break;
+        ready = tile;
       }
-      if (!have_ws_next) {
-        for (int i = tid; i < C::kATiles * kb_total; i += kEpiThreads) {
-          const int which = i / kb_total, kb = i - which * kb_total;
-          const int brow = which == 0 ? j : (a.F / 128 + j);
-          sh.ws_sm[which * kb_total + kb] = ws[((size_t)e * wsb + brow) * nsb + kb];
-        }
-      } else if (tid < C::kATiles * kb_total) {
-        sh.ws_sm[tid] = ws_next;   // fetched while the previous item was in its k-loop
-      }
-      have_ws_next = false;
-      if (w + step < last && C::kATiles * kb_total <= kEpiThreads) {
-        // weight scales of the NEXT item: the load is in flight during this item's k-loop
-        int e2, r2, m2;
-        const int w2 = w + step;
-        locate_tile(sh.tile_pref, sh.goff, a.G, w2 / NT, &e2, &r2, &m2);
-        if (tid < C::kATiles * kb_total) {
-          const int which = tid / kb_total, kb = tid - which * kb_total;
-          const int brow = which == 0 ? (w2 % NT) : (a.F / 128 + (w2 % NT));
-          ws_next = ws[((size_t)e2 * wsb + brow) * nsb + kb];
-        }
-        have_ws_next = true;
-      }
-      bar_epi();
-      float acc_g[HC];
-      float acc_u[PH == 1 ? HC : 1];
+      // written by other SMs during this launch: past L1
+      const float* xrow = xs + (size_t)(row0 + t) * nsb;
+      const int wi = (t >> 1) & (kScaleKb - 1);   // threads 0..15: K block and gate / up row of a weight scale
+      const float* wrow = ws + ((size_t)e * wsb + j + ((t & 1) && PH == 1 ? a.F / 128 : 0)) * nsb + wi;
+      for (int kb0 = 0; kb0 < kb_total; kb0 += kScaleKb) {
+        float x[kScaleKb];
 #pragma unroll
-      for (int c = 0; c < HC; ++c) acc_g[c] = 0.f;
-      if (PH == 1) {
-#pragma unroll
-        for (int c = 0; c < HC; ++c) acc_u[c] = 0.f;
-      }
-      for (int kb = 0; kb < kb_total; ++kb, ++kbc) {
-        const int ts = kbc & 1;
-        const uint32_t tph = (kbc >> 1) & 1;
-        if (!mbar_wait(&tfull[ts], tph)) {
-          umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, w, kb);
+        for (int i = 0; i < kScaleKb; ++i) x[i] = t < m && kb0 + i < kb_total ? __ldcg(xrow + kb0 + i) : 0.f;
+        const float wv = t < 2 * kScaleKb && kb0 + wi < kb_total ? __ldg(wrow + kb0) : 0.f;
+        if (!__all_sync(0xffffffffu, mbar_wait(&sempty[ss], sph ^ 1))) {
+          umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_EMPTY, w, 10000 + kb0);
           ok = false;
           break;
         }
-        tc_fence_after();
-        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + ts * C::kTmemStageCols + hh * HC;
-        uint32_t rg[HC];
-        uint32_t ru[PH == 1 ? HC : 1];
-        tmem_ld_x32(taddr, rg);
-        if constexpr (PH == 1) tmem_ld_x32(taddr + TT, ru);
-        const float wg = sh.ws_sm[kb];
-        const float wu = PH == 1 ? sh.ws_sm[kb_total + kb] : 0.f;
-        const float4* xsk = reinterpret_cast<const float4*>(sh.xs_sm + kb * TT + hh * HC);
-        tmem_ld_wait();
-        // the accumulator stage is free as soon as its values are in registers
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty[ts]);
+        float* dst = sh.scales + ss * kScaleFloats;
 #pragma unroll
-        for (int c4 = 0; c4 < HC / 4; ++c4) {
-          const float4 x4 = xsk[c4];
-          acc_g[4 * c4 + 0] = fmaf(__uint_as_float(rg[4 * c4 + 0]), x4.x * wg, acc_g[4 * c4 + 0]);
-          acc_g[4 * c4 + 1] = fmaf(__uint_as_float(rg[4 * c4 + 1]), x4.y * wg, acc_g[4 * c4 + 1]);
-          acc_g[4 * c4 + 2] = fmaf(__uint_as_float(rg[4 * c4 + 2]), x4.z * wg, acc_g[4 * c4 + 2]);
-          acc_g[4 * c4 + 3] = fmaf(__uint_as_float(rg[4 * c4 + 3]), x4.w * wg, acc_g[4 * c4 + 3]);
-          if constexpr (PH == 1) {
-            acc_u[4 * c4 + 0] = fmaf(__uint_as_float(ru[4 * c4 + 0]), x4.x * wu, acc_u[4 * c4 + 0]);
-            acc_u[4 * c4 + 1] = fmaf(__uint_as_float(ru[4 * c4 + 1]), x4.y * wu, acc_u[4 * c4 + 1]);
-            acc_u[4 * c4 + 2] = fmaf(__uint_as_float(ru[4 * c4 + 2]), x4.z * wu, acc_u[4 * c4 + 2]);
-            acc_u[4 * c4 + 3] = fmaf(__uint_as_float(ru[4 * c4 + 3]), x4.w * wu, acc_u[4 * c4 + 3]);
-          }
+        for (int i = 0; i < kScaleKb; ++i) dst[i * TT + t] = x[i];
+        if (t < 2 * kScaleKb) dst[kScaleKb * TT + t] = wv;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sfull[ss]);
+        if (++ss == kScaleStages) {
+          ss = 0;
+          sph ^= 1;
         }
       }
-      if (!ok) break;
-      // transpose through shared memory: trans[token][weight row]
+    }
+  } else {
+    // Eight promotion / epilogue warps. TMEM lane = weight row of the tile; a warp may only touch the 32 lanes
+    // selected by (warp index mod 4), so warps 4..7 and 8..11 cover the same rows and split the token columns.
+    const int ew = warp - 4;
+    const int q = warp & 3, hh = ew >> 2;
+    const int tid = ew * 32 + lane;         // 0..255 inside the epilogue group
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+    int ss = 0;
+    uint32_t sph = 0, kbc = 0;
+    bool ok = true;
+    for (int w = first; w < last && ok; w += step) {
+      int e, row0, m;
+      const int tile = w / NT, j = w - tile * NT;
+      locate_tile(sh.tile_pref, sh.goff, a.G, tile, &e, &row0, &m);
+      const int t = tid & 63, qtr = tid >> 6;     // of the epilogue: token, 32-column quarter of the 128 output columns
+      int2 meta = make_int2(-1, -1);              // phase 2: owner rank and slot of row t
+      // A warp covers 32 weight rows x HC tokens, a thread four of the rows x two of every eight tokens: with one row and all
+      // HC tokens the scales (16-byte broadcast loads) took 256 of the shared-memory port's cycles a K block, which with the
+      // operands' way in and out made 960 cycles in phase 1 and 640 in phase 2.
+      auto item = [&](auto hc) {
+        constexpr int HC = decltype(hc)::value;
+        uint64_t acc_g[2][HC / 4], acc_u[2][PH == 1 ? HC / 4 : 1];   // [lane half][8-token group, row t / 4 or t / 4 + 8]
 #pragma unroll
-      for (int c = 0; c < HC; ++c) {
-        float v = acc_g[c];
-        if constexpr (PH == 1) v = (v / (1.f + __expf(-v))) * acc_u[c];
-        sh.trans[(hh * HC + c) * kTransStride + wrow] = v;
-      }
-      bar_epi();
-      const int t = tid & 63, qtr = tid >> 6;     // token, 32-column quarter of the 128 output columns
-      const float* src = sh.trans + t * kTransStride + qtr * 32;
+        for (int c = 0; c < HC / 4; ++c) {
+          acc_g[0][c] = acc_g[1][c] = 0;
+          if (PH == 1) acc_u[0][c] = acc_u[1][c] = 0;
+        }
+        for (int kb0 = 0; kb0 < kb_total && ok; kb0 += kScaleKb) {
+          if (!mbar_wait(&sfull[ss], sph)) {
+            umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, 10000 + kb0);
+            ok = false;
+            break;
+          }
+          if (PH == 2 && kb0 == 0 && t < m) meta = __ldcg(reinterpret_cast<const int2*>(a.row_meta) + row0 + t);
+          const float* sc = sh.scales + ss * kScaleFloats;
+          const int kb1 = min(kb_total, kb0 + kScaleKb);
+          for (int kb = kb0; kb < kb1; ++kb, ++kbc) {
+            const int ts = kbc % kTmemStages;
+            if (!mbar_wait(&tfull[ts], (kbc / kTmemStages) & 1)) {
+              umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, w, kb);
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t taddr = lane_addr + ts * C::kTmemStageCols + hh * HC;
+            uint32_t rg[2][HC / 2], ru[2][HC / 2];
+            tmem_ld<HC>(taddr, rg);
+            if constexpr (PH == 1) tmem_ld<HC>(taddr + TT, ru);
+            const float2 wf = reinterpret_cast<const float2*>(sc + kScaleKb * TT)[kb - kb0];
+            const uint64_t wg = pack_f32x2(__float_as_uint(wf.x), __float_as_uint(wf.x));
+            const uint64_t wu = pack_f32x2(__float_as_uint(wf.y), __float_as_uint(wf.y));
+            uint64_t x2[HC / 8];
+#pragma unroll
+            for (int g = 0; g < HC / 8; ++g)
+              x2[g] = *reinterpret_cast<const uint64_t*>(sc + (kb - kb0) * TT + hh * HC + 8 * g + 2 * (lane & 3));
+            tmem_ld_wait();
+            // the accumulator stage is free as soon as its values are in registers
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty[ts]);
+#pragma unroll
+            for (int g = 0; g < HC / 8; ++g) {
+              const uint64_t fg = mul_f32x2(x2[g], wg), fu = mul_f32x2(x2[g], wu);
+#pragma unroll
+              for (int h = 0; h < 4; ++h) {   // lane half, row
+                const int i = 4 * g + 2 * (h & 1);
+                uint64_t& dg = acc_g[h >> 1][2 * g + (h & 1)];
+                dg = fma_f32x2(pack_f32x2(rg[h >> 1][i], rg[h >> 1][i + 1]), fg, dg);
+                if constexpr (PH == 1) {
+                  uint64_t& du = acc_u[h >> 1][2 * g + (h & 1)];
+                  du = fma_f32x2(pack_f32x2(ru[h >> 1][i], ru[h >> 1][i + 1]), fu, du);
+                }
+              }
+            }
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sempty[ss]);
+          if (++ss == kScaleStages) {
+            ss = 0;
+            sph ^= 1;
+          }
+        }
+        // transpose through shared memory: trans[token][weight row]
+#pragma unroll
+        for (int g = 0; g < HC / 8; ++g) {
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            float v[2];
+            unpack_f32x2(acc_g[h >> 1][2 * g + (h & 1)], &v[0], &v[1]);
+            if constexpr (PH == 1) {
+              float u[2];
+              unpack_f32x2(acc_u[h >> 1][2 * g + (h & 1)], &u[0], &u[1]);
+              v[0] = silu(v[0]) * u[0];
+              v[1] = silu(v[1]) * u[1];
+            }
+            float* dst = sh.trans + (hh * HC + 8 * g + 2 * (lane & 3)) * kTransStride + q * 32 + h * 8 + (lane >> 2);
+            dst[0] = v[0];
+            dst[kTransStride] = v[1];
+          }
+        }
+      };
+      const int cols = tile_columns(m);
+      if (cols == 16) item(std::integral_constant<int, 8>());
+      else if (cols == 32) item(std::integral_constant<int, 16>());
+      else item(std::integral_constant<int, 32>());
+      ok = bar_epi_and(ok);
+      if (!ok) break;
+      const float4* src = reinterpret_cast<const float4*>(sh.trans + t * kTransStride + qtr * 32);
       const int row = row0 + t;
       if (PH == 1) {
+        float4 h[8];
         float amax = 0.f;
-#pragma unroll 8
-        for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(src[i]));
+        if (t < m) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            h[i] = src[i];
+            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(h[i].x), fabsf(h[i].y)), fmaxf(fabsf(h[i].z), fabsf(h[i].w))));
+          }
+        }
         sh.amax_sm[tid] = amax;
         bar_epi();
-        amax = fmaxf(fmaxf(fmaxf(sh.amax_sm[t], sh.amax_sm[t + 64]), fmaxf(sh.amax_sm[t + 128], sh.amax_sm[t + 192])),
-                     1e-4f);
-        const float inv = 448.f / amax;
         if (t < m) {
-          uint8_t* dst = a.hq + (size_t)row * a.F + j * BMW + qtr * 32;
+          amax = fmaxf(fmaxf(fmaxf(sh.amax_sm[t], sh.amax_sm[t + 64]), fmaxf(sh.amax_sm[t + 128], sh.amax_sm[t + 192])),
+                       1e-4f);
+          const float inv = 448.f / amax;
+          uint32_t o[8];
 #pragma unroll
-          for (int qq = 0; qq < 2; ++qq) {
-            int4 o;
-            const float* s4 = src + qq * 16;
-            o.x = pack_fp8x4(s4[0] * inv, s4[1] * inv, s4[2] * inv, s4[3] * inv);
-            o.y = pack_fp8x4(s4[4] * inv, s4[5] * inv, s4[6] * inv, s4[7] * inv);
-            o.z = pack_fp8x4(s4[8] * inv, s4[9] * inv, s4[10] * inv, s4[11] * inv);
-            o.w = pack_fp8x4(s4[12] * inv, s4[13] * inv, s4[14] * inv, s4[15] * inv);
-            reinterpret_cast<int4*>(dst)[qq] = o;
-          }
+          for (int i = 0; i < 8; ++i) o[i] = pack_fp8x4(h[i].x * inv, h[i].y * inv, h[i].z * inv, h[i].w * inv);
+          int4* dst = reinterpret_cast<int4*>(a.hq + (size_t)row * a.F + j * BMW + qtr * 32);
+          dst[0] = make_int4(o[0], o[1], o[2], o[3]);
+          dst[1] = make_int4(o[4], o[5], o[6], o[7]);
           if (qtr == 0) a.hs[(size_t)row * (a.F / 128) + j] = amax * (1.f / 448.f);
         }
-        // publish: the rows of this item are in global memory -> one more phase-1 item of this token tile is done
-        __threadfence();
+        // publish: one more phase-1 item of this token tile is done. The barrier orders everybody's stores before the release
+        // (which is cumulative), so only the publishing thread waits for them.
         bar_epi();
-        if (tid == 0) red_add_release_gpu(&a.tile_done[tile], 1u);
+        if (tid == 0) {
+          __threadfence();
+          red_add_release_gpu(&a.tile_done[tile], 1u);
+        }
       } else {
         if (t < m) {
-          const int owner = sh.meta_sm[2 * t], slot = sh.meta_sm[2 * t + 1];
+          const int owner = meta.x, slot = meta.y;
           if (owner < 0 || owner >= a.R || slot < 0 || slot >= a.T_cap * a.Kt) {
             umdk_set_status(a.status, UMDK_ERR_OVERFLOW, UMDK_PH_COMBINE_DATA, owner, slot);
           } else {
@@ -389,7 +461,11 @@ __device__ __forceinline__ void run_phase(const CUtensorMap* tmW, const CUtensor
               int4 o;
               __nv_bfloat162* po = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-              for (int i = 0; i < 4; ++i) po[i] = __floats2bfloat162_rn(src[qq * 8 + 2 * i], src[qq * 8 + 2 * i + 1]);
+              for (int i = 0; i < 2; ++i) {
+                const float4 v = src[qq * 2 + i];
+                po[2 * i] = __floats2bfloat162_rn(v.x, v.y);
+                po[2 * i + 1] = __floats2bfloat162_rn(v.z, v.w);
+              }
               st_na_v4(dst + qq * 16, o);
             }
           }
@@ -405,33 +481,32 @@ moe_fused_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constant
                  const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmH, const FusedArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int kb_max = (a.H > a.F ? a.H : a.F) / BKB;
   Shared sh;
   sh.ring = smem;
   sh.trans = reinterpret_cast<float*>(smem + kRingBytes);
-  sh.xs_sm = sh.trans + TT * kTransStride;
-  sh.ws_sm = sh.xs_sm + kb_max * TT;
-  sh.amax_sm = sh.ws_sm + 2 * kb_max;
+  sh.scales = sh.trans + TT * kTransStride;
+  sh.amax_sm = sh.scales + kScaleStages * kScaleFloats;
   sh.tile_pref = reinterpret_cast<int*>(sh.amax_sm + kEpiThreads);
   sh.goff = sh.tile_pref + (a.G + 1);
-  sh.epi_flag = sh.goff + (a.G + 1);
-  sh.meta_sm = sh.epi_flag + 1;
-  sh.bars = reinterpret_cast<uint64_t*>((reinterpret_cast<uintptr_t>(sh.meta_sm + 2 * TT) + 15) & ~uintptr_t(15));
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sh.bars + 32);
+  sh.bars = reinterpret_cast<uint64_t*>((reinterpret_cast<uintptr_t>(sh.goff + a.G + 1) + 15) & ~uintptr_t(15));
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sh.bars + 2 * kPhaseBars);
   __shared__ int s_ok;
   __shared__ uint32_t s_epoch;
   const int warp = threadIdx.x >> 5;
 
   if (threadIdx.x == 0) {
     for (int p = 0; p < 2; ++p) {
-      uint64_t* b = sh.bars + p * 16;
-      for (int s = 0; s < 6; ++s) {
-        mbar_init(&b[s], 1);
-        mbar_init(&b[6 + s], 1);
+      uint64_t* b = sh.bars + p * kPhaseBars;
+      for (int s = 0; s < 12; ++s) mbar_init(&b[s], 1);   // full, empty
+      b += 12;
+      for (int i = 0; i < kTmemStages; ++i) {
+        mbar_init(&b[i], 1);
+        mbar_init(&b[kTmemStages + i], 8);
       }
-      for (int i = 0; i < 2; ++i) {
-        mbar_init(&b[12 + i], 1);
-        mbar_init(&b[14 + i], 8);
+      b += 2 * kTmemStages;
+      for (int i = 0; i < kScaleStages; ++i) {
+        mbar_init(&b[i], 2);
+        mbar_init(&b[kScaleStages + i], 8);
       }
     }
     mbar_fence_init();
@@ -530,26 +605,25 @@ moe_fused_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constant
   tc_fence_after();
 
   // ---- phase 2: contiguous ranges sized so that all CTAs finish together ----
-  // Costs in weight bytes / 128: a phase-1 item streams two 128 x H tiles, a phase-2 item one 128 x F tile.
-  // CTAs [0, extra) hold one more phase-1 item than the others ("heavy"); the light CTAs come first in the order of
-  // ranges, so they take the phase-2 items whose token tiles were finished in the early phase-1 waves.
+  // Costs in K blocks of 128 weight rows: a phase-1 item streams two 128 x H tiles, a phase-2 item one 128 x F tile; 4 and 2 for
+  // what every item takes besides (3000 and 1500 cycles).
+  // CTAs [0, extra) hold one more phase-1 item than the others ("heavy"). While they work on it the light CTAs take phase-2
+  // items whose token tiles were finished in the earlier waves; what is left when the heavy ones come is dealt evenly. (Shares
+  // by weight bytes alone gave ALL phase-2 items to the light CTAs where phase 1 is one wave: 36 us for phase 2 of 10 tokens on
+  // 16 experts, 4864 x 640.)
   {
-    const long long c1 = 2LL * a.H, c2 = a.F;
     const int n1_lo = items1 / grid, extra = items1 % grid, n_light = grid - extra;
-    const long long total = (long long)items1 * c1 + (long long)items2 * c2;
-    const long long target = (total + grid - 1) / grid;
-    long long bl = target - (long long)n1_lo * c1, bh = target - (long long)(n1_lo + 1) * c1;
-    if (bl < 0) bl = 0;
-    if (bh < 0) bh = 0;
+    const int cost1 = 2 * (a.H / BKB) + 4, cost2 = a.F / BKB + 2;
+    const long long ready = (long long)(n1_lo * grid / NT1) * NT2;   // items of the tiles that the full waves finish
+    long long early = extra > 0 ? (long long)n_light * cost1 / cost2 : 0;
+    if (early > ready) early = ready;
+    if (early > items2) early = items2;
     const int pos = c >= extra ? c - extra : n_light + c;
-    auto start_cost = [&](int p) -> long long {
-      return p <= n_light ? (long long)p * bl : (long long)n_light * bl + (long long)(p - n_light) * bh;
+    auto start = [&](int p) -> int {
+      return (int)(early * (p < n_light ? p : n_light) / n_light + (items2 - early) * p / grid);
     };
-    long long lo = (start_cost(pos) + c2 - 1) / c2;
-    long long hi = pos == grid - 1 ? (long long)items2 : (start_cost(pos + 1) + c2 - 1) / c2;
-    if (lo > items2) lo = items2;
-    if (hi > items2) hi = items2;
-    run_phase<2>(&tmW2, &tmH, a, sh, tmem_base, (int)lo, (int)hi, 1);
+    const int lo = start(pos), hi = start(pos + 1);
+    run_phase<2>(&tmW2, &tmH, a, sh, tmem_base, lo, hi, 1);
   }
 
   tc_fence_before();
@@ -734,10 +808,12 @@ UMDK_API int umdk_moe_fused(const UmdkMoeFusedParams* p, void* stream) {
       make_tmap_2d(&tmX, TMAP_U8, p->x, p->H, p->n_rows_cap, p->H, BKB, TT, TMAP_SW_128B) ||
       make_tmap_2d(&tmH, TMAP_U8, p->hq, p->F, p->n_rows_cap, p->F, BKB, TT, TMAP_SW_128B))
     return -UMDK_ERR_BAD_ARG;
+  const size_t smem = 1024 + (size_t)kRingBytes + TT * kTransStride * 4 + kScaleStages * kScaleFloats * 4 + kEpiThreads * 4 +
+                      2 * (size_t)(p->G + 1) * 4 + 16 + 2 * kPhaseBars * 8 + 16;
+  // rows of up to 15616 elements with 32 experts: as long as the scales of a whole row fitted beside the ring
   const int kb_max = (p->H > p->F ? p->H : p->F) / BKB;
-  const size_t smem = 1024 + (size_t)kRingBytes + TT * kTransStride * 4 + (size_t)kb_max * TT * 4 + 2 * kb_max * 4 +
-                      256 * 4 + 2 * (size_t)(p->G + 1) * 4 + 4 + 2 * TT * 4 + 16 + 32 * 8 + 16;
-  if (smem > 227 * 1024) return -UMDK_ERR_BAD_ARG;
+  if (smem > 227 * 1024 || (size_t)kb_max * (TT + 2) * 4 + 2 * (size_t)(p->G + 1) * 4 > 227 * 1024 - 199716)
+    return -UMDK_ERR_BAD_ARG;
   UMDK_CUDA_CHECK(cudaFuncSetAttribute(moe_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int grid = sm_count();
   if (p->max_ctas > 0 && p->max_ctas < grid) grid = p->max_ctas;

@@ -156,18 +156,6 @@ __device__ __forceinline__ Item locate(const int* tile_pref, const int* goff, in
   return it;
 }
 
-// v / (1 + exp(-v)) with the quotient rounded once more through its remainder (Markstein), which gives the rounded division
-// without its branches: 64 divisions a thread took 8 % of MODE 0 of the 256-token
-// tiles. A remainder that is not a number (v or the
-// divisor infinite) leaves the first quotient as it is.
-__device__ __forceinline__ float silu(float v) {
-  const float d = 1.f + __expf(-v);
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
-  const float q = v * r, e = fmaf(-q, d, v);
-  return fmaf(e == e ? e : -0.f, r, q);
-}
-
 // Everything behind the set-up, for 64-token tiles.
 template <int MODE>
 __device__ __forceinline__ void weight_body(uint8_t* smem, const CUtensorMap& tmW, const CUtensorMap& tmX, const MoePairArgs& a,
