@@ -330,11 +330,11 @@ __device__ __forceinline__ void run_phase(const CUtensorMap* tmW, const CUtensor
       // operands' way in and out made 960 cycles in phase 1 and 640 in phase 2.
       auto item = [&](auto hc) {
         constexpr int HC = decltype(hc)::value;
-        uint64_t acc_g[2][HC / 4], acc_u[2][PH == 1 ? HC / 4 : 1];   // [lane half][8-token group, row t / 4 or t / 4 + 8]
+        uint64_t acc_g[2][HC / 4], acc_u[2][HC / 4];   // [lane half][8-token group, row t / 4 or t / 4 + 8]
 #pragma unroll
         for (int c = 0; c < HC / 4; ++c) {
           acc_g[0][c] = acc_g[1][c] = 0;
-          if (PH == 1) acc_u[0][c] = acc_u[1][c] = 0;
+          acc_u[0][c] = acc_u[1][c] = 0;
         }
         for (int kb0 = 0; kb0 < kb_total && ok; kb0 += kScaleKb) {
           if (!mbar_wait(&sfull[ss], sph)) {
@@ -354,35 +354,40 @@ __device__ __forceinline__ void run_phase(const CUtensorMap* tmW, const CUtensor
             }
             tc_fence_after();
             const uint32_t taddr = lane_addr + ts * C::kTmemStageCols + hh * HC;
-            uint32_t rg[2][HC / 2], ru[2][HC / 2];
-            tmem_ld<HC>(taddr, rg);
-            if constexpr (PH == 1) tmem_ld<HC>(taddr + TT, ru);
+            uint32_t r[2][HC / 2];
+            tmem_ld<HC>(taddr, r);
             const float2 wf = reinterpret_cast<const float2*>(sc + kScaleKb * TT)[kb - kb0];
-            const uint64_t wg = pack_f32x2(__float_as_uint(wf.x), __float_as_uint(wf.x));
-            const uint64_t wu = pack_f32x2(__float_as_uint(wf.y), __float_as_uint(wf.y));
             uint64_t x2[HC / 8];
 #pragma unroll
             for (int g = 0; g < HC / 8; ++g)
               x2[g] = *reinterpret_cast<const uint64_t*>(sc + (kb - kb0) * TT + hh * HC + 8 * g + 2 * (lane & 3));
+            auto promote = [&](float wv, uint64_t (*acc)[HC / 4]) {
+              const uint64_t w2 = pack_f32x2(__float_as_uint(wv), __float_as_uint(wv));
+#pragma unroll
+              for (int g = 0; g < HC / 8; ++g) {
+                const uint64_t f = mul_f32x2(x2[g], w2);
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {   // lane half, row
+                  const int i = 4 * g + 2 * (h & 1);
+                  uint64_t& d = acc[h >> 1][2 * g + (h & 1)];
+                  d = fma_f32x2(pack_f32x2(r[h >> 1][i], r[h >> 1][i + 1]), f, d);
+                }
+              }
+            };
             tmem_ld_wait();
+            if constexpr (PH == 1) {
+              // one after the other: with both in flight the registers do not suffice (124 bytes in local memory, phase 1 of 128
+              // tokens, 32 experts, 7168 x 2048: 162 us against 150)
+              promote(wf.x, acc_g);
+              tmem_ld<HC>(taddr + TT, r);
+              tmem_ld_wait();
+            }
             // the accumulator stage is free as soon as its values are in registers
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&tempty[ts]);
-#pragma unroll
-            for (int g = 0; g < HC / 8; ++g) {
-              const uint64_t fg = mul_f32x2(x2[g], wg), fu = mul_f32x2(x2[g], wu);
-#pragma unroll
-              for (int h = 0; h < 4; ++h) {   // lane half, row
-                const int i = 4 * g + 2 * (h & 1);
-                uint64_t& dg = acc_g[h >> 1][2 * g + (h & 1)];
-                dg = fma_f32x2(pack_f32x2(rg[h >> 1][i], rg[h >> 1][i + 1]), fg, dg);
-                if constexpr (PH == 1) {
-                  uint64_t& du = acc_u[h >> 1][2 * g + (h & 1)];
-                  du = fma_f32x2(pack_f32x2(ru[h >> 1][i], ru[h >> 1][i + 1]), fu, du);
-                }
-              }
-            }
+            if constexpr (PH == 1) promote(wf.y, acc_u);
+            else promote(wf.x, acc_g);
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(&sempty[ss]);
