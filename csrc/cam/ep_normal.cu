@@ -36,17 +36,21 @@ constexpr int kEpWarps = kEpThreads / 32;
 // Every warp owns `per_warp` consecutive chunks of 32 tokens and a private histogram in shared memory. 32 (token, k)
 // entries are placed per step: lanes that hold the same expert find each other with a match instruction, take consecutive
 // positions in entry order, and the lowest of them advances the counter. What bounds this is the chain of steps, so the
-// walk goes over K entry groups of a chunk instead of its 32 tokens, and the histograms meet once per CTA (32 warps,
-// 1024 tokens) in shared memory and once over the grid, behind ONE barrier; a single CTA needs none. From two ranks on lane
+// walk goes over K entry groups of a chunk instead of its 32 tokens, and the histograms meet once per CTA in shared memory and
+// once over the cluster or grid, behind ONE barrier; a single CTA needs none. From two ranks on lane
 // r keeps the chunk's ballot of rank r and 32 / R tokens leave per step with a lane for each rank: neither a chain of R
-// dependent steps nor stores R words apart. Measured against the token-by-token walk with a scan over all chunks between
+// dependent steps nor stores R words apart. Measured in CTAs of 32 warps against the token-by-token walk with a scan over all chunks between
 // two barriers: 4096 tokens, top-8 of 256 experts on 1 / 8 / 32 ranks 32.4 / 36.5 / 41.4 -> 22.6 / 26.7 / 32.9 us (a step
 // per rank: 82 on 32); 1024 tokens 21.6 / 25.5 / 35.0 -> 16.2 / 18.0 / 27.0; top-16 27.4 / 30.5 / 38.7 -> 28.4 / 31.2 /
 // 39.1, bound by 16 match instructions in 32 warps of one SM. The ranks of a token come from loads K entries apart up to
 // top-8 (L1 hits, but each touches 32 lines), behind it through shared memory: 1024 tokens, one rank, top-8 16.1 / 17.0 us,
 // top-16 31.9 / 28.9.
+constexpr int kLayoutCluster = 8;
 constexpr int kDirectTopk = 8;
 __host__ __device__ constexpr int layout_rank_words(int K) { return K > kDirectTopk ? ((K + 3) / 4) | 1 : 0; }   // odd: no conflicts
+// kCluster: one chunk per warp and one cluster of several CTAs; what the first pass finds stays in registers until the bases are
+// known. Else the CTAs meet at a grid barrier.
+template <bool kCluster>
 __global__ void __launch_bounds__(kLayoutWarps * 32)
 ep_layout_kernel(const int64_t* __restrict__ topk_idx, int T, int K, int E, int R, int per_warp,
                  int* __restrict__ num_per_expert, int* __restrict__ num_per_rank, uint8_t* __restrict__ in_rank,
@@ -58,7 +62,7 @@ ep_layout_kernel(const int64_t* __restrict__ topk_idx, int T, int K, int E, int 
   const int cols = E + R;
   const int E_local = E / R;
   int* hist = sm_layout + warp * cols;
-  int* s_base = sm_layout + warps * cols;
+  int* s_base = sm_layout + warps * cols;   // at first this CTA's sums, which the others of its cluster read
   // destination rank of every entry of the warp's chunk, one byte each (0xff: none)
   const int rw = layout_rank_words(K);
   uint32_t* rank_words = reinterpret_cast<uint32_t*>(sm_layout + (warps + 1) * cols) + warp * 32 * rw;
@@ -74,10 +78,10 @@ ep_layout_kernel(const int64_t* __restrict__ topk_idx, int T, int K, int E, int 
   if (K > kDirectTopk)
     for (int i = lane; i < 32 * rw; i += 32) rank_words[i] = 0xffffffffu;
   __syncwarp();
+  int ids[kMaxTopk], spot[kMaxTopk], slot = -1;
   for (int c = c_begin; c < c_end; ++c) {
     const int t0 = c * 32;
     const int nt = min(32, T - t0);
-    int ids[kMaxTopk];
 #pragma unroll
     for (int u = 0; u < kMaxTopk; ++u) {
       const int i = u * 32 + lane;
@@ -129,7 +133,8 @@ ep_layout_kernel(const int64_t* __restrict__ topk_idx, int T, int K, int E, int 
       __syncwarp();
       if (e >= 0 && (same & lower) == 0) hist[e] += __popc(same);
       __syncwarp();
-      if (i < nt * K) send_idx[(size_t)t0 * K + i] = pos;   // position among the entries of this warp
+      spot[u] = pos;   // position among the entries of this warp
+      if (!kCluster && i < nt * K) send_idx[(size_t)t0 * K + i] = pos;
     }
     if (R == 1) {
       const uint32_t b = __ballot_sync(0xffffffffu, ranks);
@@ -137,7 +142,8 @@ ep_layout_kernel(const int64_t* __restrict__ topk_idx, int T, int K, int E, int 
       __syncwarp();
       if (lane == 0) hist[E] = first + __popc(b);
       if (lane < nt) {
-        rank_slot[t0 + lane] = ranks ? first + __popc(b & lower) : -1;
+        slot = ranks ? first + __popc(b & lower) : -1;
+        if (!kCluster) rank_slot[t0 + lane] = slot;
         in_rank[t0 + lane] = ranks ? 1 : 0;
       }
     } else {
@@ -178,7 +184,8 @@ ep_layout_kernel(const int64_t* __restrict__ topk_idx, int T, int K, int E, int 
         run += v[u];
       }
     }
-    s_base[col] = 0;
+    s_base[col] = kCluster ? run : 0;
+    if (kCluster) continue;
     if (gridDim.x > 1) {
       scratch[(size_t)blockIdx.x * cols + col] = run;
     } else {
@@ -186,7 +193,32 @@ ep_layout_kernel(const int64_t* __restrict__ topk_idx, int T, int K, int E, int 
       else num_per_rank[col - E] = run;
     }
   }
-  if (gridDim.x > 1) {
+  if constexpr (kCluster) {
+    cluster_sync_all();
+    constexpr int kCols = 2;   // columns of a thread whose base stays in registers until every CTA has read (E + R <= 2 x threads)
+    int base[kCols];
+#pragma unroll
+    for (int u = 0; u < kCols; ++u) {
+      const int col = threadIdx.x + u * blockDim.x;
+      base[u] = 0;
+      if (col >= cols) continue;
+      int v[kLayoutCluster];
+#pragma unroll
+      for (int c = 0; c < kLayoutCluster; ++c)
+        v[c] = c < (int)blockIdx.x ? ld_cluster_u32(map_to_cta(s_base + col, c)) : 0;
+#pragma unroll
+      for (int c = 0; c < kLayoutCluster; ++c) base[u] += v[c];
+      if (blockIdx.x == gridDim.x - 1) {
+        const int run = base[u] + s_base[col];
+        if (col < E) num_per_expert[col] = run;
+        else num_per_rank[col - E] = run;
+      }
+    }
+    cluster_sync_all();
+#pragma unroll
+    for (int u = 0; u < kCols; ++u)
+      if (threadIdx.x + u * blockDim.x < cols) s_base[threadIdx.x + u * blockDim.x] = base[u];
+  } else if (gridDim.x > 1) {
     if (!grid_barrier(bar, gridDim.x)) {
       umdk_set_status(status, UMDK_ERR_TIMEOUT, UMDK_PH_BARRIER, 0, 0);
       return;
@@ -213,12 +245,22 @@ ep_layout_kernel(const int64_t* __restrict__ topk_idx, int T, int K, int E, int 
   for (int c = c_begin; c < c_end; ++c) {
     const int t0 = c * 32;
     const int nt = min(32, T - t0);
+    if (kCluster) {
+#pragma unroll
+      for (int u = 0; u < kMaxTopk; ++u) {
+        const int i = u * 32 + lane;
+        if (u < K && i < nt * K) send_idx[(size_t)t0 * K + i] = ids[u] >= 0 ? spot[u] + hist[ids[u]] + s_base[ids[u]] : -1;
+      }
+    } else {
 #pragma unroll 4
-    for (int i = lane; i < nt * K; i += 32) {
-      const long long e = topk_idx[(size_t)t0 * K + i];
-      if (e >= 0 && e < E) send_idx[(size_t)t0 * K + i] += hist[e] + s_base[e];
+      for (int i = lane; i < nt * K; i += 32) {
+        const long long e = topk_idx[(size_t)t0 * K + i];
+        if (e >= 0 && e < E) send_idx[(size_t)t0 * K + i] += hist[e] + s_base[e];
+      }
     }
-    if (out_t < out_step) {
+    if (kCluster && R == 1) {
+      if (lane < nt) rank_slot[t0 + lane] = slot >= 0 ? slot + hist[E] + s_base[E] : -1;
+    } else if (out_t < out_step) {
       const int base = hist[E + out_r] + s_base[E + out_r];
 #pragma unroll 4
       for (int i = out_t; i < nt; i += out_step) {
@@ -1236,18 +1278,48 @@ static int launch_layout(const int64_t* topk_idx, int T, int K, int E, int R, in
                          uint8_t* in_rank, int* send_idx, int* rank_slot, int* scratch, uint32_t* bar, int* status,
                          cudaStream_t s) {
   const int chunks = (T + 31) / 32;
-  int warps = kLayoutWarps;
   const size_t rank_bytes = 32 * sizeof(uint32_t) * layout_rank_words(K);   // per warp
-  while (warps > 1 && sizeof(int) * (size_t)(warps + 1) * (E + R) + warps * rank_bytes > 200 * 1024) warps /= 2;
-  const size_t smem = sizeof(int) * (size_t)(warps + 1) * (E + R) + warps * rank_bytes;
+  auto smem_of = [&](int warps) { return sizeof(int) * (size_t)(warps + 1) * (E + R) + warps * rank_bytes; };
+  // 385 to 8192 tokens: a cluster of at most eight CTAs of 8, 16 or 32 warps, one chunk per warp. The walk is bound by the match instructions of an SM's warps, and the CTAs meet in the cluster's
+  // barrier and each other's shared memory instead of a grid barrier whose words have to be cleared first. CTAs of 32 warps
+  // at a grid barrier / this, one rank, us: 1003 tokens, top-6 of 64 experts 11.4 / 7.4, 1024, top-8 of 256 16.2 / 9.3, top-16
+  // 28.4 / 13.3, 2000, top-4 of 16 12.5 / 6.1, 4096, top-8 of 256 22.5 / 11.7 (32 ranks 32.9 / 20.7), 8192 22.7 / 18.2; a cluster
+  // of two loses for 300 tokens, top-8 of 64: 7.0 / 8.3.
+  if (chunks > 12) {
+    int warps = 8;
+    while (warps * kLayoutCluster < chunks && warps < 32) warps *= 2;
+    const int grid = (chunks + warps - 1) / warps;
+    if (grid <= kLayoutCluster && E + R <= 64 * warps && smem_of(warps) <= 200 * 1024) {
+      const size_t smem = smem_of(warps);
+      if (smem > 48 * 1024)
+        UMDK_CUDA_CHECK(cudaFuncSetAttribute(ep_layout_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(grid);
+      cfg.blockDim = dim3(warps * 32);
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = s;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = grid;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      UMDK_CUDA_CHECK(cudaLaunchKernelEx(&cfg, ep_layout_kernel<true>, topk_idx, T, K, E, R, 1, num_per_expert, num_per_rank, in_rank,
+                                         send_idx, rank_slot, scratch, bar, status));
+      return 0;
+    }
+  }
+  int warps = kLayoutWarps;
+  while (warps > 1 && smem_of(warps) > 200 * 1024) warps /= 2;
+  const size_t smem = smem_of(warps);
   int grid = (chunks + warps - 1) / warps;
   if (grid > sm_count()) grid = sm_count();
   const int per_warp = (chunks + grid * warps - 1) / (grid * warps);
   if (smem > 48 * 1024) {
-    UMDK_CUDA_CHECK(cudaFuncSetAttribute(ep_layout_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    UMDK_CUDA_CHECK(cudaFuncSetAttribute(ep_layout_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   }
   if (grid > 1) UMDK_CUDA_CHECK(cudaMemsetAsync(bar, 0, 2 * sizeof(uint32_t), s));
-  ep_layout_kernel<<<grid, warps * 32, smem, s>>>(topk_idx, T, K, E, R, per_warp, num_per_expert, num_per_rank, in_rank,
+  ep_layout_kernel<false><<<grid, warps * 32, smem, s>>>(topk_idx, T, K, E, R, per_warp, num_per_expert, num_per_rank, in_rank,
                                                   send_idx, rank_slot, scratch, bar, status);
   UMDK_CUDA_CHECK(cudaGetLastError());
   return 0;

@@ -207,6 +207,14 @@ def test_layout_cta_and_warp_edges(T, K, E, R):
     test_layout_matches_reference(T, K, E, R)
 
 
+# one CTA and one token more, the last CTA of a cluster with one token, clusters of 8, 16 and 32 warps exactly full, more than a
+# cluster takes, more columns than two for every thread of a cluster's CTA
+@pytest.mark.parametrize("T,K,E,R", [(384, 8, 64, 1), (385, 1, 64, 1), (1793, 5, 256, 2), (2048, 16, 64, 4), (2049, 8, 256, 1),
+                                     (4096, 2, 96, 32), (8192, 3, 128, 8), (8193, 2, 64, 1), (500, 2, 511, 1), (500, 2, 512, 1)])
+def test_layout_clusters(T, K, E, R):
+    test_layout_matches_reference(T, K, E, R)
+
+
 @pytest.mark.parametrize("T,H,E,K,quant", [
     (1, 128, 8, 1, True), (33, 2176, 16, 4, True), (300, 7168, 64, 8, True), (33, 2176, 16, 4, False),
     (129, 128, 5, 3, False),
