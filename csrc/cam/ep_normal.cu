@@ -301,6 +301,8 @@ struct DispatchArgs {
                                // index of the first arrival of every source
   volatile int* counts_host;   // same 4 ints in mapped pinned host memory + [4] = epoch stamp (may be null)
   volatile int64_t* per_expert_host;   // optional copy of recv_per_expert in mapped pinned host memory
+  volatile int* status_host;   // one rank, with host_tag: copy of the status record in mapped host memory (may be null)
+  int host_tag;                // one rank: the last CTA sets counts_host[5] to it when everything is in memory (0: nobody waits)
   int n_cap, a_cap;
   // control
   uint32_t* ctrl;              // [0] epoch, [2] recv-done counter, [10] staging gate (tag of the last staged call),
@@ -892,7 +894,17 @@ __global__ void __launch_bounds__(kEpThreads, 1) ep_dispatch_local_kernel(const 
     a.counts_host[4] = (int)(a.ctrl[0] + 1);
   }
   // the epoch advances as in the exchanging kernel, so that the two can follow each other
-  if (cta_done_is_last(&a.ctrl[2], gridDim.x, false) && threadIdx.x == 0) a.ctrl[0] += 1;
+  if (cta_done_is_last(&a.ctrl[2], gridDim.x, false) && threadIdx.x == 0) {
+    a.ctrl[0] += 1;
+    if (a.host_tag != 0 && a.counts_host) {
+      // The host waits for this word (umdk_wait_host_word): no copy of the status record behind the kernel and no wait for
+      // the stream, 10 us of a call. Everything written by the call is ordered before it.
+      if (a.status_host)
+        for (int i = 0; i < 4; ++i) a.status_host[i] = *(volatile int*)(a.status + i);
+      __threadfence_system();
+      a.counts_host[5] = a.host_tag;
+    }
+  }
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -1366,6 +1378,8 @@ struct UmdkEpDispatchParams {
   int64_t* row_expert;        // optional [n_cap] local expert per row (-1 behind the received rows), with
   float* row_weight;          // [n_cap] routing weight per row (0 behind them)
   int64_t* per_expert_host;   // optional [E/R] copy of recv_per_expert in mapped host memory
+  int* status_host;           // optional [4] copy of the status record in mapped host memory, written with the tag
+  int host_tag;               // one rank: counts_host[5] becomes this when everything the call writes is in memory (0: not)
 };
 
 UMDK_API int umdk_ep_dispatch(const UmdkEpDispatchParams* p, void* stream) {
@@ -1399,6 +1413,8 @@ UMDK_API int umdk_ep_dispatch(const UmdkEpDispatchParams* p, void* stream) {
   a.row_expert = p->row_expert;
   a.row_weight = p->row_weight;
   a.per_expert_host = p->per_expert_host;
+  a.status_host = p->status_host;
+  a.host_tag = p->host_tag;
   a.phase_mask = p->phase_mask ? p->phase_mask : 3;
   int grid = p->num_ctas > 0 ? p->num_ctas : sm_count();
   if (grid > sm_count()) grid = sm_count();  // CTAs wait on peers: the whole grid must be resident
@@ -1413,6 +1429,27 @@ UMDK_API int umdk_ep_dispatch(const UmdkEpDispatchParams* p, void* stream) {
   ep_dispatch_kernel<<<grid, kEpThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
   UMDK_CUDA_CHECK(cudaGetLastError());
   return 0;
+}
+
+// Waits until *word (mapped host memory) is `value`, which work on `stream` writes there. 0, or a negative error: the stream is
+// being captured, has failed, or has run dry without writing it.
+UMDK_API int umdk_wait_host_word(const int* word, int value, void* stream) {
+  const cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  UMDK_CUDA_CHECK(cudaStreamIsCapturing(s, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return -(int)cudaErrorStreamCaptureUnsupported;
+  for (;;) {
+    for (int i = 0; i < 4096; ++i) {
+      if (__atomic_load_n(word, __ATOMIC_ACQUIRE) == value) return 0;
+#if defined(__x86_64__)
+      __builtin_ia32_pause();
+#endif
+    }
+    const cudaError_t q = cudaStreamQuery(s);
+    if (q == cudaErrorNotReady) continue;
+    if (q != cudaSuccess) return -(int)q;
+    return __atomic_load_n(word, __ATOMIC_ACQUIRE) == value ? 0 : -UMDK_ERR_TIMEOUT;
+  }
 }
 
 struct UmdkEpCombineParams {

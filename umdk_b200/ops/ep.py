@@ -35,6 +35,7 @@ class _DispatchParams(ctypes.Structure):
         ("counts_dev", ctypes.c_void_p), ("counts_host", ctypes.c_void_p),
         ("ctrl", ctypes.c_void_p), ("status", ctypes.c_void_p), ("diag", ctypes.c_void_p),
         ("row_expert", ctypes.c_void_p), ("row_weight", ctypes.c_void_p), ("per_expert_host", ctypes.c_void_p),
+        ("status_host", ctypes.c_void_p), ("host_tag", ctypes.c_int),
     ]
 
 
@@ -243,7 +244,8 @@ class EpNormal(Recoverable):
         self.layout_scratch = torch.empty(((cap + 31) // 32) * (num_experts + self.R), dtype=torch.int32, device=dev)
         # what the host reads of the last call, in mapped host memory: 8 ints of counts, the rows per local expert (int64) and
         # a copy of the status record
-        n = 8 + 2 * (num_experts // self.R)
+        n = self.status_at = 8 + 2 * (num_experts // self.R)
+        self.tag = 0   # of the last dispatch that the host waited for
         self.mirror = HostMirror(n + 4)
         with torch.inference_mode(False):   # an inference tensor could not be written by a call outside of that mode
             self.status_host = torch.frombuffer(self.mirror.host, dtype=torch.int32)[n:]
@@ -353,15 +355,25 @@ class EpNormal(Recoverable):
         if out.row_expert is not None:
             p.row_expert, p.row_weight = out.row_expert.data_ptr(), out.row_weight.data_ptr()
         p.per_expert_host = self.mirror.dev_ptr + 32
+        wait = sync_counts and bool(phase_mask & 2)
+        local = wait and self.R == 1 and (phase_mask or 3) & 3 == 3
+        if local:   # the kernel says itself when it is through
+            self.tag = self.tag % 0x7ffffffe + 1
+            p.status_host, p.host_tag = self.mirror.dev_ptr + 4 * self.status_at, self.tag
         rc = self.lib.umdk_ep_dispatch(ctypes.byref(p), _native.stream_ptr())
         if rc != 0:
             raise RuntimeError(f"umdk_ep_dispatch failed: {rc}")
-        if sync_counts and (phase_mask & 2):
+        if wait:
             # one wait for everything the host reads: the counts lie in mapped memory, the status record comes along
-            self.status_host.copy_(self.status, non_blocking=True)
-            torch.cuda.current_stream().synchronize()
-            _raise_status(self.status_host.tolist(), self.status, "ep_dispatch", owner=self)
             host = self.mirror.host
+            if local:
+                rc = self.lib.umdk_wait_host_word(ctypes.byref(host, 20), self.tag, _native.stream_ptr())
+                if rc != 0:
+                    raise RuntimeError(f"waiting for the dispatch failed: {rc}")
+            else:
+                self.status_host.copy_(self.status, non_blocking=True)
+                torch.cuda.current_stream().synchronize()
+            _raise_status(host[self.status_at:], self.status, "ep_dispatch", owner=self)
             out.num_recv = int(host[0])
             out.per_expert = host[8:8 + 2 * (self.E // self.R):2]   # low words: counts are far below 2^31
         return out
