@@ -77,6 +77,25 @@ def _targets():
                 out=LIB / "libumdk_cam_torch.so")
         except Exception:   # no torch in this interpreter: the Python package then registers the schemas itself
             pass
+    # call path from Python to the short kernels (a CPython module)
+    pc = sorted((CSRC / "pycalls").glob("*.cpp"))
+    if pc:
+        try:
+            import sysconfig
+            import torch
+            from torch.utils import cpp_extension as _ce
+            cuda = Path(NVCC).resolve().parent.parent
+            tlib = Path(torch.__file__).resolve().parent / "lib"
+            t["umdk_calls"] = dict(
+                kind="cxx_shared", sources=pc,
+                includes=[CSRC / "cam", *(Path(p) for p in _ce.include_paths()), Path(sysconfig.get_paths()["include"]),
+                          cuda / "include"],
+                cxxflags=["-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), "-Wno-attributes"],
+                libs=["-L" + str(LIB), "-Wl,-rpath,$ORIGIN", "-lumdk_cam", "-L" + str(tlib), "-Wl,-rpath," + str(tlib),
+                      "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10_cuda", "-lc10"],
+                deps=["umdk_cam"], out=LIB / "umdk_calls.so")
+        except ImportError:   # no torch in this interpreter: nothing to call from
+            pass
     pre = CSRC / "usock" / "ums_preload.cpp"
     if pre.exists():
         t["ums_preload"] = dict(kind="cxx_shared", sources=[pre], includes=[CSRC / "usock", CSRC / "common"],
@@ -141,7 +160,7 @@ def build_all(force: bool = False, verbose: bool = False, only=None) -> dict:
     OBJ.mkdir(parents=True, exist_ok=True)
     targets = _targets()
     order = ["umdk_cam", "umdk_urma", "urma_cuda_ipc", "umdk_umq", "umdk_usock", "umdk_dlock", "umdk_urpc",
-             "ums_preload", "umdk_cam_torch"]
+             "ums_preload", "umdk_cam_torch", "umdk_calls"]
     order += [n for n in targets if n.startswith("tool_")]
     outs = {}
     # compile all objects of all targets in parallel first

@@ -81,6 +81,31 @@ def cam():
     return _cam_proxy
 
 
+_calls = None
+
+
+def calls():
+    """The CPython module behind the operators whose kernels last microseconds (csrc/pycalls/calls.cpp). The caller counts
+    its kernels in LAUNCH_COUNT."""
+    global _calls
+    if _calls is None:
+        import importlib.util
+        import torch  # noqa: F401  (its libraries, before the module that is linked against them)
+        cam()
+        path = _LIB_DIR / "umdk_calls.so"
+        if not path.exists():
+            if os.environ.get("UMDK_AUTO_BUILD", "1") == "1":
+                from . import _build
+                _build.build_all(only=["umdk_cam", "umdk_calls"])
+            if not path.exists():
+                raise NativeLibraryMissing(f"{path} not built; run `python -m umdk_b200._build`")
+        spec = importlib.util.spec_from_file_location("umdk_calls", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _calls = module
+    return _calls
+
+
 def urma() -> ctypes.CDLL:
     return _load("umdk_urma", "umdk_urma")
 

@@ -2,7 +2,6 @@
 CTAs per (sequence, key-list split), the feature dimensions divided between them."""
 from __future__ import annotations
 
-import ctypes
 import functools
 from typing import Optional, Tuple
 
@@ -15,6 +14,7 @@ DIM = 576
 DIM_V = 512
 PAGE = 64
 CHUNK = 48   # keys per step of the kernel; a split takes whole chunks
+MAX_KEYS = 43 * CHUNK   # of a split
 
 
 @functools.lru_cache(maxsize=None)
@@ -51,38 +51,21 @@ def sparse_mla_decode(q: torch.Tensor, kv_pages: torch.Tensor, block_table: torc
     puts a CTA pair on every SM with one).
     ``diag`` (int64 [16], device): the first CTA records how many cycles its roles spent in each of their waits and
     work sections (see MlaArgs::diag in the kernel source); for finding what bounds the pipeline."""
-    lib = _native.cam()
     assert q.is_cuda and q.dtype == torch.bfloat16 and q.is_contiguous() and q.shape[1:] == (HEADS, DIM)
     assert kv_pages.dtype == torch.bfloat16 and kv_pages.is_contiguous() and kv_pages.shape[1:] == (PAGE, DIM)
     assert block_table.dtype == torch.int32 and indices.dtype == torch.int32
     assert block_table.is_contiguous() and indices.is_contiguous()
     B = q.shape[0]
     topk = indices.shape[1]
-    dev = q.device
-    if out is None:
-        out = torch.empty(B, HEADS, DIM_V, dtype=torch.bfloat16, device=dev)
-    lse = torch.empty(B, HEADS, dtype=torch.float32, device=dev)
-    if status is None:
-        status = torch.zeros(4, dtype=torch.int32, device=dev)
     # one CTA pair resolves at most 2064 selected rows up front: longer key lists need more splits
-    least = int(lib.umdk_sparse_mla_min_splits(topk))
-    num_splits = max(num_splits, least) if num_splits > 0 else default_splits(B, topk, _sm_count(dev.index), least)
-    if workspace is not None and workspace[0].shape[1] != num_splits:
+    least = -(-topk // MAX_KEYS)
+    num_splits = max(num_splits, least) if num_splits > 0 else default_splits(B, topk, _sm_count(q.device.index), least)
+    if workspace is not None and (num_splits == 1 or workspace[0].shape[1] != num_splits):
         workspace = None
-    po = pl = None
-    if num_splits > 1:
-        if workspace is None:
-            workspace = (torch.empty(B, num_splits, HEADS, DIM_V, dtype=torch.float32, device=dev),
-                         torch.empty(B, num_splits, HEADS, dtype=torch.float32, device=dev))
-        po, pl = workspace
-    rc = lib.umdk_sparse_mla_decode(
-        _native.ptr(q), _native.ptr(kv_pages), _native.ptr(block_table), _native.ptr(indices),
-        _native.ptr(seq_lens), _native.ptr(out), _native.ptr(lse), _native.ptr(po), _native.ptr(pl),
-        B, topk, block_table.shape[1], kv_pages.shape[0], num_splits, ctypes.c_float(sm_scale),
-        _native.ptr(status), _native.stream_ptr(), _native.ptr(diag))
-    if rc != 0:
-        raise RuntimeError(f"umdk_sparse_mla_decode failed: {rc}")
-    return out, lse
+    po, pl = workspace if workspace is not None else (None, None)
+    _native.LAUNCH_COUNT += 1
+    return _native.calls().sparse_mla_decode(q, kv_pages, block_table, indices, sm_scale, seq_lens, num_splits, out, status, po, pl,
+                                             diag)
 
 
 def ref_sparse_mla_decode(q, kv_pages, block_table, indices, sm_scale, seq_lens=None):

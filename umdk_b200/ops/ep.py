@@ -154,7 +154,6 @@ class LayoutResult:
     send_token_idx: torch.Tensor
     rank_slot: torch.Tensor
 
-
 @dataclass
 class NotifyResult:
     """What a rank learns from the count exchange before any token moves (the outputs of the reference's
@@ -195,16 +194,6 @@ def layout(topk_idx: torch.Tensor, num_experts: int, num_ranks: int, scratch=Non
     T, K = topk_idx.shape
     dev = topk_idx.device
     E, R = num_experts, num_ranks
-    if out is not None:
-        npe, npr, sidx, rslot = out.num_tokens_per_expert, out.num_tokens_per_rank, out.send_token_idx, out.rank_slot
-        inr = out.is_token_in_rank.view(torch.uint8)
-        assert sidx.shape == (T, K) and rslot.shape == (T, R) and npe.numel() == E
-    else:
-        npe = torch.empty(E, dtype=torch.int32, device=dev)
-        npr = torch.empty(R, dtype=torch.int32, device=dev)
-        inr = torch.empty(T, R, dtype=torch.uint8, device=dev)
-        sidx = torch.empty(T, K, dtype=torch.int32, device=dev)
-        rslot = torch.empty(T, R, dtype=torch.int32, device=dev)
     chunks = (T + 31) // 32
     if scratch is None or scratch.numel() < max(1, chunks) * (E + R):
         scratch = torch.empty(max(1, chunks) * (E + R), dtype=torch.int32, device=dev)
@@ -212,12 +201,18 @@ def layout(topk_idx: torch.Tensor, num_experts: int, num_ranks: int, scratch=Non
         bar = torch.zeros(2, dtype=torch.int32, device=dev)
     if status is None:
         status = torch.zeros(4, dtype=torch.int32, device=dev)
+    if out is None:
+        _native.LAUNCH_COUNT += 1
+        return LayoutResult(*_native.calls().ep_layout(topk_idx, E, R, scratch, bar, status))
+    npe, npr, sidx, rslot = out.num_tokens_per_expert, out.num_tokens_per_rank, out.send_token_idx, out.rank_slot
+    inr = out.is_token_in_rank.view(torch.uint8)
+    assert sidx.shape == (T, K) and rslot.shape == (T, R) and npe.numel() == E
     rc = lib.umdk_ep_layout(_native.ptr(topk_idx), T, K, E, R, _native.ptr(npe), _native.ptr(npr), _native.ptr(inr),
                             _native.ptr(sidx), _native.ptr(rslot), _native.ptr(scratch), _native.ptr(bar),
                             _native.ptr(status), _native.stream_ptr())
     if rc != 0:
         raise RuntimeError(f"umdk_ep_layout failed: {rc}")
-    return out if out is not None else LayoutResult(npe, npr, inr.view(torch.bool), sidx, rslot)
+    return out
 
 
 class EpNormal(Recoverable):
@@ -255,6 +250,18 @@ class EpNormal(Recoverable):
         self.diagnose = False
         self.diag_dispatch = torch.zeros(self.R, dtype=torch.int64, device=dev)
         self.diag_combine = torch.zeros(self.R, dtype=torch.int64, device=dev)
+
+        # what never changes of the argument blocks
+        p, c = _DispatchParams(), _CombineParams()
+        for b in (p, c):
+            b.R, b.rank, b.E, b.K, b.H, b.cap = self.R, self.rank, num_experts, top_k, hidden, cap
+            for i, pp in enumerate(heap.peer_ptrs):
+                b.peers[i] = pp
+            b.ctrl, b.status = self.ctrl.data_ptr(), self.status.data_ptr()
+        p.counts_host, p.per_expert_host = self.mirror.dev_ptr, self.mirror.dev_ptr + 32
+        p.status_host = self.mirror.dev_ptr + 4 * self.status_at
+        self._dispatch_params, self._combine_params = p, c
+        self._dispatch_base, self._combine_base = ctypes.addressof(p), ctypes.addressof(c)
 
     def wait_times_us(self):
         """(dispatch, combine) wait time per source rank in microseconds from the last diagnosed calls."""
@@ -314,55 +321,42 @@ class EpNormal(Recoverable):
         K = self.K
         if lay is None:
             lay = out.layout if out is not None else self.layout(topk_idx)
-        if out is None:
-            n_cap = n_cap if n_cap is not None else self.R * self.cap * min(K, self.E // self.R)
-            a_cap = a_cap if a_cap is not None else self.R * self.cap
-            dev = x.device
-            if quant:
-                recv_x = torch.empty(n_cap, H, dtype=torch.uint8, device=dev).view(torch.float8_e4m3fn)
-                recv_s = torch.empty(n_cap, H // 128, dtype=torch.float32, device=dev)
-            else:
-                recv_x = torch.empty(n_cap, H, dtype=torch.bfloat16, device=dev)
-                recv_s = None
-            out = DispatchResult(
-                recv_x, recv_s, torch.empty(n_cap, 3, dtype=torch.int32, device=dev),
-                torch.empty(self.E, dtype=torch.int32, device=dev),
-                torch.empty(self.E // self.R, dtype=torch.int64, device=dev),
-                torch.empty(a_cap, 2 * K + 2, dtype=torch.int32, device=dev),
-                torch.empty(4 + MAX_RANKS, dtype=torch.int32, device=dev), lay, topk_idx, topk_weights, T, quant)
-            if row_info:
-                out.row_expert = torch.empty(n_cap, dtype=torch.int64, device=dev)
-                out.row_weight = torch.empty(n_cap, dtype=torch.float32, device=dev)
-        elif self.R == 1 and (phase_mask or 3) & 3 == 3 and overlap(x, out.recv_x):
-            x = x.clone()   # one rank stores its rows while other tokens are still read
-        p = _DispatchParams()
-        p.R, p.rank, p.E, p.K, p.H, p.cap, p.quant, p.T = self.R, self.rank, self.E, K, H, self.cap, int(quant), T
-        p.n_cap, p.a_cap = out.recv_x.shape[0], out.recv_meta.shape[0]
-        p.num_ctas, p.phase_mask = self.num_ctas, phase_mask
-        for i, pp in enumerate(self.heap.peer_ptrs):
-            p.peers[i] = pp
-        p.x, p.topk_idx = x.data_ptr(), topk_idx.data_ptr()
-        p.topk_w = topk_weights.data_ptr() if topk_weights is not None else None
-        p.send_idx, p.rank_slot = lay.send_token_idx.data_ptr(), lay.rank_slot.data_ptr()
-        p.num_per_expert, p.num_per_rank = lay.num_tokens_per_expert.data_ptr(), lay.num_tokens_per_rank.data_ptr()
-        p.recv_x = out.recv_x.data_ptr()
-        p.recv_scales = out.recv_scales.data_ptr() if out.recv_scales is not None else None
-        p.expand_idx, p.recv_count = out.expand_idx.data_ptr(), out.recv_count.data_ptr()
-        p.recv_per_expert, p.recv_meta = out.recv_tokens_per_expert.data_ptr(), out.recv_meta.data_ptr()
-        p.counts_dev, p.counts_host = out.counts.data_ptr(), self.mirror.dev_ptr
-        p.ctrl, p.status = self.ctrl.data_ptr(), self.status.data_ptr()
-        p.diag = self.diag_dispatch.data_ptr() if self.diagnose else None
-        if out.row_expert is not None:
-            p.row_expert, p.row_weight = out.row_expert.data_ptr(), out.row_weight.data_ptr()
-        p.per_expert_host = self.mirror.dev_ptr + 32
         wait = sync_counts and bool(phase_mask & 2)
         local = wait and self.R == 1 and (phase_mask or 3) & 3 == 3
         if local:   # the kernel says itself when it is through
             self.tag = self.tag % 0x7ffffffe + 1
-            p.status_host, p.host_tag = self.mirror.dev_ptr + 4 * self.status_at, self.tag
-        rc = self.lib.umdk_ep_dispatch(ctypes.byref(p), _native.stream_ptr())
-        if rc != 0:
-            raise RuntimeError(f"umdk_ep_dispatch failed: {rc}")
+        tag = self.tag if local else 0
+        diag = self.diag_dispatch if self.diagnose else None
+        if out is None:
+            n_cap = n_cap if n_cap is not None else self.R * self.cap * min(K, self.E // self.R)
+            a_cap = a_cap if a_cap is not None else self.R * self.cap
+            _native.LAUNCH_COUNT += 1
+            rx, rs, expand, count, per_expert, meta, counts, row_expert, row_weight = _native.calls().ep_dispatch(
+                self._dispatch_base, x, topk_idx, topk_weights, lay.send_token_idx, lay.rank_slot, lay.num_tokens_per_expert,
+                lay.num_tokens_per_rank, quant, n_cap, a_cap, row_info, self.num_ctas, phase_mask, tag, diag)
+            out = DispatchResult(rx, rs, expand, count, per_expert, meta, counts, lay, topk_idx, topk_weights, T, quant, None,
+                                 row_expert, row_weight)
+        else:
+            if self.R == 1 and (phase_mask or 3) & 3 == 3 and overlap(x, out.recv_x):
+                x = x.clone()   # one rank stores its rows while other tokens are still read
+            p = _DispatchParams.from_buffer_copy(self._dispatch_params)
+            p.quant, p.T, p.n_cap, p.a_cap = int(quant), T, out.recv_x.shape[0], out.recv_meta.shape[0]
+            p.num_ctas, p.phase_mask, p.host_tag = self.num_ctas, phase_mask, tag
+            p.x, p.topk_idx = x.data_ptr(), topk_idx.data_ptr()
+            p.topk_w = topk_weights.data_ptr() if topk_weights is not None else None
+            p.send_idx, p.rank_slot = lay.send_token_idx.data_ptr(), lay.rank_slot.data_ptr()
+            p.num_per_expert, p.num_per_rank = lay.num_tokens_per_expert.data_ptr(), lay.num_tokens_per_rank.data_ptr()
+            p.recv_x = out.recv_x.data_ptr()
+            p.recv_scales = out.recv_scales.data_ptr() if out.recv_scales is not None else None
+            p.expand_idx, p.recv_count = out.expand_idx.data_ptr(), out.recv_count.data_ptr()
+            p.recv_per_expert, p.recv_meta = out.recv_tokens_per_expert.data_ptr(), out.recv_meta.data_ptr()
+            p.counts_dev = out.counts.data_ptr()
+            p.diag = diag.data_ptr() if diag is not None else None
+            if out.row_expert is not None:
+                p.row_expert, p.row_weight = out.row_expert.data_ptr(), out.row_weight.data_ptr()
+            rc = self.lib.umdk_ep_dispatch(ctypes.byref(p), _native.stream_ptr())
+            if rc != 0:
+                raise RuntimeError(f"umdk_ep_dispatch failed: {rc}")
         if wait:
             # one wait for everything the host reads: the counts lie in mapped memory, the status record comes along
             host = self.mirror.host
@@ -385,26 +379,14 @@ class EpNormal(Recoverable):
         self._guard()
         assert y.is_cuda and y.dtype == torch.bfloat16 and y.is_contiguous() and y.shape[1] == self.H
         T = disp.num_tokens
-        if out is None:
-            out = torch.empty(T, self.H, dtype=torch.bfloat16, device=y.device)
-        elif self.R == 1 and (phase_mask or 3) & 3 == 3 and overlap(out, y):
+        if out is not None and self.R == 1 and (phase_mask or 3) & 3 == 3 and overlap(out, y):
             # one rank stores each sum while others are still formed: not into the rows they are formed from
             out.as_strided((T, self.H), (self.H, 1)).copy_(self.combine(y, disp, apply_weights))
             return out
-        p = _CombineParams()
-        p.R, p.rank, p.E, p.K, p.H, p.cap, p.T = self.R, self.rank, self.E, self.K, self.H, self.cap, T
-        p.mode, p.apply_weights, p.n_rows, p.a_cap = 0, int(apply_weights), y.shape[0], disp.recv_meta.shape[0]
-        p.num_ctas, p.phase_mask = self.num_ctas, phase_mask
-        for i, pp in enumerate(self.heap.peer_ptrs):
-            p.peers[i] = pp
-        p.y, p.recv_meta, p.counts_dev = y.data_ptr(), disp.recv_meta.data_ptr(), disp.counts.data_ptr()
-        p.in_rank = disp.layout.is_token_in_rank.data_ptr()
-        p.out, p.ctrl, p.status = out.data_ptr(), self.ctrl.data_ptr(), self.status.data_ptr()
-        p.diag = self.diag_combine.data_ptr() if self.diagnose else None
-        rc = self.lib.umdk_ep_combine(ctypes.byref(p), _native.stream_ptr())
-        if rc != 0:
-            raise RuntimeError(f"umdk_ep_combine failed: {rc}")
-        return out
+        _native.LAUNCH_COUNT += 1
+        return _native.calls().ep_combine(self._combine_base, y, disp.recv_meta, disp.counts, disp.layout.is_token_in_rank, T,
+                                          apply_weights, self.num_ctas, phase_mask, out,
+                                          self.diag_combine if self.diagnose else None)
 
     @_trace.traced("umdk.ep.combine_rows")
     def combine_rows(self, y: torch.Tensor, src_idx: torch.Tensor, topk_idx: torch.Tensor,
