@@ -355,7 +355,7 @@ static int tile_columns(int mode, int R, int Ts, int N, int K, int phase_mask, i
   for (int i = 0; i < 3; ++i) {
     const int bn = 256 >> i;
     const long waves = (rows * (N / bn) + pairs - 1) / pairs, t = waves * (K / BK) * step[i] + ends[i];
-    if (i == 0 || t < least) {
+    if (i == 0 || t + t / 20 < least) {   // 5 %: at equal times the wider tiles read less
       least = t;
       best = bn;
     }
