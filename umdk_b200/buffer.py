@@ -109,7 +109,7 @@ class Buffer:
         if key not in self._ll:
             nbytes = EpLowLatency.heap_bytes(self.group_size, E, K, H, T)
             heap = SymmetricHeap(nbytes, self.group) if self.group_size > 1 else SymmetricHeap(nbytes)
-            self._ll[key] = (heap, EpLowLatency(heap, E, K, H, F, T))
+            self._ll[key] = (heap, EpLowLatency(heap, E, K, H, F, T, dispatch_ctas=0))
         return self._ll[key][1]
 
     def destroy(self):
