@@ -15,9 +15,10 @@
 //   runs the online softmax (one head per thread; both CTAs arrive at the same P),
 //   and accumulates its own 256 output columns O[128 x 256] += P[128 x 48] * V[48 x own latent dims]  (3 MMAs),
 //   reading V from the SAME gathered tile through an MN-major descriptor.
-// Splitting by dimension halves the resident Q (80 KB instead of 144 KB), which makes room for a three-stage ring
-// of key tiles, and halves the Q*K^T work of each SM. Q moves to TMEM before the first chunk and P never leaves it: both
-// are A operands read out of TMEM, so that shared memory (128 bytes a clock) only feeds the key tiles to the MMAs.
+// Splitting by dimension halves the resident Q (80 KB instead of 144 KB), which makes room for a ring of key tiles, and
+// halves the Q*K^T work of each SM. Q moves to TMEM before the first chunk and P never leaves it: both are A operands read
+// out of TMEM, so that shared memory (128 bytes a clock) only feeds the key tiles to the MMAs; one of the four stages of the
+// ring lies where Q was.
 // TMEM columns: two S buffers of 48 (P takes the first 24 of its S), Q 160, O 256. Roles inside a CTA (20 warps):
 //   warps 0-7  softmax in two sets of four (half of a chunk's keys each): tcgen05.ld of S, add the partner's partial,
 //              common maximum of the sets, exp2, P to TMEM, lazy rescale of O
@@ -30,9 +31,15 @@
 //              48-key tiles of 640-byte pieces from 128 CTAs take 96 us for 2048 keys out of one warp, 57 us out of two,
 //              45 us out of four or more (3.7 TB/s of random 640-byte reads; 22 bytes per SM and clock when they hit
 //              L2). Gathering with 16-byte cp.async reaches the same 15 - 19 bytes with 16 warps, plain loads half of it.
-// What bounds it now: the softmax chain of a chunk (about 2600 cycles with its waits, the exp2 part 1240 of them), next
-// to 1600 cycles of DRAM time for the rows and some 1200 of MMAs. Batch 64, 2048 of 32768 keys: 94 -> 79 us; Q as an A
-// operand in shared memory alone kept one thread issuing MMAs for 2240 cycles a chunk.
+// What bounds it now: the softmax chain of a chunk (about 2600 cycles with its waits, the exp2 part 1250 of them), next
+// to 1600 cycles of DRAM time for the rows and some 1200 of MMAs. Every wait in it costs 250 - 500 cycles although its
+// barrier is complete by then (counted): barriers, the partials on their way to the partner and the gathers' issue share the
+// shared-memory queue. Batch 64, 2048 of 32768 keys: 94 -> 79 us; Q as an A operand in shared memory alone kept one thread
+// issuing MMAs for 2240 cycles a chunk. Three stages and a wait for the previous P * V in every chunk / three and a wait only where O
+// is rescaled / four / five (rows not in L2): 64 x 2048 keys 77.6 / 75.9 / 73.9 / 73.9 us, 23 x 1000 in three splits 35.0 / 34.8 /
+// 34.8 / 35.7 (copies that run further ahead keep the first tiles waiting). Tried and left out:
+// a second exchange buffer (73.6), partials sent by bulk copies out of a sending buffer (79.7), the merge launched while the
+// splits run (1 x 2048 18.9 / 18.7, 23 x 1000 30.3 / 31.4).
 // All row addresses of the split are resolved once, up front, into shared memory (index -> page -> row).
 // The running maximum is only raised when it grows by more than 8 (in log2 units); P then stays below 2^8 and the
 // accumulated O needs rescaling only a few times per row instead of in most chunks.
@@ -49,7 +56,8 @@ constexpr int kDim = 576;
 constexpr int kDimV = 512;
 constexpr int kPage = 64;
 constexpr int kChunk = 48;                       // keys per pipeline step
-constexpr int kStages = 3;
+constexpr int kStages = 4;
+constexpr int kFreeStages = 3;   // the last one lies where Q is until it has moved to TMEM
 constexpr int kMaxSlabs = 5;                     // 64-dim slabs per CTA: 4 latent (+ 1 rope in CTA 0)
 constexpr int kQSlabBytes = kHeads * 128;        // 16 KB
 constexpr int kKSlabBytes = kChunk * 128;        // 6 KB
@@ -72,14 +80,16 @@ constexpr int kColS = 0;                         // two S buffers of kChunk colu
 constexpr int kColQ = 2 * kChunk;                // Q as bf16 pairs, 32 columns per 64-dim slab
 constexpr int kColO = 256;
 static_assert(kColQ + kMaxSlabs * 32 <= kColO, "TMEM budget");
-constexpr int kOffK = kQBytes;
-constexpr int kOffX = kOffK + kStages * kStageBytes;
+constexpr int kOffK = 0;
+constexpr int kOffQ = kFreeStages * kStageBytes;
+constexpr int kOffX = kOffQ + kQBytes;
 constexpr int kOffRows = kOffX + kXBytes;
 constexpr int kOffMask = kOffRows + kMaxKeys * 4;   // one 64-bit validity mask per chunk
 constexpr int kOffMax = kOffMask + ((kMaxChunks * 8 + 63) / 64) * 64;   // [2][kSets][128] chunk maxima of the sets
 constexpr int kOffTail = kOffMax + 2 * kSets * kHeads * 4;
 constexpr int kSmemBytes = 1024 + kOffTail + 256;
 static_assert(kSmemBytes <= 232448, "shared memory budget");
+static_assert(kStages * kStageBytes <= kOffX, "the stages end in Q's memory");
 static_assert(kStageBytes % 1024 == 0 && kKSlabBytes % 1024 == 0, "swizzle atoms must stay 1024-byte aligned");
 
 struct MlaArgs {
@@ -187,7 +197,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
                          const MlaArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* q_sm = smem;
+  uint8_t* q_sm = smem + kOffQ;
   uint8_t* k_sm = smem + kOffK;
   float* x_sm = reinterpret_cast<float*>(smem + kOffX);
   int* rows_sm = reinterpret_cast<int*>(smem + kOffRows);
@@ -199,16 +209,16 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   // barrier sees 4 arrivals per phase instead of 128 (128 arrivals on one barrier, remote ones above all, cost
   // more than the work they guard).
   uint64_t* bar_full = bars + 1;     // kStages, one arrival that expects the tile's bytes from the TMA gathers
-  uint64_t* bar_empty = bars + 4;    // kStages, one commit
-  uint64_t* bar_s = bars + 7;        // 2, one commit
-  uint64_t* bar_xld = bars + 9;      // 2, 4 exchange-warp arrivals: they have read this S buffer, P may take its place
-  uint64_t* bar_p = bars + 11;       // 8 softmax-warp arrivals
-  uint64_t* bar_o = bars + 12;       // one commit
-  uint64_t* bar_xfull = bars + 13;   // one local arrival that expects the 24 KB the partner's st.async stores deliver
-  uint64_t* bar_xfree = bars + 14;   // 8 arrivals from the partner's softmax warps: its X may be overwritten
-  uint64_t* bar_fin = bars + 15;     // one commit (drain on the abort path)
-  uint64_t* bar_qt = bars + 16;      // 8 softmax-warp arrivals: Q is in TMEM
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
+  uint64_t* bar_empty = bar_full + kStages;    // kStages, one commit
+  uint64_t* bar_s = bar_empty + kStages;       // 2, one commit
+  uint64_t* bar_xld = bar_s + 2;     // 2, 4 exchange-warp arrivals: they have read this S buffer, P may take its place
+  uint64_t* bar_p = bar_s + 4;       // 8 softmax-warp arrivals
+  uint64_t* bar_o = bar_s + 5;       // one commit
+  uint64_t* bar_xfull = bar_s + 6;   // one local arrival that expects the 24 KB the partner's st.async stores deliver
+  uint64_t* bar_xfree = bar_s + 7;   // 8 arrivals from the partner's softmax warps: its X may be overwritten
+  uint64_t* bar_fin = bar_s + 8;     // one commit (drain on the abort path)
+  uint64_t* bar_qt = bar_s + 9;      // 8 softmax-warp arrivals: Q is in TMEM
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_s + 10);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -415,8 +425,10 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       }
       l_run = l_run * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));   // of this set's keys
       lap(5);
-      // P(c) overwrites P(c-1) and O may be rescaled: P(c-1) * V must have finished
-      if (c >= 1) {
+      // O is rescaled only when P(c-1) * V has finished (P(c-2) * V has: S(c) was made behind it). P(c) itself goes into the
+      // other buffer than P(c-1), and its product queues up behind that one.
+      const bool scale_o = c >= 1 && __any_sync(0xffffffffu, alpha != 1.f);
+      if (scale_o) {
         ok = __all_sync(0xffffffffu, wait_bar<false>(bar_o, (c - 1) & 1, s_abort));
         if (!ok) {
           give_up(UMDK_PH_TMEM_EMPTY, c);
@@ -431,7 +443,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       }
       lap(6);
       tc_fence_after();
-      if (c >= 1 && __any_sync(0xffffffffu, alpha != 1.f)) {
+      if (scale_o) {
 #pragma unroll 1
         for (int c0 = set * 128; c0 < set * 128 + 128; c0 += 32) {   // each set scales its half of the columns
           uint32_t o[32];
@@ -650,6 +662,13 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     const int n_inst = (kChunk / 4) * n_slabs;   // gather4 copies per tile
     for (int c = 0; c < num_chunks && ok; ++c) {
       const int st = c % kStages;
+      if (c == kFreeStages) {   // from here on in Q's memory
+        ok = __all_sync(0xffffffffu, wait_bar<false>(bar_qt, 0, s_abort));
+        if (!ok) {
+          if (lane == 0) give_up(UMDK_PH_TMA_EMPTY, 4000);
+          break;
+        }
+      }
       if (c >= kStages) {
         ok = __all_sync(0xffffffffu, wait_bar<false>(&bar_empty[st], ((c / kStages) - 1) & 1, s_abort));
         if (!ok) {

@@ -82,6 +82,13 @@ def test_sparse_mla_decode_chunk_edges(B, topk, splits, kind):
     assert torch.allclose(lse.cpu()[ok], want_lse[ok], atol=2e-2, rtol=1e-3)
 
 
+# chunks around the stages of the ring: the first stages, those in the memory that Q leaves, and their second use
+@pytest.mark.parametrize("topk", [144, 145, 192, 193, 240, 241, 288, 481, 529])
+@pytest.mark.parametrize("kind", ["plain", "growing"])
+def test_sparse_mla_decode_stage_edges(topk, kind):
+    test_sparse_mla_decode_chunk_edges(2, topk, 1, kind)
+
+
 @pytest.mark.parametrize("B,topk,splits,live", [(2, 1000, 10, 7), (1, 100, 13000, 3), (2, 40, 4, 1)])
 def test_sparse_mla_decode_splits_without_keys(B, topk, splits, live):
     """Splits take whole chunks of keys, so the last ones may have none: their part of the scratch is neither needed nor read,
