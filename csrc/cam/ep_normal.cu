@@ -1293,11 +1293,11 @@ static int launch_layout(const int64_t* topk_idx, int T, int K, int E, int R, in
   const int chunks = (T + 31) / 32;
   const size_t rank_bytes = 32 * sizeof(uint32_t) * layout_rank_words(K);   // per warp
   auto smem_of = [&](int warps) { return sizeof(int) * (size_t)(warps + 1) * (E + R) + warps * rank_bytes; };
-  // 385 to 8192 tokens: a cluster of at most eight CTAs of 8, 16 or 32 warps, one chunk per warp. The walk is bound by the match instructions of an SM's warps, and the CTAs meet in the cluster's
-  // barrier and each other's shared memory instead of a grid barrier whose words have to be cleared first. CTAs of 32 warps
-  // at a grid barrier / this, one rank, us: 1003 tokens, top-6 of 64 experts 11.4 / 7.4, 1024, top-8 of 256 16.2 / 9.3, top-16
-  // 28.4 / 13.3, 2000, top-4 of 16 12.5 / 6.1, 4096, top-8 of 256 22.5 / 11.7 (32 ranks 32.9 / 20.7), 8192 22.7 / 18.2; a cluster
-  // of two loses for 300 tokens, top-8 of 64: 7.0 / 8.3.
+  // 385 to 8192 tokens: a cluster of at most eight CTAs of 8, 16 or 32 warps, one chunk per warp. The walk is bound by the match
+  // instructions of an SM's warps, and the CTAs meet in the cluster's barrier and each other's shared memory instead of a grid
+  // barrier whose words have to be cleared first. CTAs of 32 warps at a grid barrier / this, one rank, us: 1003 tokens, top-6
+  // of 64 experts 11.4 / 7.4, 1024, top-8 of 256 16.2 / 9.3, top-16 28.4 / 13.3, 2000, top-4 of 16 12.5 / 6.1, 4096, top-8 of
+  // 256 22.5 / 11.7 (32 ranks 32.9 / 20.7), 8192 22.7 / 18.2; a cluster of two loses for 300 tokens, top-8 of 64: 7.0 / 8.3.
   if (chunks > 12) {
     int warps = 8;
     while (warps * kLayoutCluster < chunks && warps < 32) warps *= 2;

@@ -64,6 +64,11 @@ struct Args {
     if (v == -1 && PyErr_Occurred()) throw python_error();
     return v;
   }
+  bool truth() {
+    const int v = PyObject_IsTrue(next());
+    if (v < 0) throw python_error();
+    return v != 0;
+  }
   double real() {
     const double v = PyFloat_AsDouble(next());
     if (v == -1.0 && PyErr_Occurred()) throw python_error();
@@ -227,9 +232,9 @@ PyObject* ep_dispatch(Args v) {
   UmdkEpDispatchParams p = *reinterpret_cast<const UmdkEpDispatchParams*>(v.integer());
   const Tensor x = v.tensor(), idx = v.tensor(), w = v.maybe(), sidx = v.tensor(), slot = v.tensor(), npe = v.tensor(),
                npr = v.tensor();
-  p.quant = v.integer() != 0;
+  p.quant = v.truth();
   const int64_t n_cap = v.integer(), a_cap = v.integer();
-  const bool row_info = v.integer() != 0;
+  const bool row_info = v.truth();
   p.num_ctas = (int)v.integer();
   p.phase_mask = (int)v.integer();
   p.host_tag = (int)v.integer();
@@ -278,7 +283,7 @@ PyObject* ep_combine(Args v) {   // base, y (checked), recv_meta, counts, in_ran
   UmdkEpCombineParams p = *reinterpret_cast<const UmdkEpCombineParams*>(v.integer());
   const Tensor y = v.tensor(), meta = v.tensor(), counts = v.tensor(), in_rank = v.tensor();
   p.T = (int)v.integer();
-  p.apply_weights = (int)v.integer();
+  p.apply_weights = v.truth();
   p.num_ctas = (int)v.integer();
   p.phase_mask = (int)v.integer();
   Tensor out = v.maybe();

@@ -154,6 +154,7 @@ class LayoutResult:
     send_token_idx: torch.Tensor
     rank_slot: torch.Tensor
 
+
 @dataclass
 class NotifyResult:
     """What a rank learns from the count exchange before any token moves (the outputs of the reference's
