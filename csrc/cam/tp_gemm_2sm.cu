@@ -1,7 +1,8 @@
 // Tensor-parallel fused GEMM + collective kernels with CTA pairs (one `tcgen05.mma.cta_group::2` per 256 x 256 output
-// tile; 128 or 64 columns where that ends sooner, see tile_columns). Same protocol, heap layout and arguments as tp_gemm.cu - copy CTAs that gather peer shards for
-// MODE 0, push epilogue + owner reduce for MODE 1 - with the main loop of gemm_bf16_2sm.cu: each CTA of a pair stages
-// 128 rows of A and half the rows of B per k-block and keeps its half of the accumulator in its own TMEM.
+// tile; 128 or 64 columns where that ends sooner, see tile_columns). Same protocol, heap layout and arguments as tp_gemm.cu
+// - copy CTAs that gather peer shards for MODE 0, push epilogue + owner reduce for MODE 1 - with the main loop of
+// gemm_bf16_2sm.cu: each CTA of a pair stages 128 rows of A and half the rows of B per k-block and keeps its half of the
+// accumulator in its own TMEM.
 //
 // The own shard never passes through the heap on its way to the tensor cores: MODE 0 reads it from the caller's tensor at once
 // (the copy CTAs still publish it to the peers), and a group of one rank gives all 74 pairs to the GEMM. MODE 1 with one
