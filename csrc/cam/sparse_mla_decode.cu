@@ -46,6 +46,7 @@
 // Every wait is bounded; a CTA that gives up raises the abort flag of both CTAs so the partner leaves at once.
 // There is no attention code in the reference project; the op is specified by the serving configuration only.
 #include "common.h"
+#include "mla_waits.h"
 #include "ptx.cuh"
 
 namespace umdk {
@@ -210,15 +211,12 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   // more than the work they guard).
   uint64_t* bar_full = bars + 1;     // kStages, one arrival that expects the tile's bytes from the TMA gathers
   uint64_t* bar_empty = bar_full + kStages;    // kStages, one commit
-  uint64_t* bar_s = bar_empty + kStages;       // 2, one commit
-  uint64_t* bar_xld = bar_s + 2;     // 2, 4 exchange-warp arrivals: they have read this S buffer, P may take its place
-  uint64_t* bar_p = bar_s + 4;       // 8 softmax-warp arrivals
-  uint64_t* bar_o = bar_s + 5;       // one commit
-  uint64_t* bar_xfull = bar_s + 6;   // one local arrival that expects the 24 KB the partner's st.async stores deliver
-  uint64_t* bar_xfree = bar_s + 7;   // 8 arrivals from the partner's softmax warps: its X may be overwritten
-  uint64_t* bar_fin = bar_s + 8;     // one commit (drain on the abort path)
-  uint64_t* bar_qt = bar_s + 9;      // 8 softmax-warp arrivals: Q is in TMEM
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_s + 10);
+  uint64_t* bar_step = bar_empty + kStages;    // kMlaBars: see mla_waits.h
+  uint64_t* bar_xld = bar_step + kMlaBars;     // 2, 4 exchange-warp arrivals: they have read this S buffer, P may take its place
+  uint64_t* bar_xfull = bar_xld + 2;   // one local arrival that expects the 24 KB the partner's st.async stores deliver
+  uint64_t* bar_xfree = bar_xld + 3;   // 8 arrivals from the partner's softmax warps: its X may be overwritten
+  uint64_t* bar_qt = bar_xld + 4;      // 8 softmax-warp arrivals: Q is in TMEM
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_xld + 5);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -238,15 +236,10 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       mbar_init(&bar_full[i], 1);
       mbar_init(&bar_empty[i], 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&bar_s[i], 1);
-      mbar_init(&bar_xld[i], 4);
-    }
-    mbar_init(bar_p, kSoftWarps);
-    mbar_init(bar_o, 1);
+    for (int i = 0; i < kMlaBars; ++i) mbar_init(&bar_step[i], mla_of_softmax(i) ? kSoftWarps : 1);
+    for (int i = 0; i < 2; ++i) mbar_init(&bar_xld[i], 4);
     mbar_init(bar_xfull, 1);
     mbar_init(bar_xfree, kSoftWarps);
-    mbar_init(bar_fin, 1);
     mbar_init(bar_qt, kSoftWarps);
     mbar_fence_init();
     *s_abort = 0;
@@ -309,6 +302,9 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     st_cluster_u32(peer_abort, 1u);
   };
 
+  auto step_bar = [&](MlaStep step, int c) { return &bar_step[mla_wait(step, c).bar]; };
+  auto step_over = [&](MlaStep step, int c) { return wait_bar<false>(step_bar(step, c), mla_wait(step, c).parity, s_abort); };
+
   if (warp < kSoftWarps) {
     // ===================================== softmax ======================================================
     // Two sets of four warps share the heads (a thread per head and set) and split the keys of a chunk: one thread
@@ -357,7 +353,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     for (int c = 0; c < num_chunks; ++c) {
       const int sb = c & 1;
       if (ok) {
-        ok = __all_sync(0xffffffffu, wait_bar<false>(&bar_s[sb], (c >> 1) & 1, s_abort));
+        ok = __all_sync(0xffffffffu, step_over(kMlaS, c));
         if (!ok) give_up(UMDK_PH_TMEM_FULL, c);
       }
       lap(0);
@@ -426,10 +422,11 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       l_run = l_run * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));   // of this set's keys
       lap(5);
       // O is rescaled only when P(c-1) * V has finished (P(c-2) * V has: S(c) was made behind it). P(c) itself goes into the
-      // other buffer than P(c-1), and its product queues up behind that one.
+      // other buffer than P(c-1), and its product queues up behind that one: without a rescale nothing here waits for P(c-1) * V,
+      // which may then still be open behind the last chunk.
       const bool scale_o = c >= 1 && __any_sync(0xffffffffu, alpha != 1.f);
       if (scale_o) {
-        ok = __all_sync(0xffffffffu, wait_bar<false>(bar_o, (c - 1) & 1, s_abort));
+        ok = __all_sync(0xffffffffu, step_over(kMlaO, c - 1));
         if (!ok) {
           give_up(UMDK_PH_TMEM_EMPTY, c);
           continue;
@@ -462,7 +459,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_p);
+      if (lane == 0) mbar_arrive(step_bar(kMlaP, c));
       lap(7);
     }
     if (dg) {
@@ -472,7 +469,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     // ---- epilogue: this CTA's 256 output columns, half of them per set ----
     // (every decision below is the same for all eight warps: the TMEM loads are warp-collective)
     if (ok) {
-      ok = __all_sync(0xffffffffu, wait_bar<false>(bar_o, (num_chunks - 1) & 1, s_abort));
+      ok = __all_sync(0xffffffffu, step_over(kMlaEnd, 0));
       if (!ok) give_up(UMDK_PH_TMEM_EMPTY, 2000);
     }
     // both sets' sums; the last chunk used the other half of max_sm
@@ -550,7 +547,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         }
         lap(0);
         // S(c) overwrites S(c-2) and the P(c-2) in its place: P(c-2) * V has finished, and with it every reader of both
-        if (c >= 2 && !wait_bar<false>(bar_o, c & 1, s_abort)) {
+        if (c >= 2 && !step_over(kMlaO, c - 2)) {
           give_up(UMDK_PH_TMEM_EMPTY, 100 + c);
           return false;
         }
@@ -567,7 +564,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           for (int k = 0; k < 4; ++k)
             umma_f16_ta(d, q + j * 32 + k * 8, bd + j * (kKSlabBytes >> 4) + 2 * k, idesc_qk, (j | k) ? 1u : 0u);
         }
-        umma_commit(&bar_s[c & 1]);
+        umma_commit(step_bar(kMlaS, c));
         lap(3);
         return true;
       };
@@ -575,7 +572,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       for (int c = 0; c < num_chunks && ok; ++c) {
         if (c + 1 < num_chunks) ok = issue_qk(c + 1);
         if (!ok) break;
-        if (!wait_bar<false>(bar_p, c & 1, s_abort)) {
+        if (!step_over(kMlaP, c)) {
           give_up(UMDK_PH_GROUP_READY, 200 + c);
           ok = false;
           break;
@@ -589,17 +586,16 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           umma_f16_ta(tmem_base + kColO, tmem_base + kColS + (c & 1) * kChunk + k * 8, vd + k * (2048 >> 4), idesc_pv,
                       (c | k) ? 1u : 0u);
         umma_commit(&bar_empty[st]);
-        umma_commit(bar_o);
+        umma_commit(step_bar(kMlaO, c));
         lap(3);
       }
       if (dg) {
         for (int i = 0; i < 4; ++i) a.diag[8 + i] = dt[i];
         a.diag[15] = clock64() - t_begin;
       }
-      if (!ok) {   // leave only after every MMA already issued has retired (they read smem and write TMEM)
-        umma_commit(bar_fin);
-        mbar_wait(bar_fin, 0);
-      }
+      // the softmax warps read O behind this; and leave only after every MMA issued has retired (they read smem and write TMEM)
+      umma_commit(step_bar(kMlaEnd, 0));
+      mbar_wait(step_bar(kMlaEnd, 0), mla_wait(kMlaEnd, 0).parity);
     }
   } else if (warp >= kExchangeWarp && warp < kMmaWarp) {
     // ===================================== exchange (warps 8..11) =======================================
@@ -612,7 +608,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     long long t_prev = dg ? clock64() : 0;
     for (int c = 0; c < num_chunks; ++c) {
       const int sb = c & 1;
-      if (!__all_sync(0xffffffffu, wait_bar<false>(&bar_s[sb], (c >> 1) & 1, s_abort))) {
+      if (!__all_sync(0xffffffffu, step_over(kMlaS, c))) {
         give_up(UMDK_PH_TMEM_FULL, 3000 + c);
         break;
       }
@@ -828,4 +824,11 @@ UMDK_API int umdk_sparse_mla_decode(const void* q, const void* kv, const int* bl
     UMDK_CUDA_CHECK(cudaGetLastError());
   }
   return 0;
+}
+
+// Barrier and parity (2 * barrier + parity) of a wait of the kernel's: for the test that walks through the roles' orders.
+UMDK_API int umdk_sparse_mla_wait(int step, int c) {
+  if (step < kMlaS || step > kMlaEnd || c < 0) return -UMDK_ERR_BAD_ARG;
+  const MlaWait w = mla_wait(static_cast<MlaStep>(step), c);
+  return 2 * w.bar + static_cast<int>(w.parity);
 }
