@@ -97,6 +97,20 @@ def test_the_result_is_read_behind_the_last_product(n):
         assert not any(f[0] == "early" for f in faults(n, rescaled)), rescaled
 
 
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5])
+def test_no_phase_is_missed(n):
+    for rescaled in patterns(n):
+        assert faults(n, rescaled) == set(), rescaled
+
+
+@pytest.mark.parametrize("n", [2, 3, 4])
+def test_the_walk_sees_a_missed_phase(n):
+    """One barrier for every P: chunks that rescale nothing let the softmax warps get two phases ahead of the issuer."""
+    one = lambda step, c: (2, c & 1) if step == P else kernel_wait(step, c)
+    assert ("stuck",) in faults(n, set(), one)
+    assert ("stuck",) not in faults(n, set(range(1, n)), one)
+
+
 @pytest.mark.parametrize("n", [2, 3, 4])
 def test_the_walk_sees_a_result_read_too_soon(n):
     """Behind chunks that rescale nothing the barrier of the single products may be two phases back: the same parity."""
