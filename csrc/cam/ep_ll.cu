@@ -259,6 +259,19 @@ struct UmdkEpLLDispatchParams {
   int* status;
 };
 
+// CTAs of a dispatch on a GPU with `sms` SMs. num_ctas 0, one rank: an item (2 KiB of a token) for every warp, 32 CTAs at least.
+// 32 / as many as that, us, with the combine: 142 tokens of 6656, top-1 of 160 16.3 / 13.0, 256 of 7168, top-8 of 256
+// 40.4 / 34.5; no difference where 32 hold all items. With more ranks always 32: every CTA waits for the peers' counts, and
+// while they are late the other SMs belong to whatever runs beside it (a GEMM, another micro-batch's dispatch, for which a
+// peer may be waiting).
+UMDK_API int umdk_ep_ll_dispatch_grid(int R, int T, int H, int num_ctas, int sms) {
+  const int items = T * ((H / 128 + 15) / 16);
+  int grid = 32;
+  if (num_ctas > 0) grid = num_ctas;
+  else if (R == 1 && items > 32 * kLLWarps) grid = (items + kLLWarps - 1) / kLLWarps;
+  return grid < sms ? grid : sms;
+}
+
 UMDK_API int umdk_ep_ll_dispatch(const UmdkEpLLDispatchParams* p, void* stream) {
   LLDispatchArgs a;
   if (int rc = fill_ll_geom(&a.g, p->R, p->rank, p->E, p->K, p->H, p->T_cap)) return rc;
@@ -276,11 +289,7 @@ UMDK_API int umdk_ep_ll_dispatch(const UmdkEpLLDispatchParams* p, void* stream) 
   a.io.status = p->status;
   a.io.meet_cycles = umdk_rendezvous_cycles();
   a.io.phase_mask = p->phase_mask ? p->phase_mask : 3;
-  // num_ctas 0: an item (2 KiB of a token) for every warp, 32 CTAs at least. 32 / as many as that, us, with the combine: 142 tokens
-  // of 6656, top-1 of 160 16.3 / 13.0, 256 of 7168, top-8 of 256 40.4 / 34.5; no difference where 32 hold all items.
-  const int items = p->T * ((p->H / 128 + 15) / 16);
-  int grid = p->num_ctas > 0 ? p->num_ctas : items > 32 * kLLWarps ? (items + kLLWarps - 1) / kLLWarps : 32;
-  if (grid > sm_count()) grid = sm_count();
+  const int grid = umdk_ep_ll_dispatch_grid(p->R, p->T, p->H, p->num_ctas, sm_count());
   if (!p->send_idx) {
     // layout inside the kernel: 16-bit counters and positions, so at most 65535 entries per expert and a table that
     // fits in shared memory
