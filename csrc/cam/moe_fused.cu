@@ -292,7 +292,7 @@ __device__ __forceinline__ void run_phase(const CUtensorMap* tmW, const CUtensor
 #pragma unroll
         for (int i = 0; i < kScaleKb; ++i) x[i] = t < m && kb0 + i < kb_total ? __ldcg(xrow + kb0 + i) : 0.f;
         const float wv = t < 2 * kScaleKb && kb0 + wi < kb_total ? __ldg(wrow + kb0) : 0.f;
-        if (!__all_sync(0xffffffffu, mbar_wait(&sempty[ss], sph ^ 1))) {
+        if (!mbar_wait_warp(&sempty[ss], sph ^ 1)) {
           umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_EMPTY, w, 10000 + kb0);
           ok = false;
           break;
@@ -337,7 +337,7 @@ __device__ __forceinline__ void run_phase(const CUtensorMap* tmW, const CUtensor
           acc_u[0][c] = acc_u[1][c] = 0;
         }
         for (int kb0 = 0; kb0 < kb_total && ok; kb0 += kScaleKb) {
-          if (!mbar_wait(&sfull[ss], sph)) {
+          if (!mbar_wait_warp(&sfull[ss], sph)) {
             umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, 10000 + kb0);
             ok = false;
             break;
@@ -347,7 +347,7 @@ __device__ __forceinline__ void run_phase(const CUtensorMap* tmW, const CUtensor
           const int kb1 = min(kb_total, kb0 + kScaleKb);
           for (int kb = kb0; kb < kb1; ++kb, ++kbc) {
             const int ts = kbc % kTmemStages;
-            if (!mbar_wait(&tfull[ts], (kbc / kTmemStages) & 1)) {
+            if (!mbar_wait_warp(&tfull[ts], (kbc / kTmemStages) & 1)) {
               umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, w, kb);
               ok = false;
               break;

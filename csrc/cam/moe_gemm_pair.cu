@@ -277,7 +277,7 @@ __device__ __forceinline__ void weight_body(uint8_t* smem, const CUtensorMap& tm
 #pragma unroll
           for (int i = 0; i < C::kScaleKb; ++i)
             xv[i] = t64 < it.m && kb0 + i < kb_total ? a.xs[(size_t)(it.row0 + t64) * nsb + kb0 + i] : 0.f;
-          if (!__all_sync(0xffffffffu, mbar_wait(&sempty[ss], sph ^ 1))) {
+          if (!mbar_wait_warp(&sempty[ss], sph ^ 1)) {
             umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_EMPTY, w, 10000 + kb0);
             ok = false;
             break;
@@ -318,7 +318,7 @@ __device__ __forceinline__ void weight_body(uint8_t* smem, const CUtensorMap& tm
 #pragma unroll
       for (int c = 0; c < 16; ++c) acc[c] = 0;
       for (int kb0 = 0; kb0 < kb_total && ok; kb0 += C::kScaleKb) {
-        if (!__all_sync(0xffffffffu, mbar_wait(&sfull[ss], sph))) {
+        if (!mbar_wait_warp(&sfull[ss], sph)) {
           umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, 10000 + kb0);
           ok = false;
           break;
@@ -327,7 +327,7 @@ __device__ __forceinline__ void weight_body(uint8_t* smem, const CUtensorMap& tm
         const int kb1 = min(kb_total, kb0 + C::kScaleKb);
         for (int kb = kb0; kb < kb1; ++kb, ++kbc, sc += C::kW * kTok) {
           const int ts = kbc % C::kTmemStages;
-          if (!__all_sync(0xffffffffu, mbar_wait(&tfull[ts], (kbc / C::kTmemStages) & 1))) {
+          if (!mbar_wait_warp(&tfull[ts], (kbc / C::kTmemStages) & 1)) {
             umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, w, kb);
             ok = false;
             break;
@@ -400,7 +400,7 @@ __device__ __forceinline__ void weight_body(uint8_t* smem, const CUtensorMap& tm
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         if (qq == 0 && t4 < nh) st_async_b32(peer_amax + tok * 4, __float_as_uint(mx), peer_bar);
-        ok = mbar_wait_cluster(&abar[par], (n_it >> 1) & 1);
+        ok = mbar_wait_cluster_warp(&abar[par], (n_it >> 1) & 1);
         if (!ok) umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_GROUP_READY, w, 20000);
         ok = bar_half_and(half, ok);   // also: every read of the transposition buffer is done
         if (!ok) break;
@@ -565,7 +565,7 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
             w1[i] = in ? __ldg(ws1 + kb0 + i) : 0.f;
             xv[i] = in && rows > 0 ? xs[i] : 0.f;
           }
-          if (!__all_sync(0xffffffffu, mbar_wait(&bars->sempty[ss], sph ^ 1))) {
+          if (!mbar_wait_warp(&bars->sempty[ss], sph ^ 1)) {
             umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_EMPTY, w, 10000 + kb0);
             ok = false;
             break;
@@ -616,8 +616,11 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
     };
     // waits for the accumulator of K block i and starts the load of its first columns
     auto take = [&](uint32_t i, int w) {
-      ok = mbar_wait(tfull + (i & 1) * 16, (i >> 1) & 1);
-      if (!ok) umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, w, (int)i);
+      ok = mbar_wait_warp(tfull + (i & 1) * 16, (i >> 1) & 1);
+      if (!ok) {
+        umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, w, (int)i);
+        return;
+      }
       tc_fence_after();
       load(cols + (i & 1) * 256, r[0]);
     };
@@ -627,8 +630,9 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
       for (int c = 0; c < 64; ++c) acc[c] = 0;
       take(n, w);
       for (int left = kb_total; left > 0 && ok;) {
-        if (!__all_sync(0xffffffffu, mbar_wait(bars_sm + (uint32_t)offsetof(Bars, sfull) + ss * 8, sph))) {
+        if (!mbar_wait_warp(bars_sm + (uint32_t)offsetof(Bars, sfull) + ss * 8, sph)) {
           umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, 10000 + left);
+          tmem_ld_wait();   // the load that take() has started
           ok = false;
           break;
         }

@@ -71,6 +71,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return true;
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) { return mbar_wait(smem_u32(bar), parity); }
+// The same wait of a whole warp, with one answer for all its lanes. Each lane counts its own cycles, so they can disagree about
+// whether the budget ran out; behind a wait of theirs stand instructions that all lanes have to reach together.
+template <class Bar>
+__device__ __forceinline__ bool mbar_wait_warp(Bar bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+}
 __device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
@@ -390,6 +396,9 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
     if (clock64() - t0 > kSpinLimitCycles) return false;
   }
   return true;
+}
+__device__ __forceinline__ bool mbar_wait_cluster_warp(uint64_t* bar, uint32_t parity) {   // as mbar_wait_warp
+  return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity));
 }
 // Asynchronous store into another CTA's shared memory, its bytes counted on that CTA's mbarrier (complete_tx).
 __device__ __forceinline__ void st_async_b32(uint32_t cluster_addr, uint32_t v, uint32_t cluster_bar) {
