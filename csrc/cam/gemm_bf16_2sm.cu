@@ -180,7 +180,7 @@ gemm_bf16_2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       const int m0 = m_blk * 2 * BMH + (int)cta * BMH, n0 = n_blk * BN;
       const int ab = it & 1;
       const uint32_t aph = (it >> 1) & 1;
-      if (!mbar_wait(&tfull[ab], aph)) {
+      if (!mbar_wait_warp(&tfull[ab], aph)) {
         umdk_set_status(status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, t, 0);
         break;
       }

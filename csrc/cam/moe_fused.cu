@@ -100,22 +100,6 @@ struct Shared {
 };
 
 __device__ __forceinline__ void bar_epi() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
-// The same barrier, joining a decision: true on all 256 threads or on none (a wait that ran out in one warp must not leave the
-// others at the next barrier).
-__device__ __forceinline__ bool bar_epi_and(bool ok) {
-  uint32_t r;
-  asm volatile(
-      "{\n"
-      ".reg .pred p, q;\n"
-      "setp.ne.u32 q, %1, 0;\n"
-      "barrier.cta.red.and.pred p, 1, 256, q;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(r)
-      : "r"(ok ? 1u : 0u)
-      : "memory");
-  return r != 0;
-}
 // Token columns that the MMAs of a tile of m rows cover; the halves of the promoting warps take 8, 16 or 32 of them.
 __device__ __forceinline__ int tile_columns(int m) { return m <= 16 ? 16 : m <= 32 ? 32 : TT; }
 
@@ -419,7 +403,7 @@ __device__ __forceinline__ void run_phase(const CUtensorMap* tmW, const CUtensor
       if (cols == 16) item(std::integral_constant<int, 8>());
       else if (cols == 32) item(std::integral_constant<int, 16>());
       else item(std::integral_constant<int, 32>());
-      ok = bar_epi_and(ok);
+      ok = bar_and<kEpiThreads>(1, ok);
       if (!ok) break;
       const float4* src = reinterpret_cast<const float4*>(sh.trans + t * kTransStride + qtr * 32);
       const int row = row0 + t;

@@ -287,7 +287,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
       for (int kb = 0; kb < kb_total; ++kb, ++kbc) {
         const int ts = kbc & 1;
         const uint32_t tph = (kbc >> 1) & 1;
-        if (!mbar_wait(&tfull[ts], tph)) {
+        if (!mbar_wait_warp(&tfull[ts], tph)) {
           umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, w, kb);
           ok = false;
           break;
@@ -315,7 +315,6 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         __syncwarp();
         if (lane == 0) mbar_arrive(&tempty[ts]);
       }
-      if (!ok) break;
       // ---- tile epilogue: transpose through shared memory so that each thread owns half a token row ----
 #pragma unroll
       for (int c = 0; c < TT; ++c) {
@@ -323,7 +322,8 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
         if (MODE == 0) v = (v / (1.f + __expf(-v))) * acc_u[c];
         trans[c * kTransStride + tid] = v;
       }
-      bar_epi();
+      ok = bar_and<128>(1, ok);
+      if (!ok) break;
       const int t = tid & 63, half = tid >> 6;
       const float* src = trans + t * kTransStride + half * 64;
       const int row = row0 + t;

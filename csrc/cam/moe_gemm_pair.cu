@@ -112,23 +112,6 @@ __device__ __forceinline__ void bar_half(int half) {
   asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
 }
 
-// The same barrier, joining a decision: true on all 128 threads or on none (a wait that ran out in one warp must not
-// leave the others at the next barrier).
-__device__ __forceinline__ bool bar_half_and(int half, bool ok) {
-  uint32_t r;
-  asm volatile(
-      "{\n"
-      ".reg .pred p, q;\n"
-      "setp.ne.u32 q, %2, 0;\n"
-      "barrier.cta.red.and.pred p, %1, 128, q;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(r)
-      : "r"(1 + half), "r"(ok ? 1u : 0u)
-      : "memory");
-  return r != 0;
-}
-
 struct Item {
   int e, j, row0, m, n;   // expert, feature tile, first row, valid rows, rows the MMA covers (multiple of 32)
 };
@@ -354,7 +337,7 @@ __device__ __forceinline__ void weight_body(uint8_t* smem, const CUtensorMap& tm
           sph ^= 1;
         }
       }
-      ok = bar_half_and(half, ok);
+      ok = bar_and<128>(1 + half, ok);
       if (!ok) break;
       float v[32];
 #pragma unroll
@@ -402,7 +385,7 @@ __device__ __forceinline__ void weight_body(uint8_t* smem, const CUtensorMap& tm
         if (qq == 0 && t4 < nh) st_async_b32(peer_amax + tok * 4, __float_as_uint(mx), peer_bar);
         ok = mbar_wait_cluster_warp(&abar[par], (n_it >> 1) & 1);
         if (!ok) umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_GROUP_READY, w, 20000);
-        ok = bar_half_and(half, ok);   // also: every read of the transposition buffer is done
+        ok = bar_and<128>(1 + half, ok);   // also: every read of the transposition buffer is done
         if (!ok) break;
         if (t4 < nh && tok < it.m) {
           const float amax = fmaxf(fmaxf(mx, amax_in[par * kTok + tok]), 1e-4f);
@@ -438,22 +421,6 @@ __device__ __forceinline__ Item locate_tokens(const int* tile_pref, const int* g
   it.m = min(256, goff[lo + 1] - it.row0);
   it.n = 256;
   return it;
-}
-
-// Barrier of the two warps that share a quarter's tokens, joining a decision.
-__device__ __forceinline__ bool bar_quarter_and(int q, bool ok) {
-  uint32_t r;
-  asm volatile(
-      "{\n"
-      ".reg .pred p, q;\n"
-      "setp.ne.u32 q, %2, 0;\n"
-      "barrier.cta.red.and.pred p, %1, 64, q;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(r)
-      : "r"(1 + q), "r"(ok ? 1u : 0u)
-      : "memory");
-  return r != 0;
 }
 
 template <int MODE>
@@ -717,7 +684,7 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
         }
         float* am = amax_sm + (n_it & 1) * 256;
         am[u * 128 + tid] = mx;
-        ok = bar_quarter_and(q, ok);
+        ok = bar_and<64>(1 + q, ok);   // the two warps that share a quarter's tokens
         if (!ok) break;
         const float amax = fmaxf(fmaxf(mx, am[(u ^ 1) * 128 + tid]), 1e-4f);
         const float inv = 448.f / amax;

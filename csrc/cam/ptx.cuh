@@ -61,6 +61,23 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {  
       : "memory");
   return ok != 0;
 }
+// Barrier `id` of kThreads threads that joins a decision: true on all of them or on none (a wait that ran out in one warp must not
+// leave the others at the next barrier).
+template <int kThreads>
+__device__ __forceinline__ bool bar_and(int id, bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.u32 q, %2, 0;\n"
+      "barrier.cta.red.and.pred p, %1, %3, q;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(r)
+      : "r"(id), "r"(ok ? 1u : 0u), "n"(kThreads)
+      : "memory");
+  return r != 0;
+}
 // Bounded wait on a phase parity. Returns false when the cycle budget ran out.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return true;

@@ -177,22 +177,6 @@ __device__ __forceinline__ void st_cluster_u32(uint32_t cluster_addr, uint32_t v
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
 
-// Barrier of the softmax warps that also joins a decision: true on all of them or on none.
-__device__ __forceinline__ bool bar_softmax_and(bool ok) {
-  uint32_t r;
-  asm volatile(
-      "{\n"
-      ".reg .pred p, q;\n"
-      "setp.ne.u32 q, %1, 0;\n"
-      "barrier.cta.red.and.pred p, 1, %2, q;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(r)
-      : "r"(ok ? 1u : 0u), "n"(32 * kSoftWarps)
-      : "memory");
-  return r != 0;
-}
-
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV,
                          const MlaArgs a) {
@@ -392,7 +376,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       // every lane's loads of x_sm have returned (mx depends on them); keep the arrival behind that dependence
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 0));
       max_sm[(sb * kSets + set) * kHeads + head] = mx;
-      ok = bar_softmax_and(ok);   // both sets' maxima are in place
+      ok = bar_and<32 * kSoftWarps>(1, ok);   // both sets' maxima are in place
       if (!ok) break;
       // re-armed before the partner may send again (its permission needs this warp's arrival below)
       if (tid == 0 && c + 1 < num_chunks) mbar_expect_tx(bar_xfull, kXBytes);
@@ -474,7 +458,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     }
     // both sets' sums; the last chunk used the other half of max_sm
     max_sm[((num_chunks & 1) * kSets + set) * kHeads + head] = l_run;
-    ok = bar_softmax_and(ok);
+    ok = bar_and<32 * kSoftWarps>(1, ok);
     l_run += max_sm[((num_chunks & 1) * kSets + (set ^ 1)) * kHeads + head];
     tc_fence_after();
     if (ok) {

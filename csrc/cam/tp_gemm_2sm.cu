@@ -213,7 +213,7 @@ tp_gemm_2sm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         tile_coords(t, &m0, &n0, &peer, &rows);
         const int ab = it & 1;
         const uint32_t aph = (it >> 1) & 1;
-        if (!mbar_wait(&tfull[ab], aph)) {
+        if (!mbar_wait_warp(&tfull[ab], aph)) {
           umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, t, 0);
           break;
         }

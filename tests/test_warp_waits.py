@@ -27,7 +27,8 @@ def single_lane_waits_of_warps(text):
     return found
 
 
-@pytest.mark.parametrize("name", ["moe_gemm_pair.cu", "moe_fused.cu"])
+@pytest.mark.parametrize("name", [
+    "moe_gemm_pair.cu", "moe_fused.cu", "moe_gemm.cu", "tp_gemm.cu", "tp_gemm_2sm.cu", "gemm_bf16.cu", "gemm_bf16_2sm.cu"])
 def test_waits_of_warps_are_joined(name):
     assert single_lane_waits_of_warps((CAM / name).read_text()) == []
 
