@@ -16,7 +16,7 @@ namespace umdk {
 enum MlaStep : int {
   kMlaS,     // S(c) = Q * K(c) is in TMEM: one commit
   kMlaP,     // P(c) has taken its place: an arrival of every softmax warp
-  kMlaO,     // P(c) * V(c) has been added to O: one commit
+  kMlaO,     // P(c) * V(c) has been added to O: one commit, for all chunks but the last
   kMlaEnd,   // every MMA of the split is through: one commit, c is ignored
 };
 constexpr int kMlaBars = 6;

@@ -569,17 +569,17 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         for (int k = 0; k < kChunk / 16; ++k)   // 16 keys per step: A advances 8 columns, B two 8-key groups
           umma_f16_ta(tmem_base + kColO, tmem_base + kColS + (c & 1) * kChunk + k * 8, vd + k * (2048 >> 4), idesc_pv,
                       (c | k) ? 1u : 0u);
-        umma_commit(&bar_empty[st]);
-        umma_commit(step_bar(kMlaO, c));
+        if (c + 1 < num_chunks) {   // behind the last chunk one commit, below, is for everybody
+          umma_commit(&bar_empty[st]);
+          umma_commit(step_bar(kMlaO, c));
+        }
         lap(3);
       }
       if (dg) {
         for (int i = 0; i < 4; ++i) a.diag[8 + i] = dt[i];
         a.diag[15] = clock64() - t_begin;
       }
-      // the softmax warps read O behind this; and leave only after every MMA issued has retired (they read smem and write TMEM)
-      umma_commit(step_bar(kMlaEnd, 0));
-      mbar_wait(step_bar(kMlaEnd, 0), mla_wait(kMlaEnd, 0).parity);
+      umma_commit(step_bar(kMlaEnd, 0));   // also where it gave up: see the end of the kernel
     }
   } else if (warp >= kExchangeWarp && warp < kMmaWarp) {
     // ===================================== exchange (warps 8..11) =======================================
@@ -682,6 +682,8 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   tc_fence_before();
   __syncthreads();
   if (warp == kMmaWarp) {
+    // every MMA issued has retired (they read shared memory and write TMEM), also where the softmax warps gave up on them
+    mbar_wait_warp(step_bar(kMlaEnd, 0), mla_wait(kMlaEnd, 0).parity);
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
   }

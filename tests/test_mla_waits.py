@@ -26,8 +26,7 @@ def faults(n, rescaled, wait=kernel_wait, last=END):
         return ([("wait", O, c - 2)] if c >= 2 else []) + [("mma", S, c)]
     issuer = qk(0)
     for c in range(n):
-        issuer += (qk(c + 1) if c + 1 < n else []) + [("wait", P, c), ("mma", O, c)]
-    issuer += [("mma", END, n - 1)]
+        issuer += (qk(c + 1) if c + 1 < n else []) + [("wait", P, c), ("mma", O if c + 1 < n else last, c)]
     softmax = []
     for c in range(n):
         softmax += [("wait", S, c), ("meet", c)] + ([("wait", O, c - 1)] if c in rescaled else []) + [("arrive", P, c)]
@@ -50,7 +49,7 @@ def faults(n, rescaled, wait=kernel_wait, last=END):
     def happened(step, c, pcs, done):
         if step == P:
             return all(pc > softmax.index(("arrive", P, c)) for pc in pcs[1:])
-        return ("mma", step, c) in mmas[:done] and (step != END or done == len(mmas))
+        return ("mma", step, c) in mmas[:done]
 
     while todo:
         state = todo.pop()

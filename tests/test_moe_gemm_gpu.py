@@ -1,4 +1,6 @@
 """Grouped fp8 expert GEMMs (tcgen05) against an fp32 PyTorch statement of the same block-scaled math."""
+import ctypes
+
 import pytest
 import torch
 
@@ -133,7 +135,6 @@ def test_single_ctas_match_the_pairs(G, counts, K, F, H):
 def test_token_major_tiles_match_single_ctas(G, counts, K, F, H):
     """One CTA pair takes the 256-token tiles here; ``max_ctas=1`` is the single-CTA kernel, which promotes the K blocks in the
     same order: the same bytes. The oracle as in the tests above."""
-    import ctypes
     from umdk_b200 import _native
     from umdk_b200.ops import moe_gemm
     c = _case(G, counts, K, F, H, seed=G + 2)
@@ -190,3 +191,62 @@ def test_more_experts_than_the_pairs_take():
     assert ref.mean_rel_err(ref.dequant_fp8_1x128(hq[:N].cpu(), hs[:N].cpu()), r_h[:N]) < 0.04
     r_y = ref.ref_gemm2(hq.cpu(), hs.cpu(), small["off"], small["w2q"], small["w2s"])
     assert ref.mean_rel_err(y[:N].float().cpu(), r_y[:N]) < 5e-3
+
+
+def _silu_case(v, up, G):
+    """Rows whose only feature that is not zero is silu(v) * up, up a power of two: one-hot tokens, the values in their scales
+    (gate v / 2 + v / 2, so that an overflow makes the infinities)."""
+    N, K, F = v.numel(), 384, 128
+    x = torch.zeros(N + 7, K)   # with room for more than 64 rows an expert: the pairs, whatever the experts hold
+    x[:, 0] = x[:, 128] = x[:, 256] = 1.0
+    w1 = torch.zeros(G, 2 * F, K)
+    w1[:, 0, 0] = w1[:, 0, 128] = w1[:, F, 256] = 1.0
+    xs = torch.zeros(N + 7, 3)
+    xs[:N] = torch.stack((v / 2, v / 2, up), 1)
+    big = v.isinf()
+    xs[:N][big, :2] = torch.finfo(torch.float32).max * v[big, None].sign()
+    off = torch.arange(G + 1, dtype=torch.int32) * (N // G)
+    return (x.to(torch.float8_e4m3fn).cuda(), xs.cuda(), off.cuda(), w1.to(torch.float8_e4m3fn).cuda(),
+            torch.ones(G, 2, 3).cuda())
+
+
+def test_swiglu_quotient_against_the_division():
+    """SwiGLU of the pair kernel, with either kind of tile, against the division of the single-CTA kernel: over all exponents,
+    where exp(-v) and the divisor overflow and the reciprocal is subnormal, zero, infinities and NaN. The row's scale shows
+    the absolute value to the last bit but one. One unit in the last place: the quotient is rounded from its remainder, but with a
+    reciprocal that is one unit off the result may be the neighbour where the quotient lies next to a rounding boundary."""
+    from umdk_b200 import _native
+    from umdk_b200.ops import moe_gemm
+    g = torch.Generator().manual_seed(5)
+    n = 4096
+    v = torch.cat((
+        torch.randn(n, generator=g) * 2, torch.rand(n, generator=g) * 24 - 104, torch.rand(n, generator=g) * 208 - 104,
+        torch.ldexp(1 + torch.rand(n - 8, generator=g), torch.randint(-100, 127, (n - 8,), generator=g)),
+        torch.tensor([0.0, -0.0, float("inf"), float("-inf"), float("nan"), 88.7228, -88.7228, -103.97])))
+    v[3 * n::2] *= -1
+    mag = (v.double() / (1 + torch.exp(-v.double()))).abs().clamp(2.0 ** -110, 2.0 ** 110)
+    up = torch.where(v.isfinite(), torch.ldexp(torch.ones(4 * n), -torch.log2(mag).floor().nan_to_num().int()), torch.ones(()))
+    res = {}
+    for kind, G, ctas in (("division", 1, 1), ("256 tokens", 1, 2), ("64 tokens", 256, 2)):
+        status = torch.zeros(4, dtype=torch.int32, device="cuda")
+        xq, xs, off, w1q, w1s = _silu_case(v, up, G)
+        assert _native.cam().umdk_moe_gemm_uses_pairs(0, G, 128, 384, 4 * n + 7, ctas) == (kind != "division")
+        if kind != "division":
+            offs = (ctypes.c_int * (G + 1))(*off.tolist())
+            assert _native.cam().umdk_moe_gemm_tokens_on_m(0, G, 128, offs, ctas) == (kind == "256 tokens")
+        hq, hs = moe_gemm.gemm1_swiglu_quant(xq, xs, off, w1q, w1s, status, max_ctas=ctas)
+        torch.cuda.synchronize()
+        assert status.tolist()[0] == 0, status.tolist()
+        res[kind] = hq.view(torch.uint8)[:4 * n].cpu(), hs.flatten()[:4 * n].cpu()
+    codes, scales = res["division"]
+    want = (v.double() / (1 + torch.exp(-v.double()))).abs() * up.double() / 448
+    fin = v.isfinite() & (v > -88.7) & (want > 1e-4 / 448)   # beyond, exp(-v) overflows and both give zero
+    # exp as in the kernel (__expf: 2 + 1.173 |v| units), then three roundings
+    tol = (2 + 1.173 * v.double().abs() + 4) * 2.0 ** -23
+    assert (((scales.double() - want).abs() / want)[fin] <= tol[fin]).all() and int(fin.sum()) > 2 * n
+    for kind in ("256 tokens", "64 tokens"):
+        c, s = res[kind]
+        apart = (s.view(torch.int32).long() - scales.view(torch.int32).long()).abs()
+        print(kind, "rows that differ:", int((apart > 0).sum()), "of", v.numel(), "codes", int((c != codes).any(1).sum()), v[apart>0][:8], int(apart.max()))
+        assert int(apart.max()) <= 1
+        assert torch.equal(c, codes)
