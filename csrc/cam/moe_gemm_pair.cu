@@ -864,25 +864,3 @@ UMDK_API int umdk_moe_gemm_tokens_on_m(int mode, int G, int Nout, const int* gro
   const int pairs = num_ctas / 2;
   return umdk::tokens_pay(mode, umdk::feature_tiles(mode, Nout), tiles64, tiles256, pairs, 1.f / pairs) ? 1 : 0;
 }
-
-// The better width, 64 or 256 tokens, of tiles with the weight rows on the M side for these rows per expert (host memory,
-// [G + 1]): a pair's time is its number of items times what one takes, in units of a 64-token item 1.3 + 0.0105 n for one of n
-// tokens in MODE 0 and 1 + 0.0085 n in MODE 1, where n lies between the average and the widest tile. Only the 64 are launched:
-// where 256 win, and in many places where they don't, tiles with the tokens on the M side are faster still.
-UMDK_API int umdk_moe_gemm_tile_tokens(int mode, int G, int Nout, const int* group_off, int num_ctas) {
-  if (mode < 0 || mode > 1 || G < 1 || Nout < 128 || num_ctas < 2) return -UMDK_ERR_BAD_ARG;
-  int tiles64 = 0, tiles256 = 0, widest = 0;
-  for (int e = 0; e < G; ++e) {
-    const int m = group_off[e + 1] - group_off[e], tiles = (m + 255) / 256;
-    tiles64 += (m + 63) / 64;
-    tiles256 += tiles;
-    const int w = tiles > 0 ? ((m + tiles - 1) / tiles + 31) & ~31 : 0;
-    widest = w > widest ? w : widest;
-  }
-  const int pairs = num_ctas / 2, nt = umdk::feature_tiles(mode, Nout);
-  const int waves64 = (tiles64 * nt + pairs - 1) / pairs, waves256 = (tiles256 * nt + pairs - 1) / pairs;
-  const float rows = (float)(group_off[G] - group_off[0]), most = (float)widest * tiles256;
-  const float n = mode == 0 ? 0.25f * rows + 0.75f * most : 0.75f * rows + 0.25f * most;   // times the number of tiles
-  const float item = mode == 0 ? 1.3f * tiles256 + 0.0105f * n : 1.f * tiles256 + 0.0085f * n;
-  return waves256 * item < (float)waves64 * tiles256 ? 256 : 64;
-}

@@ -1,4 +1,4 @@
-"""Which kernel and which token width the grouped expert GEMMs take: from the rows of each expert and the number of work items, as
+"""Which kernel and which kind of tile the grouped expert GEMMs take: from the rows of each expert and the number of work items, as
 measured; the size of the row buffer decides nothing where it says little about the rows."""
 import ctypes
 
@@ -7,14 +7,14 @@ import pytest
 from umdk_b200 import _native
 
 
-def _tokens(mode, nout, counts, ctas=148):
+def _tokens_on_m(mode, nout, counts, ctas=148):
     off = [0]
     for c in counts:
         off.append(off[-1] + c)
-    return _native.cam().umdk_moe_gemm_tile_tokens(mode, len(counts), nout, (ctypes.c_int * len(off))(*off), ctas)
+    return _native.cam().umdk_moe_gemm_tokens_on_m(mode, len(counts), nout, (ctypes.c_int * len(off))(*off), ctas)
 
 
-# rows of 32 experts that were measured, shares as the softmax of 0.4 x normal numbers
+# rows of 32 experts, shares as the softmax of 0.4 x normal numbers
 UNEVEN_160 = [
     110, 132, 119, 83, 265, 200, 93, 239, 162, 227, 114, 316, 99, 156, 121, 120, 91, 42, 205, 87, 230, 165, 171,
     126, 156, 248, 187, 87, 232, 184, 129, 224]
@@ -23,26 +23,30 @@ UNEVEN_512 = [
     209, 333, 447, 264, 512, 407, 232, 565, 1145, 383, 614]
 
 
-# (mode, output width, rows per expert) -> the faster width as measured; loads within 3 % of each other are left out
-@pytest.mark.parametrize("mode,nout,counts,want", [
-    (0, 2048, [1] * 32, 64), (0, 2048, [30] * 32, 64), (0, 2048, [64] * 32, 64), (0, 2048, [128] * 32, 64),
-    (0, 2048, [256] * 32, 256), (0, 2048, [320] * 32, 64), (0, 2048, [512] * 32, 256), (0, 2048, UNEVEN_160, 64),
-    (0, 2048, UNEVEN_512, 64), (0, 1024, [64] * 8, 64), (0, 1024, [128] * 8, 64), (0, 1024, [320] * 8, 64),
-    (0, 512, [100] * 4, 64), (0, 512, [256] * 4, 64), (0, 512, [512] * 4, 64),
-    (1, 7168, [1] * 32, 64), (1, 7168, [30] * 32, 64), (1, 7168, [128] * 32, 64), (1, 7168, [160] * 32, 256),
-    (1, 7168, [512] * 32, 256), (1, 7168, UNEVEN_160, 256), (1, 7168, UNEVEN_512, 256), (1, 2048, [100] * 4, 64),
+# (mode, output width, rows per expert, us with 64-token tiles, us with 256-token tiles): one cold launch of either kind on 148 SMs,
+# K 7168 (mode 0) and 2048 (mode 1) for 32 experts, 2048 for 8 and 4 of mode 0, 512 for 4 of mode 1
+@pytest.mark.parametrize("mode,nout,counts,us64,us256", [
+    (0, 2048, [1] * 32, 159, 206), (0, 2048, [30] * 32, 165, 228), (0, 2048, [64] * 32, 168, 235),
+    (0, 2048, [100] * 32, 263, 241), (0, 2048, [128] * 32, 273, 249), (0, 2048, [256] * 32, 505, 251),
+    (0, 2048, [320] * 32, 626, 462), (0, 2048, [512] * 32, 1027, 472), (0, 2048, UNEVEN_160, 390, 278),
+    (0, 2048, UNEVEN_512, 1050, 587), (0, 1024, [64] * 8, 21.4, 23.6), (0, 1024, [128] * 8, 25.6, 23.5),
+    (0, 1024, [320] * 8, 46.0, 33.8), (0, 512, [100] * 4, 17.4, 21.5), (0, 512, [256] * 4, 17.4, 21.4),
+    (0, 512, [512] * 4, 23.5, 21.4),
+    (1, 7168, [1] * 32, 98, 132), (1, 7168, [30] * 32, 97, 140), (1, 7168, [64] * 32, 99, 146), (1, 7168, [160] * 32, 205, 152),
+    (1, 7168, [512] * 32, 529, 278), (1, 7168, UNEVEN_160, 202, 153), (1, 7168, UNEVEN_512, 556, 338),
+    (1, 2048, [100] * 4, 12.3, 14.4),
 ])
-def test_width_follows_the_measurements(mode, nout, counts, want):
-    assert _tokens(mode, nout, counts) == want
+def test_the_faster_kind_of_tile_is_taken(mode, nout, counts, us64, us256):
+    assert _tokens_on_m(mode, nout, counts) == (us256 < us64)
 
 
-def test_width_of_the_small_gpu_test_cases():
-    """The sizes with which the GPU tests reach either width on one CTA pair, and the narrow one on all of them."""
+def test_kind_of_tile_of_the_small_gpu_test_cases():
+    """The loads with which the GPU tests reach the 256-token tiles on one CTA pair, and the 64-token tiles on all of them."""
     for counts, f, h in (([255, 257], 128, 256), ([300, 0, 513], 256, 384), ([410, 385], 256, 128)):
-        assert 256 in (_tokens(0, f, counts, 2), _tokens(0, 128, [512] * 3, 2)) and _tokens(1, h, counts, 2) == 256
-        assert _tokens(0, f, counts) == 64 and _tokens(1, h, counts) == 64
-    assert _tokens(0, 128, [1, 31, 33], 2) == 64 and _tokens(0, 128, [0, 0]) == 64
-    assert _tokens(2, 128, [1]) < 0 and _tokens(0, 128, [1], 1) < 0
+        assert _tokens_on_m(0, f, counts, 2) == 1 and _tokens_on_m(1, h, counts, 2) == 1
+        assert _tokens_on_m(0, f, counts) == 0 and _tokens_on_m(1, h, counts) == 0
+    assert _tokens_on_m(0, 128, [1, 31, 33], 2) == 0 and _tokens_on_m(0, 128, [0, 0]) == 0
+    assert _tokens_on_m(2, 128, [1]) < 0 and _tokens_on_m(0, 128, [1], 1) < 0
 
 
 # (mode, experts, output width, K, rows of the buffer) -> pairs (1), or single CTAs (0) where they are faster for even and for
