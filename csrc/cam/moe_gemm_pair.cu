@@ -85,16 +85,18 @@ __host__ __device__ constexpr int off_tables() {
 }
 
 // Whether 256-token tiles (tokens on the M side) beat 64-token tiles (weight rows there). A pair's time is its number of items
-// times what one takes: 1.45 times as long in MODE 0 and 1.75 times in MODE 1 for a 256-token tile, however many tokens are in
-// either. 64 / 256 tokens in us (32 experts, 7168, 2048), MODE 0: 64 rows for every expert 168 / 251, uneven 72: 269 / 252,
-// 128: 315 / 256, uneven 512: 1284 / 584; MODE 1: 64 rows 90 / 143, uneven 72: 127 / 149, uneven 100: 157 / 146, uneven 512:
-// 619 / 328; 4 experts of 200 rows, 2048 of 1152: 34.5 / 16.9, 1152 of 2048: 19.9 / 18.0. Over 71 loads of six shapes the
-// choice is 6 % off the faster kind at most. From the rows that are there, not from the buffer's size. Without a division: it
-// stands between a CTA's start and its first load (inv_pairs = 1 / pairs; counts below 2^20).
+// times what one takes: 1.75 times as long in MODE 0 and twice as long in MODE 1 for a 256-token tile, however many tokens are in
+// either. 64 / 256 tokens in us, 32 experts, 7168, 2048, uneven loads of 50 - 110 rows per expert, by items per pair, a few launches
+// of either kind in turn, then hundreds of one kind, which the power limit slows down more where the tensor cores compute for
+// absent rows. MODE 0, 10 / 7: 221 / 259, 235 / 305; 11 / 7: 260 / 274, 255 / 311; 12 / 7: 263 / 258, 267 / 301; 13 / 7:
+// 286 / 263, 292 / 312; 14 / 7: 314 / 269. MODE 1, 19 / 13: 139 / 183, 134 / 183; 22 / 13: 160 / 182, 150 / 184; 25 / 13:
+// 181 / 197; 28 / 13: 198 / 183. Over 348 loads of eight shapes (4 to 64 experts, 4 to 56 K blocks), in turn, the choice is at
+// most 3 % off the faster kind in MODE 0 and 5 % in MODE 1. From the rows that are there, not from the buffer's size. Without
+// a division: it stands between a CTA's start and its first load (inv_pairs = 1 / pairs; counts below 2^20).
 __host__ __device__ __forceinline__ bool tokens_pay(int mode, int nt, int tiles64, int tiles256, int pairs, float inv_pairs) {
   const int waves64 = (int)((tiles64 * nt + pairs - 0.5f) * inv_pairs);
   const int waves256 = (int)((tiles256 * nt + pairs - 0.5f) * inv_pairs);
-  return waves256 * (mode == 0 ? 1.45f : 1.75f) < (float)waves64;
+  return waves256 * (mode == 0 ? 1.75f : 2.f) < (float)waves64;
 }
 __host__ __device__ __forceinline__ int feature_tiles(int mode, int nout) {
   return mode == 0 ? nout / 128 : (nout + 255) / 256;

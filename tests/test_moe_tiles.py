@@ -15,6 +15,9 @@ def _tokens_on_m(mode, nout, counts, ctas=148):
 
 
 # rows of 32 experts, shares as the softmax of 0.4 x normal numbers
+UNEVEN_70 = [
+    48, 57, 52, 36, 115, 87, 40, 104, 70, 98, 49, 137, 43, 68, 52, 52, 39, 18, 89, 38, 100, 72, 74,
+    55, 68, 108, 81, 38, 101, 80, 56, 97]
 UNEVEN_160 = [
     110, 132, 119, 83, 265, 200, 93, 239, 162, 227, 114, 316, 99, 156, 121, 120, 91, 42, 205, 87, 230, 165, 171,
     126, 156, 248, 187, 87, 232, 184, 129, 224]
@@ -26,13 +29,14 @@ UNEVEN_512 = [
 # (mode, output width, rows per expert, us with 64-token tiles, us with 256-token tiles): one cold launch of either kind on 148 SMs,
 # K 7168 (mode 0) and 2048 (mode 1) for 32 experts, 2048 for 8 and 4 of mode 0, 512 for 4 of mode 1
 @pytest.mark.parametrize("mode,nout,counts,us64,us256", [
-    (0, 2048, [1] * 32, 159, 206), (0, 2048, [30] * 32, 165, 228), (0, 2048, [64] * 32, 168, 235),
+    (0, 2048, [1] * 32, 159, 206), (0, 2048, [30] * 32, 165, 228), (0, 2048, [64] * 32, 168, 235), (0, 2048, UNEVEN_70, 214, 239),
     (0, 2048, [100] * 32, 263, 241), (0, 2048, [128] * 32, 273, 249), (0, 2048, [256] * 32, 505, 251),
     (0, 2048, [320] * 32, 626, 462), (0, 2048, [512] * 32, 1027, 472), (0, 2048, UNEVEN_160, 390, 278),
     (0, 2048, UNEVEN_512, 1050, 587), (0, 1024, [64] * 8, 21.4, 23.6), (0, 1024, [128] * 8, 25.6, 23.5),
     (0, 1024, [320] * 8, 46.0, 33.8), (0, 512, [100] * 4, 17.4, 21.5), (0, 512, [256] * 4, 17.4, 21.4),
     (0, 512, [512] * 4, 23.5, 21.4),
-    (1, 7168, [1] * 32, 98, 132), (1, 7168, [30] * 32, 97, 140), (1, 7168, [64] * 32, 99, 146), (1, 7168, [160] * 32, 205, 152),
+    (1, 7168, [1] * 32, 98, 132), (1, 7168, [30] * 32, 97, 140), (1, 7168, [64] * 32, 99, 146), (1, 7168, UNEVEN_70, 116, 146),
+    (1, 7168, [100] * 32, 142, 149), (1, 7168, [128] * 32, 143, 150), (1, 7168, [160] * 32, 205, 152),
     (1, 7168, [512] * 32, 529, 278), (1, 7168, UNEVEN_160, 202, 153), (1, 7168, UNEVEN_512, 556, 338),
     (1, 2048, [100] * 4, 12.3, 14.4),
 ])
