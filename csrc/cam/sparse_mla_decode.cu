@@ -752,7 +752,8 @@ __global__ void __launch_bounds__(128) mla_merge_kernel(const float* __restrict_
 
 using namespace umdk;
 
-// Smallest num_splits the kernel accepts for a key list of `topk` entries.
+// Smallest num_splits the kernel accepts for a key list of `topk` entries (umdk_b200/ops/attention.py works it out itself; a test
+// compares the two).
 UMDK_API int umdk_sparse_mla_min_splits(int topk) { return (topk + kMaxKeys - 1) / kMaxKeys; }
 
 // q: [B, 128, 576] bf16; kv: [num_pages, 64, 576] bf16; block_table: [B, max_pages]; indices: [B, topk];

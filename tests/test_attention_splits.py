@@ -47,3 +47,10 @@ def test_no_split_without_keys():
             per = -(-(-(-topk // n)) // 48) * 48   # keys per split, as the kernel rounds them
             assert least <= n <= max(least, 24, 1) and (n - 1) * per < topk <= n * per and per <= 2064
             assert n <= max(1, least, 148 // (2 * batch))
+
+
+@pytest.mark.parametrize("topk", [1, 48, 2063, 2064, 2065, 4128, 4129, 100000])
+def test_keys_of_a_split_are_those_that_the_kernel_takes(topk):
+    from umdk_b200 import _native
+    from umdk_b200.ops.attention import MAX_KEYS
+    assert _native.cam().umdk_sparse_mla_min_splits(topk) == -(-topk // MAX_KEYS)

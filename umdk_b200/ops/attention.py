@@ -14,7 +14,7 @@ DIM = 576
 DIM_V = 512
 PAGE = 64
 CHUNK = 48   # keys per step of the kernel; a split takes whole chunks
-MAX_KEYS = 43 * CHUNK   # of a split
+MAX_KEYS = 43 * CHUNK   # of a split (umdk_sparse_mla_min_splits)
 
 
 @functools.lru_cache(maxsize=None)
