@@ -705,6 +705,22 @@ struct UmdkMoeFusedParams {
 //   w1: [G][F/128][H/128][256][128]  rows 0..127 = gate rows j*128.., rows 128..255 = up rows F + j*128..
 //   w2: [G][H/128][F/128][128][128]
 // - which turns the weight stream into 32 KB / 16 KB sequential DRAM reads. Scales are unchanged.
+static size_t fused_smem_bytes(int G) {
+  return 1024 + (size_t)kRingBytes + TT * kTransStride * 4 + kScaleStages * kScaleFloats * 4 + kEpiThreads * 4 +
+         2 * (size_t)(G + 1) * 4 + 16 + 2 * kPhaseBars * 8 + 16;
+}
+
+// Limit of the layer's row lengths: kRowTableBytes hold 66 floats per 128 elements of the longer one of H and F (the scales of 64 tokens
+// and of a gate and an up tile) and two ints per expert. That is 15616 elements with 32 experts, 11776 with 1024. Nothing in
+// the kernel needs it any more, the scales pass through stages of eight K blocks; it is what callers could count on to be refused
+// while whole rows of scales lay beside the ring, and longer rows have never been run.
+constexpr size_t kRowTableBytes = 32732;
+UMDK_API int umdk_moe_fused_fits(int G, int F, int H) {
+  if (G < 1 || F < BKB || H < BKB) return 0;
+  const size_t blocks = (H > F ? H : F) / BKB;
+  return blocks * (TT + 2) * 4 + 2 * (size_t)(G + 1) * 4 <= kRowTableBytes && fused_smem_bytes(G) <= 227 * 1024;
+}
+
 UMDK_API int umdk_moe_fused(const UmdkMoeFusedParams* p, void* stream) {
   if (p->G < 1 || p->F < 128 || (p->F % 128) || p->H < 128 || (p->H % 128) || p->n_rows_cap < 1 || p->R < 1 ||
       p->R > kMaxRanks)
@@ -797,12 +813,8 @@ UMDK_API int umdk_moe_fused(const UmdkMoeFusedParams* p, void* stream) {
       make_tmap_2d(&tmX, TMAP_U8, p->x, p->H, p->n_rows_cap, p->H, BKB, TT, TMAP_SW_128B) ||
       make_tmap_2d(&tmH, TMAP_U8, p->hq, p->F, p->n_rows_cap, p->F, BKB, TT, TMAP_SW_128B))
     return -UMDK_ERR_BAD_ARG;
-  const size_t smem = 1024 + (size_t)kRingBytes + TT * kTransStride * 4 + kScaleStages * kScaleFloats * 4 + kEpiThreads * 4 +
-                      2 * (size_t)(p->G + 1) * 4 + 16 + 2 * kPhaseBars * 8 + 16;
-  // rows of up to 15616 elements with 32 experts: as long as the scales of a whole row fitted beside the ring
-  const int kb_max = (p->H > p->F ? p->H : p->F) / BKB;
-  if (smem > 227 * 1024 || (size_t)kb_max * (TT + 2) * 4 + 2 * (size_t)(p->G + 1) * 4 > 227 * 1024 - 199716)
-    return -UMDK_ERR_BAD_ARG;
+  if (!umdk_moe_fused_fits(p->G, p->F, p->H)) return -UMDK_ERR_BAD_ARG;
+  const size_t smem = fused_smem_bytes(p->G);
   UMDK_CUDA_CHECK(cudaFuncSetAttribute(moe_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int grid = sm_count();
   if (p->max_ctas > 0 && p->max_ctas < grid) grid = p->max_ctas;

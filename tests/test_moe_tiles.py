@@ -71,3 +71,10 @@ def test_what_the_pairs_cannot_take_runs_on_single_ctas():
     assert uses(0, 8, 2048, 7168, 8 * 4000, 1) == 0 and uses(1, 8, 2048, 7168, 8 * 4000, 1) == 0
     assert uses(0, 1025, 2048, 7168, 1025 * 200, 148) == 0 and uses(0, 1024, 2048, 7168, 1024 * 200, 148) == 1
     assert uses(0, 8, 2048, 7168, 8 * 4000, 3) == 1
+
+
+def test_row_lengths_of_the_fused_layer():
+    fits = _native.cam().umdk_moe_fused_fits
+    for G, longest in ((1, 123 * 128), (32, 15616), (1024, 11776)):
+        assert fits(G, 128, longest) == 1 and fits(G, longest, 128) == 1
+        assert fits(G, 128, longest + 128) == 0 and fits(G, longest + 128, 128) == 0
