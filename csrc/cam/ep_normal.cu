@@ -49,8 +49,8 @@ constexpr int kEpWarps = kEpThreads / 32;
 constexpr int kLayoutCluster = 8;
 constexpr int kDirectTopk = 8;
 __host__ __device__ constexpr int layout_rank_words(int K) { return K > kDirectTopk ? ((K + 3) / 4) | 1 : 0; }   // odd: no conflicts
-// kCluster: one chunk per warp and one cluster of several CTAs; what the first pass finds stays in registers until the bases are
-// known. Else the CTAs meet at a grid barrier.
+// kCluster: one chunk per warp and one cluster of several CTAs; what the first pass finds stays with the thread until the bases are
+// known (32 registers of it, 60 bytes of which the compiler keeps in local memory). Else the CTAs meet at a grid barrier.
 template <bool kCluster>
 __global__ void __launch_bounds__(kLayoutWarps * 32)
 ep_layout_kernel(const int64_t* __restrict__ topk_idx, int T, int K, int E, int R, int per_warp,

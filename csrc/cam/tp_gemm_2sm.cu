@@ -10,7 +10,8 @@
 // the tensor cores from there on. Measured with one rank, 8192 x 8192 times 7168 and 8192 x 3584 times 8192: 1510 -> 974 us
 // of kernel time for the two (1.48 PFLOP/s in a burst), 1627 -> 1145 us back to back under the power limit.
 // An odd number of 128-row blocks leaves the last tile's second CTA without rows (it repeats the leader's and stores nothing):
-// 8064 x 6656 times 4096 and 8064 x 1536 times 6656 took 1677 us on single CTAs through the heap, 415 here.
+// 8064 x 6656 times 4096 and 8064 x 1536 times 6656 took 1720 us on single CTAs through the heap and take 438 here (8 passes behind a
+// pause; 400 back to back 1685 and 460).
 #include "tp_common.cuh"
 
 #include <cuda_runtime.h>
