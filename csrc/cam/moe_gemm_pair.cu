@@ -567,7 +567,7 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
     uint8_t* trans = smem + C::kOffTrans + (warp - 4) * C::kTransBytes;
     // 32-bit addresses only: the accumulators and the loads in flight take 160 to 192 registers, and one value kept in local memory
     // costs a cache access in every K block. Compiled apart, the loop over the K blocks keeps none there in MODE 1 and eight in
-    // MODE 0 (32 bytes stored, 128 loaded), with the epilogue 36 / 144 and 48 / 208; the whole kernels 40 / 176 and 64 / 308.
+    // MODE 0 (32 bytes stored, 128 loaded), with the epilogue 44 / 160 and 48 / 208; the whole kernels 48 / 192 and 68 / 316.
     const uint32_t bars_sm = smem_u32(bars);
     const uint32_t tfull = bars_sm + offsetof(Bars, tfull) + u * 8;
     const uint32_t tempty = map_to_cta(&bars->tempty[u], 0);

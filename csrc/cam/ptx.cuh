@@ -89,11 +89,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) { return mbar_wait(smem_u32(bar), parity); }
 // The same wait of a whole warp, with one answer for all its lanes. Each lane counts its own cycles, so they can disagree about
-// whether the budget ran out; behind a wait of theirs stand instructions that all lanes have to reach together.
-template <class Bar>
-__device__ __forceinline__ bool mbar_wait_warp(Bar bar, uint32_t parity) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+// whether the budget ran out; behind a wait of theirs stand instructions that all lanes have to reach together. The vote is part
+// of every poll: one vote behind a wait that each lane ends by itself made the fused layer 1 % slower (286.0 -> 289.6 us, this way
+// 285.7 -> 285.6).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const long long t0 = clock64();
+  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+    if (__any_sync(0xffffffffu, clock64() - t0 > kSpinLimitCycles)) return false;
+  }
+  return true;
 }
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) { return mbar_wait_warp(smem_u32(bar), parity); }
 __device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
