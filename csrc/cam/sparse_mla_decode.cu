@@ -41,6 +41,10 @@
 // a second exchange buffer (73.6), partials sent by bulk copies out of a sending buffer (79.7), the merge launched while the
 // splits run (1 x 2048 18.9 / 18.7, 23 x 1000 30.3 / 31.4).
 // All row addresses of the split are resolved once, up front, into shared memory (index -> page -> row).
+// What a call costs around its chunks (us of a call in a CUDA graph, before / after): the first tiles are on their way as soon as
+// their rows are known and while Q moves, the partner is only waited for where it is first written to; one warp sets the barriers up;
+// the result leaves through shared memory in whole pieces of rows; the last meeting of the two CTAs is signed up for before the
+// epilogue. 1 x 2048 keys in 22 splits 18.8 / 15.2, 23 x 1000 in 3 29.5 / 26.0, 61 x 70 13.0 / 11.1, 64 x 2048 71.9 / 70.9.
 // The running maximum is only raised when it grows by more than 8 (in log2 units); P then stays below 2^8 and the
 // accumulated O needs rescaling only a few times per row instead of in most chunks.
 // Every wait is bounded; a CTA that gives up raises the abort flag of both CTAs so the partner leaves at once.
@@ -85,12 +89,16 @@ constexpr int kOffK = 0;
 constexpr int kOffQ = kFreeStages * kStageBytes;
 constexpr int kOffX = kOffQ + kQBytes;
 constexpr int kOffRows = kOffX + kXBytes;
-constexpr int kOffMask = kOffRows + kMaxKeys * 4;   // one 64-bit validity mask per chunk
-constexpr int kOffMax = kOffMask + ((kMaxChunks * 8 + 63) / 64) * 64;   // [2][kSets][128] chunk maxima of the sets
+constexpr int kMaskWords = ((kMaxKeys + 31) / 32 + 2) / 2 * 2;   // a bit per key, and the word that the last chunk's 64 bits end in
+constexpr int kOffMask = kOffRows + kMaxKeys * 4;
+constexpr int kOffMax = kOffMask + (kMaskWords * 4 + 63) / 64 * 64;   // [2][kSets][128] chunk maxima of the sets
 constexpr int kOffTail = kOffMax + 2 * kSets * kHeads * 4;
 constexpr int kSmemBytes = 1024 + kOffTail + 256;
 static_assert(kSmemBytes <= 232448, "shared memory budget");
 static_assert(kStages * kStageBytes <= kOffX, "the stages end in Q's memory");
+// The epilogue's way out: 32 rows of 512 bytes per softmax warp, a pitch that keeps both directions free of bank conflicts.
+constexpr int kOutPitch = 512 + 16, kOutPitch16 = 256 + 16;
+static_assert(kSoftWarps * 32 * kOutPitch <= kOffX, "the epilogue's rows end in front of the exchange buffer");
 static_assert(kStageBytes % 1024 == 0 && kKSlabBytes % 1024 == 0, "swizzle atoms must stay 1024-byte aligned");
 
 struct MlaArgs {
@@ -186,7 +194,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   uint8_t* k_sm = smem + kOffK;
   float* x_sm = reinterpret_cast<float*>(smem + kOffX);
   int* rows_sm = reinterpret_cast<int*>(smem + kOffRows);
-  unsigned long long* mask_sm = reinterpret_cast<unsigned long long*>(smem + kOffMask);
+  uint32_t* mask_sm = reinterpret_cast<uint32_t*>(smem + kOffMask);
   float* max_sm = reinterpret_cast<float*>(smem + kOffMax);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kOffTail);
   uint64_t* bar_q = bars;            // 1
@@ -214,26 +222,29 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   const int num_chunks = (k_end - k_begin + kChunk - 1) / kChunk;   // at least one: splits without keys are not launched
   const int seq_len = a.seq_lens ? a.seq_lens[b] : 0x7fffffff;
 
-  if (tid == 0) {
-    mbar_init(bar_q, 1);
-    for (int i = 0; i < kStages; ++i) {
-      mbar_init(&bar_full[i], 1);
-      mbar_init(&bar_empty[i], 1);
-    }
-    for (int i = 0; i < kMlaBars; ++i) mbar_init(&bar_step[i], mla_of_softmax(i) ? kSoftWarps : 1);
-    for (int i = 0; i < 2; ++i) mbar_init(&bar_xld[i], 4);
-    mbar_init(bar_xfull, 1);
-    mbar_init(bar_xfree, kSoftWarps);
-    mbar_init(bar_qt, kSoftWarps);
+  if (warp == kThreads / 32 - 1) {
+    auto init = [&](uint64_t* bar, int n, uint32_t count) {
+      if (lane < n) mbar_init(bar + lane, count);
+    };
+    init(bar_q, 1, 1);
+    init(bar_full, 2 * kStages, 1);   // and bar_empty
+    if (lane < kMlaBars) mbar_init(&bar_step[lane], mla_of_softmax(lane) ? kSoftWarps : 1);
+    init(bar_xld, 2, 4);
+    init(bar_xfull, 1, 1);
+    init(bar_xfree, 1, kSoftWarps);
+    init(bar_qt, 1, kSoftWarps);
     mbar_fence_init();
-    *s_abort = 0;
-    fence_proxy_async_smem();   // the barrier's initial state, before the copy engine counts on it
-    mbar_expect_tx(bar_q, static_cast<uint32_t>(n_slabs) * kQSlabBytes);   // Q is on its way while the rows are resolved
-    for (int j = 0; j < n_slabs; ++j) {
-      const int dim0 = j < 4 ? half * 256 + j * 64 : 512;
-      tma_load_2d(q_sm + j * kQSlabBytes, &tmQ, bar_q, dim0, b * kHeads);
+    fence_proxy_async_smem();   // the barriers' initial state, before the copy engine counts on it
+    __syncwarp();
+    if (lane == 0) {
+      *s_abort = 0;
+      mbar_expect_tx(bar_q, static_cast<uint32_t>(n_slabs) * kQSlabBytes);   // Q is on its way while the rows are resolved
+      for (int j = 0; j < n_slabs; ++j) {
+        const int dim0 = j < 4 ? half * 256 + j * 64 : 512;
+        tma_load_2d(q_sm + j * kQSlabBytes, &tmQ, bar_q, dim0, b * kHeads);
+      }
+      tma_prefetch_desc(&tmKV);
     }
-    tma_prefetch_desc(&tmKV);
   }
   if (warp == kMmaWarp) {
     tmem_alloc(tmem_slot, kTmemCols);
@@ -257,24 +268,20 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
 #pragma unroll
     for (int i = 0; i < kRowsPerThread; ++i) {
       const int k = tid + i * kThreads;
-      if (k >= num_chunks * kChunk) break;
+      if (k - lane >= num_chunks * kChunk) break;   // whole warps
       int row = -1;
       if (idx[i] >= 0) {
         if (page[i] < 0 || page[i] >= a.num_pages) umdk_set_status(a.status, UMDK_ERR_OVERFLOW, UMDK_PH_NONE, b, idx[i]);
         else row = page[i] * kPage + (idx[i] % kPage);
       }
-      rows_sm[k] = row;
+      if (k < num_chunks * kChunk) rows_sm[k] = row;
+      const uint32_t takes_part = __ballot_sync(0xffffffffu, row >= 0);
+      if (lane == 0) mask_sm[k >> 5] = takes_part;
     }
-  }
-  __syncthreads();
-  for (int c = warp; c < num_chunks; c += kThreads / 32) {   // bit j of mask c: key j of chunk c takes part
-    const uint32_t lo = __ballot_sync(0xffffffffu, rows_sm[c * kChunk + lane] >= 0);
-    const uint32_t hi = __ballot_sync(0xffffffffu, lane < kChunk - 32 && rows_sm[c * kChunk + 32 + (lane & 15)] >= 0);
-    if (lane == 0) mask_sm[c] = static_cast<unsigned long long>(hi) << 32 | lo;
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();   // the partner's barriers exist before anything is signalled across
+  cluster_arrive();   // this CTA's barriers exist; a role waits for the partner's before it first signals across
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t peer = static_cast<uint32_t>(half ^ 1);
@@ -304,7 +311,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     // of shared memory again for each chunk (80 KB for 48 keys, more than everything else together), and the shared
     // memory's 128 bytes a clock are what this kernel runs out of first.
     bool ok = __all_sync(0xffffffffu, wait_bar<false>(bar_q, 0, s_abort));
-    if (!ok) give_up(UMDK_PH_TMA_FULL, 0);
+    const bool q_here = ok;
     for (int j = set; j < n_slabs; j += kSets) {
       const uint8_t* qrow = q_sm + j * kQSlabBytes + head * 128;
       uint32_t w[32];
@@ -322,6 +329,8 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(bar_qt);
+    cluster_wait();
+    if (!q_here) give_up(UMDK_PH_TMA_FULL, 0);
     const bool dg = a.diag != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0;
     long long dt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     long long t_prev = dg ? clock64() : 0;
@@ -364,7 +373,9 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         sr[4 * j4 + 2] = __float_as_uint(__uint_as_float(sr[4 * j4 + 2]) + xv.z);
         sr[4 * j4 + 3] = __float_as_uint(__uint_as_float(sr[4 * j4 + 3]) + xv.w);
       }
-      const uint32_t valid = static_cast<uint32_t>(mask_sm[c] >> key0) & ((1u << kSetKeys) - 1u);
+      const int key = c * kChunk + key0;   // a multiple of 8
+      const uint32_t valid = static_cast<uint32_t>((static_cast<uint64_t>(mask_sm[(key >> 5) + 1]) << 32 | mask_sm[key >> 5]) >> (key & 31)) &
+                             ((1u << kSetKeys) - 1u);
       if (valid != (1u << kSetKeys) - 1u) {   // the same for every thread of the set
 #pragma unroll
         for (int j = 0; j < kSetKeys; ++j)
@@ -450,11 +461,15 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       for (int i = 0; i < 8; ++i)
         if (i != 2 && i != 3) a.diag[i] = dt[i];
     }
+    cluster_arrive();   // the last word to the partner has been said
     // ---- epilogue: this CTA's 256 output columns, half of them per set ----
     // (every decision below is the same for all eight warps: the TMEM loads are warp-collective)
     if (ok) {
       ok = __all_sync(0xffffffffu, step_over(kMlaEnd, 0));
-      if (!ok) give_up(UMDK_PH_TMEM_EMPTY, 2000);
+      if (!ok) {   // the partner may have left
+        if (!*s_abort) umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_EMPTY, b, 2000);
+        *s_abort = 1;
+      }
     }
     // both sets' sums; the last chunk used the other half of max_sm
     max_sm[((num_chunks & 1) * kSets + set) * kHeads + head] = l_run;
@@ -464,13 +479,15 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     if (ok) {
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
       const float lse2 = l_run > 0.f ? m_run + log2f(l_run) : -INFINITY;
+      // A thread has a row of its own: stored from here, a warp's 16 bytes per lane would touch 32 rows each time (128 x 256 fp32:
+      // 11000 cycles, bf16 5000). The rows go through the memory of the key tiles and out in pieces of 512 or 256 bytes.
       const int col0 = set * 128;
+      uint8_t* const rows = smem + warp * (32 * kOutPitch);
       if (a.num_splits == 1) {
-        __nv_bfloat16* dst = a.out + ((size_t)b * kHeads + head) * kDimV + half * 256;
 #pragma unroll 1
-        for (int c0 = col0; c0 < col0 + 128; c0 += 32) {
+        for (int c0 = 0; c0 < 128; c0 += 32) {
           uint32_t o[32];
-          tmem_ld_x32(lane_addr + kColO + c0, o);
+          tmem_ld_x32(lane_addr + kColO + col0 + c0, o);
           tmem_ld_wait();
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
@@ -481,29 +498,41 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
                                                               __uint_as_float(o[q * 8 + 2 * i + 1]) * inv);
               w4[i] = *reinterpret_cast<const uint32_t*>(&hh);
             }
-            *reinterpret_cast<uint4*>(dst + c0 + q * 8) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+            *reinterpret_cast<uint4*>(rows + lane * kOutPitch16 + (c0 + q * 8) * 2) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
           }
         }
+        __syncwarp();
+        __nv_bfloat16* dst = a.out + ((size_t)b * kHeads + (warp & 3) * 32) * kDimV + half * 256 + col0;
+#pragma unroll 8
+        for (int r = lane >> 4; r < 32; r += 2)
+          *reinterpret_cast<uint4*>(dst + (size_t)r * kDimV + (lane & 15) * 8) =
+              *reinterpret_cast<const uint4*>(rows + r * kOutPitch16 + (lane & 15) * 16);
         if (half == 0 && set == 0 && a.lse) a.lse[(size_t)b * kHeads + head] = lse2 * 0.6931471805599453f;
       } else {
-        float* dst = a.part_o + (((size_t)b * a.num_splits + split) * kHeads + head) * kDimV + half * 256;
 #pragma unroll 1
-        for (int c0 = col0; c0 < col0 + 128; c0 += 32) {
+        for (int c0 = 0; c0 < 128; c0 += 32) {
           uint32_t o[32];
-          tmem_ld_x32(lane_addr + kColO + c0, o);
+          tmem_ld_x32(lane_addr + kColO + col0 + c0, o);
           tmem_ld_wait();
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
-            *reinterpret_cast<float4*>(dst + c0 + q * 4) =
+            *reinterpret_cast<float4*>(rows + lane * kOutPitch + (c0 + q * 4) * 4) =
                 make_float4(__uint_as_float(o[q * 4]) * inv, __uint_as_float(o[q * 4 + 1]) * inv,
                             __uint_as_float(o[q * 4 + 2]) * inv, __uint_as_float(o[q * 4 + 3]) * inv);
           }
         }
+        __syncwarp();
+        float* dst = a.part_o + (((size_t)b * a.num_splits + split) * kHeads + (warp & 3) * 32) * kDimV + half * 256 + col0;
+#pragma unroll 8
+        for (int r = 0; r < 32; ++r)
+          *reinterpret_cast<float4*>(dst + (size_t)r * kDimV + lane * 4) =
+              *reinterpret_cast<const float4*>(rows + r * kOutPitch + lane * 16);
         if (half == 0 && set == 0) a.part_lse[((size_t)b * a.num_splits + split) * kHeads + head] = lse2;
       }
     }
   } else if (warp == kMmaWarp) {
     // ===================================== MMA issuer ===================================================
+    cluster_wait();
     if (elect_one()) {
       constexpr uint32_t idesc_qk = umma_idesc(kFmtBF16, kFmtBF16, kHeads, kChunk);
       constexpr uint32_t idesc_pv = umma_idesc(kFmtBF16, kFmtBF16, kHeads, 256, 0, 1);
@@ -583,6 +612,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     }
   } else if (warp >= kExchangeWarp && warp < kMmaWarp) {
     // ===================================== exchange (warps 8..11) =======================================
+    cluster_wait();
     const int head = (warp & 3) * 32 + lane;   // == TMEM lane
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
     const uint32_t peer_x = map_to_cta(x_sm, peer) + static_cast<uint32_t>(head) * 16u;
@@ -643,6 +673,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     for (int c = 0; c < num_chunks && ok; ++c) {
       const int st = c % kStages;
       if (c == kFreeStages) {   // from here on in Q's memory
+        cluster_wait();         // the first tiles are on their way without the partner
         ok = __all_sync(0xffffffffu, wait_bar<false>(bar_qt, 0, s_abort));
         if (!ok) {
           if (lane == 0) give_up(UMDK_PH_TMA_EMPTY, 4000);
@@ -675,10 +706,13 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       }
       lap(1);
     }
+    if (num_chunks <= kFreeStages) cluster_wait();
     if (dg) {
       for (int i = 0; i < 2; ++i) a.diag[13 + i] = dt[i];
     }
   }
+  __syncwarp();
+  if (warp >= kSoftWarps) cluster_arrive();
   tc_fence_before();
   __syncthreads();
   if (warp == kMmaWarp) {
@@ -687,7 +721,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
   }
-  cluster_sync_all();   // neither CTA leaves while the other may still write into its shared memory
+  cluster_wait();   // neither CTA leaves while the other may still write into its shared memory
 }
 
 // Joins the key-list splits that have keys (the first `live` of num_splits): out = sum_i exp2(lse_i - lse) * o_i. One CTA per
