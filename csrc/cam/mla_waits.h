@@ -1,4 +1,4 @@
-// Barriers between the softmax warps, the MMA issuer and the tensor core of sparse_mla_decode.cu, and the phase of them that says
+// Barriers between the softmax warps, the MMA issuers and the tensor core of sparse_mla_decode.cu, and the phase of them that says
 // that a step of chunk c is over. A wait names only the parity of a phase: it may stand only where the phase BEFORE the one that
 // it means is known to be over (else it returns at once) and the one AFTER it cannot be (else it never returns). The kernel takes
 // its barriers and parities from here; tests/test_mla_waits.py walks through all orders in which the roles can run.
@@ -15,12 +15,17 @@ namespace umdk {
 
 enum MlaStep : int {
   kMlaS,     // S(c) = Q * K(c) is in TMEM: one commit
-  kMlaP,     // P(c) has taken its place: an arrival of every softmax warp
+  kMlaP,     // P(c) is in TMEM: an arrival of every warp of the set that has the chunk
   kMlaO,     // P(c) * V(c) has been added to O: one commit, for all chunks but the last
-  kMlaEnd,   // every MMA of the split is through: one commit, c is ignored
+  kMlaEnd,   // every MMA of the split is through: a commit of each issuer, c is ignored
+  kMlaRead,  // S(c) has been read: the warps of the chunk's set and the exchange warps
+  kMlaFree,  // the issuer of P * V has seen kMlaO of c: P(c + 2) may be written
+  kMlaMax,   // the maximum that P(c) is relative to is known: one warp of the set (this barrier + the number of its 32 heads)
 };
-constexpr int kMlaBars = 6;
-MLA_HD constexpr bool mla_of_softmax(int bar) { return bar == 2 || bar == 3; }   // which of them the softmax warps arrive at
+constexpr int kMlaBars = 13;
+MLA_HD constexpr int mla_arrivals(int bar) {
+  return bar == 2 || bar == 3 ? 4 : bar == 5 ? 2 : bar == 6 ? 8 : 1;
+}
 
 struct MlaWait {
   int bar;   // of kMlaBars
@@ -29,17 +34,24 @@ struct MlaWait {
 
 MLA_HD constexpr MlaWait mla_wait(MlaStep step, int c) {
   switch (step) {
-    // Two barriers in turn: S(c) is made only when P(c-2) * V is through, so everybody has seen S(c-2) and P(c-2) by then.
+    // Two barriers in turn, as the sets are: with one, a set that waits for S(c) could take S(c-2) for it. S(c+2) is made behind
+    // the reads of S(c+1), and that one behind those of S(c), so nobody misses a phase.
     case kMlaS: return {c & 1, (uint32_t)(c >> 1) & 1u};
-    // With a single one the softmax warps, who need only S(c+1) for it, could all arrive for P(c+1) before the issuer has looked
-    // for P(c): a phase that is gone by, and both would wait for each other.
+    // With a single one both sets could be through with their chunks before the issuer has looked for the first: a phase that is
+    // gone by, and everybody would wait for each other.
     case kMlaP: return {2 + (c & 1), (uint32_t)(c >> 1) & 1u};
-    // The issuer waits for c - 2 before it makes S(c), the softmax warps for c - 1 where they rescale O behind S(c): in both places
-    // the phase before is over, and the next one needs the S or P that the waiting role still has to make.
+    // The issuer waits for every phase. The softmax warps wait for c - 1 where they rescale O for P(c): kMlaFree has told them that
+    // c - 2 is over, and c needs their P.
     case kMlaO: return {4, (uint32_t)c & 1u};
     // A barrier with a single phase: behind the last chunk only P(n-3) * V is known to be through, and kMlaO's barrier in that
     // phase would let a wait for P(n-1) * V pass before the last two products.
-    default: return {5, 0u};
+    case kMlaEnd: return {5, 0u};
+    // S(c+1) is made behind this phase, so the next one cannot be over; the issuer has waited for all before.
+    case kMlaRead: return {6, (uint32_t)c & 1u};
+    // Two barriers in turn: P(c+1) may be through before the set of P(c) looks for its buffer.
+    case kMlaFree: return {7 + (c & 1), (uint32_t)(c >> 1) & 1u};
+    // Waited for by the warp that ends the phases before and after it.
+    default: return {9, (uint32_t)c & 1u};
   }
 }
 
