@@ -9,6 +9,7 @@
 // disappears; rows of one expert are ordered by source rank, then by (token, k) - the same order as the reference's
 // compacted expandX (status index = localExpert * R + srcRank, :625-633).
 #include "ep_ll_dispatch.cuh"
+#include "ep_params.h"
 
 namespace umdk {
 namespace {
@@ -246,19 +247,6 @@ UMDK_API int umdk_ep_ll_layout(int R, int E, int K, int H, int T_cap, UmdkEpLLLa
   return 0;
 }
 
-struct UmdkEpLLDispatchParams {
-  int R, rank, E, K, H, T_cap, T, num_ctas, phase_mask;
-  void* peers[kMaxRanks];
-  const void* x;
-  const int64_t* topk_idx;
-  const int* send_idx;
-  const int* num_per_expert;
-  int* group_off;
-  int64_t* recv_per_expert;
-  uint32_t* ctrl;
-  int* status;
-};
-
 // CTAs of a dispatch on a GPU with `sms` SMs. num_ctas 0, one rank: an item (2 KiB of a token) for every warp, 32 CTAs at least.
 // 32 / as many as that, us, with the combine: 142 tokens of 6656, top-1 of 160 16.3 / 13.0, 256 of 7168, top-8 of 256
 // 40.4 / 34.5; no difference where 32 hold all items. With more ranks always 32: every CTA waits for the peers' counts, and
@@ -271,6 +259,8 @@ UMDK_API int umdk_ep_ll_dispatch_grid(int R, int T, int H, int num_ctas, int sms
   else if (R == 1 && items > 32 * kLLWarps) grid = (items + kLLWarps - 1) / kLLWarps;
   return grid < sms ? grid : sms;
 }
+
+static_assert(kUmdkMaxRanks == kMaxRanks, "parameter blocks");
 
 UMDK_API int umdk_ep_ll_dispatch(const UmdkEpLLDispatchParams* p, void* stream) {
   LLDispatchArgs a;
@@ -306,18 +296,6 @@ UMDK_API int umdk_ep_ll_dispatch(const UmdkEpLLDispatchParams* p, void* stream) 
   UMDK_CUDA_CHECK(cudaGetLastError());
   return 0;
 }
-
-struct UmdkEpLLCombineParams {
-  int R, rank, E, K, H, T_cap, T, num_ctas, phase_mask;
-  void* peers[kMaxRanks];
-  const void* y;
-  const int* group_off;
-  const int64_t* topk_idx;
-  const float* topk_w;
-  void* out;
-  uint32_t* ctrl;
-  int* status;
-};
 
 UMDK_API int umdk_ep_ll_combine(const UmdkEpLLCombineParams* p, void* stream) {
   LLCombineArgs a;

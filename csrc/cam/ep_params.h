@@ -1,4 +1,4 @@
-// Argument blocks of the normal-mode expert-parallel entry points, shared with the Python call path (csrc/pycalls/calls.cpp).
+// Argument blocks of the expert-parallel entry points that the Python call path (csrc/pycalls/calls.cpp) uses too.
 #pragma once
 #include <stdint.h>
 
@@ -49,4 +49,29 @@ struct UmdkEpCombineParams {
   int* status;
   long long* diag;   // optional [R] per-source wait times in ns (diagnose mode), else null
   int a_cap;         // mode 0: arrivals that recv_meta has room for
+};
+
+struct UmdkEpLLDispatchParams {
+  int R, rank, E, K, H, T_cap, T, num_ctas, phase_mask;
+  void* peers[kUmdkMaxRanks];
+  const void* x;
+  const int64_t* topk_idx;
+  const int* send_idx;         // null: the dispatch derives positions and sizes itself
+  const int* num_per_expert;
+  int* group_off;
+  int64_t* recv_per_expert;
+  uint32_t* ctrl;
+  int* status;
+};
+
+struct UmdkEpLLCombineParams {
+  int R, rank, E, K, H, T_cap, T, num_ctas, phase_mask;
+  void* peers[kUmdkMaxRanks];
+  const void* y;
+  const int* group_off;
+  const int64_t* topk_idx;
+  const float* topk_w;
+  void* out;
+  uint32_t* ctrl;
+  int* status;
 };

@@ -204,6 +204,7 @@ class EpLowLatency(Recoverable):
         # the fields of the argument blocks that no call changes; every call works on a copy
         self._dispatch_base = self._base(_LLDispatchParams(), recv_per_expert=self.recv_per_expert)
         self._combine_base = self._base(_LLCombineParams())
+        self._dispatch_addr, self._combine_addr = ctypes.addressof(self._dispatch_base), ctypes.addressof(self._combine_base)
 
     def _base(self, p, **tensors):
         p.R, p.rank, p.E, p.K, p.H, p.T_cap = self.R, self.rank, self.E, self.K, self.H, self.T_cap
@@ -263,16 +264,9 @@ class EpLowLatency(Recoverable):
             2 * (((T + 31) // 32) * self.E + 2 * T * self.K) <= 160 * 1024
         if lay is None and not inline:
             lay = ep_layout(topk_idx, self.E, self.R, self.layout_scratch, self.layout_bar, self.status)
-        p = _LLDispatchParams.from_buffer_copy(self._dispatch_base)
-        p.T, p.num_ctas, p.phase_mask = T, self.dispatch_ctas, phase_mask
-        p.x, p.topk_idx = x.data_ptr(), topk_idx.data_ptr()
-        if lay is not None:
-            p.send_idx, p.num_per_expert = lay.send_token_idx.data_ptr(), lay.num_tokens_per_expert.data_ptr()
-        else:
-            p.send_idx = p.num_per_expert = None
-        rc = self.lib.umdk_ep_ll_dispatch(ctypes.byref(p), _native.stream_ptr())
-        if rc != 0:
-            raise RuntimeError(f"umdk_ep_ll_dispatch failed: {rc}")
+        _native.LAUNCH_COUNT += 1
+        sidx, npe = (lay.send_token_idx, lay.num_tokens_per_expert) if lay is not None else (None, None)
+        _native.calls().ll_dispatch(self._dispatch_addr, x, topk_idx, sidx, npe, self.dispatch_ctas, phase_mask)
         return lay
 
     @_trace.traced("umdk.ep_ll.combine")
@@ -285,19 +279,12 @@ class EpLowLatency(Recoverable):
         assert y.is_cuda and y.dtype == torch.bfloat16 and y.is_contiguous() and y.shape[1] == self.H
         assert y.shape[0] >= min(self.n_cap, y.shape[0]) and topk_idx.dtype == torch.int64 and topk_idx.is_contiguous()
         T = topk_idx.shape[0]
-        if out is None:
-            out = torch.empty(T, self.H, dtype=torch.bfloat16, device=y.device)
-        elif self.R == 1 and (phase_mask or 3) == 3 and overlap(out, y):
+        if out is not None and self.R == 1 and (phase_mask or 3) == 3 and overlap(out, y):
             # one rank stores each sum while others are still formed: not into the rows they are formed from
             out.as_strided((T, self.H), (self.H, 1)).copy_(self.combine(y, topk_idx, topk_w, num_ctas=num_ctas))
             return out
-        p = _LLCombineParams.from_buffer_copy(self._combine_base)
-        p.T, p.num_ctas, p.phase_mask = T, num_ctas, phase_mask
-        p.y, p.topk_idx, p.topk_w, p.out = y.data_ptr(), topk_idx.data_ptr(), topk_w.data_ptr(), out.data_ptr()
-        rc = self.lib.umdk_ep_ll_combine(ctypes.byref(p), _native.stream_ptr())
-        if rc != 0:
-            raise RuntimeError(f"umdk_ep_ll_combine failed: {rc}")
-        return out
+        _native.LAUNCH_COUNT += 1
+        return _native.calls().ll_combine(self._combine_addr, y, topk_idx, topk_w, out, num_ctas, phase_mask)
 
     def _gemm1(self, w: ExpertWeights):
         p = moe_gemm.MoeGemmParams()
