@@ -15,7 +15,7 @@ namespace umdk {
 
 enum MlaStep : int {
   kMlaS,     // S(c) = Q * K(c) is in TMEM: one commit
-  kMlaP,     // P(c) is in TMEM: an arrival of every warp of the set that has the chunk
+  kMlaP,     // P(c) is in TMEM: an arrival of every warp of the set that has the chunk and of those that take the partner's in
   kMlaO,     // P(c) * V(c) has been added to O: one commit, for all chunks but the last
   kMlaEnd,   // every MMA of the split is through: a commit of each issuer, c is ignored
   kMlaRead,  // S(c) has been read: the warps of the chunk's set and the exchange warps
@@ -24,7 +24,7 @@ enum MlaStep : int {
 };
 constexpr int kMlaBars = 13;
 MLA_HD constexpr int mla_arrivals(int bar) {
-  return bar == 2 || bar == 3 ? 4 : bar == 5 ? 2 : bar == 6 ? 8 : 1;
+  return bar == 2 || bar == 3 ? 8 : bar == 5 ? 2 : bar == 6 ? 8 : 1;
 }
 
 struct MlaWait {

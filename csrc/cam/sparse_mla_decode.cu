@@ -11,40 +11,46 @@
 // Per chunk of 48 selected keys each CTA
 //   gathers only ITS dims of the 48 rows (640 or 512 bytes per row; no byte of the cache is read twice),
 //   computes a PARTIAL S[128 x 48] = Q[:, own dims] * K[:, own dims]^T   (20 or 16 MMAs of K = 16),
-//   sends the partial to its partner through distributed shared memory and adds the partner's partial,
-//   runs the online softmax (one head per thread; both CTAs arrive at the same P),
+//   sends the partial of half of the heads (16 of every 32) to its partner through distributed shared memory and adds the partner's
+//   partial to the other half,
+//   runs the online softmax of that half and sends P (and, where the maximum rises, the factors for O) to the partner,
 //   and accumulates its own 256 output columns O[128 x 256] += P[128 x 48] * V[48 x own latent dims]  (3 MMAs),
 //   reading V from the SAME gathered tile through an MN-major descriptor.
 // Splitting by dimension halves the resident Q (80 KB instead of 144 KB), which makes room for a ring of key tiles, and
 // halves the Q*K^T work of each SM. Q moves to TMEM before the first chunk and P never leaves it: both are A operands read
-// out of TMEM, so that shared memory (128 bytes a clock) only feeds the key tiles to the MMAs; two of the five stages of the
+// out of TMEM, so that shared memory (128 bytes a clock) only feeds the key tiles to the MMAs; three of the six stages of the
 // ring lie where Q was.
-// TMEM columns: S 48, two P of 24, Q 160, O 256. Roles inside a CTA (20 warps):
-//   warps 0-7  softmax in two sets of four, which take whole chunks in turn: tcgen05.ld of S, add the partner's partial,
-//              maximum (passed on from set to set), exp2, P to TMEM, lazy rescale of O
-//   warps 8-11 exchange: tcgen05.ld of the same S and asynchronous stores of it into the partner's shared memory,
-//              so that the round trip between the two CTAs is off the softmax warps' critical path
-//   warps 12, 13 MMA issuers (one elected thread each), of Q * K^T and of P * V: S(c + 2) is made while the softmax of c runs
-//   warps 14-19 gather producers: TMA tile::gather4 copies (four selected rows x 128 bytes per instruction, written
+// TMEM columns: S 48, two P of 24, Q 160, O 256. Roles inside a CTA (24 warps):
+//   warps 0-7  softmax in two sets of four, which take whole chunks in turn: tcgen05.ld of S, add the partner's partial, maximum
+//              (passed on from set to set), exp2, P to the partner and to TMEM, lazy rescale of O
+//   warps 8-11 tcgen05.ld of the other heads' S and asynchronous stores of it into the partner's shared memory
+//   warps 12-15 the partner's P from shared memory to TMEM, its rescale of O
+//   warps 16, 17 MMA issuers (one elected thread each), of Q * K^T and of P * V: S(c + 2) is made while the softmax of c runs
+//   warps 18-23 gather producers: TMA tile::gather4 copies (four selected rows x 128 bytes per instruction, written
 //              in the 128-byte-swizzled layout the MMA descriptors expect), completion counted in bytes on the
-//              stage's barrier. A warp issues its lanes' copies some 80 cycles apart and different warps side by side:
+//              stage's barrier. A warp issues its lanes' copies some 100 cycles apart and different warps side by side:
 //              48-key tiles of 640-byte pieces from 128 CTAs take 96 us for 2048 keys out of one warp, 57 us out of two,
 //              45 us out of four or more (3.7 TB/s of random 640-byte reads; 22 bytes per SM and clock when they hit
-//              L2). Gathering with 16-byte cp.async reaches the same 15 - 19 bytes with 16 warps, plain loads half of it.
-// What bounds it now: a stage of the ring is filled in 3100 cycles (1200 of issue, 1900 until the last row is there) and held for
-// 6400 (Q * K^T 600, 1250 of it waiting for S's columns; partials on their way 1400; add and maximum 900, exp2 750, P to TMEM 950,
-// P * V 600): five stages give one chunk per 1930 cycles. The st.async of the partials (24 KB a chunk, 24 bytes a clock) keep the
-// shared-memory queue that every barrier and load of the softmax goes through busy half of the time. With one set of eight
-// warps a chunk (24 keys a thread) the softmax chain itself was the limit, 2600 cycles. Batch 64, 2048 of 32768 keys: 70.9 / 62.5 us,
-// 128 x 1024 79.9 / 69.8, 23 x 1000 in three splits 26.0 / 24.7 (the rope dims in CTA 0 alone: 62.6, 71.3, 24.9); splits of one or two
-// chunks have nothing to overlap and pay for a thread's 48 keys: 61 x 70 11.1 / 11.4, 1 x 2048 15.2 / 15.5. In between (one set): Q
-// as an A operand in shared memory kept one thread issuing MMAs for 2240 cycles a chunk; copies by cp.async or plain loads, partials
-// by bulk copies out of a sending buffer (79.7 against 73.9 us), the merge launched while the splits run were no faster, nor (two
-// sets) are rows fetched into L2 ahead of the gather (62.5 / 66.9).
-// What a call costs around its chunks (us of a call in a CUDA graph, before / after): the first tiles are on their way as soon as
-// their rows are known and while Q moves, the partner is only waited for where it is first written to; one warp sets the barriers up;
-// the result leaves through shared memory in whole pieces of rows; the last meeting of the two CTAs is signed up for before the
-// epilogue. 1 x 2048 keys in 22 splits 18.8 / 15.2, 23 x 1000 in 3 29.5 / 26.0, 61 x 70 13.0 / 11.1, 64 x 2048 71.9 / 70.9.
+//              L2). Gathering with 16-byte cp.async reaches 15 - 19 bytes with 16 warps, plain loads half of it.
+// What bounds it now: the gather. A tile is filled in 2950 cycles (1050 of issue, 1900 until the last row is there) and held until
+// P * V is through; six stages give one chunk per 1600 cycles, of which the copies' issue alone takes 1080. How it got there (us in a CUDA
+// graph, 64 x 2048 / 128 x 1024 / 23 x 1000 in three splits / 61 x 70 keys):
+//   both sets on one chunk, 24 keys a thread (a chain of 2600 cycles a chunk)           70.9 / 79.9 / 26.0 / 11.1
+//   sets in turn, S in one buffer that is free once read, P in two, two MMA issuers      62.6 / 71.3 / 24.9 / 11.7
+//   the rope dims in turn (54 copies a chunk for both CTAs instead of 60 and 48)         62.5 / 69.8 / 24.7 / 11.4
+//   softmax of half of the heads (24 KB of st.async a chunk had filled the queue that every barrier and load goes through)
+//                                                                                        57.5 / 65.5 / 24.1 / 11.7
+//   six stages                                                                           56.3 / 64.5 / 24.1 / 11.8
+//   relaxed arrivals of the cluster barriers, descriptors fetched first                  56.4 / 64.0 / 23.5 / 11.2
+//   masked keys read another key's row instead of row 0, which had been the same few lines of L2 for all; nothing is fetched or
+//   multiplied behind the end of a list                                                  56.5 / 63.5 / 23.2 /  9.6
+// Tried and left out: rows fetched into L2 ahead of the gather (62.5 / 66.9), copies by cp.async or plain loads, partials by bulk copies
+// out of a sending buffer, the merge launched while the splits run; the epilogue from 16 warps or by bulk stores: it stores 32
+// bytes a clock (64 KB of result or 128 KB of partials per CTA, 2000 or 4000 cycles) whoever issues them.
+// Around its chunks a call starts the first tiles as soon as their rows are known and while Q moves; the partner is only waited for
+// where it is first written to; one warp sets the barriers up; the result leaves through shared memory in whole pieces of rows; the
+// last meeting of the two CTAs is signed up for before the epilogue. All row addresses of a split are resolved once, up front, into
+// shared memory (index -> page -> row).
 // The running maximum is only raised when it grows by more than 8 (in log2 units); P then stays below 2^8 and the
 // accumulated O needs rescaling only a few times per row instead of in most chunks.
 // Every wait is bounded; a CTA that gives up raises the abort flag of both CTAs so the partner leaves at once.
@@ -61,22 +67,26 @@ constexpr int kDim = 576;
 constexpr int kDimV = 512;
 constexpr int kPage = 64;
 constexpr int kChunk = 48;                       // keys per pipeline step
-constexpr int kStages = 5;
+constexpr int kStages = 6;                       // an even number: a stage has the rope slab always or never
 constexpr int kFreeStages = 3;   // the others lie where Q is until it has moved to TMEM
-constexpr int kMaxSlabs = 5;                     // 64-dim slabs per CTA: 4 latent (+ 1 rope in CTA 0)
+constexpr int kMaxSlabs = 5;                     // 64-dim slabs of a chunk in a CTA: 4 latent, and rope in every other one
 constexpr int kQSlabBytes = kHeads * 128;        // 16 KB
 constexpr int kKSlabBytes = kChunk * 128;        // 6 KB
 constexpr int kQBytes = kMaxSlabs * kQSlabBytes; // 81920
-constexpr int kStageBytes = kMaxSlabs * kKSlabBytes;  // 30720
-constexpr int kXBytes = kChunk * kHeads * 4;     // 24 KB, [key / 4][head][4] fp32; two of them, for chunks in turn
+constexpr int kTwoStages = (2 * kMaxSlabs - 1) * kKSlabBytes;   // 55296
+constexpr int kOwnHeads = kHeads / 2;             // heads whose softmax a CTA makes: 16 of every 32
+constexpr int kXBytes = kChunk * kOwnHeads * 4;   // 12 KB, [6][128 threads][4] fp32; two of them, for chunks in turn
+constexpr int kPBytes = kChunk * kOwnHeads * 2;   // 6 KB, [3][128 threads][4] pairs of bf16
+constexpr int kPinBytes = kPBytes + 128 * 8;      // and what O is rescaled by, for the two heads of a thread; two of them
 constexpr int kMaxChunks = 43;                   // 2064 keys per split at most
 constexpr int kMaxKeys = kMaxChunks * kChunk;
 constexpr int kSets = 2;            // softmax warp sets: set s (warps 4s .. 4s + 3) takes chunks s, s + 2, ...
 constexpr int kSoftWarps = 4 * kSets;
 constexpr int kExchangeWarp = kSoftWarps;        // warps 8..11
-constexpr int kMmaWarp = kExchangeWarp + 4;      // warp 12: Q * K^T
-constexpr int kPvWarp = kMmaWarp + 1;            // warp 13: P * V
-constexpr int kProducerWarp = kPvWarp + 1;       // warps 14..19
+constexpr int kPinWarp = kExchangeWarp + 4;      // warps 12..15
+constexpr int kMmaWarp = kPinWarp + 4;           // warp 16: Q * K^T
+constexpr int kPvWarp = kMmaWarp + 1;            // warp 17: P * V
+constexpr int kProducerWarp = kPvWarp + 1;       // warps 18..23
 constexpr int kProducerWarps = 6;
 constexpr int kThreads = 32 * (kProducerWarp + kProducerWarps);
 constexpr int kRowsPerThread = (kMaxKeys + kThreads - 1) / kThreads;
@@ -87,22 +97,24 @@ constexpr int kColQ = 2 * kChunk;                // Q as bf16 pairs, 32 columns 
 constexpr int kColO = 256;
 static_assert(kColQ + kMaxSlabs * 32 <= kColO, "TMEM budget");
 constexpr int kOffK = 0;
-constexpr int kOffQ = kFreeStages * kStageBytes;
-constexpr int kOffX1 = kStages * kStageBytes;      // begins in Q's memory: the partner writes there once Q has left it
-constexpr int kOffX0 = kOffX1 + kXBytes;
-constexpr int kOffRows = kOffX0 + kXBytes;
+constexpr int kOffQ = kFreeStages * kMaxSlabs * kKSlabBytes;
+// What the partner sends. Its P may lie where Q was: the softmax behind it had this CTA's S, which was made of Q in TMEM.
+constexpr int kOffPin = kStages / 2 * kTwoStages;
+constexpr int kOffX = kOffPin + 2 * kPinBytes;
+constexpr int kOffRows = kOffX + 2 * kXBytes;
 constexpr int kMaskWords = ((kMaxKeys + 31) / 32 + 2) / 2 * 2;   // a bit per key, and the word that the last chunk's 64 bits end in
 constexpr int kOffMask = kOffRows + kMaxKeys * 4;
-constexpr int kOffMax = kOffMask + (kMaskWords * 4 + 63) / 64 * 64;   // [2][128] running maxima of the last two chunks
-constexpr int kOffSum = kOffMax + 2 * kHeads * 4;   // [kSets][128] (sum, its maximum) of the sets
-constexpr int kOffTail = kOffSum + kSets * kHeads * 8;
+constexpr int kOffMax = kOffMask + (kMaskWords * 4 + 63) / 64 * 64;   // [2][64] running maxima of the last two chunks
+constexpr int kOffSum = kOffMax + 2 * kOwnHeads * 4;   // [kSets][64] (sum, its maximum) of the sets
+constexpr int kOffInv = kOffSum + kSets * kOwnHeads * 8;   // [128] factors of the result's rows
+constexpr int kOffTail = kOffInv + kHeads * 4;
 constexpr int kSmemBytes = 1024 + kOffTail + 512;
 static_assert(kSmemBytes <= 232448, "shared memory budget");
-static_assert(kStages * kStageBytes <= kOffQ + kQBytes && kOffQ + kQBytes <= kOffX0, "what lies in Q's memory waits for it");
+static_assert(kStages % 2 == 0 && kOffQ + kQBytes <= kOffX, "partials come in while Q is where it was");
 // The epilogue's way out: 32 rows of 512 bytes per softmax warp, a pitch that keeps both directions free of bank conflicts.
 constexpr int kOutPitch = 512 + 16, kOutPitch16 = 256 + 16;
-static_assert(kSoftWarps * 32 * kOutPitch <= kOffX1, "the epilogue's rows end in front of the exchange buffers");
-static_assert(kStageBytes % 1024 == 0 && kKSlabBytes % 1024 == 0, "swizzle atoms must stay 1024-byte aligned");
+static_assert(kSoftWarps * 32 * kOutPitch <= kOffPin, "the epilogue's rows end in front of the exchange buffers");
+static_assert(kOffQ % 1024 == 0 && kKSlabBytes % 1024 == 0, "swizzle atoms must stay 1024-byte aligned");
 
 struct MlaArgs {
   const __nv_bfloat16* kv;   // [num_pages, 64, 576]
@@ -117,8 +129,8 @@ struct MlaArgs {
   float scale_log2;
   int* status;
   // optional [16] cycle counters of the first CTA (diagnose mode). Softmax thread 0 (chunks 0, 2, ...): [0] wait S, [1] TMEM
-  // load, [4] wait partner's partial, [5] add + max, wait for the other set's maximum, exp2, [6] wait for P's buffer (and for the
-  // P*V before a rescale), [7] rescale + P store. Exchange thread 0: [2] wait partner-free, [3] remote stores. Q*K thread: [8]
+  // load, [4] wait partner's partial, [5] add + max, wait for the other set's maximum, exp2, [6] send P, wait for P's buffer (and
+  // for the P*V before a rescale), [7] rescale + P store. Exchange thread 0: [2] wait partner-free, [3] remote stores. Q*K thread: [8]
   // wait tile, [9] wait until S has been read, [11] issue, [15] all of it once Q is in TMEM. P*V thread: [10] wait P, [12] issue
   // and wait for the product before. First producer warp: [13] wait free stage, [14] issue.
   long long* diag;
@@ -137,6 +149,20 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatil
     }
   }
   return true;
+}
+// Whether the phase is over, without waiting for it.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
 }
 // Asynchronous 16-byte store into the partner CTA's shared memory; the bytes are counted on the partner's mbarrier
 // (complete_tx), so the sender needs no release fence that would wait for every store to be acknowledged.
@@ -168,16 +194,51 @@ __device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, ui
       "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void tmem_st_x8(uint32_t taddr, const uint32_t* r) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
-               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
-__device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t* r) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+// registers -> TMEM of 16 lanes; see tmem_ld_16x256b_x1 for the lanes and columns of a thread
+__device__ __forceinline__ void tmem_st_16x256b_x4(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
                "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
                "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
                : "memory");
+}
+// the same for 4 N columns: a thread has one column of every four, of lanes t / 4 (first register) and t / 4 + 8 (the next)
+__device__ __forceinline__ void tmem_st_16x128b_x4(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st_16x128b_x2(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
+               : "memory");
+}
+__device__ __forceinline__ void st_async_v2(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t cluster_bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(cluster_addr), "r"(a),
+               "r"(b), "r"(cluster_bar)
+               : "memory");
+}
+// S of 16 heads (lanes) x 48 keys: register 4 i + j of thread t is head t / 4 (j < 2) or t / 4 + 8, key 8 i + 2 (t % 4) + j % 2.
+__device__ __forceinline__ void load_scores(uint32_t taddr, uint32_t* r) {
+  tmem_ld_16x256b_x4(taddr, r);
+  tmem_ld_16x256b_x2(taddr + 32, r + 16);
+  tmem_ld_wait();
+}
+// P of the same heads and keys, a pair of keys per register: 2 i of head t / 4, 2 i + 1 of head t / 4 + 8.
+__device__ __forceinline__ void store_probs(uint32_t taddr, const uint32_t* pk) {
+  tmem_st_16x128b_x4(taddr, pk);
+  tmem_st_16x128b_x2(taddr + 16, pk + 8);
+}
+// O (256 columns) of 16 heads, `a` for head t / 4 and `b` for head t / 4 + 8 of thread t.
+__device__ __forceinline__ void rescale_o(uint32_t taddr, float a, float b) {
+#pragma unroll 1
+  for (int c0 = 0; c0 < 256; c0 += 32) {
+    uint32_t o[16];
+    tmem_ld_16x256b_x4(taddr + c0, o);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * ((j & 2) ? b : a));
+    tmem_st_16x256b_x4(taddr + c0, o);
+  }
+  tmem_st_wait();
 }
 // 2^x with the special-function unit's native approximation (2 ulp; -inf gives 0): P is rounded to bf16 anyway.
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -199,6 +260,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   int* rows_sm = reinterpret_cast<int*>(smem + kOffRows);
   uint32_t* mask_sm = reinterpret_cast<uint32_t*>(smem + kOffMask);
   float* max_sm = reinterpret_cast<float*>(smem + kOffMax);
+  float* inv_sm = reinterpret_cast<float*>(smem + kOffInv);
   float2* sum_sm = reinterpret_cast<float2*>(smem + kOffSum);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kOffTail);
   uint64_t* bar_q = bars;            // 1
@@ -208,11 +270,13 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   uint64_t* bar_full = bars + 1;     // kStages, one arrival that expects the tile's bytes from the TMA gathers
   uint64_t* bar_empty = bar_full + kStages;    // kStages, one commit
   uint64_t* bar_step = bar_empty + kStages;    // kMlaBars: see mla_waits.h
-  uint64_t* bar_xfull = bar_step + kMlaBars;   // 2, one local arrival that expects the 24 KB the partner's st.async stores deliver
-  uint64_t* bar_xfree = bar_xfull + 2;   // 2, 4 arrivals from a set of the partner's softmax warps: its X may be overwritten
-  uint64_t* bar_xq = bar_xfull + 4;      // 8 arrivals from the partner's softmax warps: Q has left the memory of its second X
-  uint64_t* bar_qt = bar_xfull + 5;      // 8 softmax-warp arrivals: Q is in TMEM
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_xfull + 6);
+  uint64_t* bar_xfull = bar_step + kMlaBars;   // 2, one local arrival that expects the partial that the partner's st.async deliver
+  uint64_t* bar_pfull = bar_xfull + 2;   // 2, the same for the partner's P
+  uint64_t* bar_inv = bar_xfull + 4;     // the same for the partner's factors of the result
+  uint64_t* bar_xfree = bar_xfull + 5;   // 2, 4 arrivals from a set of the partner's softmax warps: its X may be overwritten
+  uint64_t* bar_pfree = bar_xfull + 7;   // 2, 4 arrivals from the partner's warps that take P in
+  uint64_t* bar_qt = bar_xfull + 9;      // 8 softmax-warp arrivals: Q is in TMEM
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_xfull + 10);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -225,8 +289,16 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   const int num_chunks = (k_end - k_begin + kChunk - 1) / kChunk;   // at least one: splits without keys are not launched
   // 64-dim slabs of chunk c in this CTA: its 4 latent ones, and the rope one in turn with the partner
   auto slabs_of = [&](int c) { return (c & 1) == half ? 5 : 4; };
+  // Groups of 16 keys of chunk c, the K of one MMA: behind the end of the list nothing is fetched, and P * V leaves out what would be
+  // there (the scores of those keys, made of what the stage held before, are masked).
+  auto key_groups = [&](int c) { return min(kChunk, k_end - k_begin - c * kChunk + 15) >> 4; };
+  auto stage_at = [&](int st) { return (st >> 1) * kTwoStages + ((st & 1) ? slabs_of(0) * kKSlabBytes : 0); };
   const int seq_len = a.seq_lens ? a.seq_lens[b] : 0x7fffffff;
 
+  if (warp == kMmaWarp && lane == 0) {
+    tma_prefetch_desc(&tmQ);
+    tma_prefetch_desc(&tmKV);
+  }
   if (warp == kThreads / 32 - 1) {
     auto init = [&](uint64_t* bar, int n, uint32_t count) {
       if (lane < n) mbar_init(bar + lane, count);
@@ -234,9 +306,9 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     init(bar_q, 1, 1);
     init(bar_full, 2 * kStages, 1);   // and bar_empty
     if (lane < kMlaBars) mbar_init(&bar_step[lane], mla_arrivals(lane));
-    init(bar_xfull, 2, 1);
-    init(bar_xfree, 2, kSoftWarps / kSets);
-    init(bar_xq, 2, kSoftWarps);   // and bar_qt
+    init(bar_xfull, 5, 1);   // bar_pfull and bar_inv
+    init(bar_xfree, 4, 4);   // and bar_pfree
+    init(bar_qt, 1, kSoftWarps);
     mbar_fence_init();
     fence_proxy_async_smem();   // the barriers' initial state, before the copy engine counts on it
     __syncwarp();
@@ -247,7 +319,6 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         const int dim0 = j < 4 ? half * 256 + j * 64 : 512;
         tma_load_2d(q_sm + j * kQSlabBytes, &tmQ, bar_q, dim0, b * kHeads);
       }
-      tma_prefetch_desc(&tmKV);
     }
   }
   if (warp == kMmaWarp) {
@@ -285,7 +356,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   }
   tc_fence_before();
   __syncthreads();
-  cluster_arrive();   // this CTA's barriers exist; a role waits for the partner's before it first signals across
+  cluster_arrive_relaxed();   // this CTA's barriers exist; a role waits for the partner's before it first signals across
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t peer = static_cast<uint32_t>(half ^ 1);
@@ -297,25 +368,41 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     st_cluster_u32(peer_abort, 1u);
   };
 
+  // The last word to the partner has been said. What a warp sends or signals across is waited for there (nothing is signalled that
+  // nobody waits for) unless somebody has given up: only then the arrival has to order it, 1000 cycles and more.
+  auto leave = [&]() {
+    __syncwarp();
+    if (__any_sync(0xffffffffu, *s_abort)) cluster_arrive();
+    else cluster_arrive_relaxed();
+  };
+
   // `group`: which of the warps that share 32 heads, for kMlaMax
   auto step_bar = [&](MlaStep step, int c, int group = 0) { return &bar_step[mla_wait(step, c).bar + group]; };
   auto step_over = [&](MlaStep step, int c, int group = 0) {
     return wait_bar<false>(step_bar(step, c, group), mla_wait(step, c).parity, s_abort);
   };
-  auto x_buf = [&](int c) { return reinterpret_cast<float*>(smem + ((c & 1) ? kOffX1 : kOffX0)); };
+  auto x_buf = [&](int c) { return reinterpret_cast<uint4*>(smem + kOffX + (c & 1) * kXBytes); };
+  auto p_in = [&](int c) { return smem + kOffPin + (c & 1) * kPinBytes; };
 
   if (warp < kSoftWarps) {
     // ===================================== softmax ======================================================
-    // Two sets of four warps (a thread per head and set) take whole chunks in turn, so that the waits and latencies of two chunks
-    // overlap. What they share is the maximum that P and O are relative to: the set of chunk c needs the one of chunk c - 1 once
-    // it has its own scores, and passes its own on before the exponentials.
+    // A CTA makes the softmax of 64 heads, 16 of every 32 lanes of TMEM, and sends P to its partner: half of the additions and
+    // exponentials, and 19 KB between the CTAs for a chunk instead of 24. Two sets of four warps take whole chunks in turn, so that
+    // the waits and latencies of two chunks overlap. What they share is the maximum that P and O are relative to: the set of chunk
+    // c needs the one of chunk c - 1 once it has its own scores, and passes its own on before the exponentials. A thread has two
+    // heads (16 x 256b TMEM loads) and 12 keys of each.
     const int set = warp >> 2, group = warp & 3;
     const int head = group * 32 + lane;   // == TMEM lane
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(group * 32) << 16);
+    const uint32_t own_addr = lane_addr + (static_cast<uint32_t>(half * 16) << 16);
+    const int slot = group * 32 + lane;             // this thread's place in what the CTAs exchange
+    const int h0 = group * 16 + (lane >> 2), h1 = h0 + 8;   // its heads, among the CTA's 64
     if (group == 0 && lane == 0 && set < num_chunks) mbar_expect_tx(&bar_xfull[set], kXBytes);   // re-armed after every chunk
+    if (tid == 0) mbar_expect_tx(bar_inv, kOwnHeads * 4);
     const uint32_t peer_xfree = map_to_cta(&bar_xfree[set], peer);
-    const uint32_t peer_xq = map_to_cta(bar_xq, peer);
-    float m_own = -INFINITY, l_run = 0.f;   // l_run: this set's chunks, relative to m_own
+    const uint32_t peer_pfull = map_to_cta(&bar_pfull[set], peer);
+    const uint32_t peer_p = map_to_cta(p_in(set), peer);
+    float m0_own = -INFINITY, m1_own = -INFINITY, l0_run = 0.f, l1_run = 0.f;   // sums of this set's chunks and this thread's keys
     // Q moves from shared memory into TMEM once: as the A operand of every Q * K^T step it would otherwise be read out
     // of shared memory again for each chunk (80 KB for 48 keys, more than everything else together), and the shared
     // memory's 128 bytes a clock are what this kernel runs out of first.
@@ -339,7 +426,6 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     __syncwarp();
     if (lane == 0) mbar_arrive(bar_qt);
     cluster_wait();
-    if (lane == 0) mbar_arrive_cluster_relaxed(peer_xq);
     if (!q_here) give_up(UMDK_PH_TMA_FULL, 0);
     const bool dg = a.diag != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0;
     int dt[8] = {0, 0, 0, 0, 0, 0, 0, 0};   // 32 bits: registers are short
@@ -360,11 +446,8 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       }
       lap(0);
       tc_fence_after();
-      uint32_t sr[kChunk];
-      tmem_ld_x16(lane_addr + kColS, sr);
-      tmem_ld_x16(lane_addr + kColS + 16, sr + 16);
-      tmem_ld_x16(lane_addr + kColS + 32, sr + 32);
-      tmem_ld_wait();
+      uint32_t sr[kChunk / 2];
+      load_scores(own_addr + kColS, sr);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(step_bar(kMlaRead, c));
@@ -377,75 +460,111 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       }
       lap(4);
       // S = own partial + partner's partial (raw dot products; the scale is folded into the exponent below)
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-      const float4* xp = reinterpret_cast<const float4*>(x_buf(c)) + head;
+      const uint4* xp = x_buf(c) + slot;
 #pragma unroll
-      for (int j4 = 0; j4 < kChunk / 4; ++j4) {
-        const float4 xv = xp[j4 * kHeads];
-        sr[4 * j4] = __float_as_uint(__uint_as_float(sr[4 * j4]) + xv.x);
-        sr[4 * j4 + 1] = __float_as_uint(__uint_as_float(sr[4 * j4 + 1]) + xv.y);
-        sr[4 * j4 + 2] = __float_as_uint(__uint_as_float(sr[4 * j4 + 2]) + xv.z);
-        sr[4 * j4 + 3] = __float_as_uint(__uint_as_float(sr[4 * j4 + 3]) + xv.w);
+      for (int i = 0; i < kChunk / 8; ++i) {
+        const uint4 xv = xp[i * 128];
+        sr[4 * i] = __float_as_uint(__uint_as_float(sr[4 * i]) + __uint_as_float(xv.x));
+        sr[4 * i + 1] = __float_as_uint(__uint_as_float(sr[4 * i + 1]) + __uint_as_float(xv.y));
+        sr[4 * i + 2] = __float_as_uint(__uint_as_float(sr[4 * i + 2]) + __uint_as_float(xv.z));
+        sr[4 * i + 3] = __float_as_uint(__uint_as_float(sr[4 * i + 3]) + __uint_as_float(xv.w));
       }
       const int word = c + (c >> 1);   // bits 48 c ...
       const unsigned long long valid =
           (static_cast<unsigned long long>(mask_sm[word + 1]) << 32 | mask_sm[word]) >> ((c & 1) * 16) & ((1ull << kChunk) - 1ull);
       if (valid != (1ull << kChunk) - 1ull) {   // the same for every thread of the set
+        const unsigned long long mine = valid >> (2 * (lane & 3));
 #pragma unroll
-        for (int j = 0; j < kChunk; ++j)
-          if (!((valid >> j) & 1ull)) sr[j] = __float_as_uint(-INFINITY);
+        for (int i = 0; i < kChunk / 8; ++i) {
+          if (!((mine >> (8 * i)) & 1ull)) sr[4 * i] = sr[4 * i + 2] = __float_as_uint(-INFINITY);
+          if (!((mine >> (8 * i + 1)) & 1ull)) sr[4 * i + 1] = sr[4 * i + 3] = __float_as_uint(-INFINITY);
+        }
       }
+      float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
-      for (int j = 0; j < kChunk; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], __uint_as_float(sr[j]));
-      float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      // every lane's loads of X have returned (mx depends on them); keep the arrival behind that dependence
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 0));
+      for (int i = 0; i < kChunk / 8; ++i) {
+        mx0 = fmaxf(mx0, fmaxf(__uint_as_float(sr[4 * i]), __uint_as_float(sr[4 * i + 1])));
+        mx1 = fmaxf(mx1, fmaxf(__uint_as_float(sr[4 * i + 2]), __uint_as_float(sr[4 * i + 3])));
+      }
+      // the four threads of a head; every lane's loads of X have returned (the maxima depend on them), the arrival below stays
+      // behind that dependence
+      mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+      mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+      mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+      mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
       // re-armed before the partner may send again (its permission needs this warp's arrival below)
       if (group == 0 && lane == 0 && c + kSets < num_chunks) mbar_expect_tx(&bar_xfull[c & 1], kXBytes);
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster_relaxed(peer_xfree);
-      mx *= a.scale_log2;   // scale_log2 > 0: the maximum of the scaled scores
-      float m_run = -INFINITY;
+      if (lane == 0 && c + kSets < num_chunks) mbar_arrive_cluster_relaxed(peer_xfree);
+      mx0 *= a.scale_log2;   // scale_log2 > 0: the maximum of the scaled scores
+      mx1 *= a.scale_log2;
+      float m0 = -INFINITY, m1 = -INFINITY;
       if (c >= 1) {
         ok = __all_sync(0xffffffffu, step_over(kMlaMax, c - 1, group));
         if (!ok) {
           give_up(UMDK_PH_GROUP_READY, 4000 + c);
           break;
         }
-        m_run = max_sm[((c - 1) & 1) * kHeads + head];
+        m0 = max_sm[((c - 1) & 1) * kOwnHeads + h0];
+        m1 = max_sm[((c - 1) & 1) * kOwnHeads + h1];
       }
       // lazy maximum: raise it only when it grows by more than 8 (P stays below 2^8)
-      const float m_new = mx > m_run + 8.f || m_run == -INFINITY ? fmaxf(m_run, mx) : m_run;
-      max_sm[(c & 1) * kHeads + head] = m_new;
+      const float m0_new = mx0 > m0 + 8.f || m0 == -INFINITY ? fmaxf(m0, mx0) : m0;
+      const float m1_new = mx1 > m1 + 8.f || m1 == -INFINITY ? fmaxf(m1, mx1) : m1;
+      if ((lane & 3) == 0) {
+        max_sm[(c & 1) * kOwnHeads + h0] = m0_new;
+        max_sm[(c & 1) * kOwnHeads + h1] = m1_new;
+      }
       __syncwarp();
       if (lane == 0) mbar_arrive(step_bar(kMlaMax, c, group));
-      const float neg_m = m_new == -INFINITY ? 0.f : -m_new;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-      uint32_t pk[kChunk / 2];
+      // Asked for before the exponentials, awaited behind them: the partner has taken P(c-2) in, and P(c-2) * V is through.
+      bool p_sent = c < 2, p_used = c < 2;
+      if (c >= 2) {
+        p_sent = mbar_test(&bar_pfree[set], ((c >> 1) - 1) & 1);
+        p_used = mbar_test(step_bar(kMlaFree, c - 2), mla_wait(kMlaFree, c - 2).parity);
+      }
+      const float neg0 = m0_new == -INFINITY ? 0.f : -m0_new, neg1 = m1_new == -INFINITY ? 0.f : -m1_new;
+      float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
+      uint32_t pk[kChunk / 4];
 #pragma unroll
-      for (int j = 0; j < kChunk / 2; ++j) {
-        const float p0 = ex2_approx(fmaf(__uint_as_float(sr[2 * j]), a.scale_log2, neg_m));
-        const float p1 = ex2_approx(fmaf(__uint_as_float(sr[2 * j + 1]), a.scale_log2, neg_m));
-        sum4[j & 3] += p0 + p1;
-        const __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);
-        pk[j] = *reinterpret_cast<const uint32_t*>(&hh);
+      for (int i = 0; i < kChunk / 8; ++i) {
+        const float p0 = ex2_approx(fmaf(__uint_as_float(sr[4 * i]), a.scale_log2, neg0));
+        const float p1 = ex2_approx(fmaf(__uint_as_float(sr[4 * i + 1]), a.scale_log2, neg0));
+        const float p2 = ex2_approx(fmaf(__uint_as_float(sr[4 * i + 2]), a.scale_log2, neg1));
+        const float p3 = ex2_approx(fmaf(__uint_as_float(sr[4 * i + 3]), a.scale_log2, neg1));
+        ((i & 1) ? sum2 : sum0) += p0 + p1;
+        ((i & 1) ? sum3 : sum1) += p2 + p3;
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(p0, p1), hi = __floats2bfloat162_rn(p2, p3);
+        pk[2 * i] = *reinterpret_cast<const uint32_t*>(&lo);
+        pk[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&hi);
       }
       // (a sum relative to -inf is 0)
-      l_run = l_run * (m_own == m_new ? 1.f : ex2_approx(m_own - m_new)) + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
-      m_own = m_new;
+      l0_run = l0_run * (m0_own == m0_new ? 1.f : ex2_approx(m0_own - m0_new)) + (sum0 + sum2);
+      l1_run = l1_run * (m1_own == m1_new ? 1.f : ex2_approx(m1_own - m1_new)) + (sum1 + sum3);
+      m0_own = m0_new;
+      m1_own = m1_new;
+      // What O (P(0) .. P(c-1), relative to m0 and m1) is multiplied by in front of P(c) * V. Where nothing has been seen yet
+      // (-inf) O is zero.
+      const float alpha0 = m0 == m0_new || m0 == -INFINITY ? 1.f : ex2_approx(m0 - m0_new);
+      const float alpha1 = m1 == m1_new || m1 == -INFINITY ? 1.f : ex2_approx(m1 - m1_new);
       lap(5);
-      // P(c) goes where P(c-2) was: its product is through
-      if (c >= 2) {
-        ok = __all_sync(0xffffffffu, step_over(kMlaFree, c - 2));
-        if (!ok) {
-          give_up(UMDK_PH_TMEM_EMPTY, 500 + c);
-          break;
-        }
+      ok = __all_sync(0xffffffffu, p_sent || wait_bar<false>(&bar_pfree[set], ((c >> 1) - 1) & 1, s_abort));
+      if (!ok) {
+        give_up(UMDK_PH_GROUP_READY, 5000 + c);
+        break;
       }
-      // O (P(0) .. P(c-1), relative to m_run) is rescaled when P(c-1) * V has been added to it; without a rescale nothing here
-      // waits for that product. Where nothing has been seen yet (m_run = -inf) O is zero.
-      const float alpha = m_run == m_new || m_run == -INFINITY ? 1.f : ex2_approx(m_run - m_new);
-      const bool scale_o = c >= 1 && __any_sync(0xffffffffu, alpha != 1.f);
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        st_async_v4(peer_p + (i * 128 + slot) * 16, pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3], peer_pfull);
+      st_async_v2(peer_p + kPBytes + slot * 8, __float_as_uint(alpha0), __float_as_uint(alpha1), peer_pfull);
+      // P(c) goes where P(c-2) was: its product is through
+      ok = __all_sync(0xffffffffu, p_used || step_over(kMlaFree, c - 2));
+      if (!ok) {
+        give_up(UMDK_PH_TMEM_EMPTY, 500 + c);
+        break;
+      }
+      // O is rescaled when P(c-1) * V has been added to it; without a rescale nothing here waits for that product
+      const bool scale_o = c >= 1 && __any_sync(0xffffffffu, alpha0 != 1.f || alpha1 != 1.f);
       if (scale_o) {
         ok = __all_sync(0xffffffffu, step_over(kMlaO, c - 1));
         if (!ok) {
@@ -455,22 +574,10 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       }
       lap(6);
       tc_fence_after();
-      if (scale_o) {
-#pragma unroll 1
-        for (int c0 = 0; c0 < 256; c0 += 32) {
-          uint32_t o[32];
-          tmem_ld_x32(lane_addr + kColO + c0, o);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
-          tmem_st_x32(lane_addr + kColO + c0, o);
-        }
-        tmem_st_wait();
-      }
-      // P as the A operand of P * V, key pairs in 24 columns: through shared memory the store and its proxy fence alone took some
-      // 800 cycles a chunk next to the MMAs' operand reads
-      tmem_st_x16(lane_addr + kColP + (c & 1) * (kChunk / 2), pk);
-      tmem_st_x8(lane_addr + kColP + (c & 1) * (kChunk / 2) + 16, pk + 16);
+      if (scale_o) rescale_o(own_addr + kColO, alpha0, alpha1);
+      // P as the A operand of P * V: through shared memory the store and its proxy fence alone took some 800 cycles a chunk next
+      // to the MMAs' operand reads
+      store_probs(own_addr + kColP + (c & 1) * (kChunk / 2), pk);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -481,26 +588,42 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       for (int i = 0; i < 8; ++i)
         if (i != 2 && i != 3) a.diag[i] = dt[i];
     }
-    cluster_arrive();   // the last word to the partner has been said
+    // ---- sums and factors: the CTA's 64 heads, both sets, relative to the last maximum ----
+    l0_run += __shfl_xor_sync(0xffffffffu, l0_run, 1);
+    l1_run += __shfl_xor_sync(0xffffffffu, l1_run, 1);
+    l0_run += __shfl_xor_sync(0xffffffffu, l0_run, 2);
+    l1_run += __shfl_xor_sync(0xffffffffu, l1_run, 2);
+    if ((lane & 3) == 0) {
+      sum_sm[set * kOwnHeads + h0] = make_float2(l0_run, m0_own);
+      sum_sm[set * kOwnHeads + h1] = make_float2(l1_run, m1_own);
+    }
+    ok = bar_and<32 * kSoftWarps>(1, ok);
+    if (ok && tid < kOwnHeads) {
+      const float2 u = sum_sm[tid], v = sum_sm[kOwnHeads + tid];
+      const float m = fmaxf(u.y, v.y);
+      const float l = u.x * (u.y == m ? 1.f : ex2_approx(u.y - m)) + v.x * (v.y == m ? 1.f : ex2_approx(v.y - m));
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const float lse2 = l > 0.f ? m + log2f(l) : -INFINITY;
+      const int h = (tid >> 4) * 32 + half * 16 + (tid & 15);
+      inv_sm[h] = inv;
+      st_async_b32(map_to_cta(inv_sm + h, peer), __float_as_uint(inv), map_to_cta(bar_inv, peer));
+      if (a.num_splits > 1) a.part_lse[((size_t)b * a.num_splits + split) * kHeads + h] = lse2;
+      else if (a.lse) a.lse[(size_t)b * kHeads + h] = lse2 * 0.6931471805599453f;
+    }
+    leave();
     // ---- epilogue: this CTA's 256 output columns, half of them per set ----
     // (every decision below is the same for all eight warps: the TMEM loads are warp-collective)
     if (ok) {
-      ok = __all_sync(0xffffffffu, step_over(kMlaEnd, 0));
+      ok = __all_sync(0xffffffffu, step_over(kMlaEnd, 0) && wait_bar<true>(bar_inv, 0, s_abort));
       if (!ok) {   // the partner may have left
         if (!*s_abort) umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_EMPTY, b, 2000);
         *s_abort = 1;
       }
     }
-    // both sets' sums, relative to the last maximum
-    sum_sm[set * kHeads + head] = make_float2(l_run, m_own);
     ok = bar_and<32 * kSoftWarps>(1, ok);
-    const float2 other = sum_sm[(set ^ 1) * kHeads + head];
-    const float m_run = fmaxf(m_own, other.y);
-    l_run = l_run * (m_own == m_run ? 1.f : ex2_approx(m_own - m_run)) + other.x * (other.y == m_run ? 1.f : ex2_approx(other.y - m_run));
     tc_fence_after();
     if (ok) {
-      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-      const float lse2 = l_run > 0.f ? m_run + log2f(l_run) : -INFINITY;
+      const float inv = inv_sm[head];
       // A thread has a row of its own: stored from here, a warp's 16 bytes per lane would touch 32 rows each time (128 x 256 fp32:
       // 11000 cycles, bf16 5000). The rows go through the memory of the key tiles and out in pieces of 512 or 256 bytes.
       const int col0 = set * 128;
@@ -529,7 +652,6 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         for (int r = lane >> 4; r < 32; r += 2)
           *reinterpret_cast<uint4*>(dst + (size_t)r * kDimV + (lane & 15) * 8) =
               *reinterpret_cast<const uint4*>(rows + r * kOutPitch16 + (lane & 15) * 16);
-        if (half == 0 && set == 0 && a.lse) a.lse[(size_t)b * kHeads + head] = lse2 * 0.6931471805599453f;
       } else {
 #pragma unroll 1
         for (int c0 = 0; c0 < 128; c0 += 32) {
@@ -549,7 +671,6 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         for (int r = 0; r < 32; ++r)
           *reinterpret_cast<float4*>(dst + (size_t)r * kDimV + lane * 4) =
               *reinterpret_cast<const float4*>(rows + r * kOutPitch + lane * 16);
-        if (half == 0 && set == 0) a.part_lse[((size_t)b * a.num_splits + split) * kHeads + head] = lse2;
       }
     }
   } else if (warp == kMmaWarp) {
@@ -587,7 +708,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         lap(1);
         tc_fence_after();
         // one add per step: everything else about the operands is constant
-        const uint64_t bd = k_desc + st * (kStageBytes >> 4);
+        const uint64_t bd = k_desc + (stage_at(st) >> 4);
         const uint32_t q = tmem_base + kColQ;
 #pragma unroll
         for (int j = 0; j < kMaxSlabs; ++j) {
@@ -644,11 +765,13 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           t_prev = t;
         }
         tc_fence_after();
-        const uint64_t vd = v_desc + st * (kStageBytes >> 4);
+        const uint64_t vd = v_desc + (stage_at(st) >> 4);
 #pragma unroll
-        for (int k = 0; k < kChunk / 16; ++k)   // 16 keys per step: A advances 8 columns, B two 8-key groups
+        for (int k = 0; k < kChunk / 16; ++k) {   // 16 keys per step: A advances 8 columns, B two 8-key groups
+          if (k >= key_groups(c)) break;
           umma_f16_ta(tmem_base + kColO, tmem_base + kColP + (c & 1) * (kChunk / 2) + k * 8, vd + k * (2048 >> 4), idesc_pv,
                       (c | k) ? 1u : 0u);
+        }
         if (c + 1 < num_chunks) {   // behind the last chunk one commit, below, is for everybody
           umma_commit(&bar_empty[st]);
           umma_commit(step_bar(kMlaO, c));
@@ -660,15 +783,14 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       }
       umma_commit(step_bar(kMlaEnd, 0));   // also where it gave up
     }
-  } else if (warp >= kExchangeWarp && warp < kMmaWarp) {
-    // ===================================== exchange (warps 8..11) =======================================
+  } else if (warp >= kExchangeWarp && warp < kPinWarp) {
+    // ===================================== partials to the partner (warps 8..11) ========================
     cluster_wait();
-    const int head = (warp & 3) * 32 + lane;   // == TMEM lane
-    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-    const uint32_t peer_x[2] = {map_to_cta(x_buf(0), peer) + static_cast<uint32_t>(head) * 16u,
-                                map_to_cta(x_buf(1), peer) + static_cast<uint32_t>(head) * 16u};
+    const int slot = (warp & 3) * 32 + lane;
+    const uint32_t other_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32 + (half ^ 1) * 16) << 16);   // the partner's heads
+    const uint32_t peer_x = map_to_cta(x_buf(0), peer) + static_cast<uint32_t>(slot) * 16u;
     const uint32_t peer_xfull = map_to_cta(bar_xfull, peer);
-    const bool dg = a.diag != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && head == 0;
+    const bool dg = a.diag != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && slot == 0;
     long long dt[2] = {0, 0};
     long long t_prev = dg ? clock64() : 0;
     for (int c = 0; c < num_chunks; ++c) {
@@ -677,19 +799,14 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         break;
       }
       tc_fence_after();
-      uint32_t sr[kChunk];
-      tmem_ld_x16(lane_addr + kColS, sr);
-      tmem_ld_x16(lane_addr + kColS + 16, sr + 16);
-      tmem_ld_x16(lane_addr + kColS + 32, sr + 32);
-      tmem_ld_wait();
+      uint32_t sr[kChunk / 2];
+      load_scores(other_addr + kColS, sr);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(step_bar(kMlaRead, c));
       if (dg) t_prev = clock64();
-      // the partner's softmax warps must have read the partial of two chunks ago out of their exchange buffer; the second buffer
-      // is Q's memory to begin with
-      if (c >= 1 && !__all_sync(0xffffffffu, c == 1 ? wait_bar<false>(bar_xq, 0, s_abort)
-                                                    : wait_bar<false>(&bar_xfree[c & 1], ((c >> 1) - 1) & 1, s_abort))) {
+      // the partner's softmax warps must have read the partial of two chunks ago out of their exchange buffer
+      if (c >= 2 && !__all_sync(0xffffffffu, wait_bar<false>(&bar_xfree[c & 1], ((c >> 1) - 1) & 1, s_abort))) {
         give_up(UMDK_PH_GROUP_READY, c);
         break;
       }
@@ -699,8 +816,8 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         t_prev = t;
       }
 #pragma unroll
-      for (int j4 = 0; j4 < kChunk / 4; ++j4)
-        st_async_v4(peer_x[c & 1] + j4 * (kHeads * 16), sr[4 * j4], sr[4 * j4 + 1], sr[4 * j4 + 2], sr[4 * j4 + 3],
+      for (int i = 0; i < kChunk / 8; ++i)
+        st_async_v4(peer_x + (c & 1) * kXBytes + i * (128 * 16), sr[4 * i], sr[4 * i + 1], sr[4 * i + 2], sr[4 * i + 3],
                     peer_xfull + (c & 1) * 8);
       if (dg) dt[1] += clock64() - t_prev;
     }
@@ -708,8 +825,54 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       a.diag[2] = dt[0];
       a.diag[3] = dt[1];
     }
+  } else if (warp >= kPinWarp && warp < kMmaWarp) {
+    // ===================================== P of the partner's heads (warps 12..15) ======================
+    cluster_wait();
+    const int slot = (warp & 3) * 32 + lane;
+    const uint32_t other_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32 + (half ^ 1) * 16) << 16);
+    const uint32_t peer_pfree = map_to_cta(bar_pfree, peer);
+    if (slot == 0) {
+      for (int c = 0; c < min(num_chunks, 2); ++c) mbar_expect_tx(&bar_pfull[c], kPinBytes);   // re-armed after every chunk
+    }
+    for (int c = 0; c < num_chunks; ++c) {
+      if (!__all_sync(0xffffffffu, wait_bar<true>(&bar_pfull[c & 1], (c >> 1) & 1, s_abort))) {
+        give_up(UMDK_PH_GROUP_READY, 6000 + c);
+        break;
+      }
+      uint32_t pk[kChunk / 4];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const uint4 v = reinterpret_cast<const uint4*>(p_in(c))[i * 128 + slot];
+        pk[4 * i] = v.x;
+        pk[4 * i + 1] = v.y;
+        pk[4 * i + 2] = v.z;
+        pk[4 * i + 3] = v.w;
+      }
+      const float2 alpha = reinterpret_cast<const float2*>(p_in(c) + kPBytes)[slot];
+      // (the same value on every lane, from all of them: the loads of alpha have returned; those of P are stored below and the
+      // arrival stands behind that store)
+      const bool scale_o = c >= 1 && __any_sync(0xffffffffu, alpha.x != 1.f || alpha.y != 1.f);
+      if (c >= 2 && !__all_sync(0xffffffffu, step_over(kMlaFree, c - 2))) {
+        give_up(UMDK_PH_TMEM_EMPTY, 6000 + c);
+        break;
+      }
+      if (scale_o && !__all_sync(0xffffffffu, step_over(kMlaO, c - 1))) {
+        give_up(UMDK_PH_TMEM_EMPTY, 7000 + c);
+        break;
+      }
+      tc_fence_after();
+      store_probs(other_addr + kColP + (c & 1) * (kChunk / 2), pk);
+      if (slot == 0 && c + 2 < num_chunks) mbar_expect_tx(&bar_pfull[c & 1], kPinBytes);   // before the partner may send again
+      __syncwarp();
+      if (lane == 0 && c + 2 < num_chunks) mbar_arrive_cluster_relaxed(peer_pfree + (c & 1) * 8);
+      if (scale_o) rescale_o(other_addr + kColO, alpha.x, alpha.y);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(step_bar(kMlaP, c));
+    }
   } else {
-    // ===================================== gather producers (warps 14..19) ==================================
+    // ===================================== gather producers (warps 18..23) ==================================
     bool ok = true;
     const bool dg = a.diag != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && lane == 0 && warp == kProducerWarp;
     long long dt[2] = {0, 0};
@@ -723,7 +886,8 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     };
     for (int c = 0; c < num_chunks && ok; ++c) {
       const int st = c % kStages, n_slabs = slabs_of(c);
-      const int n_inst = (kChunk / 4) * n_slabs;   // gather4 copies per tile
+      const int n_keys = key_groups(c) * 16;
+      const int n_inst = (n_keys / 4) * n_slabs;   // gather4 copies per tile
       if (c == kFreeStages) {   // from here on in Q's memory
         cluster_wait();         // the first tiles are on their way without the partner
         ok = __all_sync(0xffffffffu, wait_bar<false>(bar_qt, 0, s_abort));
@@ -740,19 +904,23 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         }
       }
       lap(0);
-      if (warp == kProducerWarp && lane == 0) mbar_expect_tx(&bar_full[st], static_cast<uint32_t>(n_slabs) * kKSlabBytes);
+      if (warp == kProducerWarp && lane == 0) mbar_expect_tx(&bar_full[st], static_cast<uint32_t>(n_slabs * n_keys) * 128u);
       __syncwarp();
-      uint8_t* stage = k_sm + st * kStageBytes;
+      uint8_t* stage = k_sm + stage_at(st);
       const int4* rows4 = reinterpret_cast<const int4*>(rows_sm + c * kChunk);
       // A warp issues its lanes' copies one after the other, about 80 cycles apart, and different warps issue side by
       // side: the copies of a tile are dealt over all producer warps (nine each) instead of filling two of them.
       for (int u = lane * kProducerWarps + warp - kProducerWarp; u < n_inst; u += 32 * kProducerWarps) {
         const int grp = n_slabs == 4 ? u >> 2 : u / 5, slab = u - grp * n_slabs;
         int4 r = rows4[grp];
-        r.x = max(r.x, 0);   // masked keys read row 0: their scores are set to -inf before the softmax
-        r.y = max(r.y, 0);
-        r.z = max(r.z, 0);
-        r.w = max(r.w, 0);
+        // masked keys read what one of the others is there for (their scores are set to -inf before the softmax): row 0 for all of
+        // them would be the same few lines of L2 for every CTA
+        int any = max(max(r.x, r.y), max(r.z, r.w));
+        if (any < 0) any = max(rows_sm[c * kChunk], 0);
+        r.x = r.x < 0 ? any : r.x;
+        r.y = r.y < 0 ? any : r.y;
+        r.z = r.z < 0 ? any : r.z;
+        r.w = r.w < 0 ? any : r.w;
         const int col = slab < 4 ? half * 256 + slab * 64 : 512;
         tma_gather4(stage + slab * kKSlabBytes + grp * 512, &tmKV, &bar_full[st], col, r);
       }
@@ -763,8 +931,7 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       for (int i = 0; i < 2; ++i) a.diag[13 + i] = dt[i];
     }
   }
-  __syncwarp();
-  if (warp >= kSoftWarps) cluster_arrive();
+  if (warp >= kSoftWarps) leave();
   tc_fence_before();
   __syncthreads();
   if (warp == kMmaWarp) {
@@ -777,21 +944,26 @@ sparse_mla_decode_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
 }
 
 // Joins the key-list splits that have keys (the first `live` of num_splits): out = sum_i exp2(lse_i - lse) * o_i. One CTA per
-// (sequence, head), four columns per thread; the weights are made once per CTA and eight splits' partials are in flight at a
-// time (bound by the latency of reading live x 2 KB per head out of L2).
-__global__ void __launch_bounds__(128) mla_merge_kernel(const float* __restrict__ part_o,
-                                                        const float* __restrict__ part_lse,
-                                                        __nv_bfloat16* __restrict__ out, float* __restrict__ lse,
-                                                        int num_splits, int live) {
+// (sequence, head), four columns per thread, and kGroups threads per column that share the splits; the weights are made once per CTA
+// and eight splits' partials are in flight per thread at a time. Bound by the latency of reading live x 2 KB per head out of L2. Four
+// groups where a CTA has an SM to itself and more than eight splits: one round trip instead of three (one sequence, 2048 keys in 22
+// splits, the whole call 15.5 / 14.9 us). CTAs of 512 threads that have to take turns lose (4 sequences 16.2 / 21.0; two groups for 2
+// and 3 sequences 14.9 / 15.3, 15.6 / 15.9).
+template <int kGroups>
+__global__ void __launch_bounds__(128 * kGroups) mla_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse,
+                                                                  __nv_bfloat16* __restrict__ out, float* __restrict__ lse,
+                                                                  int num_splits, int live) {
   extern __shared__ float w_sm[];   // [live]
+  __shared__ float4 acc_sm[kGroups > 1 ? kGroups - 1 : 1][128];
   const int bh = blockIdx.x;        // b * 128 + head
   const int b = bh / kHeads, head = bh % kHeads;
-  const float4* po = reinterpret_cast<const float4*>(part_o + ((size_t)b * num_splits * kHeads + head) * kDimV) + threadIdx.x;
+  const int col = threadIdx.x & 127, group = threadIdx.x >> 7;
+  const float4* po = reinterpret_cast<const float4*>(part_o + ((size_t)b * num_splits * kHeads + head) * kDimV) + col;
   const size_t step = (size_t)kHeads * kDimV / 4;
   float4 v[8];
 #pragma unroll
   for (int u = 0; u < 8; ++u)
-    if (u < live) v[u] = __ldg(po + u * step);
+    if (group + u * kGroups < live) v[u] = __ldg(po + (group + u * kGroups) * step);
   if (threadIdx.x < 32) {
     const float* pl = part_lse + (size_t)b * num_splits * kHeads + head;
     float mx = -INFINITY;
@@ -813,24 +985,37 @@ __global__ void __launch_bounds__(128) mla_merge_kernel(const float* __restrict_
   }
   __syncthreads();
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int s0 = 0; s0 < live; s0 += 8) {
+  for (int s0 = group; s0 < live; s0 += 8 * kGroups) {
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      if (s0 + u >= live) break;
-      if (s0 > 0) v[u] = __ldg(po + (s0 + u) * step);
+      if (s0 + u * kGroups >= live) break;
+      if (s0 > group) v[u] = __ldg(po + (s0 + u * kGroups) * step);
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      if (s0 + u >= live) break;
-      const float w = w_sm[s0 + u];
+      if (s0 + u * kGroups >= live) break;
+      const float w = w_sm[s0 + u * kGroups];
       acc.x = fmaf(w, v[u].x, acc.x);
       acc.y = fmaf(w, v[u].y, acc.y);
       acc.z = fmaf(w, v[u].z, acc.z);
       acc.w = fmaf(w, v[u].w, acc.w);
     }
   }
+  if constexpr (kGroups > 1) {
+    if (group > 0) acc_sm[group - 1][col] = acc;
+    __syncthreads();
+    if (group > 0) return;
+#pragma unroll
+    for (int g = 0; g < kGroups - 1; ++g) {
+      const float4 o = acc_sm[g][col];
+      acc.x += o.x;
+      acc.y += o.y;
+      acc.z += o.z;
+      acc.w += o.w;
+    }
+  }
   __nv_bfloat162 o2[2] = {__floats2bfloat162_rn(acc.x, acc.y), __floats2bfloat162_rn(acc.z, acc.w)};
-  *reinterpret_cast<uint2*>(out + (size_t)bh * kDimV + threadIdx.x * 4) = *reinterpret_cast<const uint2*>(o2);
+  *reinterpret_cast<uint2*>(out + (size_t)bh * kDimV + col * 4) = *reinterpret_cast<const uint2*>(o2);
 }
 
 }  // namespace
@@ -891,9 +1076,10 @@ UMDK_API int umdk_sparse_mla_decode(const void* q, const void* kv, const int* bl
   UMDK_CUDA_CHECK(cudaGetLastError());
   if (num_splits > 1) {
     const size_t smem = sizeof(float) * live;
-    if (smem > 48 * 1024)
-      UMDK_CUDA_CHECK(cudaFuncSetAttribute(mla_merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    mla_merge_kernel<<<B * kHeads, 128, smem, s>>>(part_o, part_lse, static_cast<__nv_bfloat16*>(out), lse, num_splits, live);
+    const int groups = live > 8 && B * kHeads <= sm_count() ? 4 : 1;   // (see the kernel)
+    const auto merge = groups == 4 ? mla_merge_kernel<4> : mla_merge_kernel<1>;
+    if (smem > 40 * 1024) UMDK_CUDA_CHECK(cudaFuncSetAttribute(merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    merge<<<B * kHeads, 128 * groups, smem, s>>>(part_o, part_lse, static_cast<__nv_bfloat16*>(out), lse, num_splits, live);
     UMDK_CUDA_CHECK(cudaGetLastError());
   }
   return 0;

@@ -110,3 +110,24 @@ def test_sparse_mla_decode_splits_without_keys(B, topk, splits, live):
     else:   # one split alone rounds its sum to bf16 directly, without the detour over a weight of one
         assert torch.allclose(out.float(), want.float(), rtol=2 ** -7, atol=1e-6) and torch.allclose(lse, want_lse, rtol=1e-5)
     assert bool(torch.isnan(ws[0][:, live:]).all()) and not bool(torch.isnan(ws[0][:, :live]).any())
+
+
+# the last groups of 16 keys, one and several chunks behind them; quads of keys with none, one and all masked; the merge's ways
+@pytest.mark.parametrize("B,topk,splits", [(1, 16, 1), (2, 17, 1), (1, 32, 1), (2, 33, 1), (1, 64, 1), (3, 65, 1), (1, 81, 1), (1, 800, 17),
+                                           (2, 800, 17), (1, 384, 8)])
+@pytest.mark.parametrize("first", [0, 3, 4])
+def test_sparse_mla_decode_last_keys_and_masked_quads(B, topk, splits, first):
+    from umdk_b200.ops.attention import ref_sparse_mla_decode, sparse_mla_decode
+    q, kv, bt, idx = _case(B, 4096, topk, seed=topk + splits)
+    pos = torch.arange(topk)
+    idx[:, (pos % 16 >= 4) & (pos % 16 < 4 + first)] = -1
+    idx[:, pos % 7 == 3] = -1
+    scale = 576 ** -0.5
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    out, lse = sparse_mla_decode(q.cuda(), kv.cuda(), bt.cuda(), idx.cuda(), scale, num_splits=splits, status=status)
+    torch.cuda.synchronize()
+    assert status.tolist()[0] == 0, status.tolist()
+    want, want_lse = ref_sparse_mla_decode(q, kv, bt, idx, scale)
+    # P and the result are rounded to bf16 once each (2^-9 relative); the scores are exact fp32 sums of bf16 products
+    assert ((out.float().cpu() - want).norm() / want.norm()).item() < 2e-2
+    assert torch.allclose(lse.cpu(), want_lse, atol=2e-2, rtol=1e-3)

@@ -9,27 +9,24 @@ import pytest
 from umdk_b200 import _native
 
 S, P, O, END, READ, FREE, MAX = range(7)
-XFULL, XFREE, XQ = range(7, 10)   # barriers of the exchange, two and two in turn and one
+XFULL, XFREE, PFULL, PFREE = range(7, 11)   # barriers of the exchange, each two in turn
 
 
 def kernel_wait(step, c):
     """(barrier, parity) of a wait, as the kernel has it; the exchange's barriers stand behind the others."""
-    if step == XFULL:
-        return 20 + (c & 1), (c >> 1) & 1
-    if step == XFREE:
-        return 22 + (c & 1), (c >> 1) & 1
-    if step == XQ:
-        return 24, 0
+    if step >= XFULL:
+        return 20 + 2 * (step - XFULL) + (c & 1), (c >> 1) & 1
     w = _native.cam().umdk_sparse_mla_wait(step, c)
     assert w >= 0
     return w >> 1, w & 1
 
 
-BARS = 25
+BARS = 28
 
 
 def programs(n, rescaled, groups, ctas):
-    """Roles of a CTA: lists of ("wait", step, c), ("arrive", step, c, cta), ("mma", step, c). `groups`: warps of a set."""
+    """Roles of a CTA: lists of ("wait", step, c), ("arrive", step, c, cta), ("mma", step, c). `groups`: warps of a set (and of those
+    that take the partner's P in)."""
     out = []
     for cta in range(ctas):
         qk, pv, exchange = [], [], []
@@ -38,19 +35,28 @@ def programs(n, rescaled, groups, ctas):
             pv += ([("wait", O, c - 1), ("arrive", FREE, c - 1, cta)] if c else []) + [("wait", P, c), ("mma", O, c)]
             exchange += [("wait", S, c), ("arrive", READ, c, cta)]
             if ctas == 2:
-                exchange += [("wait", XQ, 0)] if c == 1 else [("wait", XFREE, c - 2)] if c else []
+                exchange += [("wait", XFREE, c - 2)] if c >= 2 else []
                 exchange += [("arrive", XFULL, c, 1 - cta)]
         qk, pv = qk + [("mma", END, 0)], pv + [("mma", END, 0)]
         out += [(cta, 0, qk), (cta, 1, pv), (cta, None, exchange)]
+        rescale = lambda c: [("wait", O, c - 1)] if c in rescaled else []
+        free = lambda c: [("wait", FREE, c - 2)] if c >= 2 else []
+        for g in range(groups):
+            taken = []
+            for c in range(n):
+                taken += [("wait", PFULL, c)] if ctas == 2 else []
+                taken += free(c) + rescale(c) if ctas == 1 else free(c) + rescale(c) + [("arrive", PFREE, c, 1 - cta)]
+                taken += [("arrive", P, c, cta)]
+            out.append((cta, None, taken))
         for s, g in itertools.product(range(2), range(groups)):
-            soft = [("arrive", XQ, 0, 1 - cta)] if ctas == 2 else []
+            soft = []
             for c in range(s, n, 2):
                 soft += [("wait", S, c), ("arrive", READ, c, cta)]
                 soft += [("wait", XFULL, c), ("arrive", XFREE, c, 1 - cta)] if ctas == 2 else []
                 soft += ([("wait", MAX, c - 1, g)] if c else []) + [("arrive", MAX, c, cta, g)]
-                soft += [("wait", FREE, c - 2)] if c >= 2 else []
-                soft += [("wait", O, c - 1)] if c in rescaled else []
-                soft += [("arrive", P, c, cta)]
+                if ctas == 2:
+                    soft += ([("wait", PFREE, c - 2)] if c >= 2 else []) + [("arrive", PFULL, c, 1 - cta)]
+                soft += free(c) + rescale(c) + [("arrive", P, c, cta)]
             out.append((cta, None, soft + [("wait", END, 0)]))
     return out
 
@@ -62,7 +68,7 @@ class Walk:
         self.progs = [p for _, _, p in self.roles]
         self.queues = sorted({(cta, q) for cta, q, _ in self.roles if q is not None})
         self.mmas = {(cta, q): [op for op in p if op[0] == "mma"] for cta, q, p in self.roles if q is not None}
-        self.counts = {P: groups, READ: groups + 1, END: 2, XFREE: groups, XQ: 2 * groups}
+        self.counts = {P: 2 * groups, READ: groups + 1, END: 2, XFREE: groups, PFULL: groups, PFREE: groups}
         z = len(self.progs)
         self.start = ((0,) * z, (0,) * len(self.queues), tuple((0, 0) for _ in range(ctas * BARS + ctas * 4)))
         # every arrival that a step of chunk c needs, to tell whether it has happened: (role, place) or (queue, place)
