@@ -736,78 +736,134 @@ __global__ void __launch_bounds__(kEpThreads, 1) ep_dispatch_kernel(const Dispat
   }
 }
 
+// First work item of a warp (the next is a grid of warps further on). Items of a round (dispatch: two) go to all SMs in turn, more
+// are dealt by CTAs, neighbours in memory to neighbouring warps. Dealt by CTAs / over the SMs, us: dispatch of 300 tokens of 2048, top-8,
+// fp8 12.1 / 7.5, 16 of 2048, top-2, bf16 8.5 / 5.8, 2500 of 1280, top-3, fp8 (1.1 rounds) 11.4 / 10.0; 4096 of 7168, top-8, bf16 (7)
+// 98.9 / 102.8; combine of 300 tokens 8.5 / 8.2, of 1003 of 4096 (1.7 rounds) 12.6 / 13.1, of 4096 85.8 / 88.2.
+__device__ __forceinline__ int first_item(int items, int rounds, int warp) {
+  return items <= (int)gridDim.x * kEpWarps * rounds ? warp * gridDim.x + blockIdx.x : blockIdx.x * kEpWarps + warp;
+}
+
 // Dispatch of a group of ONE rank: nothing is exchanged, the layout already says which row every (token, k) gets, so
 // each token is read once, quantised in registers and stored straight into its rows. Same outputs as ep_dispatch_kernel
 // (the arrivals of the only source are the routed tokens in order) without the arrival buffers, the flags and the
 // hand-over between sending and expanding warps. Bound by the row stores: K rows leave for one that comes in. A work item
 // is a 4 KB piece of a token (2 KB of fp8 out), so that a thousand tokens still spread over every warp of the grid and a
-// warp has its eight 16-byte loads per lane in flight together. Measured on one rank: 4096 tokens of 7168, top-8, fp8: 110 ->
-// 70 us (300 MB, 4.3 TB/s); 1003 tokens of 4096, top-6, bf16: 33 -> 17 us.
+// warp has its eight 16-byte loads per lane in flight together, while it stores the item before. A row's 2 KB and its scales are
+// stored one after the other, not 512 bytes of every row in turn. Measured on one rank (through the exchanging kernel / with no
+// prefetch, 512 bytes of each row at a time, expert counts scanned by one warp / this), us: 4096 tokens of 7168, top-8, fp8 110 / 66.5
+// / 60.8 (301 MB, 5.0 TB/s; plain stores in row order reach 7.3), bf16 - / 102.7 / 98.9, 600 tokens - / 18.2 / 15.4, 2500 of 1280, top-3
+// - / 12.9 / 10.0, 1003 of 4096, top-6, bf16 33 / 12.9 / 11.8.
 template <bool kQuant>
 __global__ void __launch_bounds__(kEpThreads, 1) ep_dispatch_local_kernel(const DispatchArgs a) {
   const EpGeom& g = a.g;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __shared__ int s_off[1024];
-  __shared__ int s_row[kEpWarps][kMaxTopk];
-  __shared__ int s_total;
-  if (warp == 0) {   // first row of every expert
-    int run = 0;
-    for (int e0 = 0; e0 < g.E; e0 += 32) {
-      const int e = e0 + lane;
-      const int n = e < g.E ? a.num_per_expert[e] : 0;
-      int x = n;
+  __shared__ int s_warp[1024 / 32];
+  // First row of every expert: threads scan their counts by warps, then the warps' sums. (One warp walking over 256 experts, 32 at a
+  // time, was eight round trips to memory, 3 us.)
+  constexpr int kScan = 1024 / kEpThreads;   // experts of a thread
+  int count[kScan], incl[kScan];
 #pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, d);
-        if (lane >= d) x += y;
-      }
-      if (e < g.E) {
-        s_off[e] = run + x - n;
-        if (blockIdx.x == 0) {
-          a.recv_count[e] = run + x;
-          a.recv_per_expert[e] = (int64_t)n;
-          if (a.per_expert_host) a.per_expert_host[e] = (int64_t)n;
-        }
-      }
-      run += __shfl_sync(0xffffffffu, x, 31);
+  for (int i = 0; i < kScan; ++i) {
+    const int e = i * kEpThreads + threadIdx.x;
+    count[i] = e < g.E ? a.num_per_expert[e] : 0;
+  }
+  const int arrivals = a.num_per_rank[0];
+  const int nblk = g.H / 128;
+  const int nvec = g.H / 8;
+  const int nparts = kQuant ? (nblk + 15) / 16 : (nvec + 255) / 256;
+  const int mw2 = 2 * g.K + 2;
+  // What an item needs from memory is asked for while the one before is stored: its 4 KB of the token, and the expert and position
+  // that lane k finds for slot k.
+  struct Item {
+    int4 x[8];
+    long long expert;
+    int pos;
+  };
+  const int items = a.T * nparts, stride = gridDim.x * kEpWarps;
+  auto fetch = [&](int item, Item* it) {
+    const int t = item / nparts, part = item - t * nparts;
+    it->expert = -1;
+    it->pos = -1;
+    if (lane < g.K) {
+      it->expert = a.topk_idx[(size_t)t * g.K + lane];
+      it->pos = a.send_idx[(size_t)t * g.K + lane];
     }
-    if (lane == 0) s_total = run;
-    if (lane == 0 && blockIdx.x == 0) {
-      const int arrivals = a.num_per_rank[0];
-      a.counts_dev[0] = run;
-      a.counts_dev[1] = arrivals;
-      a.counts_dev[2] = arrivals;
-      a.counts_dev[3] = 0;
-      a.counts_dev[4] = 0;
-      if (a.diag) a.diag[0] = 0;
-      if (run > a.n_cap || arrivals > a.a_cap)
-        umdk_set_status(a.status, UMDK_ERR_OVERFLOW, UMDK_PH_DISPATCH_COUNT, run, arrivals);
+    const int4* xrow = reinterpret_cast<const int4*>(a.x + (size_t)t * g.H);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      // quantised: two neighbouring vectors of a lane, 8 lanes per 1x128 block; else whole 512-byte pieces
+      const int v = kQuant ? part * 256 + (u >> 1) * 64 + lane * 2 + (u & 1) : part * 256 + u * 32 + lane;
+      it->x[u] = v < nvec ? __ldg(xrow + v) : make_int4(0, 0, 0, 0);
     }
+  };
+  Item cur, next;
+  int item = first_item(items, 2, warp);
+  if (item < items) fetch(item, &cur);
+#pragma unroll
+  for (int i = 0; i < kScan; ++i) {
+    int x = count[i];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, d);
+      if (lane >= d) x += y;
+    }
+    incl[i] = x;
+    if (lane == 31) s_warp[i * kEpWarps + warp] = x;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int x = lane < kScan * kEpWarps ? s_warp[lane] : 0;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, d);
+      if (lane >= d) x += y;
+    }
+    if (lane < kScan * kEpWarps) s_warp[lane] = x;
+  }
+  __syncthreads();
+  const int total = s_warp[kScan * kEpWarps - 1];
+#pragma unroll
+  for (int i = 0; i < kScan; ++i) {
+    const int e = i * kEpThreads + threadIdx.x, w = i * kEpWarps + warp;
+    if (e >= g.E) continue;
+    const int end = incl[i] + (w > 0 ? s_warp[w - 1] : 0);
+    s_off[e] = end - count[i];
+    if (blockIdx.x == 0) {
+      a.recv_count[e] = end;
+      a.recv_per_expert[e] = (int64_t)count[i];
+      if (a.per_expert_host) a.per_expert_host[e] = (int64_t)count[i];
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.counts_dev[0] = total;
+    a.counts_dev[1] = arrivals;
+    a.counts_dev[2] = arrivals;
+    a.counts_dev[3] = 0;
+    a.counts_dev[4] = 0;
+    if (a.diag) a.diag[0] = 0;
+    if (total > a.n_cap || arrivals > a.a_cap)
+      umdk_set_status(a.status, UMDK_ERR_OVERFLOW, UMDK_PH_DISPATCH_COUNT, total, arrivals);
   }
   __syncthreads();
   if (a.row_expert) {
-    for (long long r = (long long)s_total + blockIdx.x * kEpThreads + threadIdx.x; r < a.n_cap;
+    for (long long r = (long long)total + blockIdx.x * kEpThreads + threadIdx.x; r < a.n_cap;
          r += (long long)gridDim.x * kEpThreads) {
       a.row_expert[r] = -1;
       a.row_weight[r] = 0.f;
     }
   }
-  const int nblk = g.H / 128;
-  const int nvec = g.H / 8;
-  const int nparts = kQuant ? (nblk + 15) / 16 : (nvec + 255) / 256;
-  const int mw2 = 2 * g.K + 2;
-  for (int item = blockIdx.x * kEpWarps + warp; item < a.T * nparts; item += gridDim.x * kEpWarps) {
+  for (; item < items; item += stride) {
+    if (item + stride < items) fetch(item + stride, &next);
     const int t = item / nparts, part = item - t * nparts;
     int e = -1, row = -1;
-    if (lane < g.K) {
-      const long long ee = a.topk_idx[(size_t)t * g.K + lane];
-      if (ee >= 0 && ee < g.E) {
-        e = (int)ee;
-        row = s_off[e] + a.send_idx[(size_t)t * g.K + lane];
-        if (row >= a.n_cap) {
-          umdk_set_status(a.status, UMDK_ERR_OVERFLOW, UMDK_PH_DISPATCH_DATA, 0, row);
-          row = -1;
-        }
+    if (cur.expert >= 0 && cur.expert < g.E) {
+      e = (int)cur.expert;
+      row = s_off[e] + cur.pos;
+      if (row >= a.n_cap) {
+        umdk_set_status(a.status, UMDK_ERR_OVERFLOW, UMDK_PH_DISPATCH_DATA, 0, row);
+        row = -1;
       }
     }
     const uint32_t kmask = __ballot_sync(0xffffffffu, row >= 0);
@@ -836,59 +892,45 @@ __global__ void __launch_bounds__(kEpThreads, 1) ep_dispatch_local_kernel(const 
         }
       }
     }
-    __syncwarp();
-    if (lane < g.K) s_row[warp][lane] = row;
-    __syncwarp();
-    if (kmask == 0) continue;
-    const int4* xrow = reinterpret_cast<const int4*>(a.x + (size_t)t * g.H);
-    if (kQuant) {
-      int4 raw[4][2];
+    if (kmask != 0) {
+      if (kQuant) {
+        int4 q[4];
+        float scale = 0.f;   // lanes 0 .. 15: of block part * 16 + lane
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int blk = part * 16 + 4 * u + (lane >> 3);
-        if (blk < nblk) {
-          raw[u][0] = __ldg(xrow + blk * 16 + (lane & 7) * 2);
-          raw[u][1] = __ldg(xrow + blk * 16 + (lane & 7) * 2 + 1);
-        } else {
-          raw[u][0] = raw[u][1] = make_int4(0, 0, 0, 0);
+        for (int u = 0; u < 4; ++u) {
+          float f[16];
+          bf16x8_to_float(cur.x[2 * u], f);
+          bf16x8_to_float(cur.x[2 * u + 1], f + 8);
+          float su;
+          q[u] = quant16(f, &su);   // shuffles inside: executed by all lanes
+          su = __shfl_sync(0xffffffffu, su, (lane & 3) * 8);
+          if ((lane >> 2) == u) scale = su;
         }
-      }
+        const int blk = part * 16 + lane;
+        for (uint32_t m = kmask; m; m &= m - 1) {   // a row's 2 KB together
+          const size_t r = __shfl_sync(0xffffffffu, row, __ffs(m) - 1);
+          uint8_t* dst = a.recv_x + r * g.row_bytes + part * 2048 + lane * 16;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int blk = part * 16 + 4 * u + (lane >> 3);
-        float f[16];
-        bf16x8_to_float(raw[u][0], f);
-        bf16x8_to_float(raw[u][1], f + 8);
-        float scale;
-        const int4 q = quant16(f, &scale);   // shuffles inside: executed by all lanes
-        if (blk < nblk) {
-          for (uint32_t m = kmask; m; m &= m - 1) {
-            const size_t r = s_row[warp][__ffs(m) - 1];
-            st_na_v4(a.recv_x + r * g.row_bytes + blk * 128 + (lane & 7) * 16, q);
-            if ((lane & 7) == 0) a.recv_scales[r * g.nscale + blk] = scale;
+          for (int u = 0; u < 4; ++u)
+            if (part * 16 + 4 * u + (lane >> 3) < nblk) st_na_v4(dst + u * 512, q[u]);
+          if (lane < 16 && blk < nblk) a.recv_scales[r * g.nscale + blk] = scale;
+        }
+      } else {
+        for (uint32_t m = kmask; m; m &= m - 1) {
+          const size_t r = __shfl_sync(0xffffffffu, row, __ffs(m) - 1);
+          int4* drow = reinterpret_cast<int4*>(a.recv_x + r * g.row_bytes);
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const int v = part * 256 + u * 32 + lane;
+            if (v < nvec) st_na_v4(drow + v, cur.x[u]);
           }
         }
       }
-    } else {
-      int4 val[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int v = part * 256 + u * 32 + lane;
-        if (v < nvec) val[u] = __ldg(xrow + v);
-      }
-      for (uint32_t m = kmask; m; m &= m - 1) {
-        int4* drow = reinterpret_cast<int4*>(a.recv_x + (size_t)s_row[warp][__ffs(m) - 1] * g.row_bytes);
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int v = part * 256 + u * 32 + lane;
-          if (v < nvec) st_na_v4(drow + v, val[u]);
-        }
-      }
     }
+    cur = next;
   }
   if (a.counts_host && blockIdx.x == 0 && threadIdx.x == 0) {   // last: nothing here has to wait for the host's memory
-    const int arrivals = a.num_per_rank[0];
-    a.counts_host[0] = s_total;
+    a.counts_host[0] = total;
     a.counts_host[1] = arrivals;
     a.counts_host[2] = arrivals;
     __threadfence_system();
@@ -1168,7 +1210,7 @@ __global__ void __launch_bounds__(kEpThreads, 1) ep_combine_local_kernel(const C
   const int mw2 = 2 * g.K + 2;
   const int items = arrivals_in_bounds(a) * nparts;
   if (a.diag && blockIdx.x == 0 && threadIdx.x == 0) a.diag[0] = 0;
-  for (int item = blockIdx.x * kEpWarps + warp; item < items; item += gridDim.x * kEpWarps) {
+  for (int item = first_item(items, 1, warp); item < items; item += gridDim.x * kEpWarps) {
     const int it = item / nparts, v0 = (item - it * nparts) * 128;
     const int* rm = a.recv_meta + (size_t)it * mw2;
     const int dst_rank = rm[0], dst_tok = rm[1];

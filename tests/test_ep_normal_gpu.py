@@ -377,3 +377,10 @@ def test_host_copy_of_the_counts_of_several_ranks(R, E):
     finally:
         for h in heaps:
             h.close()
+
+
+# items of less than a round of warps, of one to two, of more; counts of more experts than a CTA has threads
+@pytest.mark.parametrize("T,H,E,K,quant", [(2368, 128, 513, 2, True), (2400, 384, 1023, 3, False), (4737, 256, 512, 1, True),
+                                           (1200, 2176, 31, 5, True), (640, 6144, 33, 2, False)])
+def test_single_rank_rounds_of_items_and_many_experts(T, H, E, K, quant):
+    test_single_rank_short_path_matches_exchange(T, H, E, K, quant)
