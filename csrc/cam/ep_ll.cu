@@ -26,7 +26,7 @@ struct LLDispatchArgs {
 
 __global__ void __launch_bounds__(kLLThreads, 1) ep_ll_dispatch_kernel(const LLDispatchArgs a) {
   extern __shared__ __align__(16) uint8_t ll_scratch[];
-  ll_dispatch_body<kLLThreads>(a.g, a.off, a.peers, a.io, ll_scratch, nullptr);
+  ll_dispatch_body<kLLThreads, 32>(a.g, a.off, a.peers, a.io, ll_scratch, nullptr);
 }
 
 // Low-latency combine as an operator of its own (the counterpart of the fused kernel's tail for callers that ran
@@ -124,7 +124,11 @@ __global__ void __launch_bounds__(kLLThreads, 1) ep_ll_combine_kernel(const LLCo
 // the pass through the combine buffer, the completion flags and the grid-wide wait on them. Bound by latency: one table,
 // one round of row loads. Measured: 1024 rows of 7168 to 128 tokens 34.8 -> 12.9 us; with the metadata fetched beside the row
 // count and the call ended by the first CTA instead of the last 9.5 -> 7.7 (calls back to back in a graph), 1 token 5.8 -> 4.4.
+// With the next item's rows, weights and indices fetched while one is summed, and no row waiting for its index (inputs in turn, the
+// kernel alone) 13.5 -> 9.9, 2048 rows to 256 tokens 23.1 -> 16.7. kSlots: rows of a pass; with eight for every top-k the instructions for
+// rows that are not there cost more than the rest (142 tokens, top-1, 5.0; 6.6 with eight, 4.1 with two).
 constexpr int kLLLocalSlots = 11264;   // [T * K] ints in 44 KB of shared memory
+template <int kSlots>
 __global__ void __launch_bounds__(kLLThreads, 1) ep_ll_combine_local_kernel(const LLCombineArgs a) {
   extern __shared__ int s_rowof[];
   const EpLLGeom& g = a.g;
@@ -150,36 +154,62 @@ __global__ void __launch_bounds__(kLLThreads, 1) ep_ll_combine_local_kernel(cons
   __syncthreads();
   const int nvec = g.H / 8;
   const int nchunk = (nvec + 31) / 32;
-  for (int item = blockIdx.x * kLLWarps + warp; item < a.T * nchunk; item += gridDim.x * kLLWarps) {
-    const int t = item / nchunk;
-    const int v = (item - t * nchunk) * 32 + lane;
-    if (v >= nvec) continue;
+  // Rows, weights and indices of the next item are on their way while this one is summed: rounds of items overlap.
+  struct Rows {
+    int4 vals[kSlots];
+    float wk[kSlots];
+  };
+  auto fetch = [&](int item, int k0, Rows* r) {
+    const int t = item / nchunk, v = (item - t * nchunk) * 32 + lane;
+    long long idx[kSlots];
+#pragma unroll
+    for (int u = 0; u < kSlots; ++u) {
+      const int k = k0 + u;
+      const int row = k < g.K && v < nvec ? s_rowof[t * g.K + k] : -1;
+      idx[u] = row >= 0 ? a.topk_idx[(size_t)t * g.K + k] : -1;
+      r->wk[u] = row >= 0 ? a.topk_w[(size_t)t * g.K + k] : 0.f;
+      r->vals[u] = row >= 0 ? ld_nc_v4(reinterpret_cast<const int4*>(a.y + (size_t)row * g.H) + v) : make_int4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < kSlots; ++u) {
+      if (idx[u] < 0) {
+        r->wk[u] = 0.f;
+        r->vals[u] = make_int4(0, 0, 0, 0);
+      }
+    }
+  };
+  auto add = [&](const Rows& r, float* acc) {
+#pragma unroll
+    for (int u = 0; u < kSlots; ++u) {
+      float f[8];
+      bf16x8_to_float(r.vals[u], f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = fmaf(r.wk[u], f[i], acc[i]);
+    }
+  };
+  Rows cur, next;
+  const int stride = gridDim.x * kLLWarps;
+  int item = blockIdx.x * kLLWarps + warp;
+  if (item < a.T * nchunk) fetch(item, 0, &cur);
+  for (; item < a.T * nchunk; item += stride) {
+    const int t = item / nchunk, v = (item - t * nchunk) * 32 + lane;
+    if (item + stride < a.T * nchunk) fetch(item + stride, 0, &next);
     float acc[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-    for (int k0 = 0; k0 < g.K; k0 += 8) {
-      int4 vals[8];
-      float wk[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int k = k0 + u;
-        const int row = k < g.K && a.topk_idx[(size_t)t * g.K + k] >= 0 ? s_rowof[t * g.K + k] : -1;
-        wk[u] = row >= 0 ? a.topk_w[(size_t)t * g.K + k] : 0.f;
-        vals[u] = row >= 0 ? ld_nc_v4(reinterpret_cast<const int4*>(a.y + (size_t)row * g.H) + v) : make_int4(0, 0, 0, 0);
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        float f[8];
-        bf16x8_to_float(vals[u], f);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i] = fmaf(wk[u], f[i], acc[i]);
-      }
+    add(cur, acc);
+    for (int k0 = kSlots; k0 < g.K; k0 += kSlots) {
+      fetch(item, k0, &cur);
+      add(cur, acc);
     }
-    int4 o;
-    __nv_bfloat162* po = reinterpret_cast<__nv_bfloat162*>(&o);
+    if (v < nvec) {
+      int4 o;
+      __nv_bfloat162* po = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) po[i] = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
-    reinterpret_cast<int4*>(a.out + (size_t)t * g.H)[v] = o;
+      for (int i = 0; i < 4; ++i) po[i] = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
+      reinterpret_cast<int4*>(a.out + (size_t)t * g.H)[v] = o;
+    }
+    cur = next;
   }
   if (blockIdx.x == 0) {   // the call ends: arrival words back to zero, next epoch (nobody else reads either during this kernel)
     uint32_t* exp_cnt = reinterpret_cast<uint32_t*>(self + a.off.exp_cnt[0]);
@@ -317,7 +347,10 @@ UMDK_API int umdk_ep_ll_combine(const UmdkEpLLCombineParams* p, void* stream) {
     int grid = p->num_ctas > 0 ? p->num_ctas : (items + kLLWarps - 1) / kLLWarps;
     if (grid > sm_count()) grid = sm_count();
     if (grid < 1) grid = 1;
-    ep_ll_combine_local_kernel<<<grid, kLLThreads, sizeof(int) * p->T * p->K, static_cast<cudaStream_t>(stream)>>>(a);
+    const auto combine = p->K <= 2   ? ep_ll_combine_local_kernel<2>
+                         : p->K <= 4 ? ep_ll_combine_local_kernel<4>
+                                     : ep_ll_combine_local_kernel<8>;
+    combine<<<grid, kLLThreads, sizeof(int) * p->T * p->K, static_cast<cudaStream_t>(stream)>>>(a);
     UMDK_CUDA_CHECK(cudaGetLastError());
     return 0;
   }

@@ -543,7 +543,7 @@ moe_fused_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constant
     // dispatch prologue: the operand ring is free until phase 1 and serves as its scratch
     LLDispatchIO io = a.disp;
     io.phase_mask = (a.phase_mask >> 2) & 3;
-    const bool sent = ll_dispatch_body<kThreads>(a.ll_geom, a.ll_off, a.peers, io, sh.ring, sh.goff);
+    const bool sent = ll_dispatch_body<kThreads, 1>(a.ll_geom, a.ll_off, a.peers, io, sh.ring, sh.goff);
     goff_local = (io.phase_mask & 2) != 0 && sent;
     fence_proxy_async_smem();   // the ring is written by TMA next
     __syncthreads();
