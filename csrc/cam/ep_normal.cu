@@ -303,7 +303,8 @@ struct DispatchArgs {
   volatile int* counts_host;   // same 4 ints in mapped pinned host memory + [4] = epoch stamp (may be null)
   volatile int64_t* per_expert_host;   // optional copy of recv_per_expert in mapped pinned host memory
   volatile int* status_host;   // one rank, with host_tag: copy of the status record in mapped host memory (may be null)
-  int host_tag;                // one rank: the last CTA sets counts_host[5] to it when everything is in memory (0: nobody waits)
+  int host_tag;                // one rank: counts_host[6] becomes it when the counts are there, and [5], from the last CTA, when
+                               // everything is in memory (0: nobody waits)
   int n_cap, a_cap;
   // control
   uint32_t* ctrl;              // [0] epoch, [2] recv-done counter, [10] staging gate (tag of the last staged call),
@@ -847,6 +848,15 @@ __global__ void __launch_bounds__(kEpThreads, 1) ep_dispatch_local_kernel(const 
       umdk_set_status(a.status, UMDK_ERR_OVERFLOW, UMDK_PH_DISPATCH_COUNT, total, arrivals);
   }
   __syncthreads();
+  if (a.host_tag != 0 && a.counts_host && blockIdx.x == 0 && threadIdx.x == kEpThreads - 1) {
+    // The counts first: the host makes its result of them while the rows are stored, 13 us of a call that it would else begin with
+    // when the kernel has ended.
+    a.counts_host[0] = total;
+    a.counts_host[1] = arrivals;
+    a.counts_host[2] = arrivals;
+    __threadfence_system();
+    a.counts_host[6] = a.host_tag;
+  }
   if (a.row_expert) {
     for (long long r = (long long)total + blockIdx.x * kEpThreads + threadIdx.x; r < a.n_cap;
          r += (long long)gridDim.x * kEpThreads) {
@@ -930,10 +940,12 @@ __global__ void __launch_bounds__(kEpThreads, 1) ep_dispatch_local_kernel(const 
     cur = next;
   }
   if (a.counts_host && blockIdx.x == 0 && threadIdx.x == 0) {   // last: nothing here has to wait for the host's memory
-    a.counts_host[0] = total;
-    a.counts_host[1] = arrivals;
-    a.counts_host[2] = arrivals;
-    __threadfence_system();
+    if (a.host_tag == 0) {
+      a.counts_host[0] = total;
+      a.counts_host[1] = arrivals;
+      a.counts_host[2] = arrivals;
+      __threadfence_system();
+    }
     a.counts_host[4] = (int)(a.ctrl[0] + 1);
   }
   // the epoch advances as in the exchanging kernel, so that the two can follow each other

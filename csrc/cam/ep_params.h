@@ -30,7 +30,8 @@ struct UmdkEpDispatchParams {
   float* row_weight;          // [n_cap] routing weight per row (0 behind them)
   int64_t* per_expert_host;   // optional [E/R] copy of recv_per_expert in mapped host memory
   int* status_host;           // optional [4] copy of the status record in mapped host memory, written with the tag
-  int host_tag;               // one rank: counts_host[5] becomes this when everything the call writes is in memory (0: not)
+  int host_tag;               // one rank: counts_host[6] becomes this when the counts are in host memory, [5] when everything the call
+                              // writes is in memory (0: neither)
 };
 
 struct UmdkEpCombineParams {

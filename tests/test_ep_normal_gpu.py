@@ -384,3 +384,25 @@ def test_host_copy_of_the_counts_of_several_ranks(R, E):
                                            (1200, 2176, 31, 5, True), (640, 6144, 33, 2, False)])
 def test_single_rank_rounds_of_items_and_many_experts(T, H, E, K, quant):
     test_single_rank_short_path_matches_exchange(T, H, E, K, quant)
+
+
+@pytest.mark.parametrize("T,E", [(1, 8), (2500, 600)])
+def test_counts_come_before_the_rows_and_the_report_behind_them(T, E):
+    """A dispatch of one rank that is not finished yet has its counts; what it has to report comes from finish()."""
+    from umdk_b200.ops.ep import KernelStatusError
+    xs, idxs, ws = _make_inputs(1, T, 256, E, 2, seed=T)
+    heaps, (st,) = _virtual_states(1, E, 2, 256, cap=T)
+    try:
+        x, idx, w = xs[0].cuda(), idxs[0].cuda(), ws[0].cuda()
+        want = st.dispatch(x, idx, w, sync_counts=True)
+        n = want.num_recv
+        got = st.dispatch(x, idx, w, sync_counts=True, finish=False)
+        assert got.num_recv == n and got.per_expert == want.per_expert
+        st.finish()
+        st.finish()   # once is enough
+        assert torch.equal(got.recv_x[:n].view(torch.uint8), want.recv_x[:n].view(torch.uint8))
+        st.dispatch(x, idx, w, sync_counts=True, finish=False, n_cap=n - 1)   # room for one row less
+        with pytest.raises(KernelStatusError):
+            st.finish()
+    finally:
+        heaps[0].close()

@@ -165,11 +165,12 @@ class Buffer:
                 return self._dispatch_static(st, x, topk_idx, topk_weights, use_fp8, el, async_finish)
             out = st.dispatch(x.contiguous(), topk_idx.contiguous(),
                               topk_weights.contiguous() if topk_weights is not None else None, quant=use_fp8,
-                              sync_counts=True, row_info=True)
+                              sync_counts=True, row_info=True, finish=False)
             n, per_expert = out.num_recv, out.per_expert
             rows_le, recv_w = out.row_expert[:n], out.row_weight[:n]
             recv_x = (out.recv_x[:n], out.recv_scales[:n]) if use_fp8 else out.recv_x[:n]
             h = DispatchHandle("gpu", topk_idx, topk_weights, T, gpu=out)
+            st.finish()   # the views and the handle are made while the rows are stored
             ev = EventOverlap(torch.cuda.current_stream().record_event()) if async_finish else EventOverlap()
             return recv_x, rows_le, recv_w, per_expert, h, ev
         res = cpu_dist.cpu_dispatch(x, topk_idx, topk_weights, E, self.group, quant=use_fp8)

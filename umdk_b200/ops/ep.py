@@ -242,6 +242,7 @@ class EpNormal(Recoverable):
         # a copy of the status record
         n = self.status_at = 8 + 2 * (num_experts // self.R)
         self.tag = 0   # of the last dispatch that the host waited for
+        self._unfinished = False   # its counts are here, its rows perhaps not yet
         self.mirror = HostMirror(n + 4)
         with torch.inference_mode(False):   # an inference tensor could not be written by a call outside of that mode
             self.status_host = torch.frombuffer(self.mirror.host, dtype=torch.int32)[n:]
@@ -311,10 +312,11 @@ class EpNormal(Recoverable):
     def dispatch(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_weights: Optional[torch.Tensor],
                  lay: Optional[LayoutResult] = None, quant: bool = True, n_cap: Optional[int] = None,
                  a_cap: Optional[int] = None, phase_mask: int = 3, out: Optional[DispatchResult] = None,
-                 sync_counts: bool = False, row_info: bool = False) -> DispatchResult:
+                 sync_counts: bool = False, row_info: bool = False, finish: bool = True) -> DispatchResult:
         """Runs notify + quantise + push + expand. ``phase_mask`` 1 / 2 run only the send / receive half (used to
         drive several virtual ranks from one process on one GPU). ``row_info``: the kernel also writes the local expert
-        and the routing weight of every row (``row_expert``, ``row_weight`` of a new result)."""
+        and the routing weight of every row (``row_expert``, ``row_weight`` of a new result). ``finish`` False (with
+        ``sync_counts``): returns when the host knows the counts, and the caller calls ``finish`` before it gives the result on."""
         self._guard()
         assert x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous()
         T, H = x.shape
@@ -359,19 +361,34 @@ class EpNormal(Recoverable):
             if rc != 0:
                 raise RuntimeError(f"umdk_ep_dispatch failed: {rc}")
         if wait:
-            # one wait for everything the host reads: the counts lie in mapped memory, the status record comes along
+            # what the host reads of a call lies in mapped memory, the status record comes along
             host = self.mirror.host
             if local:
-                rc = self.lib.umdk_wait_host_word(ctypes.byref(host, 20), self.tag, _native.stream_ptr())
-                if rc != 0:
-                    raise RuntimeError(f"waiting for the dispatch failed: {rc}")
+                self._wait_word(24)
             else:
                 self.status_host.copy_(self.status, non_blocking=True)
                 torch.cuda.current_stream().synchronize()
-            _raise_status(host[self.status_at:], self.status, "ep_dispatch", owner=self)
+                _raise_status(host[self.status_at:], self.status, "ep_dispatch", owner=self)
             out.num_recv = int(host[0])
             out.per_expert = host[8:8 + 2 * (self.E // self.R):2]   # low words: counts are far below 2^31
+            self._unfinished = local
+            if finish:
+                self.finish()
         return out
+
+    def _wait_word(self, at: int):
+        """Waits until the last dispatch has put its tag into the int ``at`` bytes into the mapped host memory."""
+        rc = self.lib.umdk_wait_host_word(ctypes.byref(self.mirror.host, at), self.tag, _native.stream_ptr())
+        if rc != 0:
+            raise RuntimeError(f"waiting for the dispatch failed: {rc}")
+
+    def finish(self):
+        """Waits until everything that the last ``dispatch(sync_counts=True, finish=False)`` writes is in memory; raises what it
+        reported."""
+        if self._unfinished:
+            self._unfinished = False
+            self._wait_word(20)
+            _raise_status(self.mirror.host[self.status_at:], self.status, "ep_dispatch", owner=self)
 
     @_trace.traced("umdk.ep.combine")
     def combine(self, y: torch.Tensor, disp: DispatchResult, apply_weights: bool = True, phase_mask: int = 3,
