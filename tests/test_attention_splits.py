@@ -54,3 +54,21 @@ def test_keys_of_a_split_are_those_that_the_kernel_takes(topk):
     from umdk_b200 import _native
     from umdk_b200.ops.attention import MAX_KEYS
     assert _native.cam().umdk_sparse_mla_min_splits(topk) == -(-topk // MAX_KEYS)
+
+
+# the same of the kernel whose chunks take 0.9 us
+MEASURED_SETS = {
+    (1, 213): {1: 12.2, 2: 14.1, 3: 13.5, 5: 12.6},
+    (1, 2048): {1: 46.8, 22: 14.8},
+    (8, 2048): {1: 47.6, 9: 19.8},
+    (23, 500): {1: 17.6, 2: 20.4, 3: 19.8},
+    (23, 1000): {1: 28.4, 3: 24.3},
+    (29, 692): {1: 21.6, 2: 24.6},
+    (36, 1000): {1: 28.2, 2: 31.2},
+}
+
+
+@pytest.mark.parametrize("batch,topk", list(MEASURED_SETS))
+def test_default_is_the_fastest_count_of_the_present_kernel(batch, topk):
+    times = MEASURED_SETS[batch, topk]
+    assert times[default_splits(batch, topk, 148)] <= 1.03 * min(times.values())

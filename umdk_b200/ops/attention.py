@@ -25,16 +25,16 @@ def _sm_count(device: int) -> int:
 @functools.lru_cache(maxsize=1024)
 def default_splits(batch: int, topk: int, sms: int, least: int = 1) -> int:
     """Splits of every key list: the count (at least ``least``, at most 24, one wave of CTA pairs) that takes the shortest
-    time, none of them without keys. A chunk of a split costs 1.4 us; a second split costs the merge, 5 us + 0.1 per
-    sequence, and each split's partials 0.06 + 0.03 per sequence. Measured (us, by splits): 1 sequence of 2048 keys
-    10: 22.3, 15: 19.8, 22: 19.0, 43: 19.9; of 240 keys 1: 16.2, 2: 18.7, 5: 16.4; 23 sequences of 240 keys 1: 16.8,
-    2: 22.8, of 1000 keys 2: 34.6, 3: 29.8, 4 (a second wave): 45.1. Within 2 % of the best count at 90 sizes of
-    97 - 4000 keys and 1 - 23 sequences."""
+    time, none of them without keys. A chunk of a split costs 0.9 us, and up to 0.47 more as the pairs fill the GPU; a second split
+    costs the partials and the merge, 3.4 us + 0.19 per sequence + 0.07 per split. Measured (us, by splits): 1 sequence of 2048 keys
+    1: 46.8, 22: 14.8; of 240 keys 1: 12.7, 5: 12.7; 8 of 500 1: 18.1, 6: 15.0; 16 of 500 1: 18.4, 4: 17.8; 23 of 500 1: 18.5,
+    3: 20.9, of 1000 1: 28.4, 3: 24.3; 36 of 1000 1: 29.1, 2: 31.2. (The kernel before this one took 1.4 us for a chunk; what was measured
+    with it is in the test.)"""
     chunks = -(-topk // CHUNK)
     most = max(least, min(sms // (2 * batch), 24), 1)
 
     def us(n):
-        return 1.4 * -(-chunks // n) + (5 + 0.1 * batch + (0.06 + 0.03 * batch) * n if n > 1 else 0)
+        return (0.9 + 0.0032 * batch * n) * -(-chunks // n) + (3.4 + 0.19 * batch + 0.07 * n if n > 1 else 0)
 
     n = min(range(least, most + 1), key=us)
     return -(-chunks // -(-chunks // n))
