@@ -624,7 +624,28 @@ moe_fused_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constant
   }
 
   // ---- combine tail ----
-  if (a.phase_mask & 1) {
+  // A group of one rank waits for its own CTAs only: the last one raises the flag first and clears the words behind it (they are for
+  // the next launch), and the call ends with the first CTA that is through, since all of them have read the epoch by then.
+  const bool alone = a.R == 1 && (a.phase_mask & 3) == 3;
+  if (alone) {
+    __shared__ int s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();   // (cumulative: the whole CTA's rows, behind the barrier)
+      s_last = atomicAdd(&a.ctrl[1], 1u) == gridDim.x - 1;
+      if (s_last) {
+        __threadfence();
+        st_release_gpu(reinterpret_cast<uint64_t*>(a.peers.base[0] + a.comb_flag_off), tag);
+        a.ctrl[1] = 0;
+      }
+    }
+    __syncthreads();
+    if (s_last) {
+      if (a.exp_cnt != nullptr)
+        for (int i = threadIdx.x; i < a.G; i += blockDim.x) a.exp_cnt[i] = 0;
+      for (int i = threadIdx.x; i < tiles; i += blockDim.x) a.tile_done[i] = 0;
+    }
+  } else if (a.phase_mask & 1) {
     if (cta_done_is_last(&a.ctrl[1], gridDim.x, a.R > 1)) {
       // Every CTA is through with the slab: the arrival words go back to zero BEFORE the combine flags go out - a
       // peer starts its next call (and adds to these words again) only after it has seen this rank's flag.
@@ -655,7 +676,9 @@ moe_fused_kernel(const __grid_constant__ CUtensorMap tmW1, const __grid_constant
     ll_weighted_reduce<kThreads>(self + a.comb_buf_off, a.topk_idx, a.topk_w, a.out, a.share_out, a.T, a.Kt, a.H);
   }
   stamp(5);
-  if (cta_done_is_last(&a.ctrl[2], gridDim.x, a.R > 1)) {
+  if (alone) {   // (where the wait ran out, reset() sets the epoch)
+    if (blockIdx.x == 0 && threadIdx.x == 0 && s_ok) a.ctrl[0] = epoch + 1;
+  } else if (cta_done_is_last(&a.ctrl[2], gridDim.x, a.R > 1)) {
     if (threadIdx.x == 0) a.ctrl[0] = epoch + 1;
   }
 }
