@@ -5,7 +5,11 @@
 // PRODUCTS are made once per (K block, token) by two further warps. Two kinds of tile, picked from the rows that are there:
 //
 // 64 tokens, the 256 weight rows of a pair on the MMA's M side (each CTA owns 128 of them x all tokens). For decode sizes (tens
-// of rows per expert), where the weights bound it: the ring keeps 9 x 16 KB of them in flight per SM. In MODE 0 the 128 rows of
+// of rows per expert), where the weights bound it: the ring keeps 8 x 16 KB of them in flight per SM. Barriers cover two K blocks:
+// with one each, the issuing thread's two waits, four MMAs and two commits and the promotion's waits took 500 to 680 cycles a K block.
+// Barriers per K block, a thread with a whole TMEM row / this, kernel us: 3000 rows of 32 experts, 3584 x 1024, 82.0 / 75.0 (MODE 0)
+// and 46.0 / 41.6 (MODE 1), 1024 of 32, 7168 x 2048 148.5 / 146.5 (6.4 TB/s of weights) and 82.5 / 78.5, 64 of 4, 2048 x 512 10.4 / 8.8;
+// two K blocks' loads behind one another's FMAs 103 instead of 75 (spilled registers). In MODE 0 the 128 rows of
 // a CTA are 64 gate rows and the 64 up rows of the same features, so that a pair finishes one 1x128 scale block: the
 // per-token maxima of the two halves cross once per item through distributed shared memory.
 //
@@ -21,6 +25,8 @@
 #include "moe_gemm_pair.cuh"
 #include "ptx.cuh"
 
+#include <type_traits>
+
 namespace umdk {
 namespace {
 
@@ -35,15 +41,17 @@ struct Cfg {
   static constexpr int kABytes = 128 * kBKB;
   static constexpr int kBBytes = kTok / 2 * kBKB;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = 9;
+  static constexpr int kGroup = 2;                              // K blocks of a barrier's phase
+  static constexpr int kStages = 4;                             // groups in flight
+  static constexpr int kGroupBytes = kGroup * kStageBytes;
   static constexpr int kBoxRows = kTok / 2;                     // token rows per TMA box
   static constexpr int kW = MODE == 0 ? 2 : 1;                  // scale rows per CTA (gate, up)
   static constexpr int kScaleKb = 8;                            // K blocks per scale stage
   static constexpr int kScaleStages = 3;
   static constexpr int kScaleFloats = kScaleKb * kW * kTok;
-  static constexpr int kTmemStages = 512 / kTok;                // accumulators in flight hide the hand-over between CTAs
-  static constexpr int kTransBytes = 32 * 272;                  // per half: [32][136] bf16 or [32][65] fp32
-  static constexpr int kOffScale = kStages * kStageBytes;
+  static constexpr int kTmemStages = 512 / kTok / kGroup;       // groups of accumulators in flight hide the hand-over between CTAs
+  static constexpr int kTransBytes = 32 * 272;                  // per half: [32][136] bf16 or [32][68] fp32
+  static constexpr int kOffScale = kStages * kGroupBytes;
   static constexpr int kOffTrans = kOffScale + kScaleStages * kScaleFloats * 4;
   static constexpr int kOffAmax = kOffTrans + 2 * kTransBytes;  // [2][kTok] maxima of the partner's half
   static constexpr int kEnd = kOffAmax + 2 * kTok * 4;
@@ -175,22 +183,25 @@ __device__ __forceinline__ void weight_body(uint8_t* smem, const CUtensorMap& tm
           const int nh = it.n / 2;
           const int xrow = it.row0 + (int)cta * nh;
           const int wrow = it.e * a.w_rows + (MODE == 0 ? it.j * 128 + (int)cta * 64 : it.j * 256 + (int)cta * 128);
-          for (int kb = 0; kb < kb_total; ++kb) {
+          for (int kb0 = 0; kb0 < kb_total; kb0 += C::kGroup) {
             if (!mbar_wait(&empty[s], ph ^ 1)) {
-              umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_EMPTY, w, kb);
+              umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_EMPTY, w, kb0);
               ok = false;
               break;
             }
-            if (cta == 0) mbar_expect_tx(&full[s], 2 * C::kStageBytes);
+            const int kb1 = min(kb_total, kb0 + C::kGroup);
+            if (cta == 0) mbar_expect_tx(&full[s], (kb1 - kb0) * 2 * C::kStageBytes);
             const uint32_t leader_full = map_to_cta(&full[s], 0);
-            uint8_t* st = smem + s * C::kStageBytes;
-            if (MODE == 0) {
-              tma_load_2d_pair(st, &tmW, leader_full, kb * kBKB, wrow);
-              tma_load_2d_pair(st + 64 * kBKB, &tmW, leader_full, kb * kBKB, wrow + a.Nout);
-            } else {
-              tma_load_2d_pair(st, &tmW, leader_full, kb * kBKB, wrow);
+            uint8_t* st = smem + s * C::kGroupBytes;
+            for (int kb = kb0; kb < kb1; ++kb, st += C::kStageBytes) {
+              if (MODE == 0) {
+                tma_load_2d_pair(st, &tmW, leader_full, kb * kBKB, wrow);
+                tma_load_2d_pair(st + 64 * kBKB, &tmW, leader_full, kb * kBKB, wrow + a.Nout);
+              } else {
+                tma_load_2d_pair(st, &tmW, leader_full, kb * kBKB, wrow);
+              }
+              tma_load_2d_pair(st + C::kABytes, &tmX, leader_full, kb * kBKB, xrow);
             }
-            tma_load_2d_pair(st + C::kABytes, &tmX, leader_full, kb * kBKB, xrow);
             if (++s == C::kStages) {
               s = 0;
               ph ^= 1;
@@ -201,30 +212,34 @@ __device__ __forceinline__ void weight_body(uint8_t* smem, const CUtensorMap& tm
     } else if (warp == 1) {
       if (cta == 0 && elect_one()) {
         int s = 0;
-        uint32_t ph = 0, kbc = 0;
+        uint32_t ph = 0, n_groups = 0;
         bool ok = true;
         const uint64_t a_desc = umma_desc_k_sw128(smem_u32(smem));
         for (int w = pair; w < num_items && ok; w += num_pairs) {
           const Item it = locate(tile_pref, goff, a.G, NT, w);
           const uint32_t idesc = umma_idesc(kFmtE4M3, kFmtE4M3, 256, it.n);
-          for (int kb = 0; kb < kb_total; ++kb, ++kbc) {
-            const int ts = kbc % C::kTmemStages;
-            if (!mbar_wait(&tempty[ts], ((kbc / C::kTmemStages) & 1) ^ 1)) {
-              umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_EMPTY, w, kb);
+          for (int kb0 = 0; kb0 < kb_total; kb0 += C::kGroup, ++n_groups) {
+            const int ts = n_groups % C::kTmemStages;
+            if (!mbar_wait(&tempty[ts], ((n_groups / C::kTmemStages) & 1) ^ 1)) {
+              umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_EMPTY, w, kb0);
               ok = false;
               break;
             }
             if (!mbar_wait(&full[s], ph)) {
-              umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, kb);
+              umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, kb0);
               ok = false;
               break;
             }
             tc_fence_after();
-            const uint64_t adesc = a_desc + s * (C::kStageBytes >> 4);
-            const uint64_t bdesc = adesc + (C::kABytes >> 4);
 #pragma unroll
-            for (int k = 0; k < 4; ++k)   // 32 fp8 elements per MMA K step
-              umma_f8_pair(tmem_base + ts * kTok, adesc + 2 * k, bdesc + 2 * k, idesc, k > 0 ? 1u : 0u);
+            for (int b = 0; b < C::kGroup; ++b) {
+              if (kb0 + b >= kb_total) break;
+              const uint64_t adesc = a_desc + ((s * C::kGroupBytes + b * C::kStageBytes) >> 4);
+              const uint64_t bdesc = adesc + (C::kABytes >> 4);
+#pragma unroll
+              for (int k = 0; k < 4; ++k)   // 32 fp8 elements per MMA K step
+                umma_f8_pair(tmem_base + (ts * C::kGroup + b) * kTok, adesc + 2 * k, bdesc + 2 * k, idesc, k > 0 ? 1u : 0u);
+            }
             umma_commit_both(smem_u32(&empty[s]));
             umma_commit_both(smem_u32(&tfull[ts]));
             if (++s == C::kStages) {
@@ -292,64 +307,120 @@ __device__ __forceinline__ void weight_body(uint8_t* smem, const CUtensorMap& tm
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     const uint32_t peer = cta ^ 1u;
     int ss = 0, n_it = 0;
-    uint32_t sph = 0, kbc = 0;
+    uint32_t sph = 0, n_groups = 0;
     bool ok = true;
     for (int w = pair; w < num_items && ok; w += num_pairs, ++n_it) {
       const Item it = locate(tile_pref, goff, a.G, NT, w);
       const int nh = it.n / 2, col0 = half * nh;
       const int par = n_it & 1;
       if (MODE == 0 && warp == 4 && lane == 0) mbar_expect_tx(&abar[par], it.n * 4);
-      uint64_t acc[16];   // pairs of tokens
+      // A warp covers 32 rows x HC tokens, a thread four of the rows x two of every eight tokens (see tmem_ld_16x256b_x1): with a row
+      // and all of the tokens the scales came in 16-byte broadcast loads, 256 of the shared-memory port's cycles a K block next
+      // to 320 for the operands' way in and out. The load of the other 16 lanes, or of the next K block, runs behind the FMAs.
+      auto item = [&](auto hc) {
+        constexpr int HC = decltype(hc)::value;
+        uint64_t acc[2][HC / 4];   // [lane half][8-token group, row t / 4 or t / 4 + 8]
+        uint32_t r[2][HC / 2];
 #pragma unroll
-      for (int c = 0; c < 16; ++c) acc[c] = 0;
-      for (int kb0 = 0; kb0 < kb_total && ok; kb0 += C::kScaleKb) {
-        if (!mbar_wait_warp(&sfull[ss], sph)) {
-          umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, 10000 + kb0);
-          ok = false;
-          break;
-        }
-        const float* sc = scale_sm + ss * C::kScaleFloats + which * kTok + col0;
-        const int kb1 = min(kb_total, kb0 + C::kScaleKb);
-        for (int kb = kb0; kb < kb1; ++kb, ++kbc, sc += C::kW * kTok) {
-          const int ts = kbc % C::kTmemStages;
-          if (!mbar_wait_warp(&tfull[ts], (kbc / C::kTmemStages) & 1)) {
-            umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, w, kb);
+        for (int c = 0; c < HC / 4; ++c) acc[0][c] = acc[1][c] = 0;
+        auto load = [&](int b, int h) {   // of K block b of the group
+          const uint32_t addr = lane_addr + ((n_groups % C::kTmemStages) * C::kGroup + b) * kTok + col0 + (h << 20);
+          if constexpr (HC == 32) tmem_ld_16x256b_x4(addr, r[h]);
+          else tmem_ld_16x256b_x2(addr, r[h]);
+        };
+        auto take = [&]() {   // waits for a group of accumulators and starts the load of its first half block
+          ok = mbar_wait_warp(&tfull[n_groups % C::kTmemStages], (n_groups / C::kTmemStages) & 1);
+          if (!ok) {
+            umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, w, (int)n_groups);
+            return;
+          }
+          tc_fence_after();
+          load(0, 0);
+        };
+        auto promote = [&](const uint64_t* x2, int h) {
+#pragma unroll
+          for (int g = 0; g < HC / 8; ++g) {
+#pragma unroll
+            for (int rr = 0; rr < 2; ++rr) {
+              uint64_t& d = acc[h][2 * g + rr];
+              d = fma_f32x2(pack_f32x2(r[h][4 * g + 2 * rr], r[h][4 * g + 2 * rr + 1]), x2[g], d);
+            }
+          }
+        };
+        take();
+        for (int kb0 = 0; kb0 < kb_total && ok; kb0 += C::kScaleKb) {
+          if (!mbar_wait_warp(&sfull[ss], sph)) {
+            umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, 10000 + kb0);
+            tmem_ld_wait();   // the load that take() has started
             ok = false;
             break;
           }
-          tc_fence_after();
-          uint32_t r[32];
-          tmem_ld_x32(lane_addr + ts * kTok + col0, r);
-          tmem_ld_wait();
-          // everything of this stage is in registers: the next K block may overwrite it
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster_relaxed(map_to_cta(&tempty[ts], 0));
+          const float* sc = scale_sm + ss * C::kScaleFloats + which * kTok + col0 + 2 * (lane & 3);
+          const int kb1 = min(kb_total, kb0 + C::kScaleKb);
+          for (int kb = kb0; kb < kb1 && ok; kb += C::kGroup) {
 #pragma unroll
-          for (int c4 = 0; c4 < 8; ++c4) {
-            const ulonglong2 s4 = reinterpret_cast<const ulonglong2*>(sc)[c4];
-            acc[2 * c4] = fma_f32x2(pack_f32x2(r[4 * c4], r[4 * c4 + 1]), s4.x, acc[2 * c4]);
-            acc[2 * c4 + 1] = fma_f32x2(pack_f32x2(r[4 * c4 + 2], r[4 * c4 + 3]), s4.y, acc[2 * c4 + 1]);
+            for (int b = 0; b < C::kGroup; ++b, sc += C::kW * kTok) {
+              if (kb + b >= kb1) break;
+              uint64_t x2[HC / 8];
+#pragma unroll
+              for (int g = 0; g < HC / 8; ++g) x2[g] = *reinterpret_cast<const uint64_t*>(sc + 8 * g);
+              tmem_ld_wait();
+              load(b, 1);
+              promote(x2, 0);
+              tmem_ld_wait();
+              if (b + 1 < C::kGroup && kb + b + 1 < kb1) {
+                load(b + 1, 0);
+              } else {
+                // everything of this group is in registers: the MMAs may overwrite it
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster_relaxed(map_to_cta(&tempty[n_groups % C::kTmemStages], 0));
+                ++n_groups;
+                if (kb + b + 1 < kb_total) take();
+              }
+              promote(x2, 1);
+            }
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sempty[ss]);
+          if (++ss == C::kScaleStages) {
+            ss = 0;
+            sph ^= 1;
           }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sempty[ss]);
-        if (++ss == C::kScaleStages) {
-          ss = 0;
-          sph ^= 1;
-        }
-      }
-      ok = bar_and<128>(1 + half, ok);
-      if (!ok) break;
-      float v[32];
+        ok = bar_and<128>(1 + half, ok);
+        if (!ok) return;
+        // through shared memory to threads that have one token: bf16 results, or up values and then silu(gate) * up
+        __nv_bfloat16* tb = reinterpret_cast<__nv_bfloat16*>(trans);   // [32 tokens][136]
+        float* tf = reinterpret_cast<float*>(trans);                   // [32 tokens][68]
+        auto each = [&](auto f) {
 #pragma unroll
-      for (int c = 0; c < 16; ++c) unpack_f32x2(acc[c], &v[2 * c], &v[2 * c + 1]);
+          for (int g = 0; g < HC / 8; ++g) {
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {   // lane half, row
+              float v[2];
+              unpack_f32x2(acc[h >> 1][2 * g + (h & 1)], &v[0], &v[1]);
+              const int tok = 8 * g + 2 * (lane & 3), row = h * 8 + (lane >> 2);
+              f(tok, row, v[0]);
+              f(tok + 1, row, v[1]);
+            }
+          }
+        };
+        if constexpr (MODE == 1) {
+          each([&](int t, int row, float v) { tb[t * 136 + q * 32 + row] = __float2bfloat16(v); });
+        } else {
+          const int f0 = (q & 1) * 32;   // feature inside this CTA's 64
+          if (which == 1) each([&](int t, int row, float v) { tf[t * 68 + f0 + row] = v; });
+          bar_half(half);
+          if (which == 0) each([&](int t, int row, float v) { tf[t * 68 + f0 + row] = silu(v) * tf[t * 68 + f0 + row]; });
+        }
+        bar_half(half);
+      };
+      if (nh == 16) item(std::integral_constant<int, 16>());
+      else item(std::integral_constant<int, 32>());
+      if (!ok) break;
       if (MODE == 1) {
         const int feat0 = it.j * 256 + (int)cta * 128;
-        __nv_bfloat16* tb = reinterpret_cast<__nv_bfloat16*>(trans);
-#pragma unroll
-        for (int t = 0; t < 32; ++t) tb[t * 136 + tid] = __float2bfloat16(v[t]);
-        bar_half(half);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int i = u * 128 + tid, t = i >> 4, tok = col0 + t;
@@ -360,28 +431,22 @@ __device__ __forceinline__ void weight_body(uint8_t* smem, const CUtensorMap& tm
         }
         bar_half(half);
       } else {
-        float* tf = reinterpret_cast<float*>(trans);   // [32 tokens][65]: up values, then h
-        const int f = (q & 1) * 32 + lane;             // feature inside this CTA's 64
-        const int t4 = tid >> 2, qq = tid & 3;         // afterwards: token and 16-feature quarter of a thread
+        const float4* tf = reinterpret_cast<const float4*>(trans);   // [32 tokens][17]
+        const int t4 = tid >> 2, qq = tid & 3;         // token and 16-feature quarter of a thread
         const int tok = col0 + t4;
         const uint32_t peer_amax = map_to_cta(amax_in + par * kTok, peer);
         const uint32_t peer_bar = map_to_cta(&abar[par], peer);
-        if (which == 1) {
-#pragma unroll
-          for (int t = 0; t < 32; ++t) tf[t * 65 + f] = v[t];
-        }
-        bar_half(half);
-        if (which == 0) {
-#pragma unroll
-          for (int t = 0; t < 32; ++t) tf[t * 65 + f] = silu(v[t]) * tf[t * 65 + f];
-        }
-        bar_half(half);
         float h[16], mx = 0.f;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          h[i] = tf[t4 * 65 + qq * 16 + i];
-          mx = fmaxf(mx, fabsf(h[i]));
+        for (int i = 0; i < 4; ++i) {
+          const float4 v = tf[t4 * 17 + qq * 4 + i];
+          h[4 * i] = v.x;
+          h[4 * i + 1] = v.y;
+          h[4 * i + 2] = v.z;
+          h[4 * i + 3] = v.w;
         }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) mx = fmaxf(mx, fabsf(h[i]));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         if (qq == 0 && t4 < nh) st_async_b32(peer_amax + tok * 4, __float_as_uint(mx), peer_bar);

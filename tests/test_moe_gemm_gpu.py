@@ -249,3 +249,16 @@ def test_swiglu_quotient_against_the_division():
         apart = (s.view(torch.int32).long() - scales.view(torch.int32).long()).abs()
         assert int(apart.max()) <= 1
         assert torch.equal(c, codes)
+
+
+# odd and even numbers of K blocks around a group's two and a scale stage's eight, in tiles of 32 and of 64 tokens, one item a pair and
+# several
+@pytest.mark.parametrize("G,counts,K,F,H", [
+    (2, [5, 40], 256, 384, 128),
+    (3, [32, 33, 64], 384, 128, 256),
+    (2, [17, 50], 1024, 1152, 384),
+    (4, [1, 64, 0, 34], 1152, 128, 256),
+    (2, [30, 60], 2176, 256, 512),
+])
+def test_groups_of_k_blocks_match_single_ctas(G, counts, K, F, H):
+    test_single_ctas_match_the_pairs(G, counts, K, F, H)
