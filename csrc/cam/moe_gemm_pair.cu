@@ -19,7 +19,16 @@
 // block. Measured against 256-token tiles of the other kind (32 experts, hidden 7168, width 2048, 16384 rows spread unevenly):
 // 1188 -> 573 us (MODE 0) and 513 -> 328 us (MODE 1), 1.6 PFLOP/s; two promotions in one instruction (fma.rn.f32x2) are part
 // of it. A K block takes 900 cycles at 1.45 GHz under the power limit: the tensor cores 512, the rest is the promotion's chain
-// (wait, four to eight TMEM loads, 64 packed FMAs, release) of two warps a scheduler, which all but fills it.
+// (wait, four to eight TMEM loads, 64 packed FMAs, release) of two warps a scheduler, which all but fills it. (One barrier for both
+// accumulators of a K block instead of two: 629 / 655 us; what bounds it is the way round through TMEM, not the issuing thread.)
+// An expert's last tile of at most 128 tokens is a HALF one: an MMA of 128 rows, 64 of each CTA, whose accumulator has columns 0 - 63
+// in TMEM lanes 0 - 63 and columns 64 - 127 of the same tokens in lanes 64 - 127: half of the columns for each promoting thread, 800
+// cycles a K block instead of 1000 where nothing else runs (two experts of 7168 x 2048 on eight CTAs, MODE 0 238 / 189 us, MODE 1
+// 146 / 124). A pair takes its half tiles behind the whole ones, so that no pair has whole ones only (in the order of the experts:
+// no gain). Whole tiles for all / this, us of MODE 0 and 1: 7000 rows of 64 experts, 4096 x 1024, 171 + 112 / 156 + 96; 2500 of 8,
+// 5120 x 896, 54.5 + 32.0 / 52.1 + 30.5; 16384 of 32, 7168 x 2048, where a fifth of the tiles are half ones and their weights come
+// from memory once more, 629 + 355 / 623 + 351. With eight accumulators of 64 columns 152 + 91, 55 + 31 and 625 + 345, and the
+// registers of the whole tiles spill.
 #include "ep_common.cuh"
 #include "fp8_block.cuh"
 #include "moe_gemm_pair.cuh"
@@ -57,8 +66,8 @@ struct Cfg {
   static constexpr int kEnd = kOffAmax + 2 * kTok * 4;
 };
 
-// Tiles with the TOKENS on the MMA's M side: one item = 256 tokens x 256 weight rows of one expert, each CTA of the pair owns 128
-// of the tokens (its TMEM lanes) x all 256 rows, as two accumulators of 128 columns per K block, one for each four of the
+// Tiles with the TOKENS on the MMA's M side: one item = 256 tokens (or up to 128) x 256 weight rows of one expert, each CTA of the pair
+// owns 128 of the tokens (its TMEM lanes; or 64) x all 256 rows, as two accumulators of 128 columns per K block, one for each four of the
 // promoting warps - in MODE 0 64 gate rows and the up rows of the same features, so a thread has both factors of SwiGLU.
 template <int MODE>
 struct TokCfg {
@@ -122,8 +131,12 @@ __device__ __forceinline__ void bar_half(int half) {
   asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
 }
 
+__device__ __forceinline__ void bar_two(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+
+constexpr int kHalfBits = 11;   // enough for the 1024 experts of moe_gemm_pair_fits
+
 struct Item {
-  int e, j, row0, m, n;   // expert, feature tile, first row, valid rows, rows the MMA covers (multiple of 32)
+  int e, j, row0, m, n;   // expert, feature tile, first row, valid rows, rows the MMAs cover (a multiple of 32; 128 or 256 on the M side)
 };
 
 __device__ __forceinline__ Item locate(const int* tile_pref, const int* goff, int G, int NT, int w) {
@@ -471,22 +484,27 @@ __device__ __forceinline__ void weight_body(uint8_t* smem, const CUtensorMap& tm
   }
 }
 
-__device__ __forceinline__ Item locate_tokens(const int* tile_pref, const int* goff, int G, int NT, int w) {
-  int lo = 0, hi = G;   // largest lo with tile_pref[lo] * NT <= w
+// `pref`: whole tiles before each expert in the upper bits, half tiles (at most one per expert) in the lower kHalfBits.
+__device__ __forceinline__ Item locate_tokens(const int* pref, const int* goff, int G, int NT, int w) {
+  const int whole = (pref[G] >> kHalfBits) * NT;
+  const bool half = w >= whole;
+  if (half) w -= whole;
+  auto before = [&](int e) { return half ? pref[e] & ((1 << kHalfBits) - 1) : pref[e] >> kHalfBits; };
+  int lo = 0, hi = G;   // largest lo with before(lo) * NT <= w
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
-    if (tile_pref[mid] * NT <= w) lo = mid;
+    if (before(mid) * NT <= w) lo = mid;
     else hi = mid;
   }
-  const int ntt = tile_pref[lo + 1] - tile_pref[lo];
-  const int local = w - tile_pref[lo] * NT;
+  const int ntt = (pref[lo + 1] >> kHalfBits) - (pref[lo] >> kHalfBits);   // whole tiles
+  const int local = w - before(lo) * NT;
   Item it;
   it.e = lo;
-  it.j = local / ntt;   // token tiles fastest
-  const int first = (local - it.j * ntt) * 256;
+  it.j = half ? local : local / ntt;   // token tiles fastest
+  const int first = (half ? ntt : local - it.j * ntt) * 256;
   it.row0 = goff[lo] + first;
   it.m = min(256, goff[lo + 1] - it.row0);
-  it.n = 256;
+  it.n = half ? 128 : 256;
   return it;
 }
 
@@ -502,7 +520,7 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int NT = feature_tiles(MODE, a.Nout);
   const int kb_total = a.K / kBKB;
-  const int num_items = bars->ok ? tile_pref[a.G] * NT : 0;
+  const int num_items = bars->ok ? ((tile_pref[a.G] >> kHalfBits) + (tile_pref[a.G] & ((1 << kHalfBits) - 1))) * NT : 0;
 
   if (warp < 4) {
     regs_dec<MODE == 0 ? 56 : 80>();
@@ -513,7 +531,7 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
         bool ok = true;
         for (int w = pair; w < num_items && ok; w += num_pairs) {
           const Item it = locate_tokens(tile_pref, goff, a.G, NT, w);
-          const int xrow = it.row0 + (int)cta * 128;
+          const int xrow = it.row0 + (int)cta * (it.n / 2);
           // columns of an accumulator: 64 weight rows of the leader, 64 of its partner
           const int wrow = it.e * a.w_rows + (MODE == 0 ? it.j * 128 + (int)cta * a.Nout : it.j * 256 + (int)cta * 64);
           const int wstep = MODE == 0 ? 64 : 128;
@@ -538,12 +556,12 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
       }
     } else if (warp == 1) {
       if (cta == 0 && elect_one()) {
-        constexpr uint32_t idesc = umma_idesc(kFmtE4M3, kFmtE4M3, 256, 128);
         int s = 0;
         uint32_t ph = 0, n = 0;   // n: accumulators so far
         bool ok = true;
         const uint64_t a_desc = umma_desc_k_sw128(smem_u32(smem));
         for (int w = pair; w < num_items && ok; w += num_pairs) {
+          const uint32_t idesc = umma_idesc(kFmtE4M3, kFmtE4M3, locate_tokens(tile_pref, goff, a.G, NT, w).n, 128);
           for (int kb = 0; kb < kb_total && ok; ++kb) {
             if (!mbar_wait(&bars->full[s], ph)) {
               umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, kb);
@@ -577,7 +595,7 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
         if (!mbar_wait(&bars->fin, 0)) umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMEM_FULL, -1, 0);
       }
     } else {
-      // ---- scale products of the coming K blocks for this CTA's 128 tokens ----
+      // ---- scale products of the coming K blocks for this CTA's 128 tokens, or for 64 of which each has two lanes ----
       float* scale_sm = reinterpret_cast<float*>(smem + C::kOffScale);
       const int t64 = threadIdx.x - 64;
       const int nsb = a.K / 128, wsb = a.w_rows / 128;
@@ -590,8 +608,10 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
         const float* ws1 = MODE == 0 ? ws0 + (size_t)(a.Nout / 128) * nsb : 2 * it.j + 1 < wsb ? ws0 + nsb : ws0;
         for (int kb0 = 0; kb0 < kb_total; kb0 += C::kScaleKb) {
           float w0[C::kScaleKb], w1[C::kScaleKb], xv[C::kScaleKb];
-          const float* xs = a.xs + (size_t)(it.row0 + (int)cta * 128 + t64) * nsb + kb0;
-          const int rows = it.m - (int)cta * 128 - t64;   // token t64 + 64 u is this expert's where 64 u < rows
+          const bool few = it.n == 128;
+          const int first = (int)cta * (it.n / 2) + t64;
+          const float* xs = a.xs + (size_t)(it.row0 + first) * nsb + kb0;
+          const int rows = it.m - first;   // token t64 + 64 u is this expert's where 64 u < rows
 #pragma unroll
           for (int i = 0; i < C::kScaleKb; ++i) {
             const bool in = kb0 + i < kb_total;
@@ -609,9 +629,10 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
           for (int u = 0; u < 2; ++u) {
 #pragma unroll
             for (int i = 0; i < C::kScaleKb; ++i) {
-              dst[(i * 2) * 128 + 64 * u] = xv[i] * w0[i];
+              // (in MODE 0 the upper lanes of a half tile have the up columns)
+              dst[(i * 2) * 128 + 64 * u] = xv[i] * (MODE == 0 && u == 1 && few ? w1[i] : w0[i]);
               dst[(i * 2 + 1) * 128 + 64 * u] = xv[i] * w1[i];
-              if (u == 0) xv[i] = kb0 + i < kb_total && rows > 64 ? xs[(size_t)64 * nsb + i] : 0.f;
+              if (u == 0 && !few) xv[i] = kb0 + i < kb_total && rows > 64 ? xs[(size_t)64 * nsb + i] : 0.f;
             }
           }
           __syncwarp();
@@ -664,54 +685,63 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
 #pragma unroll
       for (int c = 0; c < 64; ++c) acc[c] = 0;
       take(n, w);
-      for (int left = kb_total; left > 0 && ok;) {
-        if (!mbar_wait_warp(bars_sm + (uint32_t)offsetof(Bars, sfull) + ss * 8, sph)) {
-          umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, 10000 + left);
-          tmem_ld_wait();   // the load that take() has started
-          ok = false;
-          break;
-        }
-        uint32_t sc = scales + ss * C::kScaleFloats * 4;
-        const uint32_t end = sc + min(left, C::kScaleKb) * 1024;
-        left -= C::kScaleKb;
+      auto accumulate = [&](auto num_loads) {
+        constexpr int kNum = decltype(num_loads)::value;
+        for (int left = kb_total; left > 0 && ok;) {
+          if (!mbar_wait_warp(bars_sm + (uint32_t)offsetof(Bars, sfull) + ss * 8, sph)) {
+            umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, 10000 + left);
+            tmem_ld_wait();   // the load that take() has started
+            ok = false;
+            break;
+          }
+          uint32_t sc = scales + ss * C::kScaleFloats * 4;
+          const uint32_t end = sc + min(left, C::kScaleKb) * 1024;
+          left -= C::kScaleKb;
 #pragma unroll 1
-        for (; sc < end && ok; ++n, sc += 1024) {
-          const uint32_t f0 = ld_shared_u32(sc + (MODE == 0 ? 0 : u * 512));
-          const uint32_t f1 = MODE == 0 ? ld_shared_u32(sc + 512) : f0;
+          for (; sc < end && ok; ++n, sc += 1024) {
+            const uint32_t f0 = ld_shared_u32(sc + (MODE == 0 ? 0 : u * 512));
+            const uint32_t f1 = MODE == 0 && kNum == kLoads ? ld_shared_u32(sc + 512) : f0;
 #pragma unroll
-          for (int b = 0; b < kLoads; ++b) {   // the load of the next columns runs behind the FMAs of these
-            tmem_ld_wait();
-            if (b + 1 < kLoads) {
-              load(cols + (n & 1) * 256 + (b + 1) * kCols, r[(b + 1) & 1]);
-            } else {   // all of it is in registers: the MMAs may overwrite it
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive_cluster_relaxed<2>(tempty + (n & 1) * 16);
-              if (left > 0 || sc + 1024 < end) take(n + 1, w);
-            }
-            const uint64_t f = b < kLoads / 2 ? pack_f32x2(f0, f0) : pack_f32x2(f1, f1);
+            for (int b = 0; b < kNum; ++b) {   // the load of the next columns runs behind the FMAs of these
+              tmem_ld_wait();
+              if (b + 1 < kNum) {
+                load(cols + (n & 1) * 256 + (b + 1) * kCols, r[(b + 1) & 1]);
+              } else {   // all of it is in registers: the MMAs may overwrite it
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster_relaxed<2>(tempty + (n & 1) * 16);
+                if (left > 0 || sc + 1024 < end) take(n + 1, w);
+              }
+              const uint64_t f = b < kLoads / 2 ? pack_f32x2(f0, f0) : pack_f32x2(f1, f1);
 #pragma unroll
-            for (int c = 0; c < kCols / 2; ++c) {
-              uint64_t& d = acc[b * (kCols / 2) + c];
-              d = fma_f32x2(pack_f32x2(r[b & 1][2 * c], r[b & 1][2 * c + 1]), f, d);
+              for (int c = 0; c < kCols / 2; ++c) {
+                uint64_t& d = acc[b * (kCols / 2) + c];
+                d = fma_f32x2(pack_f32x2(r[b & 1][2 * c], r[b & 1][2 * c + 1]), f, d);
+              }
             }
           }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->sempty[ss]);
+          if (++ss == C::kScaleStages) {
+            ss = 0;
+            sph ^= 1;
+          }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars->sempty[ss]);
-        if (++ss == C::kScaleStages) {
-          ss = 0;
-          sph ^= 1;
-        }
-      }
+      };
+      const bool few = locate_tokens(tile_pref, goff, a.G, NT, w).n == 128;
+      if (few) accumulate(std::integral_constant<int, kLoads / 2>());
+      else accumulate(std::integral_constant<int, kLoads>());
       const Item it = locate_tokens(tile_pref, goff, a.G, NT, w);
-      const int rows = min(32, it.m - ((int)cta * 128 + q * 32));   // valid tokens of this warp (may be negative)
-      const size_t row0 = (size_t)it.row0 + (int)cta * 128 + q * 32;
+      const int tok0 = (int)cta * (it.n / 2) + (few ? q & 1 : q) * 32;
+      const int rows = MODE == 0 && few && q >= 2 ? 0 : min(32, it.m - tok0);   // valid tokens of this warp (may be negative)
+      const size_t row0 = (size_t)it.row0 + tok0;
       if (MODE == 1) {
         if (!ok) break;
         const int feat0 = it.j * 256 + u * 128;
 #pragma unroll
         for (int p = 0; p < 2; ++p) {   // 64 features at a time
+          if (p == 1 && few) break;
+          const int feat = feat0 + (few ? q >> 1 : p) * 64;
           __syncwarp();
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
@@ -731,11 +761,27 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
             for (int i = 0; i < 8; ++i) {
               const int t = i * 4 + (lane >> 3), seg = lane & 7;
               const int4 o = *reinterpret_cast<const int4*>(trans + t * 128 + ((seg ^ (t & 7)) << 4));
-              if (t < rows) *reinterpret_cast<int4*>(a.y + (row0 + t) * a.Nout + feat0 + p * 64 + seg * 8) = o;
+              if (t < rows) *reinterpret_cast<int4*>(a.y + (row0 + t) * a.Nout + feat + seg * 8) = o;
             }
           }
         }
       } else {
+        if (few) {   // the up values from the upper lanes to the lower ones, 32 features at a time
+          uint64_t* const up = reinterpret_cast<uint64_t*>(smem + C::kOffTrans + (u * 4 + (q | 2)) * C::kTransBytes) + lane;
+#pragma unroll
+          for (int p = 0; p < 2; ++p) {
+            if (q >= 2) {
+#pragma unroll
+              for (int c = 0; c < 16; ++c) up[c * 32] = acc[p * 16 + c];
+            }
+            bar_two(5 + u * 2 + (q & 1));
+            if (q < 2) {
+#pragma unroll
+              for (int c = 0; c < 16; ++c) acc[32 + p * 16 + c] = up[c * 32];
+            }
+            bar_two(5 + u * 2 + (q & 1));
+          }
+        }
         float mx = 0.f;
         const bool own = lane < rows;
 #pragma unroll
@@ -752,7 +798,7 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
         }
         float* am = amax_sm + (n_it & 1) * 256;
         am[u * 128 + tid] = mx;
-        ok = bar_and<64>(1 + q, ok);   // the two warps that share a quarter's tokens
+        ok = bar_and<32 * kEpiWarps>(1, ok);   // of the two warps that share a quarter's tokens; all leave together
         if (!ok) break;
         const float amax = fmaxf(fmaxf(mx, am[(u ^ 1) * 128 + tid]), 1e-4f);
         const float inv = 448.f / amax;
@@ -792,7 +838,7 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
   Bars* bars = reinterpret_cast<Bars*>(smem + off_bars<MODE>());
   int* goff = reinterpret_cast<int*>(smem + off_tables<MODE>());   // [G + 1]
   int* pref64 = goff + a.G + 1;                                    // [G + 1] tiles of 64 tokens before each expert
-  int* pref256 = pref64 + a.G + 1;                                 // the same of 256
+  int* pref256 = pref64 + a.G + 1;                                 // whole and half tiles of 256: see locate_tokens
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();   // 0 = leader
@@ -836,7 +882,7 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         bad = 1;
         m = 0;
       }
-      const int n = (m + 63) / 64, w = (m + 255) / 256;
+      const int n = (m + 63) / 64, w = ((m + 127) / 256 << kHalfBits) + ((m - 1) % 256 < 128 && m > 0);
       int x = n, y = w;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
@@ -859,7 +905,8 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
       bars->ok = !bad;
       if (kBoth) {
         pref256[a.G] = sum256;
-        bars->tokens = tokens_pay(MODE, feature_tiles(MODE, a.Nout), sum64, sum256, gridDim.x >> 1, a.inv_pairs);
+        bars->tokens = tokens_pay(MODE, feature_tiles(MODE, a.Nout), sum64, (sum256 >> kHalfBits) + (sum256 & ((1 << kHalfBits) - 1)),
+                                  gridDim.x >> 1, a.inv_pairs);
       }
     }
   }
@@ -906,7 +953,7 @@ int launch(const void* W, const void* X, const MoePairArgs& a, int grid, cudaStr
 
 }  // namespace
 
-bool moe_gemm_pair_fits(int G, int grid) { return grid >= 2 && G <= 1024; }
+bool moe_gemm_pair_fits(int G, int grid) { return grid >= 2 && G <= 1024; }   // (kHalfBits)
 
 int moe_gemm_pair_launch(int mode, const void* W, const void* X, const MoePairArgs& args, int grid, cudaStream_t stream) {
   MoePairArgs a = args;

@@ -262,3 +262,14 @@ def test_swiglu_quotient_against_the_division():
 ])
 def test_groups_of_k_blocks_match_single_ctas(G, counts, K, F, H):
     test_single_ctas_match_the_pairs(G, counts, K, F, H)
+
+
+# 256-token tiles of which some have at most 128 tokens, 64 to a CTA and each of them in two lanes: rows around 64 and 128, such tiles
+# in front of, between and behind whole ones of the same pair, one token, a partner without any
+@pytest.mark.parametrize("G,counts,K,F,H", [
+    (3, [128, 256, 256], 256, 256, 256),
+    (5, [320, 65, 129, 193, 256], 1152, 128, 384),
+    (3, [384, 1, 511], 640, 384, 128),
+])
+def test_half_token_tiles_match_single_ctas(G, counts, K, F, H):
+    test_token_major_tiles_match_single_ctas(G, counts, K, F, H)
