@@ -21,14 +21,15 @@
 // of it. A K block takes 900 cycles at 1.45 GHz under the power limit: the tensor cores 512, the rest is the promotion's chain
 // (wait, four to eight TMEM loads, 64 packed FMAs, release) of two warps a scheduler, which all but fills it. (One barrier for both
 // accumulators of a K block instead of two: 629 / 655 us; what bounds it is the way round through TMEM, not the issuing thread.)
-// An expert's last tile of at most 128 tokens is a HALF one: an MMA of 128 rows, 64 of each CTA, whose accumulator has columns 0 - 63
-// in TMEM lanes 0 - 63 and columns 64 - 127 of the same tokens in lanes 64 - 127: half of the columns for each promoting thread, 800
-// cycles a K block instead of 1000 where nothing else runs (two experts of 7168 x 2048 on eight CTAs, MODE 0 238 / 189 us, MODE 1
-// 146 / 124). A pair takes its half tiles behind the whole ones, so that no pair has whole ones only (in the order of the experts:
-// no gain). Whole tiles for all / this, us of MODE 0 and 1: 7000 rows of 64 experts, 4096 x 1024, 171 + 112 / 156 + 96; 2500 of 8,
-// 5120 x 896, 54.5 + 32.0 / 52.1 + 30.5; 16384 of 32, 7168 x 2048, where a fifth of the tiles are half ones and their weights come
-// from memory once more, 629 + 355 / 623 + 351. With eight accumulators of 64 columns 152 + 91, 55 + 31 and 625 + 345, and the
-// registers of the whole tiles spill.
+// In MODE 0 an expert's last tile of at most 128 tokens is a HALF one: an MMA of 128 rows, 64 of each CTA, whose accumulator has
+// columns 0 - 63 in TMEM lanes 0 - 63 and columns 64 - 127 of the same tokens in lanes 64 - 127: half of the columns for each promoting
+// thread, 800 cycles a K block instead of 1000 where nothing else runs (two experts of 7168 x 2048 on eight CTAs, 238 / 189 us). A
+// pair takes its half tiles behind the whole ones, so that no pair has whole ones only (in the order of the experts: no gain). Whole
+// tiles for all / this, us: 7000 rows of 64 experts, 4096 x 1024, 171 / 151; 2500 of 8, 5120 x 896, 54.5 / 50.1; 8000 of 16,
+// 4096 x 1536, 146 / 139; 16384 of 32, 7168 x 2048, where a fifth of the tiles are half ones and their weights come from memory once
+// more, 629 / 621. With eight accumulators of 64 columns 152, 53, 146 and 625: the registers of the whole tiles spill. In MODE 1 it
+// gains as much (112 / 96, 355 / 351), but the 64-token tiles, which are in the same kernel, lose more (1024 rows of 16,
+// 2048 x 1024: 15.5 / 17.6): the compiler's registers again.
 #include "ep_common.cuh"
 #include "fp8_block.cuh"
 #include "moe_gemm_pair.cuh"
@@ -66,7 +67,7 @@ struct Cfg {
   static constexpr int kEnd = kOffAmax + 2 * kTok * 4;
 };
 
-// Tiles with the TOKENS on the MMA's M side: one item = 256 tokens (or up to 128) x 256 weight rows of one expert, each CTA of the pair
+// Tiles with the TOKENS on the MMA's M side: one item = 256 tokens (or, in MODE 0, up to 128) x 256 weight rows of one expert, each CTA of the pair
 // owns 128 of the tokens (its TMEM lanes; or 64) x all 256 rows, as two accumulators of 128 columns per K block, one for each four of the
 // promoting warps - in MODE 0 64 gate rows and the up rows of the same features, so a thread has both factors of SwiGLU.
 template <int MODE>
@@ -484,19 +485,26 @@ __device__ __forceinline__ void weight_body(uint8_t* smem, const CUtensorMap& tm
   }
 }
 
-// `pref`: whole tiles before each expert in the upper bits, half tiles (at most one per expert) in the lower kHalfBits.
+// `pref`: tiles before each expert; with half tiles (MODE 0) whole ones in the upper bits and half ones, at most one per expert, in the
+// lower kHalfBits.
+template <int MODE>
+__device__ __forceinline__ int tiles_of(int pref) {
+  return MODE == 0 ? (pref >> kHalfBits) + (pref & ((1 << kHalfBits) - 1)) : pref;
+}
+template <int MODE>
 __device__ __forceinline__ Item locate_tokens(const int* pref, const int* goff, int G, int NT, int w) {
-  const int whole = (pref[G] >> kHalfBits) * NT;
-  const bool half = w >= whole;
+  constexpr int kBits = MODE == 0 ? kHalfBits : 0;
+  const int whole = MODE == 0 ? (pref[G] >> kBits) * NT : 0;
+  const bool half = MODE == 0 && w >= whole;
   if (half) w -= whole;
-  auto before = [&](int e) { return half ? pref[e] & ((1 << kHalfBits) - 1) : pref[e] >> kHalfBits; };
+  auto before = [&](int e) { return half ? pref[e] & ((1 << kBits) - 1) : pref[e] >> kBits; };
   int lo = 0, hi = G;   // largest lo with before(lo) * NT <= w
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
     if (before(mid) * NT <= w) lo = mid;
     else hi = mid;
   }
-  const int ntt = (pref[lo + 1] >> kHalfBits) - (pref[lo] >> kHalfBits);   // whole tiles
+  const int ntt = (pref[lo + 1] >> kBits) - (pref[lo] >> kBits);   // whole tiles
   const int local = w - before(lo) * NT;
   Item it;
   it.e = lo;
@@ -516,11 +524,15 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
   // Both kinds of tile are in one kernel. What the compiler shares between them it keeps in registers all the way through the
   // promotion: hide that the addresses are the same.
   asm volatile("" : "+l"(smem), "+l"(bars));
+  if (MODE == 0) {   // with these two as well: 628 / 619 us at 16384 rows, 147 / 139 at 8000
+    asm volatile("" : "+l"(tile_pref), "+l"(goff));
+    asm volatile("" : "+r"(warp), "+r"(lane), "+r"(cta), "+r"(tmem_base));
+  }
   static_assert(C::kStages <= 9 && C::kTmemStages <= 8 && C::kScaleStages <= 3, "barriers");
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int NT = feature_tiles(MODE, a.Nout);
   const int kb_total = a.K / kBKB;
-  const int num_items = bars->ok ? ((tile_pref[a.G] >> kHalfBits) + (tile_pref[a.G] & ((1 << kHalfBits) - 1))) * NT : 0;
+  const int num_items = bars->ok ? tiles_of<MODE>(tile_pref[a.G]) * NT : 0;
 
   if (warp < 4) {
     regs_dec<MODE == 0 ? 56 : 80>();
@@ -530,7 +542,7 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
         uint32_t ph = 0;
         bool ok = true;
         for (int w = pair; w < num_items && ok; w += num_pairs) {
-          const Item it = locate_tokens(tile_pref, goff, a.G, NT, w);
+          const Item it = locate_tokens<MODE>(tile_pref, goff, a.G, NT, w);
           const int xrow = it.row0 + (int)cta * (it.n / 2);
           // columns of an accumulator: 64 weight rows of the leader, 64 of its partner
           const int wrow = it.e * a.w_rows + (MODE == 0 ? it.j * 128 + (int)cta * a.Nout : it.j * 256 + (int)cta * 64);
@@ -561,7 +573,8 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
         bool ok = true;
         const uint64_t a_desc = umma_desc_k_sw128(smem_u32(smem));
         for (int w = pair; w < num_items && ok; w += num_pairs) {
-          const uint32_t idesc = umma_idesc(kFmtE4M3, kFmtE4M3, locate_tokens(tile_pref, goff, a.G, NT, w).n, 128);
+          const uint32_t idesc =
+              umma_idesc(kFmtE4M3, kFmtE4M3, MODE == 0 ? locate_tokens<MODE>(tile_pref, goff, a.G, NT, w).n : 256, 128);
           for (int kb = 0; kb < kb_total && ok; ++kb) {
             if (!mbar_wait(&bars->full[s], ph)) {
               umdk_set_status(a.status, UMDK_ERR_TIMEOUT, UMDK_PH_TMA_FULL, w, kb);
@@ -603,12 +616,12 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
       uint32_t sph = 0;
       bool ok = true;
       for (int w = pair; w < num_items && ok; w += num_pairs) {
-        const Item it = locate_tokens(tile_pref, goff, a.G, NT, w);
+        const Item it = locate_tokens<MODE>(tile_pref, goff, a.G, NT, w);
         const float* ws0 = a.ws + ((size_t)it.e * wsb + (MODE == 0 ? it.j : 2 * it.j)) * nsb;
         const float* ws1 = MODE == 0 ? ws0 + (size_t)(a.Nout / 128) * nsb : 2 * it.j + 1 < wsb ? ws0 + nsb : ws0;
         for (int kb0 = 0; kb0 < kb_total; kb0 += C::kScaleKb) {
           float w0[C::kScaleKb], w1[C::kScaleKb], xv[C::kScaleKb];
-          const bool few = it.n == 128;
+          const bool few = MODE == 0 && it.n == 128;
           const int first = (int)cta * (it.n / 2) + t64;
           const float* xs = a.xs + (size_t)(it.row0 + first) * nsb + kb0;
           const int rows = it.m - first;   // token t64 + 64 u is this expert's where 64 u < rows
@@ -629,8 +642,8 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
           for (int u = 0; u < 2; ++u) {
 #pragma unroll
             for (int i = 0; i < C::kScaleKb; ++i) {
-              // (in MODE 0 the upper lanes of a half tile have the up columns)
-              dst[(i * 2) * 128 + 64 * u] = xv[i] * (MODE == 0 && u == 1 && few ? w1[i] : w0[i]);
+              // (the upper lanes of a half tile have the up columns)
+              dst[(i * 2) * 128 + 64 * u] = xv[i] * (u == 1 && few ? w1[i] : w0[i]);
               dst[(i * 2 + 1) * 128 + 64 * u] = xv[i] * w1[i];
               if (u == 0 && !few) xv[i] = kb0 + i < kb_total && rows > 64 ? xs[(size_t)64 * nsb + i] : 0.f;
             }
@@ -728,20 +741,18 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
           }
         }
       };
-      const bool few = locate_tokens(tile_pref, goff, a.G, NT, w).n == 128;
+      const bool few = MODE == 0 && locate_tokens<MODE>(tile_pref, goff, a.G, NT, w).n == 128;
       if (few) accumulate(std::integral_constant<int, kLoads / 2>());
       else accumulate(std::integral_constant<int, kLoads>());
-      const Item it = locate_tokens(tile_pref, goff, a.G, NT, w);
+      const Item it = locate_tokens<MODE>(tile_pref, goff, a.G, NT, w);
       const int tok0 = (int)cta * (it.n / 2) + (few ? q & 1 : q) * 32;
-      const int rows = MODE == 0 && few && q >= 2 ? 0 : min(32, it.m - tok0);   // valid tokens of this warp (may be negative)
+      const int rows = few && q >= 2 ? 0 : min(32, it.m - tok0);   // valid tokens of this warp (may be negative)
       const size_t row0 = (size_t)it.row0 + tok0;
       if (MODE == 1) {
         if (!ok) break;
         const int feat0 = it.j * 256 + u * 128;
 #pragma unroll
         for (int p = 0; p < 2; ++p) {   // 64 features at a time
-          if (p == 1 && few) break;
-          const int feat = feat0 + (few ? q >> 1 : p) * 64;
           __syncwarp();
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
@@ -761,7 +772,7 @@ __device__ __forceinline__ void token_body(uint8_t* smem, const CUtensorMap& tmW
             for (int i = 0; i < 8; ++i) {
               const int t = i * 4 + (lane >> 3), seg = lane & 7;
               const int4 o = *reinterpret_cast<const int4*>(trans + t * 128 + ((seg ^ (t & 7)) << 4));
-              if (t < rows) *reinterpret_cast<int4*>(a.y + (row0 + t) * a.Nout + feat + seg * 8) = o;
+              if (t < rows) *reinterpret_cast<int4*>(a.y + (row0 + t) * a.Nout + feat0 + p * 64 + seg * 8) = o;
             }
           }
         }
@@ -882,7 +893,7 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         bad = 1;
         m = 0;
       }
-      const int n = (m + 63) / 64, w = ((m + 127) / 256 << kHalfBits) + ((m - 1) % 256 < 128 && m > 0);
+      const int n = (m + 63) / 64, w = MODE == 1 ? (m + 255) / 256 : ((m + 127) / 256 << kHalfBits) + (m > 0 && (m - 1) % 256 < 128);
       int x = n, y = w;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
@@ -905,8 +916,7 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
       bars->ok = !bad;
       if (kBoth) {
         pref256[a.G] = sum256;
-        bars->tokens = tokens_pay(MODE, feature_tiles(MODE, a.Nout), sum64, (sum256 >> kHalfBits) + (sum256 & ((1 << kHalfBits) - 1)),
-                                  gridDim.x >> 1, a.inv_pairs);
+        bars->tokens = tokens_pay(MODE, feature_tiles(MODE, a.Nout), sum64, tiles_of<MODE>(sum256), gridDim.x >> 1, a.inv_pairs);
       }
     }
   }

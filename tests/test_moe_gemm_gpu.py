@@ -264,7 +264,7 @@ def test_groups_of_k_blocks_match_single_ctas(G, counts, K, F, H):
     test_single_ctas_match_the_pairs(G, counts, K, F, H)
 
 
-# 256-token tiles of which some have at most 128 tokens, 64 to a CTA and each of them in two lanes: rows around 64 and 128, such tiles
+# 256-token tiles of which some have at most 128 tokens (gate/up: 64 to a CTA and each of them in two lanes): rows around 64 and 128, such tiles
 # in front of, between and behind whole ones of the same pair, one token, a partner without any
 @pytest.mark.parametrize("G,counts,K,F,H", [
     (3, [128, 256, 256], 256, 256, 256),
